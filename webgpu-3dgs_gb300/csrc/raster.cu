@@ -92,22 +92,39 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // Converts the staged ProjectedSplat prefix (mean, depth, radius | conic,
 // opacity | color, valid) into the raster form.  vis = the largest Q at which
 // alpha can still reach 1/255, with a 1% margin, in the units of the splat's
-// form (-1: never visible; +inf: conic too ill-conditioned for the alpha
-// bound, or a non-finite opacity or conic: use the circle only).
-__device__ __forceinline__ void prepare(SplatStage& s) {
+// form (-1: never visible; +inf: use the circle only: a conic with a
+// non-positive diagonal, or a non-finite opacity or conic).
+//
+// vis also carries the rounding of the quadratic form, so that the cull stays
+// conservative for any conic, needles included (condition numbers of 10^3
+// and more, splats with axes more than 30:1 apart).  With u = 2^-24 and
+// t(d) = |A| dx^2 + 2 |B dx dy| + |C| dy^2, the per-pixel form in either
+// operation order and the cull's own evaluation each lie within about 4 u t
+// of the exact form, and rect_may_hit's approximate stationary points raise it
+// by far less (2^-42 t).  A pixel that passes its tests lies in the circle, and
+// the cull's points within `ext` of one (ext bounds the diagonal of a warp's
+// pixel block), so t <= (|A| + 2 |B| + |C|) (r + ext)^2; 16 u times that is
+// added, twice the sum of both.  Needles kept for every block of their circle
+// (as before the bound) are 4.8 times the blocks that hold a visible pixel on
+// a 4K close-up of heavy-tailed scales, 1.3 times on the 3M-splat orbit views:
+// raster 6.34 -> 1.61 ms there (3M splats, 32x32 tiles), 3.94 -> 3.31 ms for
+// 8 orbit views (64x32), 0.425 -> 0.362 ms for one view at 16x16.
+__device__ __forceinline__ void prepare(SplatStage& s, float ext) {
   const float4 a = s.a, b = s.b;
   const float A = b.x, B = b.y, C = b.z, op = b.w;
+  const float sum = fabsf(A) + 2.0f * fabsf(B) + fabsf(C);
   float vis;
   const float lim = op * 255.0f;
   if (lim < 0.999f) {
     vis = -1.0f;  // alpha = opacity * exp(power) <= opacity < 1/255 everywhere
-  } else if (lim > 1.0f && A * C - B * B >= 1e-3f * (A + C) * (A + C) && A > 0.0f && C > 0.0f) {
-    vis = __log2f(lim) * 1.01f + 1e-3f;
   } else {
-    vis = __int_as_float(0x7f800000);
+    const float reach = a.w + ext;
+    vis = __log2f(lim) * 1.01f + 1e-3f + (kHalfLog2e * 9.5367431640625e-07f) * sum * reach * reach;
+    // false for NaNs too
+    if (!(lim > 1.0f && A > 0.0f && C > 0.0f && vis < 3.0e38f)) vis = __int_as_float(0x7f800000);
   }
   const float r2 = a.w * a.w;
-  const float terms = (fabsf(A) + 2.0f * fabsf(B) + fabsf(C)) * r2;
+  const float terms = sum * r2;
   s.a = make_float4(a.x, a.y, r2, op);
   if (terms <= kExactFormBound) {
     s.b = make_float4(kHalfLog2e * A, 2.0f * kHalfLog2e * B, kHalfLog2e * C, vis);
@@ -116,6 +133,12 @@ __device__ __forceinline__ void prepare(SplatStage& s) {
     s.b = make_float4(A, 2.0f * B, C, vis / kHalfLog2e);
     s.c.w = 1.0f;
   }
+}
+
+// Bounds the diagonal of the pixel-centre box of any warp of the culled
+// variants: 8x8 or 8x4 blocks (9.9), else rows of the tile.
+__device__ __forceinline__ float warp_box_reach(const RasterArgs& a, bool blocks) {
+  return blocks ? 12.0f : (float)(a.tile_w + a.tile_h);
 }
 
 // rasterize_tiles.wgsl:81-98 for one (pixel, splat) pair: the splat's alpha
@@ -353,7 +376,7 @@ __device__ void raster_tile_plain(const RasterArgs& a, const TileGeom& g, SplatS
       cp_async_wait<0>();
     }
     const uint32_t cnt = min(D, end - (start + bi * D));
-    for (uint32_t k = tid; k < cnt; k += nt) prepare(cur[k]);  // own copies are complete
+    for (uint32_t k = tid; k < cnt; k += nt) prepare(cur[k], 0.0f);  // own copies are complete
     __syncthreads();
     if (!done) {
       for (uint32_t j = 0; j < cnt; ++j) {
@@ -389,7 +412,9 @@ __device__ void raster_tile_culled(const RasterArgs& a, const TileGeom& g, uint3
   const uint32_t D = a.batch ? a.batch : nt;  // splats per staged batch
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t lx, ly;
-  if ((a.tile_w % 8 == 0) && ((nthr / a.tile_w) % 4 == 0)) {  // 8x4 pixel block per warp
+  const bool blocks = (a.tile_w % 8 == 0) && ((nthr / a.tile_w) % 4 == 0);
+  const float reach = warp_box_reach(a, blocks);
+  if (blocks) {  // 8x4 pixel block per warp
     const uint32_t bw = a.tile_w / 8;
     lx = (warp % bw) * 8 + (lane & 7);
     ly = row0 + (warp / bw) * 4 + (lane >> 3);
@@ -430,7 +455,7 @@ __device__ void raster_tile_culled(const RasterArgs& a, const TileGeom& g, uint3
       cp_async_wait<0>();
     }
     const uint32_t cnt = min(D, end - (start + bi * D));
-    for (uint32_t k = tid; k < cnt; k += nthr) prepare(cur[k]);  // own copies are complete
+    for (uint32_t k = tid; k < cnt; k += nthr) prepare(cur[k], reach);  // own copies are complete
     __syncthreads();
     if (__any_sync(0xffffffffu, !done)) {
       for (uint32_t k0 = 0; k0 < cnt; k0 += 32) {
@@ -489,6 +514,7 @@ __device__ void raster_tile_culled2(const RasterArgs& a, const TileGeom& g, uint
   const uint32_t D = a.batch ? a.batch : nt;  // splats per staged batch
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t bw = a.tile_w / 8;
+  const float reach = warp_box_reach(a, true);
   const uint32_t px = g.ox + (warp % bw) * 8 + (lane & 7);
   const uint32_t py0 = g.oy + strip * strip_h + (warp / bw) * 8 + (lane >> 3), py1 = py0 + 4;
   const bool in0 = px < g.W && py0 < g.H, in1 = px < g.W && py1 < g.H;
@@ -522,7 +548,7 @@ __device__ void raster_tile_culled2(const RasterArgs& a, const TileGeom& g, uint
       cp_async_wait<0>();
     }
     const uint32_t cnt = min(D, end - (start + bi * D));
-    for (uint32_t k = tid; k < cnt; k += nthr) prepare(cur[k]);  // own copies are complete
+    for (uint32_t k = tid; k < cnt; k += nthr) prepare(cur[k], reach);  // own copies are complete
     __syncthreads();
     if (__any_sync(0xffffffffu, !(done0 && done1))) {
       for (uint32_t k0 = 0; k0 < cnt; k0 += 32) {
