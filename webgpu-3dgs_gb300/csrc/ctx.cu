@@ -22,6 +22,7 @@
 // scenes and uneven sizes, in one launch sequence.
 #include <algorithm>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -524,6 +525,8 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   CK(raster_shape(a, c->sm_count, &strips, &raster_ctas), "raster shape");
   const bool split_all = (c->flags & GS3D_FLAG_SPLIT_ALL_TILES) != 0;
   const bool learned = c->schedule == GS3D_SCHEDULE_LEARNED && c->total_tiles > 1;
+  static_assert(offsetof(Ctrl, raster_heavy) == offsetof(Ctrl, raster_queue) + 8, "cleared together");
+  CK(cudaMemsetAsync(&ctrl_of(c)->raster_queue, 0, 12, c->stream), "reset raster queue");
   const uint32_t* order = nullptr;
   const uint32_t* heavy = nullptr;
   if (c->schedule != GS3D_SCHEDULE_ROW_MAJOR && c->total_tiles > 1) {
@@ -555,7 +558,7 @@ int raster_stage(gs3d_ctx* c, bool culled) {
     order = u32(c->sched_order_a);
     heavy = &ctrl_of(c)->raster_heavy;
   } else if (split_all) {  // row-major order, every tile split
-    CK(launch_heavy_count(nullptr, c->total_tiles, raster_ctas, strips, true,
+    CK(launch_heavy_count(nullptr, c->total_tiles, raster_ctas, strips, 0.0f, true,
                           &ctrl_of(c)->raster_heavy, c->stream),
        "split all tiles");
     heavy = &ctrl_of(c)->raster_heavy;
@@ -568,7 +571,8 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   a.tile_costs = u32(c->tile_costs);
   a.order = order;
   a.queue_counter = &ctrl_of(c)->raster_queue;
-  CK(cudaMemsetAsync(a.queue_counter, 0, sizeof(uint32_t), c->stream), "reset raster queue");
+  a.ref_counter = u32(c->ref_counter);
+  a.err = &ctrl_of(c)->error;
   // the previous frame's splat target may still be copying out (captured as
   // an external event wait in graph mode; a never-recorded event is no wait)
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -576,7 +580,9 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   CK(cudaStreamWaitEvent(c->stream, c->copy_done,
                          cap == cudaStreamCaptureStatusActive ? cudaEventWaitExternal : 0),
      "wait for the previous copy-out");
-  CK(launch_raster(a, c->sm_count, c->stream), "rasterize_tiles");
+  // the row-major order's heavy tiles go where the other orders keep theirs
+  CK(launch_raster(a, u32(c->sched_order_b), &ctrl_of(c)->raster_heavy, c->sm_count, c->stream),
+     "rasterize_tiles");
   if (learned)  // the gate measures this frame's prediction error
     CK(launch_gate_update(static_cast<float*>(c->tile_preds.p), u32(c->tile_costs),
                           c->total_tiles, static_cast<SchedGate*>(c->gate.p), c->stream),

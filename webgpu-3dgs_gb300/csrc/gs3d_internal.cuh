@@ -84,9 +84,9 @@ struct Ctrl {
   uint32_t error;
   uint32_t scan_tile_counter;
   uint32_t sort_part_counter[kMaxSortPasses];
-  uint32_t raster_queue;
   uint32_t sched_counter[2];
-  uint32_t raster_heavy;  // tiles at the head of the raster order shaded as half strips
+  unsigned long long raster_queue;  // next raster work item
+  uint32_t raster_heavy;  // tiles whose raster work is split (the head of an order by cost)
   uint32_t emit_chunk;    // next 256-splat chunk of the depth-ordered emit
   uint32_t pad;
   uint32_t sort_hist[kMaxSortPasses][kRadixBins];  // global digit histograms
@@ -317,13 +317,20 @@ cudaError_t launch_schedule(uint32_t schedule, const uint32_t* tile_offsets, uin
                             uint32_t* keys_b, uint32_t* order_b, float* est, uint32_t* status,
                             Ctrl* ctrl, uint32_t raster_ctas, uint32_t strips, bool split_all,
                             int sm_count, cudaStream_t s);
+// Tiles of fewer keys, or of a smaller predicted cost, are never split.  Most
+// long lists are opaque and end after a few thousand splats, so the bound on
+// keys is high (3M splats at 16x16, key-count bound of half a fair share alone:
+// a quarter of the tiles split, raster 0.36 -> 0.43 ms); a predicted cost says
+// what is walked.
+constexpr uint32_t kHeavyKeys = 16384, kHeavyCost = 1024;
 // The per-tile split: *heavy = the number of tiles (the head of an order by
-// decreasing est) whose expected cost per strip exceeds half of one raster
-// CTA's fair share of the frame, sum(est) * strips / raster_ctas; those tiles
-// are shaded as two half-strip work items per strip.  all: every tile (est
-// may be null).
+// decreasing est) whose expected cost per work item exceeds half of one raster
+// worker's fair share of the frame, sum(est) * strips / raster_ctas, and floor;
+// those tiles are shaded as half-block work items.  all: every tile (est may be
+// null).
 cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t raster_ctas,
-                               uint32_t strips, bool all, uint32_t* heavy, cudaStream_t s);
+                               uint32_t strips, float floor, bool all, uint32_t* heavy,
+                               cudaStream_t s);
 
 // ---- learned schedule (learned.cu) ----
 constexpr int kFeatures = 16;
@@ -371,7 +378,9 @@ cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint
                             int sm_count, cudaStream_t s);
 // Rasterizes every tile of the batch.  Persistent CTAs pull tile indices
 // from a device work queue (order[k] = k-th tile to render, identity when
-// order is null) through *queue_counter, which must be zero at launch.
+// order is null) through *queue_counter, which must be zero at launch, as must
+// *heavy_count where args.heavy and args.order are null (the row-major order
+// then lists the tiles it splits in heavy_list[num_tiles]).
 struct RasterArgs {
   const ViewDesc* views;
   uint32_t n_views;
@@ -383,18 +392,25 @@ struct RasterArgs {
   uint2* image;
   uint32_t* tile_costs;   // may be null
   const uint32_t* order;  // may be null
-  uint32_t* queue_counter;
+  unsigned long long* queue_counter;
+  const uint32_t* ref_counter;
+  uint32_t* err;
   uint32_t batch;         // splats staged per batch (0 = tile_w * tile_h)
   bool culled;
-  uint32_t split;         // CTAs per tile (row strips), set by launch_raster
-  // tiles at the head of the order shaded as two half-strip items per strip
-  // (device count, two-pixel culled variant only; may be null: none)
+  // tiles at the head of the order whose blocks are shaded as two half-block
+  // items (device count, warp variant only; may be null: none)
   const uint32_t* heavy;
+  // set by launch_raster:
+  const uint32_t* heavy_list;  // row-major order: the *heavy tiles it splits
+  float heavy_share;           // ... and the share of the refs above which it does
+  uint32_t coarse;             // tiles of the order shaded by regions; the rest by blocks
 };
-cudaError_t launch_raster(const RasterArgs& a, int sm_count, cudaStream_t s);
-// Row strips per tile and resident CTAs of the raster launch for these args.
-cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* strips,
-                         uint32_t* resident_ctas);
+cudaError_t launch_raster(const RasterArgs& a, uint32_t* heavy_list, uint32_t* heavy_count,
+                          int sm_count, cudaStream_t s);
+// Work items per tile and resident workers (warps; CTAs where a CTA shades a
+// tile) of the raster launch for these args.
+cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* items_per_tile,
+                         uint32_t* resident);
 
 // Headless composite of one view's splat target over a background colour,
 // optionally through the tile heat-map overlay; out = W*H RGBA8 words.

@@ -68,7 +68,8 @@ namespace {
 // decides the result.  Below that bound the fast form's q differs from the
 // reference's by about 2^-11 at most, so each alpha differs by a relative
 // 1e-3 and a pixel, whose blend weights alpha_i T_i sum to at most 1, by
-// about that much.  b.w = vis, in q's units.
+// about that much.  b.w = vis, in q's units; its two lowest bits hold the
+// splat's kind (prepare).
 struct SplatStage {  // first 48 bytes of a ProjectedSplat, prepared in place (prepare())
   float4 a;  // mean_px.x, mean_px.y, radius_px^2, opacity
   float4 b;  // q coefficients (see above), vis
@@ -77,6 +78,10 @@ struct SplatStage {  // first 48 bytes of a ProjectedSplat, prepared in place (p
 
 constexpr float kHalfLog2e = 0.72134752044448170f;
 constexpr float kExactFormBound = 4096.0f;
+constexpr float kCircleOnly = 3.0e38f;  // vis of splats culled by their circle alone
+// How a splat's alpha is evaluated: fast form whose op exp(power) stays below
+// the 0.99 clamp; fast form with the clamp; exact form (which clamps).
+constexpr uint32_t kSimple = 0u, kClamped = 1u, kExact = 2u;
 
 struct Pixel {
   float cr, cg, cb, T;
@@ -92,8 +97,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // Converts the staged ProjectedSplat prefix (mean, depth, radius | conic,
 // opacity | color, valid) into the raster form.  vis = the largest Q at which
 // alpha can still reach 1/255, with a 1% margin, in the units of the splat's
-// form (-1: never visible; +inf: use the circle only: a conic with a
-// non-positive diagonal, or a non-finite opacity or conic).
+// form (-1: never visible; kCircleOnly or more: use the circle only: a conic
+// with a non-positive diagonal, or a non-finite opacity or conic).
 //
 // vis also carries the rounding of the quadratic form, so that the cull stays
 // conservative for any conic, needles included (condition numbers of 10^3
@@ -121,16 +126,20 @@ __device__ __forceinline__ void prepare(SplatStage& s, float ext) {
     const float reach = a.w + ext;
     vis = __log2f(lim) * 1.01f + 1e-3f + (kHalfLog2e * 9.5367431640625e-07f) * sum * reach * reach;
     // false for NaNs too
-    if (!(lim > 1.0f && A > 0.0f && C > 0.0f && vis < 3.0e38f)) vis = __int_as_float(0x7f800000);
+    if (!(lim > 1.0f && A > 0.0f && C > 0.0f && vis < 1.0e38f)) vis = kCircleOnly;
   }
   const float r2 = a.w * a.w;
   const float terms = sum * r2;
   s.a = make_float4(a.x, a.y, r2, op);
   if (terms <= kExactFormBound) {
+    // no clamp where ex2 of a value <= 0 (to 2 ulp) times op stays below it
+    const bool simple = op <= 0.9899f && fabsf(a.x) + fabsf(a.y) < 3.0e38f;
+    vis = __uint_as_float((__float_as_uint(vis) & ~3u) | (simple ? kSimple : kClamped));
     s.b = make_float4(kHalfLog2e * A, 2.0f * kHalfLog2e * B, kHalfLog2e * C, vis);
     s.c.w = 0.0f;
   } else {  // also non-finite terms
-    s.b = make_float4(A, 2.0f * B, C, vis / kHalfLog2e);
+    vis = fminf(vis * (1.0f / kHalfLog2e), kCircleOnly);
+    s.b = make_float4(A, 2.0f * B, C, __uint_as_float((__float_as_uint(vis) & ~3u) | kExact));
     s.c.w = 1.0f;
   }
 }
@@ -147,11 +156,11 @@ __device__ __forceinline__ float warp_box_reach(const RasterArgs& a, bool blocks
 // reference).  A skipped splat blends with alpha = 0 (blend_alpha), which
 // leaves C and T bit-unchanged.
 __device__ __forceinline__ float splat_alpha(float pfx, float pfy, const SplatStage& s,
-                                             bool& ok) {
+                                             bool exact, bool& ok) {
   const float4 a = s.a, b = s.b;
   const float dx = pfx - a.x;
   const float dy = pfy - a.y;
-  if (s.c.w == 0.0f) {
+  if (!exact) {
     // fast form: q < 0 cannot occur (no power > 0 test needed): these splats'
     // conics have condition numbers below 455 (their terms, at least 9 times
     // the condition number, stay within kExactFormBound), so q, computed to
@@ -196,7 +205,7 @@ __device__ __forceinline__ bool blend_one(float pfx, float pfy, const SplatStage
     if (d2 > s.a.z) return false;
   }
   bool ok;
-  const float alpha = splat_alpha(pfx, pfy, s, ok);
+  const float alpha = splat_alpha(pfx, pfy, s, s.c.w != 0.0f, ok);
   return blend_alpha(p, s.c, alpha, ok && live);
 }
 
@@ -207,17 +216,13 @@ __device__ __forceinline__ bool blend_one(float pfx, float pfy, const SplatStage
 // each pixel is bit-identical to the one-pixel variants.
 __device__ __forceinline__ float2 bcast(float x) { return make_float2(x, x); }
 
-struct Pixel2 {
-  float2 cr, cg, cb, T;
-};
-
 __device__ __forceinline__ float2 splat_alpha2(float pfx, float2 pfy, const SplatStage& s,
-                                               bool& ok0, bool& ok1) {
+                                               bool exact, bool& ok0, bool& ok1) {
   const float4 a = s.a, b = s.b;
   const float dx = pfx - a.x;
   const float2 dy = __fadd2_rn(pfy, bcast(-a.y));
   float2 d2, q, ev;
-  if (s.c.w == 0.0f) {  // fast form (splat-uniform branch; no q < 0 test, see splat_alpha)
+  if (!exact) {  // fast form (splat-uniform branch; no q < 0 test, see splat_alpha)
     d2 = __ffma2_rn(bcast(dx), bcast(dx), __fmul2_rn(dy, dy));
     q = __ffma2_rn(bcast(b.x * dx), bcast(dx),
                    __ffma2_rn(bcast(b.y * dx), dy, __fmul2_rn(__fmul2_rn(bcast(b.z), dy), dy)));
@@ -246,14 +251,116 @@ __device__ __forceinline__ float2 splat_alpha2(float pfx, float2 pfy, const Spla
   return alpha;
 }
 
-__device__ __forceinline__ void blend_alpha2(Pixel2& p, const float4 c, float2 alpha, bool ok0,
-                                             bool ok1) {
-  const float2 al = make_float2(ok0 ? alpha.x : 0.0f, ok1 ? alpha.y : 0.0f);
-  const float2 ta = __fmul2_rn(p.T, al);
-  p.cr = __ffma2_rn(ta, bcast(c.x), p.cr);
-  p.cg = __ffma2_rn(ta, bcast(c.y), p.cg);
-  p.cb = __ffma2_rn(ta, bcast(c.z), p.cb);
-  p.T = __fmul2_rn(p.T, __fadd2_rn(bcast(1.0f), make_float2(-al.x, -al.y)));
+// splat_alpha and splat_alpha2 of a simple splat, 0 where it is skipped: the
+// same operations without the clamp, which cannot act.
+__device__ __forceinline__ float simple_alpha(float pfx, float pfy, const SplatStage& s) {
+  const float4 a = s.a, b = s.b;
+  const float dx = pfx - a.x;
+  const float dy = pfy - a.y;
+  const float d2 = fmaf(dx, dx, dy * dy);
+  const float q = fmaf(b.x * dx, dx, fmaf(b.y * dx, dy, b.z * dy * dy));
+  const float alpha = a.w * ex2_approx(-q);
+  return !(d2 > a.z) && !(alpha < 1.0f / 255.0f) ? alpha : 0.0f;
+}
+__device__ __forceinline__ float2 simple_alpha(float pfx, float2 pfy, const SplatStage& s) {
+  const float4 a = s.a, b = s.b;
+  const float dx = pfx - a.x;
+  const float2 dy = __fadd2_rn(pfy, bcast(-a.y));
+  const float2 d2 = __ffma2_rn(bcast(dx), bcast(dx), __fmul2_rn(dy, dy));
+  const float2 q =
+      __ffma2_rn(bcast(b.x * dx), bcast(dx),
+                 __ffma2_rn(bcast(b.y * dx), dy, __fmul2_rn(__fmul2_rn(bcast(b.z), dy), dy)));
+  const float2 alpha = __fmul2_rn(bcast(a.w), make_float2(ex2_approx(-q.x), ex2_approx(-q.y)));
+  return make_float2(!(d2.x > a.z) && !(alpha.x < 1.0f / 255.0f) ? alpha.x : 0.0f,
+                     !(d2.y > a.z) && !(alpha.y < 1.0f / 255.0f) ? alpha.y : 0.0f);
+}
+// The same for an exact-form splat.
+__device__ __forceinline__ float exact_alpha(float pfx, float pfy, const SplatStage& s) {
+  bool ok;
+  const float alpha = splat_alpha(pfx, pfy, s, true, ok);
+  return ok ? alpha : 0.0f;
+}
+__device__ __forceinline__ float2 exact_alpha(float pfx, float2 pfy, const SplatStage& s) {
+  bool ok0, ok1;
+  const float2 alpha = splat_alpha2(pfx, pfy, s, true, ok0, ok1);
+  return make_float2(ok0 ? alpha.x : 0.0f, ok1 ? alpha.y : 0.0f);
+}
+// The same for a splat of either form: both are evaluated and one is taken, so
+// that four of a step overlap (a branch per splat costs more than the few
+// operations that the forms do not share).  The q < 0 and clamp tests cannot
+// act on a fast-form splat that has none.
+__device__ __forceinline__ float any_alpha(float pfx, float pfy, const SplatStage& s, bool exact) {
+  const float4 a = s.a, b = s.b;
+  const float dx = pfx - a.x;
+  const float dy = pfy - a.y;
+  const float u = __fmul_rn(b.x, dx), v = __fmul_rn(b.y, dx);
+  const float w = __fmul_rn(__fmul_rn(b.z, dy), dy);
+  const float dyy = __fmul_rn(dy, dy);
+  const float qe = __fadd_rn(__fadd_rn(__fmul_rn(u, dx), __fmul_rn(v, dy)), w);
+  const float qf = fmaf(u, dx, fmaf(v, dy, w));
+  const float d2 = exact ? __fadd_rn(__fmul_rn(dx, dx), dyy) : fmaf(dx, dx, dyy);
+  const float q = exact ? qe : qf;
+  const float alpha = fminf(0.99f, a.w * ex2_approx(__fmul_rn(q, exact ? -kHalfLog2e : -1.0f)));
+  return !(d2 > a.z) && !(q < 0.0f) && !(alpha < 1.0f / 255.0f) ? alpha : 0.0f;
+}
+__device__ __forceinline__ float2 any_alpha(float pfx, float2 pfy, const SplatStage& s,
+                                            bool exact) {
+  const float4 a = s.a, b = s.b;
+  const float dx = pfx - a.x;
+  const float2 dy = __fadd2_rn(pfy, bcast(-a.y));
+  const float u = __fmul_rn(b.x, dx), v = __fmul_rn(b.y, dx);
+  const float2 w = __fmul2_rn(__fmul2_rn(bcast(b.z), dy), dy);
+  const float2 dyy = __fmul2_rn(dy, dy);
+  // exact: every sum a scalar __fadd_rn (never merged into an FMA)
+  const float t1 = __fmul_rn(u, dx), dxx = __fmul_rn(dx, dx);
+  const float2 t2 = __fmul2_rn(bcast(v), dy);
+  // fast
+  const float2 qf = __ffma2_rn(bcast(u), bcast(dx), __ffma2_rn(bcast(v), dy, w));
+  const float2 df = __ffma2_rn(bcast(dx), bcast(dx), dyy);
+  const float2 q = make_float2(exact ? __fadd_rn(__fadd_rn(t1, t2.x), w.x) : qf.x,
+                               exact ? __fadd_rn(__fadd_rn(t1, t2.y), w.y) : qf.y);
+  const float2 d2 =
+      make_float2(exact ? __fadd_rn(dxx, dyy.x) : df.x, exact ? __fadd_rn(dxx, dyy.y) : df.y);
+  const float2 ev = __fmul2_rn(q, bcast(exact ? -kHalfLog2e : -1.0f));
+  const float2 am = __fmul2_rn(bcast(a.w), make_float2(ex2_approx(ev.x), ex2_approx(ev.y)));
+  const float2 alpha = make_float2(fminf(0.99f, am.x), fminf(0.99f, am.y));
+  return make_float2(
+      !(d2.x > a.z) && !(q.x < 0.0f) && !(alpha.x < 1.0f / 255.0f) ? alpha.x : 0.0f,
+      !(d2.y > a.z) && !(q.y < 0.0f) && !(alpha.y < 1.0f / 255.0f) ? alpha.y : 0.0f);
+}
+
+// The blend state of a lane's pixels: one (Px1) or two of a column (Px2).
+// T is 0 once a pixel has terminated (out-of-view pixels start so), and a
+// splat then adds exactly nothing to it; `fin` holds the T it ended with.
+constexpr float kEndT = 1.0e-4f;
+struct Px1 {
+  float y, cr = 0.f, cg = 0.f, cb = 0.f, T = 1.f, fin = 0.f;
+  using V = float;
+  static constexpr int kN = 1;
+  __device__ static V mul(V a, V b) { return a * b; }
+  __device__ static V fma(V a, float c, V b) { return fmaf(a, c, b); }
+  __device__ static V keep(V al) { return 1.0f - al; }
+  __device__ static float& at(V& v, int) { return v; }
+};
+struct Px2 {
+  float2 y, cr = {0.f, 0.f}, cg = {0.f, 0.f}, cb = {0.f, 0.f}, T = {1.f, 1.f}, fin = {0.f, 0.f};
+  using V = float2;
+  static constexpr int kN = 2;
+  __device__ static V mul(V a, V b) { return __fmul2_rn(a, b); }
+  __device__ static V fma(V a, float c, V b) { return __ffma2_rn(a, bcast(c), b); }
+  __device__ static V keep(V al) { return __ffma2_rn(al, bcast(-1.0f), bcast(1.0f)); }
+  __device__ static float& at(V& v, int i) { return i ? v.y : v.x; }
+};
+template <typename PX>
+__device__ __forceinline__ bool px_live(PX& p) {
+  bool live = false;
+#pragma unroll
+  for (int i = 0; i < PX::kN; ++i) live = live || PX::at(p.T, i) > 0.0f;
+  return live;
+}
+template <typename PX>
+__device__ __forceinline__ float px_final(PX& p, int i) {
+  return PX::at(p.T, i) > 0.0f ? PX::at(p.T, i) : PX::at(p.fin, i);
 }
 
 __device__ __forceinline__ void store_pixel(uint2* image, uint32_t W, uint32_t px, uint32_t py,
@@ -283,44 +390,186 @@ __device__ __forceinline__ void stage_batch(const gs3d_projected_splat* __restri
 }
 
 // Can the splat reach alpha >= 1/255 inside the rectangle of pixel centres
-// [x0,x1] x [y0,y1]?  Exact minimum of the splat's q over the rectangle (the
-// quadratic form's minimum over a box not holding the mean lies on an edge,
-// at the clamped stationary point of that edge; scale-invariant, so either
-// form works), compared with vis; plus the radius circle.  Conservative by
-// the margins folded into vis and the circle: vis is finite only for conics
-// of condition number below about 10^3, where the rounding of q in any
-// operation order stays far inside the 1% margin.  NaN means, radii, conics
-// or opacities are never culled (the per-pixel tests decide, as in the
-// reference).
-__device__ __forceinline__ bool rect_may_hit(const SplatStage& s, float2 xr, float2 yr) {
-  const float4 a = s.a, b = s.b;
+// [x0,x1] x [y0,y1]?  Minimum of the splat's q over the rectangle
+// (scale-invariant, so either form works), compared with vis; plus the radius
+// circle.  Any point d of a rectangle without the mean sees the mean through
+// the edge nearest to it in x or in y, and q(t d) = t^2 q(d): so where q <= vis
+// somewhere, it is on one of those two edges, also for a form that rounding
+// made indefinite.  Along an edge q is convex (the conic's diagonal is
+// positive), so its minimum there is at the clamped stationary point.
+// Conservative by the margins folded into vis (prepare) and the circle.  NaN
+// means, radii, conics or opacities are never culled (the per-pixel tests
+// decide, as in the reference).
+__device__ __forceinline__ bool rect_may_hit(const float4 a, const float4 b, float2 xr,
+                                             float2 yr) {
   // the box corners relative to the mean (x - m computed as x + (-m))
   const float2 xd = __fadd2_rn(xr, bcast(-a.x)), yd = __fadd2_rn(yr, bcast(-a.y));
   const float x0 = xd.x, x1 = xd.y, y0 = yd.x, y1 = yd.y;
   const float ex = fminf(fmaxf(0.0f, x0), x1), ey = fminf(fmaxf(0.0f, y0), y1);
-  if (ex * ex + ey * ey > a.z * 1.0001f + 1e-3f) return false;
   const float vis = b.w;
-  if (vis < 0.0f) return false;
-  if (ex == 0.0f && ey == 0.0f) return true;  // the mean lies inside
-  if (vis == __int_as_float(0x7f800000)) return true;
+  if (ex * ex + ey * ey > a.z * 1.0001f + 1e-3f || vis < 0.0f) return false;
   const float qa = b.x, qb = b.y, qc = b.z;
-  // edge stationary points, by the fast reciprocal division: an error d in
-  // the point raises q there by qa d^2 (qc d^2) over the edge minimum, far
-  // inside the margins folded into vis
-  const float sy = __fdividef(-qb, 2.0f * qc), sx = __fdividef(-qb, 2.0f * qa);
-  // q = qa x^2 + qb x y + qc y^2 at the two vertical edges (x0, x1 at their
-  // clamped stationary y) and the two horizontal ones, as pairs
-  const float2 vx = xd, hy = yd;
-  const float2 svy = __fmul2_rn(bcast(sy), vx), shx = __fmul2_rn(bcast(sx), hy);
-  const float2 vy = make_float2(fminf(fmaxf(svy.x, y0), y1), fminf(fmaxf(svy.y, y0), y1));
-  const float2 hx = make_float2(fminf(fmaxf(shx.x, x0), x1), fminf(fmaxf(shx.y, x0), x1));
-  auto Q2 = [&](float2 x, float2 y) {
-    return __ffma2_rn(__fmul2_rn(bcast(qa), x), x,
-                      __ffma2_rn(__fmul2_rn(bcast(qb), x), y,
-                                 __fmul2_rn(__fmul2_rn(bcast(qc), y), y)));
-  };
-  const float2 qv = Q2(vx, vy), qh = Q2(hx, hy);
-  return fminf(fminf(qv.x, qv.y), fminf(qh.x, qh.y)) <= vis;
+  // stationary points of the edges x = ex and y = ey, by the fast reciprocal
+  // division: an error d in the point raises q there by qa d^2 (qc d^2) over
+  // the edge minimum, far inside the margins folded into vis
+  const float vy = fminf(fmaxf(__fdividef(-0.5f * qb, qc) * ex, y0), y1);
+  const float hx = fminf(fmaxf(__fdividef(-0.5f * qb, qa) * ey, x0), x1);
+  const float2 x = make_float2(ex, hx), y = make_float2(vy, ey);
+  const float2 q = __ffma2_rn(__fmul2_rn(bcast(qa), x), x,
+                              __ffma2_rn(__fmul2_rn(bcast(qb), x), y,
+                                         __fmul2_rn(__fmul2_rn(bcast(qc), y), y)));
+  // the mean inside (ex = ey = 0): q is 0 at both, or the circle decides
+  return fminf(q.x, q.y) <= vis || (ex == 0.0f && ey == 0.0f) || vis >= kCircleOnly;
+}
+
+// ---- the culled variants' inner loops ------------------------------------------
+// A warp works on one segment of a staged batch at a time: it tests the
+// segment's splats against its pixel block, 32 a step, and queues the ones that
+// may hit in order in its list; then it blends the list four splats a step.
+// The four alphas do not depend on one another, only T's four multiplications
+// form a chain, and the cut-off is looked at once a step: T never grows, so a
+// pixel above the cut-off after the fourth splat has not ended before.  In a
+// step that ends a pixel, the products of the chain from its end on are
+// dropped.
+constexpr int kGroup = 4, kFineGroup = 8;      // splats blended a step
+constexpr uint32_t kSegment = 256;             // splats culled before they are blended
+constexpr uint32_t kListPitch = kSegment + 8;  // list entries per warp (padded steps)
+constexpr uint32_t kKindShift = 14;            // list entry: staged index | kind << 14
+constexpr uint32_t kIndexMask = (1u << kKindShift) - 1u;
+
+// Queues the splats [k0, k1) of `cur` that may hit the box; returns how many,
+// padded with `none` (an invisible staged splat) to whole steps.
+__device__ __forceinline__ uint32_t cull_segment(const SplatStage* cur, uint32_t k0, uint32_t k1,
+                                                 uint32_t none, float2 xr, float2 yr,
+                                                 uint16_t* list) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t n = 0;
+#pragma unroll 1
+  for (uint32_t k = k0; k < k1; k += 32) {
+    const uint32_t j = k + lane;
+    const uint32_t i = j < k1 ? j : none;
+    const float4 a = cur[i].a, b = cur[i].b;
+    const bool hit = rect_may_hit(a, b, xr, yr);
+    const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+    if (hit)
+      list[n + __popc(mask & lanemask_lt())] =
+          (uint16_t)(i | (__float_as_uint(b.w) << kKindShift));
+    n += __popc(mask);
+  }
+  if (lane < kGroup) list[n + lane] = (uint16_t)none;
+  __syncwarp();
+  return n;
+}
+
+// Blends the n queued splats into the lane's pixels; false once every pixel
+// of the warp has terminated, with used = 1 + the position in the tile's list
+// (position(staged index)) of the splat that ended the lane's last pixel,
+// where it ended in the last step (the warp's largest is among those).
+template <int G, typename PX, typename POS>
+__device__ __forceinline__ bool blend_list(const SplatStage* cur, const uint16_t* list,
+                                           uint32_t n, float pfx, PX& p, POS position,
+                                           uint32_t& used) {
+  using V = typename PX::V;
+  constexpr bool kAhead = G > kGroup;  // one warp's chain: the next step's entries early
+  uint32_t ahead[G / 2];               // two a word
+  if (kAhead) {
+#pragma unroll
+    for (int h = 0; h < G / 2; ++h) ahead[h] = reinterpret_cast<const uint32_t*>(list)[h];
+  }
+  for (uint32_t i = 0; i < n; i += G) {
+    uint32_t e[G / 2];
+#pragma unroll
+    for (int h = 0; h < G / 2; ++h) {
+      if (kAhead) {
+        e[h] = ahead[h];
+        ahead[h] = reinterpret_cast<const uint32_t*>(list + i + G)[h];
+      } else {
+        e[h] = reinterpret_cast<const uint32_t*>(list + i)[h];
+      }
+    }
+    uint32_t id[G], any = 0u, all = ~0u;
+#pragma unroll
+    for (int h = 0; h < G / 2; ++h) {
+      id[2 * h] = e[h] & kIndexMask;
+      id[2 * h + 1] = (e[h] >> 16) & kIndexMask;
+      any |= e[h];
+      all &= e[h];
+    }
+    constexpr uint32_t kKinds = (3u << kKindShift) | (3u << (16 + kKindShift));
+    constexpr uint32_t kAllExact = (kExact << kKindShift) | (kExact << (16 + kKindShift));
+    V al[G];
+    if ((any & kKinds) == 0u) {
+#pragma unroll
+      for (int h = 0; h < G; ++h) al[h] = simple_alpha(pfx, p.y, cur[id[h]]);
+    } else if ((all & kKinds) == kAllExact) {
+#pragma unroll
+      for (int h = 0; h < G; ++h) al[h] = exact_alpha(pfx, p.y, cur[id[h]]);
+    } else {
+#pragma unroll
+      for (int h = 0; h < G; ++h)
+        al[h] = any_alpha(pfx, p.y, cur[id[h]],
+                          ((e[h / 2] >> (16 * (h & 1))) & (kExact << kKindShift)) != 0u);
+    }
+    V t[G + 1];  // T before each splat and after the last
+    t[0] = p.T;
+#pragma unroll
+    for (int h = 0; h < G; ++h) t[h + 1] = PX::mul(t[h], PX::keep(al[h]));
+    V ta[G];
+#pragma unroll
+    for (int h = 0; h < G; ++h) ta[h] = PX::mul(t[h], al[h]);
+    bool ends = false;
+#pragma unroll
+    for (int k = 0; k < PX::kN; ++k)
+      ends = ends || (PX::at(t[G], k) < kEndT && PX::at(t[0], k) > 0.0f);
+    p.T = t[G];
+    const bool any_ends = __any_sync(0xffffffffu, ends);
+    if (any_ends) {
+#pragma unroll
+      for (int k = 0; k < PX::kN; ++k) {
+        float tn = PX::at(t[1], k);
+#pragma unroll
+        for (int h = 1; h < G; ++h) {
+          const bool before = PX::at(t[h], k) >= kEndT;
+          PX::at(ta[h], k) = before ? PX::at(ta[h], k) : 0.0f;
+          tn = before ? PX::at(t[h + 1], k) : tn;
+        }
+        const bool end = tn < kEndT;
+        if (end && PX::at(t[0], k) > 0.0f) PX::at(p.fin, k) = tn;
+        PX::at(p.T, k) = end ? 0.0f : tn;
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+      const float4 c = cur[id[h]].c;
+      p.cr = PX::fma(ta[h], c.x, p.cr);
+      p.cg = PX::fma(ta[h], c.y, p.cg);
+      p.cb = PX::fma(ta[h], c.z, p.cb);
+    }
+    if (any_ends && !__any_sync(0xffffffffu, px_live(p))) {
+#pragma unroll
+      for (int k = 0; k < PX::kN; ++k)
+#pragma unroll
+        for (int h = 0; h < G; ++h)
+          if (PX::at(t[h], k) >= kEndT && PX::at(t[h + 1], k) < kEndT)
+            used = max(used, position(id[h]) + 1);
+      return false;
+    }
+  }
+  return true;
+}
+
+// The staged splats [0, cnt) of one batch, by one warp.
+template <typename PX>
+__device__ __forceinline__ void warp_batch(const SplatStage* cur, uint32_t cnt, uint32_t none,
+                                           float2 xr, float2 yr, uint16_t* list, float pfx, PX& p,
+                                           uint32_t base, uint32_t& used) {
+  if (!__any_sync(0xffffffffu, px_live(p))) return;
+  for (uint32_t k0 = 0; k0 < cnt; k0 += kSegment) {
+    const uint32_t n = cull_segment(cur, k0, min(cnt, k0 + kSegment), none, xr, yr, list);
+    if (!blend_list<kGroup>(cur, list, n, pfx, p, [&](uint32_t i) { return base + i; }, used)) break;
+    __syncwarp();  // the list is rewritten
+  }
+  if (px_live(p)) used = base + cnt;
 }
 
 struct TileGeom {
@@ -344,6 +593,14 @@ __device__ __forceinline__ TileGeom tile_geom(const RasterArgs& a, uint32_t t) {
   g.H = __ldg(&vd.f.viewport[1]);
   g.image = a.image + __ldg(&vd.pixel_base);
   return g;
+}
+
+// Row-major order: does the tile's key count exceed half of a resident warp's
+// fair share of the launch (refs x regions / warps)?  Read on the device, where
+// the live count is.
+__device__ __forceinline__ bool tile_is_heavy(const RasterArgs& a, uint32_t t) {
+  const uint32_t lo = __ldg(a.tile_offsets + t), hi = __ldg(a.tile_offsets + t + 1);
+  return hi > lo + kHeavyKeys && (float)(hi - lo) > a.heavy_share * (float)__ldg(a.ref_counter);
 }
 
 // One thread per pixel, linear pixel order (the reference's layout).
@@ -402,13 +659,9 @@ __device__ void raster_tile_plain(const RasterArgs& a, const TileGeom& g, SplatS
 // Culled variant: warps own compact pixel blocks and skip splats that no
 // pixel of their block can blend.  blockDim.x == tile_w * tile_h, a multiple
 // of 32.
-// The tile's rows [row0, row0 + nthr / tile_w) are shaded by the CTA's nthr
-// threads, one pixel each (the whole tile in the one-pixel kernel; half a
-// row strip when the two-pixel kernel splits a heavy tile).
-__device__ void raster_tile_culled(const RasterArgs& a, const TileGeom& g, uint32_t row0,
-                                   uint32_t nthr, SplatStage* buf0, SplatStage* buf1,
-                                   uint32_t* s_cost) {
-  const uint32_t nt = a.tile_w * a.tile_h;
+__device__ void raster_tile_culled(const RasterArgs& a, const TileGeom& g, SplatStage* buf0,
+                                   SplatStage* buf1, uint16_t* lists, uint32_t* s_cost) {
+  const uint32_t nt = a.tile_w * a.tile_h, nthr = nt;
   const uint32_t D = a.batch ? a.batch : nt;  // splats per staged batch
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t lx, ly;
@@ -417,10 +670,10 @@ __device__ void raster_tile_culled(const RasterArgs& a, const TileGeom& g, uint3
   if (blocks) {  // 8x4 pixel block per warp
     const uint32_t bw = a.tile_w / 8;
     lx = (warp % bw) * 8 + (lane & 7);
-    ly = row0 + (warp / bw) * 4 + (lane >> 3);
+    ly = (warp / bw) * 4 + (lane >> 3);
   } else {
     lx = tid % a.tile_w;
-    ly = row0 + tid / a.tile_w;
+    ly = tid / a.tile_w;
   }
   const uint32_t px = g.ox + lx;
   const uint32_t py = g.oy + ly;
@@ -441,9 +694,12 @@ __device__ void raster_tile_culled(const RasterArgs& a, const TileGeom& g, uint3
   const uint32_t len = end > start ? end - start : 0u;
   const uint32_t nbatches = (len + D - 1) / D;
 
-  Pixel p{0.f, 0.f, 0.f, 1.0f};
-  bool done = !in_bounds;
+  Px1 p;
+  p.y = pfy;
+  if (!in_bounds) p.T = 0.0f;
   uint32_t used = 0;
+  const float2 xr = make_float2(xlo, xhi), yr = make_float2(ylo, yhi);
+  uint16_t* list = lists + warp * kListPitch;
 
   if (nbatches > 0) stage_batch(a.proj, a.values, start, end, D, nthr, buf0);
   for (uint32_t bi = 0; bi < nbatches; ++bi) {
@@ -457,233 +713,354 @@ __device__ void raster_tile_culled(const RasterArgs& a, const TileGeom& g, uint3
     const uint32_t cnt = min(D, end - (start + bi * D));
     for (uint32_t k = tid; k < cnt; k += nthr) prepare(cur[k], reach);  // own copies are complete
     __syncthreads();
-    if (__any_sync(0xffffffffu, !done)) {
-      for (uint32_t k0 = 0; k0 < cnt; k0 += 32) {
-        const uint32_t j = k0 + lane;
-        const bool hit = j < cnt && rect_may_hit(cur[j], make_float2(xlo, xhi), make_float2(ylo, yhi));
-        uint32_t mask = __ballot_sync(0xffffffffu, hit);
-        while (mask) {
-          const uint32_t b0 = __ffs(mask) - 1;
-          mask &= mask - 1;
-          if (mask) {
-            // two hits: both alphas first (independent work for the
-            // scheduler), then the blends in order
-            const uint32_t b1 = __ffs(mask) - 1;
-            mask &= mask - 1;
-            bool ok0, ok1;
-            const float al0 = splat_alpha(pfx, pfy, cur[k0 + b0], ok0);
-            const float al1 = splat_alpha(pfx, pfy, cur[k0 + b1], ok1);
-            if (blend_alpha(p, cur[k0 + b0].c, al0, ok0 && !done)) {
-              done = true;
-              used = bi * D + k0 + b0 + 1;
-            }
-            if (blend_alpha(p, cur[k0 + b1].c, al1, ok1 && !done)) {
-              done = true;
-              used = bi * D + k0 + b1 + 1;
-            }
-          } else if (blend_one<false>(pfx, pfy, cur[k0 + b0], p, !done)) {
-            done = true;
-            used = bi * D + k0 + b0 + 1;
-          }
-        }
-        if (__all_sync(0xffffffffu, done)) break;
-      }
-      if (!done) used = bi * D + cnt;
-    }
-    if (__syncthreads_and(done)) {
+    warp_batch(cur, cnt, D, xr, yr, list, pfx, p, bi * D, used);
+    if (__syncthreads_and(!px_live(p))) {
       cp_async_wait<0>();
       break;
     }
   }
   if (in_bounds) {
     atomicMax(s_cost, used);
-    store_pixel(g.image, g.W, px, py, p);
+    store_pixel(g.image, g.W, px, py, Pixel{p.cr, p.cg, p.cb, px_final(p, 0)});
   }
 }
 
-// Culled variant with two pixels a thread: each warp owns an 8x8 block,
-// lane (x, y) shading rows y and y + 4, so a staged splat is loaded, culled
-// and looped over once for 64 pixels.  blockDim.x == tile_w * tile_h / 2;
-// tile sides divide by 8.  Per pixel the arithmetic and the splat sequence
-// are those of the other variants (bit-identical image).
-__device__ void raster_tile_culled2(const RasterArgs& a, const TileGeom& g, uint32_t strip,
-                                    SplatStage* buf0, SplatStage* buf1, uint32_t* s_cost) {
-  const uint32_t nt = a.tile_w * a.tile_h;
-  const uint32_t strip_h = a.tile_h / a.split;  // this CTA shades rows [strip * strip_h, +strip_h)
-  const uint32_t nthr = a.tile_w * strip_h / 2;
-  const uint32_t D = a.batch ? a.batch : nt;  // splats per staged batch
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t bw = a.tile_w / 8;
-  const float reach = warp_box_reach(a, true);
-  const uint32_t px = g.ox + (warp % bw) * 8 + (lane & 7);
-  const uint32_t py0 = g.oy + strip * strip_h + (warp / bw) * 8 + (lane >> 3), py1 = py0 + 4;
-  const bool in0 = px < g.W && py0 < g.H, in1 = px < g.W && py1 < g.H;
-  const float pfx = (float)px + 0.5f, pfy0 = (float)py0 + 0.5f, pfy1 = (float)py1 + 0.5f;
-  float xlo = pfx, xhi = pfx, ylo = pfy0, yhi = pfy1;
+// The first 32 bytes of a record in one 256-bit load (records are 64-byte
+// aligned).
+__device__ __forceinline__ void load_record(const gs3d_projected_splat* p, SplatStage& s) {
+  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(s.a.x), "=f"(s.a.y), "=f"(s.a.z), "=f"(s.a.w), "=f"(s.b.x), "=f"(s.b.y), "=f"(s.b.z),
+        "=f"(s.b.w)
+      : "l"(p));
+  s.c = __ldg(reinterpret_cast<const float4*>(p) + 2);
+}
+
+// ---- the warp variant: tiles whose sides divide by 8 ---------------------------
+// A work item is one warp's: a region of up to 2x2 pixel blocks of 8x8 of a
+// tile, a lane shading rows y and y + 4 of one column of a block.  Warps share
+// nothing, so there are no block barriers (with a tile's splats staged per CTA
+// they were 26% of the warps' time, waiting for the block with the most hits)
+// and every warp takes its next item from the queue by itself.
+//
+// A warp walks the tile's splats 32 at a time: each lane fetches a record one
+// step ahead, prepares it and tests it against the whole region, and the
+// splats that may hit it (in order) are kept in shared memory.  Once they fill
+// it, each block of the region queues its hits among them and blends
+// (cull_segment, blend_list), its pixels' state parked in shared memory
+// meanwhile.  So the tests against blocks and the padded steps run on full
+// vectors: in a 64x32 tile most splats miss a given 16x16 region.
+//
+// Items of one block instead of a region (and of half a block, one pixel a
+// lane) trade those gains for a shorter chain: they serve launches with fewer
+// regions than resident warps, and the heaviest tiles.
+constexpr uint32_t kRegionRows = 2;  // blocks
+constexpr uint32_t kRegionBlocks = 4;
+constexpr uint32_t kItemWarps = 4;  // warps of a CTA (independent of one another)
+constexpr uint32_t kKept = 104;     // splats kept before they are blended (a multiple of 8)
+struct WarpSmem {
+  SplatStage kept[kKept + 1];  // c.w = position in the tile's list; [kKept] hits nothing
+  float4 state[kRegionBlocks][2][32];  // a block's pixels, per lane
+  uint16_t list[kKept + 16];
+};
+
+__device__ __forceinline__ void load_px(const float4 (&st)[2][32], uint32_t lane, Px2& p) {
+  const float4 a = st[0][lane], b = st[1][lane];  // T < 0: terminated with -T
+  p.cr = make_float2(a.x, a.y);
+  p.cg = make_float2(a.z, a.w);
+  p.cb = make_float2(b.x, b.y);
+  p.T = make_float2(fmaxf(b.z, 0.0f), fmaxf(b.w, 0.0f));
+  p.fin = make_float2(fmaxf(-b.z, 0.0f), fmaxf(-b.w, 0.0f));
+}
+__device__ __forceinline__ void store_px(float4 (&st)[2][32], uint32_t lane, const Px2& p) {
+  st[0][lane] = make_float4(p.cr.x, p.cr.y, p.cg.x, p.cg.y);
+  st[1][lane] = make_float4(p.cb.x, p.cb.y, p.T.x > 0.0f ? p.T.x : -p.fin.x,
+                            p.T.y > 0.0f ? p.T.y : -p.fin.y);
+}
+__device__ __forceinline__ void load_px(const float4 (&st)[2][32], uint32_t lane, Px1& p) {
+  const float4 a = st[0][lane];
+  p.cr = a.x;
+  p.cg = a.y;
+  p.cb = a.z;
+  p.T = fmaxf(a.w, 0.0f);
+  p.fin = fmaxf(-a.w, 0.0f);
+}
+__device__ __forceinline__ void store_px(float4 (&st)[2][32], uint32_t lane, const Px1& p) {
+  st[0][lane] = make_float4(p.cr, p.cg, p.cb, p.T > 0.0f ? p.T : -p.fin);
+}
+
+// Shades the nbx x nby blocks at pixel (x0, y0) of the view; returns the
+// region's share of the tile's cost.  FINE: one block, whose chain through the
+// list is what counts: records are fetched two steps ahead (into the states of
+// the blocks that it does not have), a splat that may hit the region is queued
+// at once, and few are kept before they are blended.
+template <typename PX, bool FINE>
+__device__ uint32_t shade_region(const RasterArgs& a, const TileGeom& g, uint32_t x0, uint32_t y0,
+                                 uint32_t nbx, uint32_t nby, WarpSmem& w) {
+  constexpr uint32_t kRows = PX::kN == 2 ? 8 : 4;  // of a block
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t nb = FINE ? 1u : nbx * nby;
+  const float bx0 = (float)x0 + 0.5f, by0 = (float)y0 + 0.5f;
+  const float2 xr = make_float2(bx0, bx0 + (float)(8 * nbx - 1));
+  const float2 yr = make_float2(by0, by0 + (float)(kRows * nby - 1));
+  auto px_of = [&](uint32_t b) { return x0 + (b % nbx) * 8 + (lane & 7); };
+  auto py_of = [&](uint32_t b) { return y0 + (b / nbx) * kRows + (lane >> 3); };
+
+  uint32_t alive = 0;  // blocks with a pixel that has not terminated
+  for (uint32_t b = 0; b < nb; ++b) {
+    PX p;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    xlo = fminf(xlo, __shfl_xor_sync(0xffffffffu, xlo, o));
-    xhi = fmaxf(xhi, __shfl_xor_sync(0xffffffffu, xhi, o));
-    ylo = fminf(ylo, __shfl_xor_sync(0xffffffffu, ylo, o));
-    yhi = fmaxf(yhi, __shfl_xor_sync(0xffffffffu, yhi, o));
+    for (int i = 0; i < PX::kN; ++i)
+      if (!(px_of(b) < g.W && py_of(b) + 4 * i < g.H)) PX::at(p.T, i) = 0.0f;
+    store_px(w.state[b], lane, p);
+    if (__any_sync(0xffffffffu, px_live(p))) alive |= 1u << b;
   }
 
   const uint32_t start = __ldg(a.tile_offsets + g.tile);
-  const uint32_t end = __ldg(a.tile_offsets + g.tile + 1);
-  const uint32_t len = end > start ? end - start : 0u;
-  const uint32_t nbatches = (len + D - 1) / D;
+  const uint32_t last = __ldg(a.tile_offsets + g.tile + 1);
+  const uint32_t end = last > start ? last : start;
+  uint32_t used = 0, n = 0;
 
-  const float2 pfy = make_float2(pfy0, pfy1);
-  Pixel2 p{bcast(0.f), bcast(0.f), bcast(0.f), bcast(1.0f)};
-  bool done0 = !in0, done1 = !in1;
-  uint32_t used0 = 0, used1 = 0;
-
-  if (nbatches > 0) stage_batch(a.proj, a.values, start, end, D, nthr, buf0);
-  for (uint32_t bi = 0; bi < nbatches; ++bi) {
-    SplatStage* cur = (bi & 1) ? buf1 : buf0;
-    if (bi + 1 < nbatches) {
-      stage_batch(a.proj, a.values, start + (bi + 1) * D, end, D, nthr, (bi & 1) ? buf0 : buf1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+  // blends the n kept splats into every block
+  auto flush = [&]() {
+    if (FINE && lane < 2 * kFineGroup) w.list[n + lane] = (uint16_t)kKept;  // whole steps
+    __syncwarp();
+    for (uint32_t b = 0; b < nb; ++b) {
+      if (!((alive >> b) & 1u)) continue;
+      const float fx = bx0 + (float)((b % nbx) * 8), fy = by0 + (float)((b / nbx) * kRows);
+      const uint32_t hits =
+          FINE ? n
+               : cull_segment(w.kept, 0, n, kKept, make_float2(fx, fx + 7.0f),
+                              make_float2(fy, fy + (float)(kRows - 1)), w.list);
+      PX p;
+      load_px(w.state[b], lane, p);
+      const float ly = fy + (float)(lane >> 3);
+      PX::at(p.y, 0) = ly;
+      if (PX::kN == 2) PX::at(p.y, 1) = ly + 4.0f;
+      if (!blend_list<FINE && PX::kN == 1 ? kFineGroup : kGroup>(w.kept, w.list, hits, fx + (float)(lane & 7), p,
+                      [&](uint32_t i) { return __float_as_uint(w.kept[i].c.w); }, used))
+        alive &= ~(1u << b);
+      store_px(w.state[b], lane, p);
+      __syncwarp();  // the list is rewritten
     }
-    const uint32_t cnt = min(D, end - (start + bi * D));
-    for (uint32_t k = tid; k < cnt; k += nthr) prepare(cur[k], reach);  // own copies are complete
-    __syncthreads();
-    if (__any_sync(0xffffffffu, !(done0 && done1))) {
-      for (uint32_t k0 = 0; k0 < cnt; k0 += 32) {
-        const uint32_t j = k0 + lane;
-        const bool hit = j < cnt && rect_may_hit(cur[j], make_float2(xlo, xhi), make_float2(ylo, yhi));
-        uint32_t mask = __ballot_sync(0xffffffffu, hit);
-        while (mask) {
-          const uint32_t b = __ffs(mask) - 1;
-          mask &= mask - 1;
-          const SplatStage& sp = cur[k0 + b];
-          bool ok0, ok1;
-          const float2 al = splat_alpha2(pfx, pfy, sp, ok0, ok1);
-          ok0 = ok0 && !done0;
-          ok1 = ok1 && !done1;
-          blend_alpha2(p, sp.c, al, ok0, ok1);
-          if (ok0 && p.T.x < 1.0e-4f) {
-            done0 = true;
-            used0 = bi * D + k0 + b + 1;
-          }
-          if (ok1 && p.T.y < 1.0e-4f) {
-            done1 = true;
-            used1 = bi * D + k0 + b + 1;
-          }
-        }
-        if (__all_sync(0xffffffffu, done0 && done1)) break;
+    n = 0;
+  };
+  // keeps the lanes' splats (list positions k + lane) that may hit the region
+  auto keep = [&](SplatStage& s, uint32_t k) {
+    prepare(s, 24.0f);  // the region's pixel centres lie within 15 sqrt(2)
+    const bool hit = k + lane < end && rect_may_hit(s.a, s.b, xr, yr);
+    const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+    if (hit) {
+      const uint32_t i = n + __popc(mask & lanemask_lt());
+      s.c.w = __uint_as_float(k - start + lane);
+      w.kept[i] = s;
+      if (FINE) w.list[i] = (uint16_t)(i | (__float_as_uint(s.b.w) << kKindShift));
+    }
+    n += __popc(mask);
+  };
+  uint32_t id = 0;  // of the record to fetch next
+  auto fetch_id = [&](uint32_t k) {
+    if (k + lane < end) id = __ldg(a.values + k + lane);
+  };
+
+  if (FINE) {
+    SplatStage* ring = reinterpret_cast<SplatStage*>(&w.state[1][0][0]);  // 2 steps of 32
+    auto fetch = [&](uint32_t k, uint32_t slot) {  // a lane reads back only what it fetched
+      if (k + lane < end) {
+        const float4* src = reinterpret_cast<const float4*>(a.proj + id);
+        SplatStage* dst = ring + slot * 32 + lane;
+        cp_async16(&dst->a, src);
+        cp_async16(&dst->b, src + 1);
+        cp_async16(&dst->c, src + 2);
       }
-      if (!done0) used0 = bi * D + cnt;
-      if (!done1) used1 = bi * D + cnt;
+      cp_async_commit();
+    };
+    fetch_id(start);
+    fetch(start, 0);
+    fetch_id(start + 32);
+    fetch(start + 32, 1);
+    fetch_id(start + 64);
+    uint32_t slot = 0;
+    for (uint32_t k = start; k < end && alive; k += 32, slot ^= 1u) {
+      cp_async_wait<1>();
+      SplatStage s = ring[slot * 32 + lane];
+      keep(s, k);
+      fetch(k + 64, slot);
+      fetch_id(k + 96);
+      if (n > kKept - 48) flush();
     }
-    if (__syncthreads_and(done0 && done1)) {
-      cp_async_wait<0>();
-      break;
+    cp_async_wait<0>();
+  } else {
+    SplatStage next{};
+    fetch_id(start);
+    if (start + lane < end) load_record(a.proj + id, next);
+    fetch_id(start + 32);
+    for (uint32_t k = start; k < end && alive; k += 32) {
+      SplatStage s = next;
+      if (k + 32 + lane < end) load_record(a.proj + id, next);
+      fetch_id(k + 64);
+      keep(s, k);
+      if (n > kKept - 32) flush();
     }
   }
-  if (in0) {
-    atomicMax(s_cost, used0);
-    store_pixel(g.image, g.W, px, py0, Pixel{p.cr.x, p.cg.x, p.cb.x, p.T.x});
+  if (n && alive) flush();
+
+  for (uint32_t b = 0; b < nb; ++b) {
+    PX p;
+    load_px(w.state[b], lane, p);
+#pragma unroll
+    for (int i = 0; i < PX::kN; ++i) {
+      const uint32_t px = px_of(b), py = py_of(b) + 4 * i;
+      if (px < g.W && py < g.H)
+        store_pixel(g.image, g.W, px, py,
+                    Pixel{PX::at(p.cr, i), PX::at(p.cg, i), PX::at(p.cb, i), px_final(p, i)});
+    }
   }
-  if (in1) {
-    atomicMax(s_cost, used1);
-    store_pixel(g.image, g.W, px, py1, Pixel{p.cr.y, p.cg.y, p.cb.y, p.T.y});
+  __syncwarp();
+  return alive ? end - start : __reduce_max_sync(0xffffffffu, used);
+}
+
+// Persistent warps.  Work items: first those of the heavy tiles, each a block
+// (row-major order, tiles from heavy_list) or half a block (the head of the
+// order by decreasing expected cost); then the regions of the next a.coarse
+// tiles in order and the blocks of the remaining ones.
+__global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(RasterArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  WarpSmem& w = reinterpret_cast<WarpSmem*>(smem)[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31;
+  if (lane == 0) {
+    w.kept[kKept].a = make_float4(0.f, 0.f, -1.f, 0.f);
+    w.kept[kKept].b = make_float4(0.f, 0.f, 0.f, -1.f);
+    w.kept[kKept].c = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __syncwarp();
+  const uint32_t bw = a.tile_w / 8, blocks = bw * (a.tile_h / 8);
+  const uint32_t rw = (bw + 1) / 2, regions = rw * ((a.tile_h / 8 + kRegionRows - 1) / kRegionRows);
+  const uint32_t heavy = a.heavy != nullptr ? min(__ldg(a.heavy), a.num_tiles) : 0u;
+  const uint32_t per_heavy = a.heavy_list != nullptr ? blocks : 2 * blocks;
+  // heavy tiles of the row-major order come up again among the others
+  const uint32_t first = a.heavy_list != nullptr ? 0u : heavy;
+  const uint32_t fine = max(first, a.coarse);  // tiles [first, fine) by regions
+  const uint64_t heavy_items = (uint64_t)heavy * per_heavy;
+  const uint64_t fine_items = heavy_items + (uint64_t)(fine - first) * regions;
+  const uint64_t items = fine_items + (uint64_t)(a.num_tiles - fine) * blocks;
+  for (;;) {
+    unsigned long long item = 0;
+    if (lane == 0) item = atomicAdd(a.queue_counter, 1ull);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (item >= items) break;
+    uint32_t t, sub;
+    const bool in_heavy = item < heavy_items;
+    if (in_heavy) {
+      const uint32_t i = (uint32_t)(item / per_heavy);
+      sub = (uint32_t)(item - (uint64_t)i * per_heavy);
+      t = a.heavy_list != nullptr ? __ldg(a.heavy_list + i)
+          : a.order != nullptr    ? __ldg(a.order + i)
+                                  : i;
+    } else {
+      const bool coarse = item < fine_items;
+      const uint64_t j = item - (coarse ? heavy_items : fine_items);
+      const uint32_t per_tile = coarse ? regions : blocks;
+      uint32_t i = (uint32_t)(j / per_tile);
+      sub = (uint32_t)(j - (uint64_t)i * per_tile);
+      i += coarse ? first : fine;
+      t = a.order != nullptr ? __ldg(a.order + i) : i;
+      if (a.heavy_list != nullptr && heavy > 0 && tile_is_heavy(a, t)) continue;
+    }
+    const TileGeom g = tile_geom(a, t);
+    uint32_t cost;
+    if (in_heavy && a.heavy_list == nullptr) {
+      const uint32_t b = sub >> 1;
+      cost = shade_region<Px1, true>(a, g, g.ox + (b % bw) * 8, g.oy + (b / bw) * 8 + (sub & 1) * 4, 1,
+                               1, w);
+    } else if (in_heavy || item >= fine_items) {
+      cost = shade_region<Px2, true>(a, g, g.ox + (sub % bw) * 8, g.oy + (sub / bw) * 8, 1, 1, w);
+    } else {
+      const uint32_t rx = 2 * (sub % rw), ry = kRegionRows * (sub / rw);
+      cost = shade_region<Px2, false>(a, g, g.ox + rx * 8, g.oy + ry * 8, min(2u, bw - rx),
+                               min(kRegionRows, a.tile_h / 8 - ry), w);
+    }
+    if (lane == 0 && a.tile_costs != nullptr && cost)
+      atomicMax(a.tile_costs + t, cost);  // zeroed before the launch; max over a tile's items
   }
 }
 
-// Persistent CTAs pull tile indices from the work queue.
-// Persistent CTAs over the queue; MODE 0: one thread per pixel, linear;
-// 1: culled, 8x4 warp blocks; 2: culled, two pixels a thread, 8x8 blocks.
+// Lists the tiles that the row-major order splits: those whose key count
+// exceeds half of a resident warp's fair share of the launch.
+__global__ void __launch_bounds__(256) heavy_list_kernel(RasterArgs a, uint32_t* list,
+                                                         uint32_t* count) {
+  const uint32_t t = blockIdx.x * 256 + threadIdx.x;
+  if (t < a.num_tiles && tile_is_heavy(a, t)) list[atomicAdd(count, 1u)] = t;
+}
+
+// Persistent CTAs over the queue of tiles; MODE 0: one thread per pixel,
+// linear; 1: culled, 8x4 warp blocks.
 template <int MODE>
 __device__ __forceinline__ void raster_loop(const RasterArgs& a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t D = a.batch ? a.batch : a.tile_w * a.tile_h;
   SplatStage* buf0 = reinterpret_cast<SplatStage*>(smem);
-  SplatStage* buf1 = buf0 + D;
+  SplatStage* buf1 = buf0 + D + 1;  // entry D of both: a splat that hits nothing
+  uint16_t* lists = reinterpret_cast<uint16_t*>(buf1 + D + 1);
   __shared__ uint32_t s_item, s_cost;
-  // work items: the first `heavy` tiles of the order as two half-strip items
-  // per strip, then one item per strip of the others
-  const uint32_t heavy = (MODE == 2 && a.heavy != nullptr) ? min(__ldg(a.heavy), a.num_tiles) : 0u;
-  const uint32_t heavy_items = 2u * a.split * heavy;
-  const uint32_t items = heavy_items + (a.num_tiles - heavy) * a.split;
+  if (MODE != 0 && threadIdx.x < 2) {
+    SplatStage& none = (threadIdx.x ? buf1 : buf0)[D];
+    none.a = make_float4(0.f, 0.f, -1.f, 0.f);
+    none.b = make_float4(0.f, 0.f, 0.f, -1.f);
+    none.c = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   while (true) {
     if (threadIdx.x == 0) {
-      s_item = atomicAdd(a.queue_counter, 1u);
+      s_item = (uint32_t)atomicAdd(a.queue_counter, 1ull);
       s_cost = 0u;
     }
     __syncthreads();
     const uint32_t item = s_item;
-    if (item >= items) break;
-    uint32_t ti, strip, half;  // half: 0 whole strip, 1 / 2 first / second half
-    if (item < heavy_items) {
-      ti = item / (2u * a.split);
-      const uint32_t sub = item - ti * 2u * a.split;
-      strip = sub >> 1;
-      half = 1u + (sub & 1u);
-    } else {
-      const uint32_t j = item - heavy_items;
-      ti = heavy + j / a.split;
-      strip = j - (ti - heavy) * a.split;
-      half = 0u;
-    }
-    const uint32_t t = a.order != nullptr ? __ldg(a.order + ti) : ti;
+    if (item >= a.num_tiles) break;
+    const uint32_t t = a.order != nullptr ? __ldg(a.order + item) : item;
     const TileGeom g = tile_geom(a, t);
-    if (MODE == 2) {
-      if (half == 0u) {
-        raster_tile_culled2(a, g, strip, buf0, buf1, &s_cost);
-      } else {  // half a row strip, one pixel a thread (the same per-pixel arithmetic)
-        const uint32_t strip_h = a.tile_h / a.split;
-        raster_tile_culled(a, g, strip * strip_h + (half - 1u) * (strip_h / 2), blockDim.x, buf0,
-                           buf1, &s_cost);
-      }
-    } else if (MODE == 1) {
-      raster_tile_culled(a, g, 0u, a.tile_w * a.tile_h, buf0, buf1, &s_cost);
+    if (MODE == 1) {
+      raster_tile_culled(a, g, buf0, buf1, lists, &s_cost);
     } else {
       raster_tile_plain(a, g, buf0, buf1, &s_cost);
     }
     __syncthreads();  // s_cost complete; shared buffers free for the next tile
-    if (threadIdx.x == 0 && a.tile_costs != nullptr)
-      atomicMax(a.tile_costs + t, s_cost);  // zeroed before the launch; max over a tile's items
+    if (threadIdx.x == 0 && a.tile_costs != nullptr) atomicMax(a.tile_costs + t, s_cost);
   }
 }
 
 __global__ void raster_kernel_plain(RasterArgs a) { raster_loop<0>(a); }
-__global__ void raster_kernel_culled(RasterArgs a) { raster_loop<1>(a); }
-// at most 512 threads (a 1024-pixel tile of unsplittable strips)
-__global__ void __launch_bounds__(512, 2) raster_kernel_culled2(RasterArgs a) {
-  raster_loop<2>(a);
-}
+__global__ void __launch_bounds__(1024) raster_kernel_culled(RasterArgs a) { raster_loop<1>(a); }
 
-// Variant, strips, block size, staged batch and resident CTAs per SM of the
-// raster launch for `a` (the occupancy is computed once per device and shape).
+// Variant, block size, staged batch and resident CTAs per SM of the raster
+// launch for `a` (the occupancy is computed once per device and shape).
 struct RasterConfig {
   int mode;
-  uint32_t split, threads, D;
+  uint32_t threads, D;
+  size_t smem;
   int per_sm;
+  uint32_t regions, blocks;  // work items per tile of the warp variant
   void (*kern)(RasterArgs);
 };
+
+// Two staged batches and, for the culled variants, a list per warp.
+size_t raster_smem(int mode, uint32_t D, uint32_t threads) {
+  if (mode == 2) return kItemWarps * sizeof(WarpSmem);
+  return 2 * ((size_t)D + 1) * sizeof(SplatStage) +
+         (mode != 0 ? (size_t)(threads / 32) * kListPitch * sizeof(uint16_t) : 0);
+}
 
 cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
   const uint32_t nt = a.tile_w * a.tile_h;
   if (a.batch % 32 != 0 || a.batch > 1024) return cudaErrorInvalidValue;
-  const uint32_t D = a.batch ? a.batch : nt;
   const bool culled = a.culled && (nt % 32 == 0);
-  // two pixels a thread where the tile splits into 8x8 blocks
+  // warp items where the tile splits into 8x8 blocks
   const int mode = !culled ? 0 : (a.tile_w % 8 == 0 && a.tile_h % 8 == 0) ? 2 : 1;
-  // two-pixel tiles of more than 512 pixels are shaded by four (else two)
-  // CTAs of row strips whose heights divide by 8, so that a block barrier
-  // waits for few warps and more CTAs interleave on an SM
-  uint32_t split = 1;
-  if (mode == 2 && nt > 512) split = (a.tile_h / 4) % 8 == 0 ? 4u : (a.tile_h / 2) % 8 == 0 ? 2u : 1u;
-  const uint32_t threads = mode == 2 ? nt / (2 * split) : nt;
-  // one thread a pixel up to 1024 pixels; two-pixel strips of at most 512
-  // threads (the kernel's launch bound)
-  if ((mode != 2 && nt > 1024) || (mode == 2 && threads > 512)) return cudaErrorInvalidValue;
-  const size_t smem = 2 * (size_t)D * sizeof(SplatStage);
-  auto kern = mode == 2 ? raster_kernel_culled2 : mode == 1 ? raster_kernel_culled
-                                                             : raster_kernel_plain;
+  if (mode != 2 && nt > 1024) return cudaErrorInvalidValue;  // one thread a pixel
+  const uint32_t D = mode == 2 ? 0u : a.batch ? a.batch : nt;
+  const uint32_t threads = mode == 2 ? kItemWarps * 32 : nt;
+  const size_t smem = raster_smem(mode, D, threads);
+  auto kern = mode == 2 ? raster_kernel_warps : mode == 1 ? raster_kernel_culled
+                                                           : raster_kernel_plain;
   // launch configuration per (device, variant, tile area, batch), computed
   // once per process (the shared-memory attribute is a per-device setting)
   static std::mutex mu;
@@ -705,7 +1082,7 @@ cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
     // one attribute per kernel, set to the largest batch's footprint so that
     // configurations cached earlier keep fitting
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(2 * 1024 * sizeof(SplatStage)));
+                                         (int)raster_smem(mode, 1024, 1024));
     if (e != cudaSuccess) return e;
     int n = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)threads, smem);
@@ -714,40 +1091,59 @@ cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
     std::lock_guard<std::mutex> lock(mu);
     cache[key] = per_sm;
   }
-  *cfg = RasterConfig{mode, split, threads, D, per_sm, kern};
+  const uint32_t bw = a.tile_w / 8, bh = a.tile_h / 8;
+  *cfg = RasterConfig{mode,   threads, D,   smem, per_sm, mode == 2 ? ((bw + 1) / 2) * ((bh + kRegionRows - 1) / kRegionRows) : 1u,
+                      mode == 2 ? bw * bh : 1u, kern};
   return cudaSuccess;
 }
+
+// The last regions of a launch, this many for each resident warp, are shaded
+// by blocks: a launch of few regions is bound by its longest item's chain, and
+// a larger one by the items under way when the queue runs empty.
+constexpr float kFineWaves = 1.75f;
 
 }  // namespace
 
-cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* strips,
-                         uint32_t* resident_ctas) {
+cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* items_per_tile,
+                         uint32_t* resident) {
   RasterConfig cfg;
   const cudaError_t e = raster_config(a, &cfg);
   if (e != cudaSuccess) return e;
-  *strips = cfg.split;
-  *resident_ctas = (uint32_t)sm_count * (uint32_t)cfg.per_sm;
+  *items_per_tile = cfg.regions;
+  *resident = (uint32_t)sm_count * (uint32_t)cfg.per_sm * (cfg.mode == 2 ? kItemWarps : 1u);
   return cudaSuccess;
 }
 
-cudaError_t launch_raster(const RasterArgs& args, int sm_count, cudaStream_t s) {
+cudaError_t launch_raster(const RasterArgs& args, uint32_t* heavy_list, uint32_t* heavy_count,
+                          int sm_count, cudaStream_t s) {
   if (args.num_tiles == 0) return cudaSuccess;
   RasterArgs a = args;
   RasterConfig cfg;
   cudaError_t e = raster_config(a, &cfg);
   if (e != cudaSuccess) return e;
-  a.split = cfg.split;
-  if (cfg.mode != 2) a.heavy = nullptr;  // half strips exist in the two-pixel variant only
   // every work item folds its cost into its tile's by maximum
   if (a.tile_costs != nullptr) {
     e = cudaMemsetAsync(a.tile_costs, 0, (size_t)a.num_tiles * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
   }
-  // up to two items per strip when tiles are split
-  const uint64_t max_items = (uint64_t)a.num_tiles * a.split * (a.heavy != nullptr ? 2 : 1);
-  const uint32_t grid = (uint32_t)std::min<uint64_t>(
-      max_items, (uint64_t)sm_count * (uint64_t)std::max(cfg.per_sm, 1));
-  cfg.kern<<<grid, cfg.threads, 2 * (size_t)cfg.D * sizeof(SplatStage), s>>>(a);
+  const uint32_t ctas = (uint32_t)sm_count * (uint32_t)cfg.per_sm;
+  uint64_t max_ctas = a.num_tiles;
+  if (cfg.mode == 2) {
+    const uint64_t warps = (uint64_t)ctas * kItemWarps;
+    a.coarse = (float)a.num_tiles * (float)cfg.regions > kFineWaves * (float)warps ? a.num_tiles : 0u;
+    if (a.order == nullptr && a.heavy == nullptr && a.coarse > 0 && cfg.blocks > 1) {
+      a.heavy_share = 0.5f * (float)cfg.regions / (float)warps;
+      heavy_list_kernel<<<(a.num_tiles + 255) / 256, 256, 0, s>>>(a, heavy_list, heavy_count);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      a.heavy_list = heavy_list;
+      a.heavy = heavy_count;
+    }
+    max_ctas = ((uint64_t)a.num_tiles * cfg.blocks * 2 + kItemWarps - 1) / kItemWarps;
+  } else {
+    a.heavy = nullptr;  // split items exist in the warp variant only
+  }
+  cfg.kern<<<(uint32_t)std::min<uint64_t>(max_ctas, ctas), cfg.threads, cfg.smem, s>>>(a);
   return cudaGetLastError();
 }
 

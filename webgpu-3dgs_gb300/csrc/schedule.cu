@@ -11,10 +11,10 @@
 // schedule the learned one falls back to).  Learned schedule: expected cost
 // = the cost MLP's prediction (learned.cu); both sort 16-bit keys.
 //
-// Both also split: the tiles whose expected cost per strip exceeds half of a
-// raster CTA's fair share of the frame (the head of the order) are shaded as
-// two half-strip work items per strip, so a tile far heavier than the rest
-// does not leave one CTA running alone at the end of the raster.
+// Both also split: the tiles whose expected cost per work item exceeds half of
+// a raster worker's fair share of the frame (the head of the order) are shaded
+// as two items per 8x8 pixel block, so a tile far heavier than the rest does not
+// leave one worker running alone at the end of the raster.
 #include "gs3d_internal.cuh"
 
 namespace gs3d {
@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(kThreads)
 constexpr int kHeavyThreads = 1024;
 __global__ void __launch_bounds__(kHeavyThreads)
     heavy_count_kernel(const float* __restrict__ est, uint32_t n, uint32_t raster_ctas,
-                       uint32_t strips, uint32_t all, uint32_t* __restrict__ heavy) {
+                       uint32_t strips, float floor, uint32_t all,
+                       uint32_t* __restrict__ heavy) {
   __shared__ float s_sum[kHeavyThreads / 32];
   __shared__ uint32_t s_cnt[kHeavyThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -59,8 +60,9 @@ __global__ void __launch_bounds__(kHeavyThreads)
   __syncthreads();
   float total = 0.0f;
   for (int w = 0; w < kHeavyThreads / 32; ++w) total += s_sum[w];
-  // a strip costs about est; the frame about sum(est) * strips
-  const float thr = 0.5f * total * (float)strips / (float)max(raster_ctas, 1u);
+  // a work item costs about est; the frame about sum(est) * strips
+  const float thr =
+      fmaxf(0.5f * total * (float)strips / (float)max(raster_ctas, 1u), floor);
   uint32_t cnt = 0;
   for (uint32_t t = threadIdx.x; t < n; t += kHeavyThreads) cnt += __ldg(est + t) > thr ? 1u : 0u;
 #pragma unroll
@@ -77,9 +79,10 @@ __global__ void __launch_bounds__(kHeavyThreads)
 }  // namespace
 
 cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t raster_ctas,
-                               uint32_t strips, bool all, uint32_t* heavy, cudaStream_t s) {
-  heavy_count_kernel<<<1, kHeavyThreads, 0, s>>>(est, n, raster_ctas, strips, all ? 1u : 0u,
-                                                 heavy);
+                               uint32_t strips, float floor, bool all, uint32_t* heavy,
+                               cudaStream_t s) {
+  heavy_count_kernel<<<1, kHeavyThreads, 0, s>>>(est, n, raster_ctas, strips, floor,
+                                                 all ? 1u : 0u, heavy);
   return cudaGetLastError();
 }
 
@@ -96,7 +99,9 @@ cudaError_t launch_schedule(uint32_t schedule, const uint32_t* tile_offsets, uin
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  e = launch_heavy_count(est, num_tiles, raster_ctas, strips, split_all, &ctrl->raster_heavy, s);
+  e = launch_heavy_count(est, num_tiles, raster_ctas, strips,
+                         schedule == GS3D_SCHEDULE_LEARNED ? (float)kHeavyCost : (float)kHeavyKeys,
+                         split_all, &ctrl->raster_heavy, s);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(ctrl->sched_counter, 0, sizeof(ctrl->sched_counter), s);
   if (e != cudaSuccess) return e;
