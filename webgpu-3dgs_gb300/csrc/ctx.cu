@@ -84,6 +84,8 @@ struct gs3d_ctx {
   DevBuf scan_status, sort_status;
   uint32_t scan_epoch = 0;
   DevBuf depth_keys_a, depth_ids_a, depth_keys_b, depth_ids_b, sorted_offsets, depth_status;
+  // binned rebin: first entry of every cell, chunks of entries, tile totals
+  DevBuf cell_start, chunk_cell, chunk_counts, tile_counts, tile_scan_status;
   DevBuf rect8;  // one-word tile rectangles per splat-view (fused rebin, small grids)
   DevBuf tile_offsets, image, tile_costs, composite_out;
   DevBuf sched_keys_a, sched_keys_b, sched_order_a, sched_order_b, sched_status;
@@ -98,7 +100,7 @@ struct gs3d_ctx {
   bool have_camera = false;
   std::vector<ViewDesc> views;       // host copy
   std::vector<gs3d_view_info> info;  // per-view layout
-  uint32_t total_splats = 0, total_tiles = 0, total_blocks = 0, max_sh = 0;
+  uint32_t total_splats = 0, total_tiles = 0, total_cells = 0, total_blocks = 0, max_sh = 0;
   uint64_t total_pixels = 0;
   DevBuf d_views;
   ViewDesc* h_upload = nullptr;  // pinned ring of view tables
@@ -197,6 +199,15 @@ uint32_t* u32(DevBuf& b) { return static_cast<uint32_t*>(b.p); }
 Ctrl* ctrl_of(gs3d_ctx* c) { return static_cast<Ctrl*>(c->ctrl.p); }
 ViewDesc* dviews(gs3d_ctx* c) { return static_cast<ViewDesc*>(c->d_views.p); }
 
+// Chunk buffers of the binned rebin: the key capacity's entries in the cells of
+// the current batch.
+int ensure_chunks(gs3d_ctx* c, uint32_t cells) {
+  const size_t slots = chunk_slots_max(c->capacity, cells);
+  TRY(ensure(c, c->chunk_cell, slots * 4, "cell chunks"));
+  TRY(ensure(c, c->chunk_counts, slots * kCellTiles * 4, "cell chunk counts"));
+  return GS3D_OK;
+}
+
 int ensure_key_capacity(gs3d_ctx* c, uint64_t want) {
   if (want > kMaxCapacity)
     return fail(c, GS3D_ERR_CAPACITY, "%llu tile refs exceed the %u-ref limit of one rebin",
@@ -211,7 +222,7 @@ int ensure_key_capacity(gs3d_ctx* c, uint64_t want) {
   TRY(ensure(c, c->sort_status, sort_status_words_max(cap) * sizeof(uint32_t),
              "sort look-back status"));
   c->capacity = cap;
-  return GS3D_OK;
+  return c->total_cells ? ensure_chunks(c, c->total_cells) : GS3D_OK;
 }
 
 // Per-splat-view buffers for a batch of `m` splat-views.
@@ -349,7 +360,7 @@ int set_views(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, bool upload
   if (n_views == 0 || !views) return fail(c, GS3D_ERR_INVALID_ARG, "empty view list");
   std::vector<ViewDesc> vds(n_views, ViewDesc{});
   std::vector<gs3d_view_info> infos(n_views, gs3d_view_info{});
-  uint64_t splats = 0, tiles = 0, pixels = 0, blocks = 0;
+  uint64_t splats = 0, tiles = 0, cells = 0, pixels = 0, blocks = 0;
   uint32_t max_sh = 0;
   for (uint32_t v = 0; v < n_views; ++v) {
     const gs3d_view& in = views[v];
@@ -382,6 +393,8 @@ int set_views(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, bool upload
     d.sh_degree = sc.sh_degree;
     d.splat_base = (uint32_t)splats;
     d.pixel_base = pixels;
+    d.cell_base = (uint32_t)cells;
+    d.cells_x = (tx + kCellSide - 1) / kCellSide;
     gs3d_view_info& vi = infos[v];
     vi.pixel_offset = pixels;
     vi.width = w;
@@ -396,6 +409,7 @@ int set_views(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, bool upload
     d.group_next = kNoView;
     splats += sc.n;
     tiles += (uint64_t)tx * ty;
+    cells += (uint64_t)d.cells_x * ((ty + kCellSide - 1) / kCellSide);
     pixels += (uint64_t)w * h;
   }
   // scene groups: views of one scene are projected by one preprocess block
@@ -436,12 +450,17 @@ int set_views(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, bool upload
   TRY(ensure(c, c->tile_est, std::max<uint64_t>(tiles, 1) * 4, "tile expected costs"));
   TRY(ensure(c, c->d_views, (size_t)n_views * sizeof(ViewDesc), "view table"));
   if (c->capacity < 1) TRY(ensure_key_capacity(c, 1));
+  TRY(ensure(c, c->tile_counts, std::max<uint64_t>(tiles, 1) * 4, "tile counts"));
+  TRY(ensure(c, c->tile_scan_status, scan_status_words((uint32_t)tiles) * 8, "tile scan status"));
+  TRY(ensure(c, c->cell_start, (cells + 1) * 4, "cell starts"));
+  TRY(ensure_chunks(c, (uint32_t)cells));
 
   if (!upload) {  // the caller uploads the table (CUDA-graph replay)
     c->views.swap(vds);
     c->info.swap(infos);
     c->total_splats = (uint32_t)splats;
     c->total_tiles = (uint32_t)tiles;
+    c->total_cells = (uint32_t)cells;
     c->total_pixels = pixels;
     c->total_blocks = (uint32_t)blocks;
     c->max_sh = max_sh;
@@ -471,6 +490,7 @@ int set_views(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, bool upload
   c->info.swap(infos);
   c->total_splats = (uint32_t)splats;
   c->total_tiles = (uint32_t)tiles;
+  c->total_cells = (uint32_t)cells;
   c->total_pixels = pixels;
   c->total_blocks = (uint32_t)blocks;
   c->max_sh = max_sh;
@@ -590,36 +610,98 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   return GS3D_OK;
 }
 
-// Fused rebin over the current batch: depth digits sorted over splat-views,
-// refs emitted in depth order, tile digits sorted over refs.  For every view
-// the sorted keys, values, tile_offsets and image equal the stage-wise
-// sequence's.
-int fused_rebin(gs3d_ctx* c) {
-  TRY(require_frame(c, "rebin"));
+// Do the refs go through cells (binning.cu) or through the digit passes over
+// the refs themselves?  Cells take three launches more, so they pay where the
+// refs outweigh a launch: sum of the stages from scan to tile ranges, passes ->
+// cells, 20k splats 51 -> 69 us, 100k 79 -> 87 us, 400k 110 -> 109 us, 3M (16x16
+// tiles) 623 -> 294 us, 8 views of 3M (64x32) 1743 -> 1306 us, 3M heavy-tailed
+// splats at 4K (32x32) 3317 -> 815 us.
+constexpr uint32_t kCellsMinSplats = 300000;
+bool use_cells(const gs3d_ctx* c) {
+  bool fits = c->total_cells <= kMaxCells && c->total_splats >= kCellsMinSplats;
+  for (const ViewDesc& v : c->views)
+    fits = fits && v.f.tile_count[0] <= 0xffffu && v.f.tile_count[1] <= 0xffffu;
+  return fits && c->total_tiles > 256;  // else one digit pass
+}
+
+void next_scan_epoch(gs3d_ctx* c) { c->scan_epoch = (c->scan_epoch % ((1u << 30) - 1)) + 1; }
+
+SortPlan cell_digit_plan(uint32_t num_cells, uint32_t digit_bits) {
+  SortPlan p = tile_digit_plan(num_cells, digit_bits);
+  for (int k = 0; k < p.passes; ++k) p.shift[k] += (int)kCellShift;
+  return p;
+}
+
+// Depth-ordered splats -> refs in (tile, depth, splat) order and tile ranges:
+// entries per (splat, cell) in depth order, sorted by cell, expanded in place.
+// The refs end in the A buffers.
+int bin_refs(gs3d_ctx* c, const uint32_t* rect8) {
+  Ctrl* k = ctrl_of(c);
+  const uint32_t nv = (uint32_t)c->views.size(), cells = c->total_cells;
+  const gs3d_projected_splat* proj = static_cast<gs3d_projected_splat*>(c->proj.p);
+  next_scan_epoch(c);
+  {
+    StageScope t(c, GS3D_STAGE_SCAN);
+    // cleared every rebin: a graph replay reuses the captured epoch
+    CK(cudaMemsetAsync(c->scan_status.p, 0, scan_status_words(c->total_splats) * 8, c->stream),
+       "clear scan status");
+    CK(launch_scan_cells(u32(c->counts), rect8, proj, u32(c->depth_ids_a), u32(c->sorted_offsets),
+                         c->total_splats, static_cast<unsigned long long*>(c->scan_status.p),
+                         &k->scan_tile_counter, c->scan_epoch, &k->entry_total, &k->ref_total,
+                         &k->error, c->stream),
+       "prefix scan (cells, depth order)");
+  }
+  const SortPlan cp = cell_digit_plan(cells, c->digit_bits);
+  // the sorted entries end in the B buffers
+  DevBuf& ka = cp.passes % 2 ? c->keys_a : c->keys_b;
+  DevBuf& kb = cp.passes % 2 ? c->keys_b : c->keys_a;
+  DevBuf& va = cp.passes % 2 ? c->vals_a : c->vals_b;
+  DevBuf& vb = cp.passes % 2 ? c->vals_b : c->vals_a;
+  {
+    StageScope t(c, GS3D_STAGE_EMIT);
+    CK(launch_emit_cells(dviews(c), nv, c->total_splats, proj, rect8, u32(c->depth_keys_a),
+                         u32(c->depth_ids_a), u32(c->sorted_offsets), &k->entry_total,
+                         &k->ref_total, u32(c->ref_counter), c->capacity,
+                         static_cast<uint2*>(ka.p), u32(va), cp, &k->tile_hist[0][0],
+                         &k->emit_chunk, &k->error, c->sm_count, c->stream),
+       "emit (cells, depth order)");
+  }
+  const uint2* entries = static_cast<uint2*>(c->keys_b.p);
+  {
+    StageScope t(c, GS3D_STAGE_SORT);
+    CK(launch_sort_tile_passes(cp, &k->entry_total, c->capacity, static_cast<uint2*>(ka.p),
+                               u32(va), static_cast<uint2*>(kb.p), u32(vb), u32(c->sort_status),
+                               &k->tile_hist[0][0], &k->sort_part_counter[4], &k->error,
+                               c->sm_count, c->stream),
+       "cell-digit sort");
+  }
+  {
+    StageScope t(c, GS3D_STAGE_IDENTIFY);
+    CK(launch_bin_count(dviews(c), nv, cells, entries, &k->entry_total, &k->ref_total, c->capacity,
+                        u32(c->cell_start), u32(c->chunk_cell), u32(c->chunk_counts),
+                        u32(c->tile_counts), c->sm_count, c->stream),
+       "tile counts");
+    CK(cudaMemsetAsync(c->tile_scan_status.p, 0, scan_status_words(c->total_tiles) * 8, c->stream),
+       "clear tile scan status");
+    CK(launch_scan_tiles(u32(c->tile_counts), u32(c->tile_offsets), c->total_tiles, &k->ref_total,
+                         static_cast<unsigned long long*>(c->tile_scan_status.p),
+                         &k->tile_scan_counter, c->scan_epoch, &k->tile_scan_total, &k->error,
+                         c->stream),
+       "tile offsets");
+    CK(launch_bin_place(dviews(c), nv, cells, entries, u32(c->vals_b), u32(c->cell_start),
+                        u32(c->chunk_cell), u32(c->chunk_counts), u32(c->tile_offsets),
+                        &k->ref_total, c->capacity, static_cast<uint2*>(c->keys_a.p),
+                        u32(c->vals_a), &k->place_chunk, &k->error, c->sm_count, c->stream),
+       "ref placement");
+  }
+  return GS3D_OK;
+}
+
+// The same by the digit passes over the refs.
+int sort_refs(gs3d_ctx* c, const uint32_t* rect8) {
   Ctrl* k = ctrl_of(c);
   const uint32_t nv = (uint32_t)c->views.size();
-  CK(cudaMemsetAsync(c->ctrl.p, 0, sizeof(Ctrl), c->stream), "reset control block");
-  // tile rectangles fit one word when every view has at most 256 tiles per axis
-  bool small_grids = true;
-  for (const ViewDesc& v : c->views)
-    small_grids = small_grids && v.f.tile_count[0] <= 256 && v.f.tile_count[1] <= 256;
-  uint32_t* rect8 = small_grids ? u32(c->rect8) : nullptr;
-  {
-    StageScope t(c, GS3D_STAGE_PREPROCESS);
-    CK(launch_preprocess(dviews(c), nv, c->total_blocks, c->max_sh,
-                         static_cast<gs3d_projected_splat*>(c->proj.p), u32(c->counts),
-                         u32(c->depth_keys_a), u32(c->depth_ids_a), rect8, &k->error, c->stream),
-       "preprocess");
-  }
-  {
-    StageScope t(c, GS3D_STAGE_DEPTH_SORT);
-    CK(launch_sort_depth_keys(&dviews(c)->batch_splats, c->total_splats, u32(c->depth_keys_a),
-                              u32(c->depth_ids_a), u32(c->depth_keys_b), u32(c->depth_ids_b),
-                              u32(c->depth_status), &k->sort_hist[0][0],
-                              &k->sort_part_counter[0], &k->error, c->sm_count, c->stream),
-       "depth sort");
-  }
-  c->scan_epoch = (c->scan_epoch % ((1u << 30) - 1)) + 1;
+  next_scan_epoch(c);
   {
     StageScope t(c, GS3D_STAGE_SCAN);
     // cleared every rebin: a graph replay reuses the captured epoch
@@ -660,6 +742,43 @@ int fused_rebin(gs3d_ctx* c) {
     CK(launch_identify(static_cast<uint2*>(c->keys_a.p), u32(c->ref_counter), c->capacity,
                        c->total_tiles, u32(c->tile_offsets), &k->error, c->sm_count, c->stream),
        "identify_tile_ranges");
+  }
+  return GS3D_OK;
+}
+
+// Fused rebin over the current batch: depth digits sorted over splat-views,
+// refs emitted in depth order, tile digits sorted over refs.  For every view
+// the sorted keys, values, tile_offsets and image equal the stage-wise
+// sequence's.
+int fused_rebin(gs3d_ctx* c) {
+  TRY(require_frame(c, "rebin"));
+  Ctrl* k = ctrl_of(c);
+  const uint32_t nv = (uint32_t)c->views.size();
+  CK(cudaMemsetAsync(c->ctrl.p, 0, sizeof(Ctrl), c->stream), "reset control block");
+  // tile rectangles fit one word when every view has at most 256 tiles per axis
+  bool small_grids = true;
+  for (const ViewDesc& v : c->views)
+    small_grids = small_grids && v.f.tile_count[0] <= 256 && v.f.tile_count[1] <= 256;
+  uint32_t* rect8 = small_grids ? u32(c->rect8) : nullptr;
+  {
+    StageScope t(c, GS3D_STAGE_PREPROCESS);
+    CK(launch_preprocess(dviews(c), nv, c->total_blocks, c->max_sh,
+                         static_cast<gs3d_projected_splat*>(c->proj.p), u32(c->counts),
+                         u32(c->depth_keys_a), u32(c->depth_ids_a), rect8, &k->error, c->stream),
+       "preprocess");
+  }
+  {
+    StageScope t(c, GS3D_STAGE_DEPTH_SORT);
+    CK(launch_sort_depth_keys(&dviews(c)->batch_splats, c->total_splats, u32(c->depth_keys_a),
+                              u32(c->depth_ids_a), u32(c->depth_keys_b), u32(c->depth_ids_b),
+                              u32(c->depth_status), &k->sort_hist[0][0],
+                              &k->sort_part_counter[0], &k->error, c->sm_count, c->stream),
+       "depth sort");
+  }
+  if (use_cells(c)) {
+    TRY(bin_refs(c, rect8));
+  } else {
+    TRY(sort_refs(c, rect8));
   }
   return raster_stage(c, true);
 }
@@ -827,7 +946,8 @@ int gs3d_destroy(gs3d_ctx* c) {
                     &c->keys_a,        &c->vals_a,        &c->keys_b,        &c->vals_b,
                     &c->scan_status,   &c->sort_status,   &c->depth_keys_a,  &c->depth_ids_a,
                     &c->depth_keys_b,  &c->depth_ids_b,   &c->sorted_offsets, &c->depth_status,
-                    &c->rect8,
+                    &c->rect8,         &c->cell_start,    &c->chunk_cell,
+                    &c->chunk_counts,  &c->tile_counts,   &c->tile_scan_status,
                     &c->tile_offsets,  &c->image,         &c->tile_costs,    &c->sched_keys_a,
                     &c->sched_keys_b,  &c->sched_order_a, &c->sched_order_b, &c->sched_status,
                     &c->d_views,       &c->ctrl,          &c->model_params,  &c->model_mean,
@@ -1279,7 +1399,9 @@ int gs3d_autotune(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, uint32_
         gs3d_tune_result r{};
         r.tuning = t;
         r.ms_per_view = ms / (float)reps / (float)n_views;
-        r.tile_passes = (uint32_t)tile_digit_plan(c->total_tiles, digit).passes;
+        r.tile_passes = (uint32_t)(use_cells(c) ? cell_digit_plan(c->total_cells, digit)
+                                                : tile_digit_plan(c->total_tiles, digit))
+                            .passes;
         r.refs = refs;
         res.push_back(r);
       }

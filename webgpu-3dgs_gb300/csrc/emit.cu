@@ -98,7 +98,16 @@ __global__ void __launch_bounds__(kThreads)
 // millions of atomics per batch on a few L2 slices) cost more than the emit's
 // own stores.  Tickets rather than a fixed stride, because the refs of a chunk
 // range from 256 to millions (near splats covering a whole view).
-template <int TP, int BINS>
+//
+// CELLS: the binned rebin's entries (binning.cu) instead of refs, one per
+// (splat-view, cell of 8x8 tiles): keys hold the cell and the part of the
+// splat's rectangle inside it, offsets count cells, and the frame's refs (which
+// the capacity is checked against: at least one per entry) are in *ref_total.
+struct CellArgs {
+  const unsigned long long* ref_total;
+  uint32_t* ref_counter;  // written: min(*ref_total, 2^32 - 1)
+};
+template <int TP, int BINS, bool CELLS>
 __global__ void __launch_bounds__(kThreads)
     emit_sorted_kernel(const ViewDesc* __restrict__ views, uint32_t n_views, uint32_t n,
                        const gs3d_projected_splat* __restrict__ proj,
@@ -106,8 +115,9 @@ __global__ void __launch_bounds__(kThreads)
                        const uint32_t* __restrict__ sorted_keys,
                        const uint32_t* __restrict__ sorted_ids,
                        const uint32_t* __restrict__ sorted_offsets,
-                       const uint32_t* __restrict__ ref_counter, uint32_t capacity,
-                       uint2* __restrict__ keys, uint32_t* __restrict__ values, int4 shifts,
+                       const uint32_t* __restrict__ ref_counter, CellArgs cells,
+                       uint32_t capacity, uint2* __restrict__ keys,
+                       uint32_t* __restrict__ values, int4 shifts,
                        uint4 masks, uint32_t* __restrict__ g_hist,
                        uint32_t* __restrict__ chunk_ticket, uint32_t* __restrict__ err) {
   __shared__ uint32_t s_off[kThreads + 1];
@@ -119,7 +129,10 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ uint32_t s_first, s_next;  // tickets: the block's first chunk, its next one
 
   const uint32_t total = *ref_counter;
-  if (total > capacity) {
+  const unsigned long long frame_refs = CELLS ? *cells.ref_total : total;
+  if (CELLS && blockIdx.x == 0 && threadIdx.x == 0)
+    *cells.ref_counter = frame_refs > 0xffffffffull ? 0xffffffffu : (uint32_t)frame_refs;
+  if (frame_refs > capacity) {
     if (blockIdx.x == 0 && threadIdx.x == 0) latch_error(err, DEVERR_CAPACITY);
     return;
   }
@@ -151,7 +164,8 @@ __global__ void __launch_bounds__(kThreads)
   auto gather = [&](uint32_t c) {
     if (c >= chunks || c * kThreads + threadIdx.x >= n) return;
     if (rect8 != nullptr) {
-      const uint32_t rr = __ldg(rect8 + p_id);
+      uint32_t rr = __ldg(rect8 + p_id);
+      if (rr == kCulledRect) rr = 0u;
       const uint32_t x0 = rr & 0xffu, y0 = (rr >> 8) & 0xffu;
       p_rect = make_uint4(x0, y0, x0 + ((rr >> 16) & 0xffu), y0 + (rr >> 24));
     } else {
@@ -174,11 +188,21 @@ __global__ void __launch_bounds__(kThreads)
       const uint32_t v =
           find_view(n_views, id, [&](uint32_t k) { return __ldg(&views[k].splat_base); });
       s_off[threadIdx.x] = p_off;
+      if (CELLS) {
+        const uint32_t cx0 = x0 / kCellSide, cy0 = y0 / kCellSide;
+        const uint32_t wc = p_rect.z / kCellSide - cx0 + 1u, hc = p_rect.w / kCellSide - cy0 + 1u;
+        const uint32_t cx = __ldg(&views[v].cells_x);
+        s_ra[threadIdx.x] =
+            make_uint4(wc | (hc << 16), __float_as_uint(1.0f / (float)wc), cx - wc, x0 | (y0 << 16));
+        s_rb[threadIdx.x] = make_uint4(__ldg(&views[v].cell_base) + cy0 * cx + cx0, p_key, id,
+                                       p_rect.z | (p_rect.w << 16));
+      } else {
       const uint32_t tx = __ldg(&views[v].f.tile_count[0]);
       // ref k of the splat: row = k / w, tile = first + row * tx + (k - row * w)
       //                                      = first + row * (tx - w) + k
       s_ra[threadIdx.x] = make_uint4(w * h, w, __float_as_uint(1.0f / (float)w), tx - w);
       s_rb[threadIdx.x] = make_uint4(__ldg(&views[v].f.tile_base) + y0 * tx + x0, p_key, id, 0u);
+      }
     }
     const uint32_t last = min(n, first + kThreads);
     if (threadIdx.x == 0) s_off[last - first] = p_end;
@@ -236,7 +260,26 @@ __global__ void __launch_bounds__(kThreads)
         if (live) {
           const uint32_t k = j - s_off[o];
           const uint4 ra = s_ra[o];
-          if (k < ra.x) {
+          if (CELLS) {
+            const uint32_t wc = ra.x & 0xffffu, hc = ra.x >> 16;
+            if (k < wc * hc) {
+              const uint32_t row = (uint32_t)(((float)k + 0.5f) * __uint_as_float(ra.y));
+              const uint32_t col = k - row * wc;
+              const uint4 rb = s_rb[o];
+              // the rectangle inside the cell: its own ends in the first and the
+              // last column and row, the cell's in between
+              const uint32_t lx0 = col == 0 ? ra.w & 7u : 0u;
+              const uint32_t ly0 = row == 0 ? (ra.w >> 16) & 7u : 0u;
+              const uint32_t lx1 = col + 1 == wc ? rb.w & 7u : 7u;
+              const uint32_t ly1 = row + 1 == hc ? (rb.w >> 16) & 7u : 7u;
+              tile = ((rb.x + row * ra.z + k) << kCellShift) | lx0 | (ly0 << 3) | (lx1 << 6) |
+                     (ly1 << 9);
+              keys[j] = make_uint2(tile, rb.y);
+              values[j] = rb.z;
+            } else {
+              live = false;
+            }
+          } else if (k < ra.x) {
             // row = floor(k / w) by a float reciprocal: exact while k + w < 2^22
             // (k < w * h <= tiles of one view)
             const uint32_t row = (uint32_t)(((float)k + 0.5f) * __uint_as_float(ra.z));
@@ -265,12 +308,12 @@ __global__ void __launch_bounds__(kThreads)
 
 // Resident blocks per SM of one emit instance (its registers and shared
 // memory decide), asked once per instance.
-template <int TP, int BINS>
+template <int TP, int BINS, bool CELLS>
 uint32_t emit_blocks_per_sm() {
   static int per_sm = 0;
   if (per_sm == 0) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, emit_sorted_kernel<TP, BINS>, kThreads,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, emit_sorted_kernel<TP, BINS, CELLS>, kThreads,
                                                       0) != cudaSuccess) {
       (void)cudaGetLastError();
       b = 1;
@@ -278,6 +321,57 @@ uint32_t emit_blocks_per_sm() {
     per_sm = b < 1 ? 1 : b;
   }
   return (uint32_t)per_sm;
+}
+
+template <bool CELLS>
+cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
+                         const gs3d_projected_splat* proj, const uint32_t* rect8,
+                         const uint32_t* sorted_keys, const uint32_t* sorted_ids,
+                         const uint32_t* sorted_offsets, const uint32_t* counter, CellArgs cells,
+                         uint32_t capacity, uint2* keys, uint32_t* values, const SortPlan& plan,
+                         uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
+                         cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  const uint32_t chunks = (n + kThreads - 1) / kThreads;
+  const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 1u;
+  int4 sh = make_int4(0, 0, 0, 0);
+  uint4 mk = make_uint4(0, 0, 0, 0);
+  int* shp = &sh.x;
+  uint32_t* mkp = &mk.x;
+  for (int p = 0; p < plan.passes && p < 4; ++p) {
+    shp[p] = plan.shift[p];
+    mkp[p] = digit_mask(plan.nbits[p]);
+  }
+  bool wide = false;  // an 11-bit digit needs 2048-bin histograms
+  for (int p = 0; p < plan.passes; ++p) wide = wide || plan.nbits[p] > 8;
+#define GS3D_EMIT_CASE(TP, BINS)                                                              \
+  case TP:                                                                                    \
+    emit_sorted_kernel<TP, BINS, CELLS>                                                       \
+        <<<std::min(chunks, sms * emit_blocks_per_sm<TP, BINS, CELLS>()), kThreads, 0, s>>>(  \
+            views, n_views, n, proj, rect8, sorted_keys, sorted_ids, sorted_offsets, counter, \
+            cells, capacity, keys, values, sh, mk, g_hist, chunk_ticket, err);                \
+    break;
+  if (wide) {
+    switch (plan.passes) {
+      GS3D_EMIT_CASE(1, 2048)
+      GS3D_EMIT_CASE(2, 2048)
+      GS3D_EMIT_CASE(3, 2048)
+      default:
+        return cudaErrorInvalidValue;
+    }
+  } else {
+    switch (plan.passes) {
+      GS3D_EMIT_CASE(0, kRadixBins)
+      GS3D_EMIT_CASE(1, kRadixBins)
+      GS3D_EMIT_CASE(2, kRadixBins)
+      GS3D_EMIT_CASE(3, kRadixBins)
+      GS3D_EMIT_CASE(4, kRadixBins)
+      default:
+        return cudaErrorInvalidValue;
+    }
+  }
+#undef GS3D_EMIT_CASE
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -291,47 +385,23 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
                                const SortPlan& tile_plan, uint32_t* g_hist,
                                uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                                cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  const uint32_t chunks = (n + kThreads - 1) / kThreads;
-  const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 1u;
-  int4 sh = make_int4(0, 0, 0, 0);
-  uint4 mk = make_uint4(0, 0, 0, 0);
-  int* shp = &sh.x;
-  uint32_t* mkp = &mk.x;
-  for (int p = 0; p < tile_plan.passes && p < 4; ++p) {
-    shp[p] = tile_plan.shift[p];
-    mkp[p] = digit_mask(tile_plan.nbits[p]);
-  }
-  bool wide = false;  // an 11-bit digit needs 2048-bin histograms
-  for (int p = 0; p < tile_plan.passes; ++p) wide = wide || tile_plan.nbits[p] > 8;
-#define GS3D_EMIT_CASE(TP, BINS)                                                              \
-  case TP:                                                                                    \
-    emit_sorted_kernel<TP, BINS><<<std::min(chunks, sms * emit_blocks_per_sm<TP, BINS>()),    \
-                                   kThreads, 0, s>>>(                                         \
-        views, n_views, n, proj, rect8, sorted_keys, sorted_ids, sorted_offsets, ref_counter, \
-        capacity, keys, values, sh, mk, g_hist, chunk_ticket, err);                           \
-    break;
-  if (wide) {
-    switch (tile_plan.passes) {
-      GS3D_EMIT_CASE(1, 2048)
-      GS3D_EMIT_CASE(2, 2048)
-      GS3D_EMIT_CASE(3, 2048)
-      default:
-        return cudaErrorInvalidValue;
-    }
-  } else {
-    switch (tile_plan.passes) {
-      GS3D_EMIT_CASE(0, kRadixBins)
-      GS3D_EMIT_CASE(1, kRadixBins)
-      GS3D_EMIT_CASE(2, kRadixBins)
-      GS3D_EMIT_CASE(3, kRadixBins)
-      GS3D_EMIT_CASE(4, kRadixBins)
-      default:
-        return cudaErrorInvalidValue;
-    }
-  }
-#undef GS3D_EMIT_CASE
-  return cudaGetLastError();
+  return emit_ordered<false>(views, n_views, n, proj, rect8, sorted_keys, sorted_ids,
+                             sorted_offsets, ref_counter, CellArgs{}, capacity, keys, values,
+                             tile_plan, g_hist, chunk_ticket, err, sm_count, s);
+}
+
+cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t n,
+                              const gs3d_projected_splat* proj, const uint32_t* rect8,
+                              const uint32_t* sorted_keys, const uint32_t* sorted_ids,
+                              const uint32_t* sorted_offsets, const uint32_t* entry_total,
+                              const unsigned long long* ref_total, uint32_t* ref_counter,
+                              uint32_t capacity, uint2* keys, uint32_t* values,
+                              const SortPlan& cell_plan, uint32_t* g_hist, uint32_t* chunk_ticket,
+                              uint32_t* err, int sm_count, cudaStream_t s) {
+  return emit_ordered<true>(views, n_views, n, proj, rect8, sorted_keys, sorted_ids,
+                            sorted_offsets, entry_total, CellArgs{ref_total, ref_counter},
+                            capacity, keys, values, cell_plan, g_hist, chunk_ticket, err,
+                            sm_count, s);
 }
 
 cudaError_t launch_emit(const FrameUniforms* d_frame, uint32_t n,

@@ -48,10 +48,24 @@ struct ViewDesc {
   uint64_t pixel_base;  // first pixel of this view's image in the batch target
   uint32_t batch_tiles;   // tiles in the whole batch (same in every view)
   uint32_t group_next;    // next view of the same scene in the batch, or kNoView
-  uint64_t pad2;
+  uint32_t cell_base;     // first cell of this view (binning.cu)
+  uint32_t cells_x;       // cells per row of its tile grid
 };
 constexpr uint32_t kNoView = 0xffffffffu;
 static_assert(sizeof(ViewDesc) % 16 == 0, "ViewDesc is copied as 16-byte words");
+
+// ---- cells: 8x8 blocks of a view's tile grid (binning.cu) ----
+constexpr uint32_t kCellSide = 8, kCellTiles = kCellSide * kCellSide;
+constexpr uint32_t kCellShift = 12;  // entry: cell << 12 | y1, x1, y0, x0 inside the cell (3 bits each)
+constexpr uint32_t kMaxCells = 1u << (32 - kCellShift);
+constexpr uint32_t kChunkEntries = 1024;
+constexpr uint32_t kNoCell = 0xffffffffu;
+constexpr uint32_t kCulledRect = 0xffffffffu;  // one-word rectangle of a culled splat
+// Where the chunks of the cell m whose first entry is a begin.  A cell's
+// ceil(n / kChunkEntries) chunks fit before those of the next one.
+__host__ __device__ inline uint32_t chunk_slot(uint32_t a, uint32_t m) {
+  return a / kChunkEntries + m;
+}
 
 // Largest v with key(v) <= x over a non-decreasing per-view field.
 template <typename F>
@@ -62,6 +76,24 @@ __device__ __forceinline__ uint32_t find_view(uint32_t n_views, uint32_t x, F ke
     if (key(mid) <= x) lo = mid; else hi = mid;
   }
   return lo;
+}
+
+struct CellGeom {
+  uint32_t tile0, tiles_x;  // global tile of the cell's first tile, tiles per row of its view
+  uint32_t w, h;            // tiles of the cell inside the grid
+};
+__device__ __forceinline__ CellGeom cell_geom(const ViewDesc* views, uint32_t n_views,
+                                              uint32_t m) {
+  const uint32_t v = find_view(n_views, m, [&](uint32_t k) { return __ldg(&views[k].cell_base); });
+  const ViewDesc& vd = views[v];
+  const uint32_t lm = m - __ldg(&vd.cell_base), cx = __ldg(&vd.cells_x);
+  const uint32_t x = lm % cx * kCellSide, y = lm / cx * kCellSide;
+  CellGeom g;
+  g.tiles_x = __ldg(&vd.f.tile_count[0]);
+  g.tile0 = __ldg(&vd.f.tile_base) + y * g.tiles_x + x;
+  g.w = min(kCellSide, g.tiles_x - x);
+  g.h = min(kCellSide, __ldg(&vd.f.tile_count[1]) - y);
+  return g;
 }
 
 // Device error latch bits (read and cleared by gs3d_synchronize).
@@ -88,6 +120,11 @@ struct Ctrl {
   unsigned long long raster_queue;  // next raster work item
   uint32_t raster_heavy;  // tiles whose raster work is split (the head of an order by cost)
   uint32_t emit_chunk;    // next 256-splat chunk of the depth-ordered emit
+  uint32_t place_chunk;   // next chunk of cell entries to place
+  unsigned long long ref_total;  // refs of the frame (binned rebin)
+  uint32_t entry_total;          // its (splat, cell) entries
+  uint32_t tile_scan_counter;
+  uint32_t tile_scan_total;
   uint32_t pad;
   uint32_t sort_hist[kMaxSortPasses][kRadixBins];  // global digit histograms
   uint32_t sched_hist[2][kRadixBins];
@@ -268,6 +305,34 @@ cudaError_t launch_scan(const uint32_t* counts, const uint32_t* gather, uint32_t
                         uint32_t n, unsigned long long* status, uint32_t* tile_counter,
                         uint32_t epoch, uint32_t* total_out, uint32_t* err, cudaStream_t s);
 size_t scan_status_words(uint32_t n);
+// Exclusive scan, in the order of `gather`, of the cells that every splat-view
+// covers: its rectangle in rect8 (all ones: culled), or where rect8 is null in
+// the projected records (counts 0: culled).  Adds the refs to *ref_total.
+cudaError_t launch_scan_cells(const uint32_t* counts, const uint32_t* rect8,
+                              const gs3d_projected_splat* proj, const uint32_t* gather,
+                              uint32_t* offsets, uint32_t n, unsigned long long* status,
+                              uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
+                              unsigned long long* ref_total, uint32_t* err, cudaStream_t s);
+// tile_offsets[n + 1] of n tile counts, in identify_tile_ranges.wgsl's
+// convention (tiles after the last populated one keep 0).
+cudaError_t launch_scan_tiles(const uint32_t* tile_counts, uint32_t* tile_offsets, uint32_t n,
+                              const unsigned long long* ref_total, unsigned long long* status,
+                              uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
+                              uint32_t* err, cudaStream_t s);
+// Binned rebin (binning.cu), over the entries sorted by cell: chunk counts and
+// tile totals; then, once the tile offsets are known, the refs.
+size_t chunk_slots_max(uint32_t capacity, uint32_t num_cells);
+cudaError_t launch_bin_count(const ViewDesc* views, uint32_t n_views, uint32_t num_cells,
+                             const uint2* entries, const uint32_t* entry_total,
+                             const unsigned long long* ref_total, uint32_t capacity,
+                             uint32_t* cell_start, uint32_t* chunk_cell, uint32_t* chunk_counts,
+                             uint32_t* tile_counts, int sm_count, cudaStream_t s);
+cudaError_t launch_bin_place(const ViewDesc* views, uint32_t n_views, uint32_t num_cells,
+                             const uint2* entries, const uint32_t* ids, const uint32_t* cell_start,
+                             const uint32_t* chunk_cell, const uint32_t* chunk_counts,
+                             const uint32_t* tile_offsets, const unsigned long long* ref_total,
+                             uint32_t capacity, uint2* keys, uint32_t* values, uint32_t* ticket,
+                             uint32_t* err, int sm_count, cudaStream_t s);
 // Message of the calling thread's last failing context-free call.
 const char* noalloc_last_error();
 // Sets the message gs3d_last_error(NULL) returns on the calling thread.
@@ -373,6 +438,16 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
                                const SortPlan& tile_plan, uint32_t* g_hist,
                                uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                                cudaStream_t s);
+// The same for cell entries: one per (splat-view, cell), keys [cell and
+// rectangle inside it | depth], and *ref_counter = the frame's refs.
+cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t total,
+                              const gs3d_projected_splat* proj, const uint32_t* rect8,
+                              const uint32_t* sorted_keys, const uint32_t* sorted_ids,
+                              const uint32_t* sorted_offsets, const uint32_t* entry_total,
+                              const unsigned long long* ref_total, uint32_t* ref_counter,
+                              uint32_t capacity, uint2* keys, uint32_t* values,
+                              const SortPlan& cell_plan, uint32_t* g_hist, uint32_t* chunk_ticket,
+                              uint32_t* err, int sm_count, cudaStream_t s);
 cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint32_t capacity,
                             uint32_t num_tiles, uint32_t* tile_offsets, uint32_t* err,
                             int sm_count, cudaStream_t s);

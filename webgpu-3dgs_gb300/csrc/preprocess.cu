@@ -278,9 +278,11 @@ __device__ __forceinline__ void preprocess_block(const ViewDesc* __restrict__ vi
         depth_keys[gi] = valid ? __float_as_uint(-r0.z) : 0xffffffffu;
         depth_ids[gi] = gi;
         // tile rectangle in one word [x0, y0, x1 - x0, y1 - y0] (8 bits each;
-        // requested only when every view has at most 256 tiles per axis)
+        // requested only when every view has at most 256 tiles per axis; kCulledRect,
+        // which no rectangle inside such a grid is, for a culled splat)
         if (rect8 != nullptr)
-          rect8[gi] = r3.x | (r3.y << 8) | ((r3.z - r3.x) << 16) | ((r3.w - r3.y) << 24);
+          rect8[gi] = !valid ? kCulledRect
+                             : r3.x | (r3.y << 8) | ((r3.z - r3.x) << 16) | ((r3.w - r3.y) << 24);
       }
     }
   }

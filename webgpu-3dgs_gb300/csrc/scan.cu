@@ -36,13 +36,33 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x, int lane) {
   return x;
 }
 
+// What is scanned: counts (through a permutation where gather is given); the
+// cells covered by splat-views (cells8: from one-word rectangles, cells16: from
+// the projected records); tile counts, written in tile_offsets' convention.
+enum class Scan { counts, cells8, cells16, tiles };
+
+struct ScanExtra {
+  const uint32_t* rect8;
+  const gs3d_projected_splat* proj;
+  unsigned long long* ref_total;  // cells: the refs are added; tiles: read
+};
+
+// Cells and refs of a splat-view's tile rectangle [x0, x1] x [y0, y1].
+__device__ __forceinline__ uint32_t rect_cells(uint32_t x0, uint32_t y0, uint32_t x1, uint32_t y1,
+                                               unsigned long long& refs) {
+  refs += (unsigned long long)(x1 - x0 + 1) * (y1 - y0 + 1);
+  return (x1 / kCellSide - x0 / kCellSide + 1) * (y1 / kCellSide - y0 / kCellSide + 1);
+}
+
+template <Scan KIND>
 __global__ void __launch_bounds__(kThreads)
     scan_kernel(const uint32_t* __restrict__ in, const uint32_t* __restrict__ gather,
-                uint32_t* __restrict__ out, uint32_t n,
+                ScanExtra ex, uint32_t* __restrict__ out, uint32_t n,
                 unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket,
                 uint32_t epoch, uint32_t* __restrict__ total_out, uint32_t* __restrict__ err) {
   __shared__ uint32_t s_tile, s_prefix;
   __shared__ uint32_t s_warp[kThreads / 32];
+  __shared__ unsigned long long s_refs[kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
@@ -56,7 +76,29 @@ __global__ void __launch_bounds__(kThreads)
   const bool vec_in = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
   const bool vec_out = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   uint32_t v[kItems];
-  if (gather != nullptr) {  // counts read through a permutation (fused rebin)
+  if (KIND == Scan::cells8 || KIND == Scan::cells16) {
+    unsigned long long refs = 0;
+    uint32_t id[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) id[k] = (base + k < n) ? __ldg(gather + base + k) : 0u;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      v[k] = 0u;
+      if (base + k >= n) continue;
+      if (KIND == Scan::cells8) {
+        const uint32_t r = __ldg(ex.rect8 + id[k]);
+        const uint32_t x0 = r & 0xffu, y0 = (r >> 8) & 0xffu;
+        if (r != kCulledRect)
+          v[k] = rect_cells(x0, y0, x0 + ((r >> 16) & 0xffu), y0 + (r >> 24), refs);
+      } else if (__ldg(in + id[k]) != 0u) {
+        const uint4 r = __ldg(reinterpret_cast<const uint4*>(ex.proj + id[k]) + 3);
+        v[k] = rect_cells(r.x, r.y, r.z, r.w, refs);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) refs += __shfl_xor_sync(0xffffffffu, refs, o);
+    if (lane == 0) s_refs[warp] = refs;
+  } else if (gather != nullptr) {  // counts read through a permutation (fused rebin)
 #pragma unroll
     for (int k = 0; k < kItems; ++k) v[k] = (base + k < n) ? __ldg(in + __ldg(gather + base + k)) : 0u;
   } else if (vec_in && base + kItems <= n) {
@@ -80,6 +122,12 @@ __global__ void __launch_bounds__(kThreads)
     const uint32_t wi = warp_inclusive(w, lane);
     if (lane < kThreads / 32) s_warp[lane] = wi - w;  // exclusive warp offsets
     const uint32_t tile_total = __shfl_sync(0xffffffffu, wi, kThreads / 32 - 1);
+    if ((KIND == Scan::cells8 || KIND == Scan::cells16) && lane == 0) {
+      unsigned long long refs = 0;
+#pragma unroll
+      for (int w8 = 0; w8 < kThreads / 32; ++w8) refs += s_refs[w8];
+      if (refs) atomicAdd(ex.ref_total, refs);
+    }
 
     // ---- decoupled look-back (warp 0) ----
     unsigned long long excl = 0;
@@ -138,7 +186,7 @@ __global__ void __launch_bounds__(kThreads)
       s_prefix = overflow ? 0xffffffffu : (uint32_t)excl;
       if (tile == num_tiles - 1) {
         *total_out = inc32;
-        out[n] = inc32;
+        if (KIND != Scan::tiles) out[n] = inc32;
       }
     }
   }
@@ -150,6 +198,18 @@ __global__ void __launch_bounds__(kThreads)
   for (int k = 0; k < kItems; ++k) {
     o[k] = run;
     run += v[k];
+  }
+  if (KIND == Scan::tiles) {
+    // a tile after the last populated one keeps 0: its predecessor is empty and
+    // every ref lies before it
+    const unsigned long long all = *ex.ref_total;
+    uint32_t before = base > 0 && base < n ? __ldg(in + base - 1) : 1u;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      if (base + k + 1 == n) out[n] = v[k] ? o[k] + v[k] : 0u;
+      if (o[k] == all && before == 0u) o[k] = 0u;
+      before = v[k];
+    }
   }
   if (vec_out && base + kItems <= n) {
     reinterpret_cast<uint4*>(out + base)[0] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -178,8 +238,39 @@ cudaError_t launch_scan(const uint32_t* counts, const uint32_t* gather, uint32_t
     return cudaGetLastError();
   }
   const uint32_t tiles = (n + kTile - 1) / kTile;
-  scan_kernel<<<tiles, kThreads, 0, s>>>(counts, gather, offsets, n, status, tile_counter, epoch,
-                                         total_out, err);
+  scan_kernel<Scan::counts><<<tiles, kThreads, 0, s>>>(counts, gather, ScanExtra{}, offsets, n,
+                                                       status, tile_counter, epoch, total_out, err);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_scan_cells(const uint32_t* counts, const uint32_t* rect8,
+                              const gs3d_projected_splat* proj, const uint32_t* gather,
+                              uint32_t* offsets, uint32_t n, unsigned long long* status,
+                              uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
+                              unsigned long long* ref_total, uint32_t* err, cudaStream_t s) {
+  if (n == 0) {
+    scan_empty_kernel<<<1, 1, 0, s>>>(offsets, total_out);
+    return cudaGetLastError();
+  }
+  const uint32_t tiles = (n + kTile - 1) / kTile;
+  const ScanExtra ex{rect8, proj, ref_total};
+  if (rect8 != nullptr)
+    scan_kernel<Scan::cells8><<<tiles, kThreads, 0, s>>>(counts, gather, ex, offsets, n, status,
+                                                         tile_counter, epoch, total_out, err);
+  else
+    scan_kernel<Scan::cells16><<<tiles, kThreads, 0, s>>>(counts, gather, ex, offsets, n, status,
+                                                          tile_counter, epoch, total_out, err);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_scan_tiles(const uint32_t* tile_counts, uint32_t* tile_offsets, uint32_t n,
+                              const unsigned long long* ref_total, unsigned long long* status,
+                              uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
+                              uint32_t* err, cudaStream_t s) {
+  const uint32_t tiles = (n + kTile - 1) / kTile;
+  const ScanExtra ex{nullptr, nullptr, const_cast<unsigned long long*>(ref_total)};
+  scan_kernel<Scan::tiles><<<tiles, kThreads, 0, s>>>(tile_counts, nullptr, ex, tile_offsets, n,
+                                                      status, tile_counter, epoch, total_out, err);
   return cudaGetLastError();
 }
 
