@@ -93,6 +93,7 @@ struct gs3d_ctx {
   bool have_model = false;
   DevBuf model_params, model_mean, model_inv_std, tile_feats, tile_preds;
   DevBuf tile_est;    // expected cost per tile of the last ordered raster
+  DevBuf raster_pool; // blocks handed on between raster warps
   DevBuf gate;        // SchedGate: the learned schedule's fallback gate
   float gate_bound = 0.5f;
 
@@ -448,6 +449,10 @@ int set_views(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, bool upload
   TRY(ensure(c, c->tile_feats, std::max<uint64_t>(tiles, 1) * kFeatures * 4, "tile features"));
   TRY(ensure(c, c->tile_preds, std::max<uint64_t>(tiles, 1) * 4, "tile cost predictions"));
   TRY(ensure(c, c->tile_est, std::max<uint64_t>(tiles, 1) * 4, "tile expected costs"));
+  if (!c->raster_pool.p) {
+    TRY(ensure(c, c->raster_pool, raster_pool_bytes(), "raster pool"));
+    CK(cudaMemsetAsync(c->raster_pool.p, 0, raster_pool_bytes(), c->stream), "raster pool");
+  }
   TRY(ensure(c, c->d_views, (size_t)n_views * sizeof(ViewDesc), "view table"));
   if (c->capacity < 1) TRY(ensure_key_capacity(c, 1));
   TRY(ensure(c, c->tile_counts, std::max<uint64_t>(tiles, 1) * 4, "tile counts"));
@@ -545,8 +550,11 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   CK(raster_shape(a, c->sm_count, &strips, &raster_ctas), "raster shape");
   const bool split_all = (c->flags & GS3D_FLAG_SPLIT_ALL_TILES) != 0;
   const bool learned = c->schedule == GS3D_SCHEDULE_LEARNED && c->total_tiles > 1;
-  static_assert(offsetof(Ctrl, raster_heavy) == offsetof(Ctrl, raster_queue) + 8, "cleared together");
-  CK(cudaMemsetAsync(&ctrl_of(c)->raster_queue, 0, 12, c->stream), "reset raster queue");
+  CK(cudaMemsetAsync(&ctrl_of(c)->raster_queue, 0,
+                     offsetof(Ctrl, raster_pool) + sizeof(Ctrl::raster_pool) -
+                         offsetof(Ctrl, raster_queue),
+                     c->stream),
+     "reset raster queue");
   const uint32_t* order = nullptr;
   const uint32_t* heavy = nullptr;
   if (c->schedule != GS3D_SCHEDULE_ROW_MAJOR && c->total_tiles > 1) {
@@ -591,7 +599,8 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   a.tile_costs = u32(c->tile_costs);
   a.order = order;
   a.queue_counter = &ctrl_of(c)->raster_queue;
-  a.ref_counter = u32(c->ref_counter);
+  a.pool = c->raster_pool.p;
+  a.pool_ctrl = &ctrl_of(c)->raster_pool;
   a.err = &ctrl_of(c)->error;
   // the previous frame's splat target may still be copying out (captured as
   // an external event wait in graph mode; a never-recorded event is no wait)
@@ -600,9 +609,7 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   CK(cudaStreamWaitEvent(c->stream, c->copy_done,
                          cap == cudaStreamCaptureStatusActive ? cudaEventWaitExternal : 0),
      "wait for the previous copy-out");
-  // the row-major order's heavy tiles go where the other orders keep theirs
-  CK(launch_raster(a, u32(c->sched_order_b), &ctrl_of(c)->raster_heavy, c->sm_count, c->stream),
-     "rasterize_tiles");
+  CK(launch_raster(a, c->sm_count, c->stream), "rasterize_tiles");
   if (learned)  // the gate measures this frame's prediction error
     CK(launch_gate_update(static_cast<float*>(c->tile_preds.p), u32(c->tile_costs),
                           c->total_tiles, static_cast<SchedGate*>(c->gate.p), c->stream),
@@ -952,7 +959,7 @@ int gs3d_destroy(gs3d_ctx* c) {
                     &c->sched_keys_b,  &c->sched_order_a, &c->sched_order_b, &c->sched_status,
                     &c->d_views,       &c->ctrl,          &c->model_params,  &c->model_mean,
                     &c->model_inv_std, &c->tile_feats,    &c->tile_preds,    &c->composite_out,
-                    &c->tile_est,      &c->gate};
+                    &c->tile_est,      &c->gate,          &c->raster_pool};
   for (DevBuf* b : bufs) release(*b);
   for (int i = 0; i < kUploadSlots; ++i)
     if (c->upload_ev[i]) cudaEventDestroy(c->upload_ev[i]);

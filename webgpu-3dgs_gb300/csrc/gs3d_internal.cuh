@@ -117,8 +117,6 @@ struct Ctrl {
   uint32_t scan_tile_counter;
   uint32_t sort_part_counter[kMaxSortPasses];
   uint32_t sched_counter[2];
-  unsigned long long raster_queue;  // next raster work item
-  uint32_t raster_heavy;  // tiles whose raster work is split (the head of an order by cost)
   uint32_t emit_chunk;    // next 256-splat chunk of the depth-ordered emit
   uint32_t place_chunk;   // next chunk of cell entries to place
   unsigned long long ref_total;  // refs of the frame (binned rebin)
@@ -129,6 +127,11 @@ struct Ctrl {
   uint32_t sort_hist[kMaxSortPasses][kRadixBins];  // global digit histograms
   uint32_t sched_hist[2][kRadixBins];
   uint32_t tile_hist[kMaxTilePasses][kTileHistStride];  // fused rebin's tile passes
+  // raster: the work queue and the line of waiting warps, on cache lines of
+  // their own (both are polled), cleared together
+  alignas(128) unsigned long long raster_queue;  // next work item
+  uint32_t raster_heavy;  // tiles whose work is split (the head of an order by cost)
+  alignas(128) uint32_t raster_pool[4];          // blocks handed on between warps
 };
 
 // Fallback gate of the learned raster schedule, kept on the device across
@@ -454,8 +457,7 @@ cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint
 // Rasterizes every tile of the batch.  Persistent CTAs pull tile indices
 // from a device work queue (order[k] = k-th tile to render, identity when
 // order is null) through *queue_counter, which must be zero at launch, as must
-// *heavy_count where args.heavy and args.order are null (the row-major order
-// then lists the tiles it splits in heavy_list[num_tiles]).
+// the four words of pool_ctrl.
 struct RasterArgs {
   const ViewDesc* views;
   uint32_t n_views;
@@ -468,20 +470,18 @@ struct RasterArgs {
   uint32_t* tile_costs;   // may be null
   const uint32_t* order;  // may be null
   unsigned long long* queue_counter;
-  const uint32_t* ref_counter;
+  void* pool;             // raster_pool_bytes(), zeroed once: blocks handed on between warps
+  void* pool_ctrl;
   uint32_t* err;
   uint32_t batch;         // splats staged per batch (0 = tile_w * tile_h)
   bool culled;
   // tiles at the head of the order whose blocks are shaded as two half-block
   // items (device count, warp variant only; may be null: none)
   const uint32_t* heavy;
-  // set by launch_raster:
-  const uint32_t* heavy_list;  // row-major order: the *heavy tiles it splits
-  float heavy_share;           // ... and the share of the refs above which it does
-  uint32_t coarse;             // tiles of the order shaded by regions; the rest by blocks
+  bool fine;              // single blocks instead of regions, set by launch_raster
 };
-cudaError_t launch_raster(const RasterArgs& a, uint32_t* heavy_list, uint32_t* heavy_count,
-                          int sm_count, cudaStream_t s);
+size_t raster_pool_bytes();
+cudaError_t launch_raster(const RasterArgs& a, int sm_count, cudaStream_t s);
 // Work items per tile and resident workers (warps; CTAs where a CTA shades a
 // tile) of the raster launch for these args.
 cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* items_per_tile,

@@ -595,14 +595,6 @@ __device__ __forceinline__ TileGeom tile_geom(const RasterArgs& a, uint32_t t) {
   return g;
 }
 
-// Row-major order: does the tile's key count exceed half of a resident warp's
-// fair share of the launch (refs x regions / warps)?  Read on the device, where
-// the live count is.
-__device__ __forceinline__ bool tile_is_heavy(const RasterArgs& a, uint32_t t) {
-  const uint32_t lo = __ldg(a.tile_offsets + t), hi = __ldg(a.tile_offsets + t + 1);
-  return hi > lo + kHeavyKeys && (float)(hi - lo) > a.heavy_share * (float)__ldg(a.ref_counter);
-}
-
 // One thread per pixel, linear pixel order (the reference's layout).
 __device__ void raster_tile_plain(const RasterArgs& a, const TileGeom& g, SplatStage* buf0,
                                   SplatStage* buf1, uint32_t* s_cost) {
@@ -753,7 +745,6 @@ __device__ __forceinline__ void load_record(const gs3d_projected_splat* p, Splat
 // Items of one block instead of a region (and of half a block, one pixel a
 // lane) trade those gains for a shorter chain: they serve launches with fewer
 // regions than resident warps, and the heaviest tiles.
-constexpr uint32_t kRegionRows = 2;  // blocks
 constexpr uint32_t kRegionBlocks = 4;
 constexpr uint32_t kItemWarps = 4;  // warps of a CTA (independent of one another)
 constexpr uint32_t kKept = 104;     // splats kept before they are blended (a multiple of 8)
@@ -788,36 +779,122 @@ __device__ __forceinline__ void store_px(float4 (&st)[2][32], uint32_t lane, con
   st[0][lane] = make_float4(p.cr, p.cg, p.cb, p.T > 0.0f ? p.T : -p.fin);
 }
 
+// ---- blocks handed on ------------------------------------------------------------
+// How far a region's warp has to walk its list is known only once its pixels
+// have terminated, and the queue may run empty while a few warps still have
+// thousands of splats before them.  A warp that finds no more items takes a
+// place in a line and waits; a warp that sees some waiting hands blocks of its
+// region on to them, with their pixels' state and the list position (the
+// pixels' arithmetic does not change, so neither do the image and the costs).
+// The n-th block handed on goes to the n-th place, so every waiting warp polls a
+// word of its own.
+constexpr uint32_t kPoolSlots = 4096;    // blocks handed on in a launch
+constexpr uint32_t kMaxWaiting = 1024;   // others leave
+constexpr uint32_t kHandOnLeft = 512;    // list entries left below which nothing is handed on
+struct PoolSlot {
+  float4 state[2][32];
+  uint32_t tile, view_x, view_y, k;
+  uint32_t ready;  // 1 from when it is written until it is read (0 between launches)
+  uint32_t pad[3];
+};
+// The counters of RasterArgs::pool_ctrl, all zero at launch: blocks handed on,
+// places taken, warps waiting, warps started and not yet gone.
+struct PoolCtrl {
+  uint32_t handed, places, waiting, present;
+};
+__device__ __forceinline__ uint4 pool_look(const RasterArgs& a) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(a.pool_ctrl)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void hand_on(const RasterArgs& a, const float4 (&st)[2][32],
+                                        uint32_t slot, uint32_t tile, uint32_t x, uint32_t y,
+                                        uint32_t k) {
+  const uint32_t lane = threadIdx.x & 31;
+  PoolSlot& s = static_cast<PoolSlot*>(a.pool)[slot];
+  __stcg(&s.state[0][lane], st[0][lane]);
+  __stcg(&s.state[1][lane], st[1][lane]);
+  if (lane == 0) __stcg(reinterpret_cast<uint4*>(&s.tile), make_uint4(tile, x, y, k));
+  __threadfence();
+  __syncwarp();
+  if (lane == 0) st_relaxed_u32(&s.ready, 1u);
+}
+// Lane 0 of a warp without work: waits for a block and returns its slot, or ~0u
+// once nobody is left who could hand one on (or enough warps wait already).
+// Blocks go to places in order and a warp that got one comes back for the next
+// place, so a block without a waiting warp is found by the next that comes, its
+// giver at the latest.
+__device__ __forceinline__ uint32_t wait_for_block(const RasterArgs& a) {
+  PoolCtrl* c = static_cast<PoolCtrl*>(a.pool_ctrl);
+  const uint32_t before = atomicAdd(&c->waiting, 1u);
+  const bool crowd = before >= kMaxWaiting &&
+                     ld_relaxed_u32(&c->places) >= ld_relaxed_u32(&c->handed) + kMaxWaiting / 2;
+  const uint32_t place = crowd ? kPoolSlots : atomicAdd(&c->places, 1u);
+  if (place < kPoolSlots) {
+    uint32_t* ready = &static_cast<PoolSlot*>(a.pool)[place].ready;
+    for (uint32_t polls = 0; polls < (1u << 22); ++polls) {  // a second and more
+      if (ld_relaxed_u32(ready) != 0u) {
+        atomicSub(&c->waiting, 1u);
+        __threadfence();
+        st_relaxed_u32(ready, 0u);
+        return place;
+      }
+      if ((polls & 3u) == 3u) {
+        const uint4 v = pool_look(a);
+        // everyone waits: nobody hands on any more
+        if (v.z >= v.w && place >= ld_relaxed_u32(&c->handed)) break;
+      }
+      __nanosleep(300);
+    }
+  }
+  atomicSub(&c->waiting, 1u);
+  atomicSub(&c->present, 1u);
+  return ~0u;
+}
+
 // Shades the nbx x nby blocks at pixel (x0, y0) of the view; returns the
 // region's share of the tile's cost.  FINE: one block, whose chain through the
 // list is what counts: records are fetched two steps ahead (into the states of
 // the blocks that it does not have), a splat that may hit the region is queued
 // at once, and few are kept before they are blended.
-template <typename PX, bool FINE>
+template <typename PX, bool FINE, bool HAND_ON>
 __device__ uint32_t shade_region(const RasterArgs& a, const TileGeom& g, uint32_t x0, uint32_t y0,
-                                 uint32_t nbx, uint32_t nby, WarpSmem& w) {
+                                 uint32_t nbx, uint32_t nby, WarpSmem& w,
+                                 uint32_t slot_in = ~0u) {
   constexpr uint32_t kRows = PX::kN == 2 ? 8 : 4;  // of a block
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t nb = FINE ? 1u : nbx * nby;
   const float bx0 = (float)x0 + 0.5f, by0 = (float)y0 + 0.5f;
-  const float2 xr = make_float2(bx0, bx0 + (float)(8 * nbx - 1));
-  const float2 yr = make_float2(by0, by0 + (float)(kRows * nby - 1));
+  float2 xr = make_float2(bx0, bx0 + (float)(8 * nbx - 1));
+  float2 yr = make_float2(by0, by0 + (float)(kRows * nby - 1));
   auto px_of = [&](uint32_t b) { return x0 + (b % nbx) * 8 + (lane & 7); };
   auto py_of = [&](uint32_t b) { return y0 + (b / nbx) * kRows + (lane >> 3); };
 
   uint32_t alive = 0;  // blocks with a pixel that has not terminated
-  for (uint32_t b = 0; b < nb; ++b) {
-    PX p;
-#pragma unroll
-    for (int i = 0; i < PX::kN; ++i)
-      if (!(px_of(b) < g.W && py_of(b) + 4 * i < g.H)) PX::at(p.T, i) = 0.0f;
-    store_px(w.state[b], lane, p);
-    if (__any_sync(0xffffffffu, px_live(p))) alive |= 1u << b;
-  }
-
+  uint32_t owned = (1u << nb) - 1u;
   const uint32_t start = __ldg(a.tile_offsets + g.tile);
   const uint32_t last = __ldg(a.tile_offsets + g.tile + 1);
   const uint32_t end = last > start ? last : start;
+  uint32_t begin = start;
+  if (HAND_ON && FINE && PX::kN == 2 && slot_in != ~0u) {  // a block handed on
+    const PoolSlot& ps = static_cast<PoolSlot*>(a.pool)[slot_in];
+    w.state[0][0][lane] = __ldcg(&ps.state[0][lane]);
+    w.state[0][1][lane] = __ldcg(&ps.state[1][lane]);
+    begin = __ldcg(&ps.k);
+    alive = 1u;
+  } else {
+    for (uint32_t b = 0; b < nb; ++b) {
+      PX p;
+#pragma unroll
+      for (int i = 0; i < PX::kN; ++i)
+        if (!(px_of(b) < g.W && py_of(b) + 4 * i < g.H)) PX::at(p.T, i) = 0.0f;
+      store_px(w.state[b], lane, p);
+      if (__any_sync(0xffffffffu, px_live(p))) alive |= 1u << b;
+    }
+  }
   uint32_t used = 0, n = 0;
 
   // blends the n kept splats into every block
@@ -874,19 +951,23 @@ __device__ uint32_t shade_region(const RasterArgs& a, const TileGeom& g, uint32_
       }
       cp_async_commit();
     };
-    fetch_id(start);
-    fetch(start, 0);
-    fetch_id(start + 32);
-    fetch(start + 32, 1);
-    fetch_id(start + 64);
+    fetch_id(begin);
+    fetch(begin, 0);
+    fetch_id(begin + 32);
+    fetch(begin + 32, 1);
+    fetch_id(begin + 64);
     uint32_t slot = 0;
-    for (uint32_t k = start; k < end && alive; k += 32, slot ^= 1u) {
-      cp_async_wait<1>();
-      SplatStage s = ring[slot * 32 + lane];
-      keep(s, k);
-      fetch(k + 64, slot);
-      fetch_id(k + 96);
-      if (n > kKept - 48) flush();
+    for (uint32_t k = begin; alive; k += 32, slot ^= 1u) {
+      const bool more = k < end;
+      if (more) {
+        cp_async_wait<1>();
+        SplatStage s = ring[slot * 32 + lane];
+        keep(s, k);
+        fetch(k + 64, slot);
+        fetch_id(k + 96);
+      }
+      if (more ? n > kKept - 48 : n > 0) flush();
+      if (!more) break;
     }
     cp_async_wait<0>();
   } else {
@@ -894,17 +975,46 @@ __device__ uint32_t shade_region(const RasterArgs& a, const TileGeom& g, uint32_
     fetch_id(start);
     if (start + lane < end) load_record(a.proj + id, next);
     fetch_id(start + 32);
-    for (uint32_t k = start; k < end && alive; k += 32) {
-      SplatStage s = next;
-      if (k + 32 + lane < end) load_record(a.proj + id, next);
-      fetch_id(k + 64);
-      keep(s, k);
-      if (n > kKept - 32) flush();
+    for (uint32_t k = start; alive; k += 32) {
+      const bool more = k < end;
+      if (more) {
+        SplatStage s = next;
+        if (k + 32 + lane < end) load_record(a.proj + id, next);
+        fetch_id(k + 64);
+        keep(s, k);
+      }
+      if (more ? n > kKept - 32 : n > 0) {
+        uint4 pool = make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t at = k + 32;
+        const bool look = HAND_ON && end > at + kHandOnLeft && (alive & (alive - 1u)) != 0u;
+        if (look && lane == 0) pool = pool_look(a);
+        flush();
+        if (look && (alive & (alive - 1u)) != 0u) {
+          const int places = __shfl_sync(0xffffffffu, (int)min(pool.y, kPoolSlots) - (int)pool.x, 0);
+          for (int i = 0; i < places && (alive & (alive - 1u)) != 0u; ++i) {
+            uint32_t slot = 0;
+            if (lane == 0) slot = atomicAdd(&static_cast<PoolCtrl*>(a.pool_ctrl)->handed, 1u);
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+            if (slot >= kPoolSlots) break;
+            const uint32_t b = 31 - __clz(alive);
+            hand_on(a, w.state[b], slot, g.tile, x0 + (b % nbx) * 8, y0 + (b / nbx) * kRows, at);
+            alive &= ~(1u << b);
+            owned &= ~(1u << b);
+          }
+          if ((alive & (alive - 1u)) == 0u) {  // one block left: test against it alone
+            const uint32_t b = 31 - __clz(alive);
+            const float fx = bx0 + (float)((b % nbx) * 8), fy = by0 + (float)((b / nbx) * kRows);
+            xr = make_float2(fx, fx + 7.0f);
+            yr = make_float2(fy, fy + (float)(kRows - 1));
+          }
+        }
+      }
+      if (!more) break;
     }
   }
-  if (n && alive) flush();
 
   for (uint32_t b = 0; b < nb; ++b) {
+    if (HAND_ON && !((owned >> b) & 1u)) continue;
     PX p;
     load_px(w.state[b], lane, p);
 #pragma unroll
@@ -919,10 +1029,11 @@ __device__ uint32_t shade_region(const RasterArgs& a, const TileGeom& g, uint32_
   return alive ? end - start : __reduce_max_sync(0xffffffffu, used);
 }
 
-// Persistent warps.  Work items: first those of the heavy tiles, each a block
-// (row-major order, tiles from heavy_list) or half a block (the head of the
-// order by decreasing expected cost); then the regions of the next a.coarse
-// tiles in order and the blocks of the remaining ones.
+// Persistent warps.  Work items: first those of the heavy tiles at the head of
+// an order by decreasing expected cost, each half a block; then the regions of
+// the other tiles in order, or their blocks where a launch has too few regions
+// (a.fine); then blocks handed on.
+template <bool HAND_ON>
 __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(RasterArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   WarpSmem& w = reinterpret_cast<WarpSmem*>(smem)[threadIdx.x >> 5];
@@ -931,65 +1042,78 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
     w.kept[kKept].a = make_float4(0.f, 0.f, -1.f, 0.f);
     w.kept[kKept].b = make_float4(0.f, 0.f, 0.f, -1.f);
     w.kept[kKept].c = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (HAND_ON) atomicAdd(&static_cast<PoolCtrl*>(a.pool_ctrl)->present, 1u);
   }
   __syncwarp();
   const uint32_t bw = a.tile_w / 8, blocks = bw * (a.tile_h / 8);
-  const uint32_t rw = (bw + 1) / 2, regions = rw * ((a.tile_h / 8 + kRegionRows - 1) / kRegionRows);
+  const uint32_t rw = (bw + 1) / 2, regions = rw * ((a.tile_h / 8 + 1) / 2);
   const uint32_t heavy = a.heavy != nullptr ? min(__ldg(a.heavy), a.num_tiles) : 0u;
-  const uint32_t per_heavy = a.heavy_list != nullptr ? blocks : 2 * blocks;
-  // heavy tiles of the row-major order come up again among the others
-  const uint32_t first = a.heavy_list != nullptr ? 0u : heavy;
-  const uint32_t fine = max(first, a.coarse);  // tiles [first, fine) by regions
-  const uint64_t heavy_items = (uint64_t)heavy * per_heavy;
-  const uint64_t fine_items = heavy_items + (uint64_t)(fine - first) * regions;
-  const uint64_t items = fine_items + (uint64_t)(a.num_tiles - fine) * blocks;
+  const uint32_t per_tile = a.fine ? blocks : regions;
+  const uint64_t heavy_items = (uint64_t)heavy * 2 * blocks;
+  const uint64_t items = heavy_items + (uint64_t)(a.num_tiles - heavy) * per_tile;
+  bool queued = true;  // the queue may still hold items
   for (;;) {
-    unsigned long long item = 0;
-    if (lane == 0) item = atomicAdd(a.queue_counter, 1ull);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= items) break;
-    uint32_t t, sub;
-    const bool in_heavy = item < heavy_items;
-    if (in_heavy) {
-      const uint32_t i = (uint32_t)(item / per_heavy);
-      sub = (uint32_t)(item - (uint64_t)i * per_heavy);
-      t = a.heavy_list != nullptr ? __ldg(a.heavy_list + i)
-          : a.order != nullptr    ? __ldg(a.order + i)
-                                  : i;
-    } else {
-      const bool coarse = item < fine_items;
-      const uint64_t j = item - (coarse ? heavy_items : fine_items);
-      const uint32_t per_tile = coarse ? regions : blocks;
-      uint32_t i = (uint32_t)(j / per_tile);
-      sub = (uint32_t)(j - (uint64_t)i * per_tile);
-      i += coarse ? first : fine;
-      t = a.order != nullptr ? __ldg(a.order + i) : i;
-      if (a.heavy_list != nullptr && heavy > 0 && tile_is_heavy(a, t)) continue;
+    unsigned long long item = items;
+    if (queued) {
+      if (lane == 0) item = atomicAdd(a.queue_counter, 1ull);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      queued = item < items;
     }
-    const TileGeom g = tile_geom(a, t);
-    uint32_t cost;
-    if (in_heavy && a.heavy_list == nullptr) {
-      const uint32_t b = sub >> 1;
-      cost = shade_region<Px1, true>(a, g, g.ox + (b % bw) * 8, g.oy + (b / bw) * 8 + (sub & 1) * 4, 1,
-                               1, w);
-    } else if (in_heavy || item >= fine_items) {
-      cost = shade_region<Px2, true>(a, g, g.ox + (sub % bw) * 8, g.oy + (sub / bw) * 8, 1, 1, w);
+    uint32_t t, x, y, nbx = 1, nby = 1, slot = ~0u;
+    const bool in_heavy = item < heavy_items;
+    bool fine = a.fine;
+    TileGeom g;
+    if (queued) {
+      uint32_t sub;
+      if (in_heavy) {
+        t = (uint32_t)(item / (2 * blocks));
+        sub = (uint32_t)(item - (uint64_t)t * (2 * blocks));
+      } else {
+        const uint64_t j = item - heavy_items;
+        t = (uint32_t)(j / per_tile);
+        sub = (uint32_t)(j - (uint64_t)t * per_tile);
+        t += heavy;
+      }
+      if (a.order != nullptr) t = __ldg(a.order + t);
+      g = tile_geom(a, t);
+      if (in_heavy) {
+        const uint32_t b = sub >> 1;
+        x = g.ox + (b % bw) * 8;
+        y = g.oy + (b / bw) * 8 + (sub & 1) * 4;
+      } else if (fine) {
+        x = g.ox + (sub % bw) * 8;
+        y = g.oy + (sub / bw) * 8;
+      } else {
+        const uint32_t rx = 2 * (sub % rw), ry = 2 * (sub / rw);
+        x = g.ox + rx * 8;
+        y = g.oy + ry * 8;
+        nbx = min(2u, bw - rx);
+        nby = min(2u, a.tile_h / 8 - ry);
+      }
     } else {
-      const uint32_t rx = 2 * (sub % rw), ry = kRegionRows * (sub / rw);
-      cost = shade_region<Px2, false>(a, g, g.ox + rx * 8, g.oy + ry * 8, min(2u, bw - rx),
-                               min(kRegionRows, a.tile_h / 8 - ry), w);
+      if (!HAND_ON) break;
+      if (lane == 0) slot = wait_for_block(a);
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      if (slot == ~0u) break;
+      const uint4 info =
+          __ldcg(reinterpret_cast<const uint4*>(&static_cast<PoolSlot*>(a.pool)[slot].tile));
+      t = info.x;
+      x = info.y;
+      y = info.z;
+      g = tile_geom(a, t);
+      fine = true;
+    }
+    uint32_t cost;
+    if (in_heavy) {
+      cost = shade_region<Px1, true, HAND_ON>(a, g, x, y, 1, 1, w);
+    } else if (fine) {
+      cost = shade_region<Px2, true, HAND_ON>(a, g, x, y, 1, 1, w, slot);
+    } else {
+      cost = shade_region<Px2, false, HAND_ON>(a, g, x, y, nbx, nby, w);
     }
     if (lane == 0 && a.tile_costs != nullptr && cost)
       atomicMax(a.tile_costs + t, cost);  // zeroed before the launch; max over a tile's items
   }
-}
-
-// Lists the tiles that the row-major order splits: those whose key count
-// exceeds half of a resident warp's fair share of the launch.
-__global__ void __launch_bounds__(256) heavy_list_kernel(RasterArgs a, uint32_t* list,
-                                                         uint32_t* count) {
-  const uint32_t t = blockIdx.x * 256 + threadIdx.x;
-  if (t < a.num_tiles && tile_is_heavy(a, t)) list[atomicAdd(count, 1u)] = t;
 }
 
 // Persistent CTAs over the queue of tiles; MODE 0: one thread per pixel,
@@ -1059,7 +1183,7 @@ cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
   const uint32_t D = mode == 2 ? 0u : a.batch ? a.batch : nt;
   const uint32_t threads = mode == 2 ? kItemWarps * 32 : nt;
   const size_t smem = raster_smem(mode, D, threads);
-  auto kern = mode == 2 ? raster_kernel_warps : mode == 1 ? raster_kernel_culled
+  auto kern = mode == 2 ? raster_kernel_warps<false> : mode == 1 ? raster_kernel_culled
                                                            : raster_kernel_plain;
   // launch configuration per (device, variant, tile area, batch), computed
   // once per process (the shared-memory attribute is a per-device setting)
@@ -1083,6 +1207,9 @@ cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
     // configurations cached earlier keep fitting
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)raster_smem(mode, 1024, 1024));
+    if (e == cudaSuccess && mode == 2)
+      e = cudaFuncSetAttribute(raster_kernel_warps<true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int n = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)threads, smem);
@@ -1092,15 +1219,18 @@ cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
     cache[key] = per_sm;
   }
   const uint32_t bw = a.tile_w / 8, bh = a.tile_h / 8;
-  *cfg = RasterConfig{mode,   threads, D,   smem, per_sm, mode == 2 ? ((bw + 1) / 2) * ((bh + kRegionRows - 1) / kRegionRows) : 1u,
+  *cfg = RasterConfig{mode,   threads, D,   smem, per_sm, mode == 2 ? ((bw + 1) / 2) * ((bh + 1) / 2) : 1u,
                       mode == 2 ? bw * bh : 1u, kern};
   return cudaSuccess;
 }
 
-// The last regions of a launch, this many for each resident warp, are shaded
-// by blocks: a launch of few regions is bound by its longest item's chain, and
-// a larger one by the items under way when the queue runs empty.
+// Launches with fewer regions than this many times the resident warps are
+// shaded by blocks: they are bound by the longest item's chain (raster of a
+// 400k-splat frame with 0.75 regions a warp: 302 -> 143 us, of a 100k-splat one
+// with 1.2: 124 -> 64 us; a 3M-splat frame with 2.7: 342 us by regions, 473 by
+// blocks).
 constexpr float kFineWaves = 1.75f;
+constexpr float kHandOnWaves = 8.0f;
 
 }  // namespace
 
@@ -1114,8 +1244,9 @@ cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* items_per_
   return cudaSuccess;
 }
 
-cudaError_t launch_raster(const RasterArgs& args, uint32_t* heavy_list, uint32_t* heavy_count,
-                          int sm_count, cudaStream_t s) {
+size_t raster_pool_bytes() { return kPoolSlots * sizeof(PoolSlot); }
+
+cudaError_t launch_raster(const RasterArgs& args, int sm_count, cudaStream_t s) {
   if (args.num_tiles == 0) return cudaSuccess;
   RasterArgs a = args;
   RasterConfig cfg;
@@ -1129,16 +1260,9 @@ cudaError_t launch_raster(const RasterArgs& args, uint32_t* heavy_list, uint32_t
   const uint32_t ctas = (uint32_t)sm_count * (uint32_t)cfg.per_sm;
   uint64_t max_ctas = a.num_tiles;
   if (cfg.mode == 2) {
-    const uint64_t warps = (uint64_t)ctas * kItemWarps;
-    a.coarse = (float)a.num_tiles * (float)cfg.regions > kFineWaves * (float)warps ? a.num_tiles : 0u;
-    if (a.order == nullptr && a.heavy == nullptr && a.coarse > 0 && cfg.blocks > 1) {
-      a.heavy_share = 0.5f * (float)cfg.regions / (float)warps;
-      heavy_list_kernel<<<(a.num_tiles + 255) / 256, 256, 0, s>>>(a, heavy_list, heavy_count);
-      e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
-      a.heavy_list = heavy_list;
-      a.heavy = heavy_count;
-    }
+    const float waves = (float)a.num_tiles * (float)cfg.regions / (float)(ctas * kItemWarps);
+    a.fine = waves <= kFineWaves;
+    if (!a.fine && (a.order == nullptr || waves < kHandOnWaves)) cfg.kern = raster_kernel_warps<true>;
     max_ctas = ((uint64_t)a.num_tiles * cfg.blocks * 2 + kItemWarps - 1) / kItemWarps;
   } else {
     a.heavy = nullptr;  // split items exist in the warp variant only
