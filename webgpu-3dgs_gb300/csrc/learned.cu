@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "gs3d_internal.cuh"
 
@@ -242,58 +243,155 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- training (f32): forward keeps activations, backward accumulates ----
+//
+// A block works on tiles of 64 samples with the weights in shared memory; the
+// layers are small matrix products of 64 x 64 outputs, 4 x 4 a thread, so an
+// operand word in shared memory serves four multiply-adds.  (One sample a step,
+// a unit a thread, read one word per multiply-add and met four block barriers a
+// sample: a step of 65,536 samples, forward and backward, took 1168 us.)  Plain
+// f32 multiply-adds: the tensor formats round the operands.  The units' sums run
+// over k in order, so h1 and h2 are those of that kernel bit for bit.
+constexpr int kTrainThreads = 256;
+constexpr int kTile = 64;            // samples
+constexpr int kPitch = kHidden + 4;  // 16-byte rows, neighbouring row groups on other banks
+constexpr int kPitchX = kFeatures + 4;
 
-// One block of kHidden threads per chunk of samples; thread j owns hidden
-// unit j of both layers.  acts[i] = h1 (64) | h2 (64) | y.
-__global__ void __launch_bounds__(kHidden)
+// acc[s][u] += sum over k in [0, K) of a[s0 + s][k] * b[k][u0 + u], k in order.
+template <int K, int PA, int PB>
+__device__ __forceinline__ void tile_product(const float* a, const float* b, int s0, int u0,
+                                             float (&acc)[4][4]) {
+#pragma unroll 4
+  for (int k = 0; k < K; k += 4) {
+    float4 av[4], bv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      av[i] = *reinterpret_cast<const float4*>(a + (s0 + i) * PA + k);
+      bv[i] = *reinterpret_cast<const float4*>(b + (k + i) * PB + u0);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        const float x = kk == 0 ? av[i].x : kk == 1 ? av[i].y : kk == 2 ? av[i].z : av[i].w;
+        acc[i][0] = fmaf(x, bv[kk].x, acc[i][0]);
+        acc[i][1] = fmaf(x, bv[kk].y, acc[i][1]);
+        acc[i][2] = fmaf(x, bv[kk].z, acc[i][2]);
+        acc[i][3] = fmaf(x, bv[kk].w, acc[i][3]);
+      }
+  }
+}
+
+// The tile's features, zero past n.
+__device__ __forceinline__ void load_x(const float* __restrict__ x, uint32_t i0, uint32_t n,
+                                       float* sx) {
+  for (int k = threadIdx.x; k < kTile * kFeatures; k += kTrainThreads) {
+    const int s = k / kFeatures, c = k % kFeatures;
+    sx[s * kPitchX + c] = i0 + s < n ? __ldg(x + (size_t)i0 * kFeatures + k) : 0.f;
+  }
+}
+
+struct ForwardSmem {
+  float w1[kFeatures][kHidden];  // [k][unit]
+  float w2[kHidden][kPitch];     // [k][unit]
+  float x[kTile * kPitchX];
+  float h[2][kTile * kPitch];    // h1, h2
+};
+__global__ void __launch_bounds__(kTrainThreads, 2)
     mlp_forward_kernel(const float* __restrict__ params, const float* __restrict__ x, uint32_t n,
                        float* __restrict__ acts, float* __restrict__ y) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  ForwardSmem& sm = *reinterpret_cast<ForwardSmem*>(smem);
   const float* W1 = params;
   const float* B1 = W1 + kHidden * kFeatures;
   const float* W2 = B1 + kHidden;
   const float* B2 = W2 + kHidden * kHidden;
   const float* W3 = B2 + kHidden;
-  const float* B3 = W3 + kHidden;
-  __shared__ float s_x[kFeatures], s_h1[kHidden], s_part[kHidden / 32];
-  const int j = threadIdx.x;
-  float w1[kFeatures];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int k = tid; k < kHidden * kFeatures; k += kTrainThreads)
+    sm.w1[k % kFeatures][k / kFeatures] = __ldg(W1 + k);
+  for (int k = tid; k < kHidden * kHidden; k += kTrainThreads)
+    sm.w2[k % kHidden][k / kHidden] = __ldg(W2 + k);
+  const int s0 = tid / 16 * 4, u0 = tid % 16 * 4;  // this thread's samples and units
+  float b1[4], b2[4], w3[4];
 #pragma unroll
-  for (int k = 0; k < kFeatures; ++k) w1[k] = __ldg(W1 + j * kFeatures + k);
-  const float b1 = __ldg(B1 + j), b2 = __ldg(B2 + j), w3 = __ldg(W3 + j), b3 = __ldg(B3);
-  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    if (j < kFeatures) s_x[j] = __ldg(x + (size_t)i * kFeatures + j);
+  for (int u = 0; u < 4; ++u) {
+    b1[u] = __ldg(B1 + u0 + u);
+    b2[u] = __ldg(B2 + u0 + u);
+    w3[u] = __ldg(W3 + u0 + u);
+  }
+  const float b3 = __ldg(W3 + kHidden);
+  for (uint32_t i0 = blockIdx.x * kTile; i0 < n; i0 += gridDim.x * kTile) {
+    load_x(x, i0, n, sm.x);
     __syncthreads();
-    float h = b1;
+    float acc[4][4];
+    auto activate = [&](float* out) {  // relu, kept for the next layer and the caller
 #pragma unroll
-    for (int k = 0; k < kFeatures; ++k) h = fmaf(w1[k], s_x[k], h);
-    h = fmaxf(0.f, h);
-    s_h1[j] = h;
-    __syncthreads();
-    float h2 = b2;
-    for (int k = 0; k < kHidden; ++k) h2 = fmaf(__ldg(W2 + j * kHidden + k), s_h1[k], h2);
-    h2 = fmaxf(0.f, h2);
-    float* a = acts + (size_t)i * (2 * kHidden + 1);
-    a[j] = h;
-    a[kHidden + j] = h2;
-    const float p = warp_sum(w3 * h2);
-    if ((j & 31) == 0) s_part[j >> 5] = p;
-    __syncthreads();
-    if (j == 0) {
-      float out = b3;
-      for (int w = 0; w < kHidden / 32; ++w) out += s_part[w];
-      a[2 * kHidden] = out;
-      y[i] = out;
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[i][u] = fmaxf(0.f, acc[i][u]);
+        *reinterpret_cast<float4*>(out + (s0 + i) * kPitch + u0) =
+            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      }
+      __syncthreads();
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[i][u] = b1[u];
+    tile_product<kFeatures, kPitchX, kHidden>(sm.x, &sm.w1[0][0], s0, u0, acc);
+    activate(sm.h[0]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[i][u] = b2[u];
+    tile_product<kHidden, kPitch, kPitch>(sm.h[0], &sm.w2[0][0], s0, u0, acc);
+    activate(sm.h[1]);
+    // y: a thread's four units, then the 16 threads of a sample (a half warp)
+    float out[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float v = 0.f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v = fmaf(w3[u], acc[i][u], v);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      out[i] = v + b3;
     }
-    __syncthreads();
+    if ((lane & 15) == 0)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i0 + s0 + i < n) {
+          y[i0 + s0 + i] = out[i];
+          acts[(size_t)(i0 + s0 + i) * (2 * kHidden + 1) + 2 * kHidden] = out[i];
+        }
+    // activations, a warp a row at a time
+    for (int s = warp; s < kTile && i0 + s < n; s += kTrainThreads / 32) {
+      float* a = acts + (size_t)(i0 + s) * (2 * kHidden + 1);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        a[h * kHidden + lane] = sm.h[h][s * kPitch + lane];
+        a[h * kHidden + 32 + lane] = sm.h[h][s * kPitch + 32 + lane];
+      }
+    }
+    __syncthreads();  // h and x are rewritten
   }
 }
 
+struct BackwardSmem {
+  float w2[kHidden][kPitch];  // [unit of layer 2][unit of layer 1]
+  float x[kTile * kPitchX];
+  float h1[kTile * kPitch], d2[kTile * kPitch], d1[kTile * kPitch];
+  float b1[kHidden];
+};
 // Gradient of the mean squared error (y - target)^2 over n samples, added
-// into grads (same layout as params; must be zeroed by the caller).
-__global__ void __launch_bounds__(kHidden)
+// into grads (same layout as params; must be zeroed by the caller).  The weight
+// gradients stay in registers over a block's tiles.
+__global__ void __launch_bounds__(kTrainThreads, 2)
     mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ x,
                         const float* __restrict__ acts, const float* __restrict__ target,
                         uint32_t n, float* __restrict__ grads) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  BackwardSmem& sm = *reinterpret_cast<BackwardSmem*>(smem);
   const float* W2 = params + kHidden * kFeatures + kHidden;
   const float* W3 = W2 + kHidden * kHidden + kHidden;
   float* gW1 = grads;
@@ -302,50 +400,119 @@ __global__ void __launch_bounds__(kHidden)
   float* gB2 = gW2 + kHidden * kHidden;
   float* gW3 = gB2 + kHidden;
   float* gB3 = gW3 + kHidden;
-  __shared__ float s_x[kFeatures], s_h1[kHidden], s_dh2[kHidden];
-  const int j = threadIdx.x;
-  float w2col[kHidden];  // W2[i][j] for all i: this thread's column
-#pragma unroll
-  for (int i = 0; i < kHidden; ++i) w2col[i] = __ldg(W2 + i * kHidden + j);
-  const float w3 = __ldg(W3 + j);
-  float acc_w1[kFeatures], acc_w2[kHidden];
-#pragma unroll
-  for (int k = 0; k < kFeatures; ++k) acc_w1[k] = 0.f;
-#pragma unroll
-  for (int k = 0; k < kHidden; ++k) acc_w2[k] = 0.f;
-  float acc_b1 = 0.f, acc_b2 = 0.f, acc_w3 = 0.f, acc_b3 = 0.f;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int k = tid; k < kHidden * kHidden; k += kTrainThreads)
+    sm.w2[k / kHidden][k % kHidden] = __ldg(W2 + k);
+  if (tid < kHidden) sm.b1[tid] = 0.f;
+  const float w3[2] = {__ldg(W3 + lane), __ldg(W3 + 32 + lane)};
+  const int s0 = tid / 16 * 4, u0 = tid % 16 * 4;
+  float g2[4][4] = {};     // d W2[s0 + i][u0 + u] (rows: units of layer 2)
+  float g1[4] = {};        // d W1[tid / 4][tid % 4 * 4 + c]
+  float gb1[4] = {};       // this thread's share of d b1[u0 + u]
+  float gb2[2] = {}, gw3[2] = {}, gb3 = 0.f;  // per lane, over the warp's samples
+  const int j1 = tid / 4, c1 = tid % 4 * 4;
   const float scale = 2.0f / (float)n;
-  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const float* a = acts + (size_t)i * (2 * kHidden + 1);
-    if (j < kFeatures) s_x[j] = __ldg(x + (size_t)i * kFeatures + j);
-    const float h1 = a[j], h2 = a[kHidden + j];
-    s_h1[j] = h1;
-    const float dy = scale * (a[2 * kHidden] - __ldg(target + i));
-    const float dh2 = h2 > 0.f ? dy * w3 : 0.f;
-    s_dh2[j] = dh2;
+  for (uint32_t i0 = blockIdx.x * kTile; i0 < n; i0 += gridDim.x * kTile) {
+    load_x(x, i0, n, sm.x);
+    for (int s = warp; s < kTile; s += kTrainThreads / 32) {  // a warp a sample at a time
+      const bool in = i0 + s < n;
+      const float* a = acts + (size_t)(i0 + s) * (2 * kHidden + 1);
+      const float dy = in ? scale * (a[2 * kHidden] - __ldg(target + i0 + s)) : 0.f;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = h * 32 + lane;
+        const float h1 = in ? a[j] : 0.f, h2 = in ? a[kHidden + j] : 0.f;
+        const float d2 = h2 > 0.f ? dy * w3[h] : 0.f;
+        sm.h1[s * kPitch + j] = h1;
+        sm.d2[s * kPitch + j] = d2;
+        gw3[h] += dy * h2;
+        gb2[h] += d2;
+      }
+      gb3 += dy;
+    }
     __syncthreads();
-    acc_w3 += dy * h2;
-    acc_b3 += dy;
-    acc_b2 += dh2;
+    float d1[4][4] = {};
+    tile_product<kHidden, kPitch, kPitch>(sm.d2, &sm.w2[0][0], s0, u0, d1);
 #pragma unroll
-    for (int k = 0; k < kHidden; ++k) acc_w2[k] = fmaf(dh2, s_h1[k], acc_w2[k]);
-    float dh1 = 0.f;
+    for (int i = 0; i < 4; ++i) {
+      const float4 h1 = *reinterpret_cast<const float4*>(sm.h1 + (s0 + i) * kPitch + u0);
+      d1[i][0] = h1.x > 0.f ? d1[i][0] : 0.f;
+      d1[i][1] = h1.y > 0.f ? d1[i][1] : 0.f;
+      d1[i][2] = h1.z > 0.f ? d1[i][2] : 0.f;
+      d1[i][3] = h1.w > 0.f ? d1[i][3] : 0.f;
 #pragma unroll
-    for (int r = 0; r < kHidden; ++r) dh1 = fmaf(w2col[r], s_dh2[r], dh1);
-    dh1 = h1 > 0.f ? dh1 : 0.f;
-    acc_b1 += dh1;
+      for (int u = 0; u < 4; ++u) gb1[u] += d1[i][u];
+      *reinterpret_cast<float4*>(sm.d1 + (s0 + i) * kPitch + u0) =
+          make_float4(d1[i][0], d1[i][1], d1[i][2], d1[i][3]);
+    }
+    __syncthreads();
+    // outer products over the tile's samples, summed by tile: shorter chains
+    float t2[4][4] = {}, t1[4] = {};
+#pragma unroll 4
+    for (int s = 0; s < kTile; ++s) {
+      const float4 r = *reinterpret_cast<const float4*>(sm.d2 + s * kPitch + s0);
+      const float4 h = *reinterpret_cast<const float4*>(sm.h1 + s * kPitch + u0);
+      const float rv[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-    for (int k = 0; k < kFeatures; ++k) acc_w1[k] = fmaf(dh1, s_x[k], acc_w1[k]);
+      for (int i = 0; i < 4; ++i) {
+        t2[i][0] = fmaf(rv[i], h.x, t2[i][0]);
+        t2[i][1] = fmaf(rv[i], h.y, t2[i][1]);
+        t2[i][2] = fmaf(rv[i], h.z, t2[i][2]);
+        t2[i][3] = fmaf(rv[i], h.w, t2[i][3]);
+      }
+      const float d = sm.d1[s * kPitch + j1];
+      const float4 f = *reinterpret_cast<const float4*>(sm.x + s * kPitchX + c1);
+      t1[0] = fmaf(d, f.x, t1[0]);
+      t1[1] = fmaf(d, f.y, t1[1]);
+      t1[2] = fmaf(d, f.z, t1[2]);
+      t1[3] = fmaf(d, f.w, t1[3]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g2[i][u] += t2[i][u];
+      g1[u] += t1[u];
+    }
     __syncthreads();
   }
 #pragma unroll
-  for (int k = 0; k < kFeatures; ++k) atomicAdd(gW1 + j * kFeatures + k, acc_w1[k]);
-  atomicAdd(gB1 + j, acc_b1);
+  for (int u = 0; u < 4; ++u) {
 #pragma unroll
-  for (int k = 0; k < kHidden; ++k) atomicAdd(gW2 + j * kHidden + k, acc_w2[k]);
-  atomicAdd(gB2 + j, acc_b2);
-  atomicAdd(gW3 + j, acc_w3);
-  if (j == 0) atomicAdd(gB3, acc_b3);
+    for (int i = 0; i < 4; ++i) atomicAdd(gW2 + (s0 + i) * kHidden + u0 + u, g2[i][u]);
+    atomicAdd(gW1 + j1 * kFeatures + c1 + u, g1[u]);
+    gb1[u] += __shfl_xor_sync(0xffffffffu, gb1[u], 16);
+    if (lane < 16) atomicAdd(&sm.b1[u0 + u], gb1[u]);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    atomicAdd(gB2 + h * 32 + lane, gb2[h]);
+    atomicAdd(gW3 + h * 32 + lane, gw3[h]);
+  }
+  if (lane == 0) atomicAdd(gB3, gb3);
+  __syncthreads();
+  if (tid < kHidden) atomicAdd(gB1 + tid, sm.b1[tid]);
+}
+
+// Blocks of a training launch: the resident ones, at most one per tile.
+template <auto KERNEL>
+cudaError_t train_blocks(size_t smem, uint32_t n, uint32_t* blocks) {
+  static std::mutex mu;
+  static int resident[kMaxDevices] = {};
+  int dev = 0;
+  cudaError_t e = current_device(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (resident[dev] == 0) {
+    int sms = 0, per_sm = 0;
+    e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, kTrainThreads, smem);
+    if (e != cudaSuccess) return e;
+    resident[dev] = sms * std::max(per_sm, 1);
+  }
+  *blocks = std::min<uint32_t>((n + kTile - 1) / kTile, (uint32_t)resident[dev]);
+  return cudaSuccess;
 }
 
 __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
@@ -447,15 +614,21 @@ cudaError_t launch_mlp_infer(const float* params, const float* x, uint32_t n, fl
 cudaError_t launch_mlp_forward(const float* params, const float* x, uint32_t n, float* acts,
                                float* y, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  mlp_forward_kernel<<<std::min<uint32_t>(n, 2048), kHidden, 0, s>>>(params, x, n, acts, y);
+  uint32_t blocks = 0;
+  const cudaError_t e = train_blocks<mlp_forward_kernel>(sizeof(ForwardSmem), n, &blocks);
+  if (e != cudaSuccess) return e;
+  mlp_forward_kernel<<<blocks, kTrainThreads, sizeof(ForwardSmem), s>>>(params, x, n, acts, y);
   return cudaGetLastError();
 }
 
 cudaError_t launch_mlp_backward(const float* params, const float* x, const float* acts,
                                 const float* target, uint32_t n, float* grads, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  mlp_backward_kernel<<<std::min<uint32_t>(n, 1024), kHidden, 0, s>>>(params, x, acts, target, n,
-                                                                      grads);
+  uint32_t blocks = 0;
+  const cudaError_t e = train_blocks<mlp_backward_kernel>(sizeof(BackwardSmem), n, &blocks);
+  if (e != cudaSuccess) return e;
+  mlp_backward_kernel<<<blocks, kTrainThreads, sizeof(BackwardSmem), s>>>(params, x, acts, target,
+                                                                          n, grads);
   return cudaGetLastError();
 }
 
