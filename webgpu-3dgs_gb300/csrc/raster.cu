@@ -787,9 +787,12 @@ __device__ __forceinline__ void store_px(float4 (&st)[2][32], uint32_t lane, con
 // region on to them, with their pixels' state and the list position (the
 // pixels' arithmetic does not change, so neither do the image and the costs).
 // The n-th block handed on goes to the n-th place, so every waiting warp polls a
-// word of its own.
+// word of its own.  Only the warps of the first kHelperCtas CTAs wait: a waiting
+// warp keeps its CTA's shared memory from kernels of other streams (3 eager
+// 1005x672 views at a time: 442 us alone and 199 us with three contexts in
+// turn; with every warp waiting 442 and 299, with none 672 and 248).
 constexpr uint32_t kPoolSlots = 4096;    // blocks handed on in a launch
-constexpr uint32_t kMaxWaiting = 1024;   // others leave
+constexpr uint32_t kHelperCtas = 64;     // the others leave when the queue is empty
 constexpr uint32_t kHandOnLeft = 512;    // list entries left below which nothing is handed on
 struct PoolSlot {
   float4 state[2][32];
@@ -823,16 +826,13 @@ __device__ __forceinline__ void hand_on(const RasterArgs& a, const float4 (&st)[
   if (lane == 0) st_relaxed_u32(&s.ready, 1u);
 }
 // Lane 0 of a warp without work: waits for a block and returns its slot, or ~0u
-// once nobody is left who could hand one on (or enough warps wait already).
-// Blocks go to places in order and a warp that got one comes back for the next
-// place, so a block without a waiting warp is found by the next that comes, its
-// giver at the latest.
+// once nobody is left who could hand one on.  Blocks go to places in order, a
+// warp that got one comes back for the next place, and none leaves while a
+// block is on its way to its place or another warp still works.
 __device__ __forceinline__ uint32_t wait_for_block(const RasterArgs& a) {
   PoolCtrl* c = static_cast<PoolCtrl*>(a.pool_ctrl);
-  const uint32_t before = atomicAdd(&c->waiting, 1u);
-  const bool crowd = before >= kMaxWaiting &&
-                     ld_relaxed_u32(&c->places) >= ld_relaxed_u32(&c->handed) + kMaxWaiting / 2;
-  const uint32_t place = crowd ? kPoolSlots : atomicAdd(&c->places, 1u);
+  atomicAdd(&c->waiting, 1u);
+  const uint32_t place = atomicAdd(&c->places, 1u);
   if (place < kPoolSlots) {
     uint32_t* ready = &static_cast<PoolSlot*>(a.pool)[place].ready;
     for (uint32_t polls = 0; polls < (1u << 22); ++polls) {  // a second and more
@@ -1092,6 +1092,10 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
       }
     } else {
       if (!HAND_ON) break;
+      if (blockIdx.x >= kHelperCtas) {
+        if (lane == 0) atomicSub(&static_cast<PoolCtrl*>(a.pool_ctrl)->present, 1u);
+        break;
+      }
       if (lane == 0) slot = wait_for_block(a);
       slot = __shfl_sync(0xffffffffu, slot, 0);
       if (slot == ~0u) break;
@@ -1230,6 +1234,10 @@ cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
 // with 1.2: 124 -> 64 us; a 3M-splat frame with 2.7: 342 us by regions, 473 by
 // blocks).
 constexpr float kFineWaves = 1.75f;
+// Blocks are handed on in the row-major order, which cannot know the long lists
+// beforehand, and in orders by cost up to this many regions a warp (16 views of
+// 640x360 with 5 regions a warp: raster 975 -> 871 us; with 20 and more the
+// tail is short and the check costs 2%).
 constexpr float kHandOnWaves = 8.0f;
 
 }  // namespace
