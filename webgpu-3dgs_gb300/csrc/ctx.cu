@@ -528,11 +528,11 @@ SortPlan tile_digit_plan(uint32_t num_tiles, uint32_t digit_bits) {
   return tp;
 }
 
-int raster_stage(gs3d_ctx* c, bool culled) {
-  if ((uint64_t)c->tile_w * c->tile_h > 1024 && !culled)
+int raster_stage(gs3d_ctx* c) {
+  if ((uint64_t)c->tile_w * c->tile_h > 1024 && (c->flags & GS3D_FLAG_STAGEWISE_REBIN))
     return fail(c, GS3D_ERR_INVALID_ARG,
-                "tiles of %ux%u pixels are shaded by the culled two-pixel raster only; the "
-                "stage-wise rebin's one-pixel raster takes at most 1024",
+                "tiles of %ux%u pixels are for the fused rebin; the stage-wise rebin takes tiles "
+                "of at most 1024 pixels",
                 c->tile_w, c->tile_h);
   StageScope t(c, GS3D_STAGE_RASTER);
   RasterArgs a{};
@@ -545,7 +545,6 @@ int raster_stage(gs3d_ctx* c, bool culled) {
   // batches of a 2048-pixel tile would not fit shared memory)
   a.batch = c->raster_batch ? c->raster_batch
                             : ((uint64_t)c->tile_w * c->tile_h > 1024 ? 1024u : 0u);
-  a.culled = culled;
   uint32_t strips = 1, raster_ctas = 1;
   CK(raster_shape(a, c->sm_count, &strips, &raster_ctas), "raster shape");
   const bool split_all = (c->flags & GS3D_FLAG_SPLIT_ALL_TILES) != 0;
@@ -787,7 +786,7 @@ int fused_rebin(gs3d_ctx* c) {
   } else {
     TRY(sort_refs(c, rect8));
   }
-  return raster_stage(c, true);
+  return raster_stage(c);
 }
 
 void destroy_graph(gs3d_ctx* c) {
@@ -1271,7 +1270,7 @@ int gs3d_rasterize_tiles(gs3d_ctx* c) {
   if (!c) return GS3D_ERR_INVALID_ARG;
   TRY(require_frame(c, "rasterize_tiles"));
   TRY(set_device(c));
-  return raster_stage(c, /*culled=*/!(c->flags & GS3D_FLAG_STAGEWISE_REBIN));
+  return raster_stage(c);
 }
 
 int gs3d_rebin(gs3d_ctx* c, const gs3d_camera* cam, uint32_t width, uint32_t height) {

@@ -474,7 +474,6 @@ struct RasterArgs {
   void* pool_ctrl;
   uint32_t* err;
   uint32_t batch;         // splats staged per batch (0 = tile_w * tile_h)
-  bool culled;
   // tiles at the head of the order whose blocks are shaded as two half-block
   // items (device count, warp variant only; may be null: none)
   const uint32_t* heavy;

@@ -1180,7 +1180,7 @@ size_t raster_smem(int mode, uint32_t D, uint32_t threads) {
 cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
   const uint32_t nt = a.tile_w * a.tile_h;
   if (a.batch % 32 != 0 || a.batch > 1024) return cudaErrorInvalidValue;
-  const bool culled = a.culled && (nt % 32 == 0);
+  const bool culled = nt % 32 == 0;  // whole warps; else pixel by pixel
   // warp items where the tile splits into 8x8 blocks
   const int mode = !culled ? 0 : (a.tile_w % 8 == 0 && a.tile_h % 8 == 0) ? 2 : 1;
   if (mode != 2 && nt > 1024) return cudaErrorInvalidValue;  // one thread a pixel
