@@ -232,13 +232,13 @@ int ensure_splat_buffers(gs3d_ctx* c, uint32_t m) {
   TRY(ensure(c, c->counts, (size_t)m * 4, "splat_ref_counts"));
   TRY(ensure(c, c->offsets, ((size_t)m + 1) * 4, "splat_ref_offsets"));
   TRY(ensure(c, c->scan_status, scan_status_words(m) * 8, "scan look-back status"));
-  const size_t md = sort_capacity_round(std::max<uint32_t>(m, 1));
+  const size_t md = depth_sort_capacity(m);
   TRY(ensure(c, c->depth_keys_a, md * 4, "depth keys"));
   TRY(ensure(c, c->depth_keys_b, md * 4, "depth keys"));
   TRY(ensure(c, c->depth_ids_a, md * 4, "depth ids"));
   TRY(ensure(c, c->depth_ids_b, md * 4, "depth ids"));
   TRY(ensure(c, c->sorted_offsets, ((size_t)m + 1) * 4, "depth-ordered offsets"));
-  TRY(ensure(c, c->depth_status, sort_status_words(m, 4) * 4, "depth sort status"));
+  TRY(ensure(c, c->depth_status, depth_sort_status_words(m) * 4, "depth sort status"));
   TRY(ensure(c, c->rect8, (size_t)m * 4, "tile rectangles"));
   return GS3D_OK;
 }
@@ -630,6 +630,11 @@ bool use_cells(const gs3d_ctx* c) {
   return fits && c->total_tiles > 256;  // else one digit pass
 }
 
+DepthSorted depth_sorted(gs3d_ctx* c) {
+  return DepthSorted{&ctrl_of(c)->depth_range, u32(c->depth_keys_a), u32(c->depth_ids_a),
+                     u32(c->depth_keys_b), u32(c->depth_ids_b)};
+}
+
 void next_scan_epoch(gs3d_ctx* c) { c->scan_epoch = (c->scan_epoch % ((1u << 30) - 1)) + 1; }
 
 SortPlan cell_digit_plan(uint32_t num_cells, uint32_t digit_bits) {
@@ -651,7 +656,7 @@ int bin_refs(gs3d_ctx* c, const uint32_t* rect8) {
     // cleared every rebin: a graph replay reuses the captured epoch
     CK(cudaMemsetAsync(c->scan_status.p, 0, scan_status_words(c->total_splats) * 8, c->stream),
        "clear scan status");
-    CK(launch_scan_cells(u32(c->counts), rect8, proj, u32(c->depth_ids_a), u32(c->sorted_offsets),
+    CK(launch_scan_cells(u32(c->counts), rect8, proj, depth_sorted(c), u32(c->sorted_offsets),
                          c->total_splats, static_cast<unsigned long long*>(c->scan_status.p),
                          &k->scan_tile_counter, c->scan_epoch, &k->entry_total, &k->ref_total,
                          &k->error, c->stream),
@@ -665,8 +670,8 @@ int bin_refs(gs3d_ctx* c, const uint32_t* rect8) {
   DevBuf& vb = cp.passes % 2 ? c->vals_b : c->vals_a;
   {
     StageScope t(c, GS3D_STAGE_EMIT);
-    CK(launch_emit_cells(dviews(c), nv, c->total_splats, proj, rect8, u32(c->depth_keys_a),
-                         u32(c->depth_ids_a), u32(c->sorted_offsets), &k->entry_total,
+    CK(launch_emit_cells(dviews(c), nv, c->total_splats, proj, rect8, depth_sorted(c),
+                         u32(c->sorted_offsets), &k->entry_total,
                          &k->ref_total, u32(c->ref_counter), c->capacity,
                          static_cast<uint2*>(ka.p), u32(va), cp, &k->tile_hist[0][0],
                          &k->emit_chunk, &k->error, c->sm_count, c->stream),
@@ -713,7 +718,8 @@ int sort_refs(gs3d_ctx* c, const uint32_t* rect8) {
     // cleared every rebin: a graph replay reuses the captured epoch
     CK(cudaMemsetAsync(c->scan_status.p, 0, scan_status_words(c->total_splats) * 8, c->stream),
        "clear scan status");
-    CK(launch_scan(u32(c->counts), u32(c->depth_ids_a), u32(c->sorted_offsets), c->total_splats,
+    const DepthSorted order = depth_sorted(c);
+    CK(launch_scan(u32(c->counts), &order, u32(c->sorted_offsets), c->total_splats,
                    static_cast<unsigned long long*>(c->scan_status.p), &k->scan_tile_counter,
                    c->scan_epoch, u32(c->ref_counter), &k->error, c->stream),
        "prefix scan (depth order)");
@@ -722,8 +728,7 @@ int sort_refs(gs3d_ctx* c, const uint32_t* rect8) {
   {
     StageScope t(c, GS3D_STAGE_EMIT);
     CK(launch_emit_sorted(dviews(c), nv, c->total_splats,
-                          static_cast<gs3d_projected_splat*>(c->proj.p), rect8, u32(c->depth_keys_a),
-                          u32(c->depth_ids_a),
+                          static_cast<gs3d_projected_splat*>(c->proj.p), rect8, depth_sorted(c),
                           u32(c->sorted_offsets), u32(c->ref_counter), c->capacity,
                           static_cast<uint2*>(c->keys_a.p), u32(c->vals_a), tp,
                           &k->tile_hist[0][0], &k->emit_chunk, &k->error, c->sm_count,
@@ -770,15 +775,16 @@ int fused_rebin(gs3d_ctx* c) {
     StageScope t(c, GS3D_STAGE_PREPROCESS);
     CK(launch_preprocess(dviews(c), nv, c->total_blocks, c->max_sh,
                          static_cast<gs3d_projected_splat*>(c->proj.p), u32(c->counts),
-                         u32(c->depth_keys_a), u32(c->depth_ids_a), rect8, &k->error, c->stream),
+                         u32(c->depth_keys_a), u32(c->depth_ids_a), rect8, &k->depth_range,
+                         &k->error, c->stream),
        "preprocess");
   }
   {
     StageScope t(c, GS3D_STAGE_DEPTH_SORT);
-    CK(launch_sort_depth_keys(&dviews(c)->batch_splats, c->total_splats, u32(c->depth_keys_a),
-                              u32(c->depth_ids_a), u32(c->depth_keys_b), u32(c->depth_ids_b),
-                              u32(c->depth_status), &k->sort_hist[0][0],
-                              &k->sort_part_counter[0], &k->error, c->sm_count, c->stream),
+    CK(launch_sort_depth(&dviews(c)->batch_splats, c->total_splats, &k->depth_range,
+                         u32(c->depth_keys_a), u32(c->depth_ids_a), u32(c->depth_keys_b),
+                         u32(c->depth_ids_b), u32(c->depth_status), &k->depth_hist[0][0],
+                         &k->sort_part_counter[0], &k->error, c->sm_count, c->stream),
        "depth sort");
   }
   if (use_cells(c)) {
@@ -1198,7 +1204,7 @@ int gs3d_preprocess(gs3d_ctx* c) {
   StageScope t(c, GS3D_STAGE_PREPROCESS);
   CK(launch_preprocess(dviews(c), 1, c->total_blocks, c->max_sh,
                        static_cast<gs3d_projected_splat*>(c->proj.p), u32(c->counts), nullptr,
-                       nullptr, nullptr, &ctrl_of(c)->error, c->stream),
+                       nullptr, nullptr, nullptr, &ctrl_of(c)->error, c->stream),
      "preprocess");
   return GS3D_OK;
 }

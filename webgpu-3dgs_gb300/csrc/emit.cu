@@ -108,12 +108,10 @@ struct CellArgs {
   uint32_t* ref_counter;  // written: min(*ref_total, 2^32 - 1)
 };
 template <int TP, int BINS, bool CELLS>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
     emit_sorted_kernel(const ViewDesc* __restrict__ views, uint32_t n_views, uint32_t n,
                        const gs3d_projected_splat* __restrict__ proj,
-                       const uint32_t* __restrict__ rect8,
-                       const uint32_t* __restrict__ sorted_keys,
-                       const uint32_t* __restrict__ sorted_ids,
+                       const uint32_t* __restrict__ rect8, DepthSorted sorted,
                        const uint32_t* __restrict__ sorted_offsets,
                        const uint32_t* __restrict__ ref_counter, CellArgs cells,
                        uint32_t capacity, uint2* __restrict__ keys,
@@ -136,6 +134,8 @@ __global__ void __launch_bounds__(kThreads)
     if (blockIdx.x == 0 && threadIdx.x == 0) latch_error(err, DEVERR_CAPACITY);
     return;
   }
+  const uint32_t* __restrict__ sorted_keys = sorted.keys();
+  const uint32_t* __restrict__ sorted_ids = sorted.ids();
   for (int k = threadIdx.x; k < TP * BINS; k += kThreads) (&s_hist[0][0])[k] = 0u;
   const int sh[4] = {shifts.x, shifts.y, shifts.z, shifts.w};
   const uint32_t mk[4] = {masks.x, masks.y, masks.z, masks.w};
@@ -326,8 +326,8 @@ uint32_t emit_blocks_per_sm() {
 template <bool CELLS>
 cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
                          const gs3d_projected_splat* proj, const uint32_t* rect8,
-                         const uint32_t* sorted_keys, const uint32_t* sorted_ids,
-                         const uint32_t* sorted_offsets, const uint32_t* counter, CellArgs cells,
+                         const DepthSorted& sorted, const uint32_t* sorted_offsets,
+                         const uint32_t* counter, CellArgs cells,
                          uint32_t capacity, uint2* keys, uint32_t* values, const SortPlan& plan,
                          uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                          cudaStream_t s) {
@@ -348,8 +348,8 @@ cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
   case TP:                                                                                    \
     emit_sorted_kernel<TP, BINS, CELLS>                                                       \
         <<<std::min(chunks, sms * emit_blocks_per_sm<TP, BINS, CELLS>()), kThreads, 0, s>>>(  \
-            views, n_views, n, proj, rect8, sorted_keys, sorted_ids, sorted_offsets, counter, \
-            cells, capacity, keys, values, sh, mk, g_hist, chunk_ticket, err);                \
+            views, n_views, n, proj, rect8, sorted, sorted_offsets, counter, cells,           \
+            capacity, keys, values, sh, mk, g_hist, chunk_ticket, err);                \
     break;
   if (wide) {
     switch (plan.passes) {
@@ -378,28 +378,27 @@ cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
 
 cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t n,
                                const gs3d_projected_splat* proj, const uint32_t* rect8,
-                               const uint32_t* sorted_keys,
-                               const uint32_t* sorted_ids,
+                               const DepthSorted& sorted,
                                const uint32_t* sorted_offsets, const uint32_t* ref_counter,
                                uint32_t capacity, uint2* keys, uint32_t* values,
                                const SortPlan& tile_plan, uint32_t* g_hist,
                                uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                                cudaStream_t s) {
-  return emit_ordered<false>(views, n_views, n, proj, rect8, sorted_keys, sorted_ids,
-                             sorted_offsets, ref_counter, CellArgs{}, capacity, keys, values,
+  return emit_ordered<false>(views, n_views, n, proj, rect8, sorted, sorted_offsets,
+                             ref_counter, CellArgs{}, capacity, keys, values,
                              tile_plan, g_hist, chunk_ticket, err, sm_count, s);
 }
 
 cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t n,
                               const gs3d_projected_splat* proj, const uint32_t* rect8,
-                              const uint32_t* sorted_keys, const uint32_t* sorted_ids,
-                              const uint32_t* sorted_offsets, const uint32_t* entry_total,
+                              const DepthSorted& sorted, const uint32_t* sorted_offsets,
+                              const uint32_t* entry_total,
                               const unsigned long long* ref_total, uint32_t* ref_counter,
                               uint32_t capacity, uint2* keys, uint32_t* values,
                               const SortPlan& cell_plan, uint32_t* g_hist, uint32_t* chunk_ticket,
                               uint32_t* err, int sm_count, cudaStream_t s) {
-  return emit_ordered<true>(views, n_views, n, proj, rect8, sorted_keys, sorted_ids,
-                            sorted_offsets, entry_total, CellArgs{ref_total, ref_counter},
+  return emit_ordered<true>(views, n_views, n, proj, rect8, sorted, sorted_offsets, entry_total,
+                            CellArgs{ref_total, ref_counter},
                             capacity, keys, values, cell_plan, g_hist, chunk_ticket, err,
                             sm_count, s);
 }

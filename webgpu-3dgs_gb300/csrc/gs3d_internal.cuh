@@ -104,6 +104,26 @@ enum : uint32_t {
   DEVERR_BUCKET = 8u,    // a radix digit held 2^30 keys or more (30-bit look-back counts)
 };
 
+// Largest depth key of the frame's valid splats and largest complement of one
+// (the smallest key), both 0 before the preprocess.
+struct DepthRange {
+  uint32_t max, max_not;
+};
+constexpr int kDepthPasses = 4;  // launched; three where the keys span less than 2^27
+__host__ __device__ inline bool depth_three_passes(uint32_t lo, uint32_t hi) {
+  return hi >= lo && hi - lo < (1u << 27);
+}
+// Where the depth sort leaves its result: the B arrays after three passes.
+struct DepthSorted {
+  const DepthRange* range;
+  const uint32_t *keys_a, *ids_a, *keys_b, *ids_b;
+  __device__ __forceinline__ bool in_b() const {
+    return depth_three_passes(~__ldg(&range->max_not), __ldg(&range->max));
+  }
+  __device__ __forceinline__ const uint32_t* keys() const { return in_b() ? keys_b : keys_a; }
+  __device__ __forceinline__ const uint32_t* ids() const { return in_b() ? ids_b : ids_a; }
+};
+
 constexpr int kMaxSortPasses = 8;
 constexpr int kRadixBins = 256;
 // Histograms of the fused rebin's tile-id passes: 2048 bins a pass (11-bit
@@ -123,7 +143,8 @@ struct Ctrl {
   uint32_t entry_total;          // its (splat, cell) entries
   uint32_t tile_scan_counter;
   uint32_t tile_scan_total;
-  uint32_t pad;
+  DepthRange depth_range;
+  uint32_t depth_hist[kDepthPasses][512];
   uint32_t sort_hist[kMaxSortPasses][kRadixBins];  // global digit histograms
   uint32_t sched_hist[2][kRadixBins];
   uint32_t tile_hist[kMaxTilePasses][kTileHistStride];  // fused rebin's tile passes
@@ -302,9 +323,9 @@ __host__ __device__ inline uint32_t digit_mask(int nbits) { return (1u << nbits)
 cudaError_t launch_preprocess(const ViewDesc* views, uint32_t n_views, uint32_t total_blocks,
                               uint32_t max_sh_degree, gs3d_projected_splat* out, uint32_t* counts,
                               uint32_t* depth_keys, uint32_t* depth_ids, uint32_t* rect8,
-                              uint32_t* err, cudaStream_t s);
-// Exclusive scan of counts[gather[i]] (counts[i] when gather is null).
-cudaError_t launch_scan(const uint32_t* counts, const uint32_t* gather, uint32_t* offsets,
+                              DepthRange* range, uint32_t* err, cudaStream_t s);
+// Exclusive scan of counts in the order of gather (as they are when it is null).
+cudaError_t launch_scan(const uint32_t* counts, const DepthSorted* gather, uint32_t* offsets,
                         uint32_t n, unsigned long long* status, uint32_t* tile_counter,
                         uint32_t epoch, uint32_t* total_out, uint32_t* err, cudaStream_t s);
 size_t scan_status_words(uint32_t n);
@@ -312,7 +333,7 @@ size_t scan_status_words(uint32_t n);
 // covers: its rectangle in rect8 (all ones: culled), or where rect8 is null in
 // the projected records (counts 0: culled).  Adds the refs to *ref_total.
 cudaError_t launch_scan_cells(const uint32_t* counts, const uint32_t* rect8,
-                              const gs3d_projected_splat* proj, const uint32_t* gather,
+                              const gs3d_projected_splat* proj, const DepthSorted& gather,
                               uint32_t* offsets, uint32_t n, unsigned long long* status,
                               uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
                               unsigned long long* ref_total, uint32_t* err, cudaStream_t s);
@@ -368,11 +389,16 @@ cudaError_t launch_sort_u32(const SortPlan& plan, const uint32_t* count, uint32_
                             uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b,
                             uint32_t* vals_b, uint32_t* status, uint32_t* g_hist,
                             uint32_t* part_counters, uint32_t* err, int sm_count, cudaStream_t s);
-// Four 8-bit passes over 32-bit per-splat depth keys (count read on device).
-cudaError_t launch_sort_depth_keys(const uint32_t* count, uint32_t capacity, uint32_t* keys_a,
-                                   uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b,
-                                   uint32_t* status, uint32_t* g_hist, uint32_t* part_counters,
-                                   uint32_t* err, int sm_count, cudaStream_t s);
+// Depth order of the splat-views (depth_sort.cu): keys_a / ids_a sorted (count
+// read on the device), the result where DepthSorted says.  The arrays hold
+// depth_sort_capacity(capacity) entries; g_hist[4][512] zeroed.
+size_t depth_sort_capacity(uint32_t n);
+size_t depth_sort_status_words(uint32_t n);
+cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const DepthRange* range,
+                              uint32_t* keys_a, uint32_t* ids_a, uint32_t* keys_b,
+                              uint32_t* ids_b, uint32_t* status, uint32_t* g_hist,
+                              uint32_t* part_counters, uint32_t* err, int sm_count,
+                              cudaStream_t s);
 // Raster work order: tile indices sorted by decreasing expected cost
 // (schedule = GS3D_SCHEDULE_KEY_COUNT: the tile's key count), so the
 // persistent raster CTAs start the longest tiles first.
@@ -434,8 +460,7 @@ cudaError_t launch_log_costs(const uint32_t* costs, uint32_t n, float* out, cuda
 // rectangles from the projected records).
 cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t total,
                                const gs3d_projected_splat* proj, const uint32_t* rect8,
-                               const uint32_t* sorted_keys,
-                               const uint32_t* sorted_ids,
+                               const DepthSorted& sorted,
                                const uint32_t* sorted_offsets, const uint32_t* ref_counter,
                                uint32_t capacity, uint2* keys, uint32_t* values,
                                const SortPlan& tile_plan, uint32_t* g_hist,
@@ -445,8 +470,8 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
 // rectangle inside it | depth], and *ref_counter = the frame's refs.
 cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t total,
                               const gs3d_projected_splat* proj, const uint32_t* rect8,
-                              const uint32_t* sorted_keys, const uint32_t* sorted_ids,
-                              const uint32_t* sorted_offsets, const uint32_t* entry_total,
+                              const DepthSorted& sorted, const uint32_t* sorted_offsets,
+                              const uint32_t* entry_total,
                               const unsigned long long* ref_total, uint32_t* ref_counter,
                               uint32_t capacity, uint2* keys, uint32_t* values,
                               const SortPlan& cell_plan, uint32_t* g_hist, uint32_t* chunk_ticket,

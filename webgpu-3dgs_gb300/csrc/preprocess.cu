@@ -90,6 +90,7 @@ __device__ __forceinline__ void preprocess_block(const ViewDesc* __restrict__ vi
                                                  uint32_t* __restrict__ depth_keys,
                                                  uint32_t* __restrict__ depth_ids,
                                                  uint32_t* __restrict__ rect8,
+                                                 DepthRange* __restrict__ range,
                                                  uint32_t* __restrict__ err) {
   constexpr int K = (DEG + 1) * (DEG + 1) - 1;
   constexpr int KC = 3 * K;  // floats of SH rest per splat
@@ -155,6 +156,11 @@ __device__ __forceinline__ void preprocess_block(const ViewDesc* __restrict__ vi
     sh_ready = false;
   }
 
+  // the frame's range so far (it only widens; read long before it is needed)
+  uint32_t seen = 0;
+  if (range != nullptr && threadIdx.x < 2)
+    seen = ld_relaxed_u32(threadIdx.x == 0 ? &range->max : &range->max_not);
+  uint32_t key_max = 0, key_max_not = 0;  // depth keys of this thread's valid splat-views
   for (uint32_t v = leader; v != kNoView; v = views[v].group_next) {
     const ViewDesc& vd = views[v];
     const FrameUniforms* fu = &vd.f;
@@ -275,7 +281,12 @@ __device__ __forceinline__ void preprocess_block(const ViewDesc* __restrict__ vi
       reinterpret_cast<uint4*>(o)[3] = r3;
       counts[gi] = count;
       if (depth_keys != nullptr) {  // per-splat depth sort keys of the fused rebin
-        depth_keys[gi] = valid ? __float_as_uint(-r0.z) : 0xffffffffu;
+        const uint32_t key = valid ? __float_as_uint(-r0.z) : 0xffffffffu;
+        depth_keys[gi] = key;
+        if (valid) {
+          key_max = max(key_max, key);
+          key_max_not = max(key_max_not, ~key);
+        }
         depth_ids[gi] = gi;
         // tile rectangle in one word [x0, y0, x1 - x0, y1 - y0] (8 bits each;
         // requested only when every view has at most 256 tiles per axis; kCulledRect,
@@ -286,14 +297,33 @@ __device__ __forceinline__ void preprocess_block(const ViewDesc* __restrict__ vi
       }
     }
   }
+  if (range != nullptr) {  // one pair per block, added where it widens the frame's
+    __shared__ uint32_t s_range[kThreads / 32][2];
+    key_max = __reduce_max_sync(0xffffffffu, key_max);
+    key_max_not = __reduce_max_sync(0xffffffffu, key_max_not);
+    if ((threadIdx.x & 31) == 0) {
+      s_range[threadIdx.x >> 5][0] = key_max;
+      s_range[threadIdx.x >> 5][1] = key_max_not;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      uint32_t m = 0;
+#pragma unroll
+      for (int w = 0; w < kThreads / 32; ++w) m = max(m, s_range[w][threadIdx.x]);
+      if (m > seen) atomicMax(threadIdx.x == 0 ? &range->max : &range->max_not, m);
+    }
+  }
 }
 
+// Four blocks per SM (64 registers a thread; the SH slices of degree 3 leave no
+// room for a fifth): with 70 registers and three blocks 8 views of 3M splats
+// took 770 us, with four 711.
 template <int MAXDEG>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
     preprocess_kernel(const ViewDesc* __restrict__ views, uint32_t n_views,
                       gs3d_projected_splat* __restrict__ out, uint32_t* __restrict__ counts,
                       uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ depth_ids,
-                      uint32_t* __restrict__ rect8,
+                      uint32_t* __restrict__ rect8, DepthRange* __restrict__ range,
                       uint32_t* __restrict__ err) {
   extern __shared__ __align__(16) float s_sh[];
   __shared__ uint64_t s_bar;
@@ -307,22 +337,22 @@ __global__ void __launch_bounds__(kThreads)
   switch (deg) {  // uniform per block
     case 0:
       preprocess_block<0>(views, v, local_first, s_sh, &s_bar, out, counts, depth_keys,
-                          depth_ids, rect8, err);
+                          depth_ids, rect8, range, err);
       break;
     case 1:
       if (MAXDEG >= 1)
         preprocess_block<MAXDEG >= 1 ? 1 : 0>(views, v, local_first, s_sh, &s_bar, out, counts,
-                                              depth_keys, depth_ids, rect8, err);
+                                              depth_keys, depth_ids, rect8, range, err);
       break;
     case 2:
       if (MAXDEG >= 2)
         preprocess_block<MAXDEG >= 2 ? 2 : 0>(views, v, local_first, s_sh, &s_bar, out, counts,
-                                              depth_keys, depth_ids, rect8, err);
+                                              depth_keys, depth_ids, rect8, range, err);
       break;
     default:
       if (MAXDEG >= 3)
         preprocess_block<MAXDEG >= 3 ? 3 : 0>(views, v, local_first, s_sh, &s_bar, out, counts,
-                                              depth_keys, depth_ids, rect8, err);
+                                              depth_keys, depth_ids, rect8, range, err);
       break;
   }
 }
@@ -332,8 +362,7 @@ __global__ void __launch_bounds__(kThreads)
 cudaError_t launch_preprocess(const ViewDesc* views, uint32_t n_views, uint32_t total_blocks,
                               uint32_t max_sh_degree, gs3d_projected_splat* out, uint32_t* counts,
                               uint32_t* depth_keys, uint32_t* depth_ids, uint32_t* rect8,
-                              uint32_t* err,
-                              cudaStream_t s) {
+                              DepthRange* range, uint32_t* err, cudaStream_t s) {
   if (total_blocks == 0) return cudaSuccess;
   const uint32_t kc = 3u * ((max_sh_degree + 1) * (max_sh_degree + 1) - 1);
   // 45 floats x 256 splats = 46,080 B at degree 3: inside the 48 KB default window
@@ -341,19 +370,19 @@ cudaError_t launch_preprocess(const ViewDesc* views, uint32_t n_views, uint32_t 
   switch (max_sh_degree) {
     case 0:
       preprocess_kernel<0><<<total_blocks, kThreads, 0, s>>>(views, n_views, out, counts,
-                                                             depth_keys, depth_ids, rect8, err);
+                                                             depth_keys, depth_ids, rect8, range, err);
       break;
     case 1:
       preprocess_kernel<1><<<total_blocks, kThreads, smem, s>>>(views, n_views, out, counts,
-                                                                depth_keys, depth_ids, rect8, err);
+                                                                depth_keys, depth_ids, rect8, range, err);
       break;
     case 2:
       preprocess_kernel<2><<<total_blocks, kThreads, smem, s>>>(views, n_views, out, counts,
-                                                                depth_keys, depth_ids, rect8, err);
+                                                                depth_keys, depth_ids, rect8, range, err);
       break;
     default:
       preprocess_kernel<3><<<total_blocks, kThreads, smem, s>>>(views, n_views, out, counts,
-                                                                depth_keys, depth_ids, rect8, err);
+                                                                depth_keys, depth_ids, rect8, range, err);
       break;
   }
   return cudaGetLastError();

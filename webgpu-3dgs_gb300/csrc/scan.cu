@@ -56,8 +56,7 @@ __device__ __forceinline__ uint32_t rect_cells(uint32_t x0, uint32_t y0, uint32_
 
 template <Scan KIND>
 __global__ void __launch_bounds__(kThreads)
-    scan_kernel(const uint32_t* __restrict__ in, const uint32_t* __restrict__ gather,
-                ScanExtra ex, uint32_t* __restrict__ out, uint32_t n,
+    scan_kernel(const uint32_t* __restrict__ in, DepthSorted order, ScanExtra ex, uint32_t* __restrict__ out, uint32_t n,
                 unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket,
                 uint32_t epoch, uint32_t* __restrict__ total_out, uint32_t* __restrict__ err) {
   __shared__ uint32_t s_tile, s_prefix;
@@ -65,6 +64,7 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ unsigned long long s_refs[kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
+  const uint32_t* gather = order.range != nullptr ? order.ids() : nullptr;
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -230,7 +230,7 @@ __global__ void scan_empty_kernel(uint32_t* out, uint32_t* total_out) {
 
 size_t scan_status_words(uint32_t n) { return (n + kTile - 1) / kTile + 1; }
 
-cudaError_t launch_scan(const uint32_t* counts, const uint32_t* gather, uint32_t* offsets,
+cudaError_t launch_scan(const uint32_t* counts, const DepthSorted* gather, uint32_t* offsets,
                         uint32_t n, unsigned long long* status, uint32_t* tile_counter,
                         uint32_t epoch, uint32_t* total_out, uint32_t* err, cudaStream_t s) {
   if (n == 0) {
@@ -238,13 +238,13 @@ cudaError_t launch_scan(const uint32_t* counts, const uint32_t* gather, uint32_t
     return cudaGetLastError();
   }
   const uint32_t tiles = (n + kTile - 1) / kTile;
-  scan_kernel<Scan::counts><<<tiles, kThreads, 0, s>>>(counts, gather, ScanExtra{}, offsets, n,
+  scan_kernel<Scan::counts><<<tiles, kThreads, 0, s>>>(counts, gather ? *gather : DepthSorted{}, ScanExtra{}, offsets, n,
                                                        status, tile_counter, epoch, total_out, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_scan_cells(const uint32_t* counts, const uint32_t* rect8,
-                              const gs3d_projected_splat* proj, const uint32_t* gather,
+                              const gs3d_projected_splat* proj, const DepthSorted& gather,
                               uint32_t* offsets, uint32_t n, unsigned long long* status,
                               uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
                               unsigned long long* ref_total, uint32_t* err, cudaStream_t s) {
@@ -269,7 +269,7 @@ cudaError_t launch_scan_tiles(const uint32_t* tile_counts, uint32_t* tile_offset
                               uint32_t* err, cudaStream_t s) {
   const uint32_t tiles = (n + kTile - 1) / kTile;
   const ScanExtra ex{nullptr, nullptr, const_cast<unsigned long long*>(ref_total)};
-  scan_kernel<Scan::tiles><<<tiles, kThreads, 0, s>>>(tile_counts, nullptr, ex, tile_offsets, n,
+  scan_kernel<Scan::tiles><<<tiles, kThreads, 0, s>>>(tile_counts, DepthSorted{}, ex, tile_offsets, n,
                                                       status, tile_counter, epoch, total_out, err);
   return cudaGetLastError();
 }

@@ -22,8 +22,8 @@
 // 8.  Passes alternate A->B->A; with an odd pass count the sorted result ends
 // in the B buffers and the host swaps the buffer names.
 //
-// The same pass kernel, instantiated for 32-bit keys, sorts the per-splat
-// depth keys of the fused rebin (fused_rebin in ctx.cu).
+// The same pass kernel, instantiated for 32-bit keys, sorts the raster's work
+// order (schedule.cu); the splats' depth keys have their own (depth_sort.cu).
 //
 // The order produced is identical to the reference's: lexicographic
 // (tile id, depth bits, emit position), since every pass is a stable
@@ -944,21 +944,6 @@ cudaError_t launch_sort_u32(const SortPlan& plan, const uint32_t* count, uint32_
                             uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b,
                             uint32_t* vals_b, uint32_t* status, uint32_t* g_hist,
                             uint32_t* part_counters, uint32_t* err, int sm_count, cudaStream_t s) {
-  return run_passes<uint32_t>(plan, count, capacity, keys_a, vals_a, keys_b, vals_b, status,
-                              g_hist, kRadixBins, part_counters, err, false, sm_count, s);
-}
-
-cudaError_t launch_sort_depth_keys(const uint32_t* count, uint32_t capacity, uint32_t* keys_a,
-                                   uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b,
-                                   uint32_t* status, uint32_t* g_hist, uint32_t* part_counters,
-                                   uint32_t* err, int sm_count, cudaStream_t s) {
-  SortPlan plan{};
-  plan.passes = 4;
-  for (int p = 0; p < 4; ++p) {
-    plan.word[p] = 1;
-    plan.shift[p] = 8 * p;
-    plan.nbits[p] = 8;
-  }
   return run_passes<uint32_t>(plan, count, capacity, keys_a, vals_a, keys_b, vals_b, status,
                               g_hist, kRadixBins, part_counters, err, false, sm_count, s);
 }
