@@ -528,7 +528,8 @@ SortPlan tile_digit_plan(uint32_t num_tiles, uint32_t digit_bits) {
   return tp;
 }
 
-int raster_stage(gs3d_ctx* c) {
+// cleared: the fused rebin has zeroed the work queue and the tile costs.
+int raster_stage(gs3d_ctx* c, bool cleared) {
   if ((uint64_t)c->tile_w * c->tile_h > 1024 && (c->flags & GS3D_FLAG_STAGEWISE_REBIN))
     return fail(c, GS3D_ERR_INVALID_ARG,
                 "tiles of %ux%u pixels are for the fused rebin; the stage-wise rebin takes tiles "
@@ -549,11 +550,16 @@ int raster_stage(gs3d_ctx* c) {
   CK(raster_shape(a, c->sm_count, &strips, &raster_ctas), "raster shape");
   const bool split_all = (c->flags & GS3D_FLAG_SPLIT_ALL_TILES) != 0;
   const bool learned = c->schedule == GS3D_SCHEDULE_LEARNED && c->total_tiles > 1;
-  CK(cudaMemsetAsync(&ctrl_of(c)->raster_queue, 0,
-                     offsetof(Ctrl, raster_pool) + sizeof(Ctrl::raster_pool) -
-                         offsetof(Ctrl, raster_queue),
-                     c->stream),
-     "reset raster queue");
+  if (!cleared) {
+    CK(cudaMemsetAsync(&ctrl_of(c)->raster_queue, 0,
+                       offsetof(Ctrl, raster_pool) + sizeof(Ctrl::raster_pool) -
+                           offsetof(Ctrl, raster_queue),
+                       c->stream),
+       "reset raster queue");
+    // every work item folds its cost into its tile's by maximum
+    CK(cudaMemsetAsync(c->tile_costs.p, 0, (size_t)c->total_tiles * sizeof(uint32_t), c->stream),
+       "clear tile costs");
+  }
   const uint32_t* order = nullptr;
   const uint32_t* heavy = nullptr;
   if (c->schedule != GS3D_SCHEDULE_ROW_MAJOR && c->total_tiles > 1) {
@@ -653,9 +659,6 @@ int bin_refs(gs3d_ctx* c, const uint32_t* rect8) {
   next_scan_epoch(c);
   {
     StageScope t(c, GS3D_STAGE_SCAN);
-    // cleared every rebin: a graph replay reuses the captured epoch
-    CK(cudaMemsetAsync(c->scan_status.p, 0, scan_status_words(c->total_splats) * 8, c->stream),
-       "clear scan status");
     CK(launch_scan_cells(u32(c->counts), rect8, proj, depth_sorted(c), u32(c->sorted_offsets),
                          c->total_splats, static_cast<unsigned long long*>(c->scan_status.p),
                          &k->scan_tile_counter, c->scan_epoch, &k->entry_total, &k->ref_total,
@@ -673,8 +676,9 @@ int bin_refs(gs3d_ctx* c, const uint32_t* rect8) {
     CK(launch_emit_cells(dviews(c), nv, c->total_splats, proj, rect8, depth_sorted(c),
                          u32(c->sorted_offsets), &k->entry_total,
                          &k->ref_total, u32(c->ref_counter), c->capacity,
-                         static_cast<uint2*>(ka.p), u32(va), cp, &k->tile_hist[0][0],
-                         &k->emit_chunk, &k->error, c->sm_count, c->stream),
+                         static_cast<uint2*>(ka.p), u32(va), cp,
+                         tile_sort_status(cp, c->capacity, u32(c->sort_status)),
+                         &k->tile_hist[0][0], &k->emit_chunk, &k->error, c->sm_count, c->stream),
        "emit (cells, depth order)");
   }
   const uint2* entries = static_cast<uint2*>(c->keys_b.p);
@@ -692,8 +696,6 @@ int bin_refs(gs3d_ctx* c, const uint32_t* rect8) {
                         u32(c->cell_start), u32(c->chunk_cell), u32(c->chunk_counts),
                         u32(c->tile_counts), c->sm_count, c->stream),
        "tile counts");
-    CK(cudaMemsetAsync(c->tile_scan_status.p, 0, scan_status_words(c->total_tiles) * 8, c->stream),
-       "clear tile scan status");
     CK(launch_scan_tiles(u32(c->tile_counts), u32(c->tile_offsets), c->total_tiles, &k->ref_total,
                          static_cast<unsigned long long*>(c->tile_scan_status.p),
                          &k->tile_scan_counter, c->scan_epoch, &k->tile_scan_total, &k->error,
@@ -715,9 +717,6 @@ int sort_refs(gs3d_ctx* c, const uint32_t* rect8) {
   next_scan_epoch(c);
   {
     StageScope t(c, GS3D_STAGE_SCAN);
-    // cleared every rebin: a graph replay reuses the captured epoch
-    CK(cudaMemsetAsync(c->scan_status.p, 0, scan_status_words(c->total_splats) * 8, c->stream),
-       "clear scan status");
     const DepthSorted order = depth_sorted(c);
     CK(launch_scan(u32(c->counts), &order, u32(c->sorted_offsets), c->total_splats,
                    static_cast<unsigned long long*>(c->scan_status.p), &k->scan_tile_counter,
@@ -731,6 +730,7 @@ int sort_refs(gs3d_ctx* c, const uint32_t* rect8) {
                           static_cast<gs3d_projected_splat*>(c->proj.p), rect8, depth_sorted(c),
                           u32(c->sorted_offsets), u32(c->ref_counter), c->capacity,
                           static_cast<uint2*>(c->keys_a.p), u32(c->vals_a), tp,
+                          tile_sort_status(tp, c->capacity, u32(c->sort_status)),
                           &k->tile_hist[0][0], &k->emit_chunk, &k->error, c->sm_count,
                           c->stream),
        "emit (depth order)");
@@ -779,20 +779,28 @@ int fused_rebin(gs3d_ctx* c) {
                          &k->error, c->stream),
        "preprocess");
   }
+  const bool cells = use_cells(c);
+  // zeroed by the depth sort's first kernel: the scans' look-back status (every
+  // rebin: a graph replay reuses the captured epoch), the tile costs and, for
+  // the boundary writes of identify, the tile offsets
+  const ClearList clear{
+      {u32(c->scan_status), u32(c->tile_scan_status), u32(c->tile_costs), u32(c->tile_offsets)},
+      {scan_status_words(c->total_splats) * 2, cells ? scan_status_words(c->total_tiles) * 2 : 0,
+       c->total_tiles, cells ? 0 : (size_t)c->total_tiles + 1}};
   {
     StageScope t(c, GS3D_STAGE_DEPTH_SORT);
     CK(launch_sort_depth(&dviews(c)->batch_splats, c->total_splats, &k->depth_range,
                          u32(c->depth_keys_a), u32(c->depth_ids_a), u32(c->depth_keys_b),
                          u32(c->depth_ids_b), u32(c->depth_status), &k->depth_hist[0][0],
-                         &k->sort_part_counter[0], &k->error, c->sm_count, c->stream),
+                         &k->sort_part_counter[0], &k->error, clear, c->sm_count, c->stream),
        "depth sort");
   }
-  if (use_cells(c)) {
+  if (cells) {
     TRY(bin_refs(c, rect8));
   } else {
     TRY(sort_refs(c, rect8));
   }
-  return raster_stage(c);
+  return raster_stage(c, true);
 }
 
 void destroy_graph(gs3d_ctx* c) {
@@ -1265,6 +1273,9 @@ int gs3d_identify_tile_ranges(gs3d_ctx* c) {
   TRY(require_frame(c, "identify_tile_ranges"));
   TRY(set_device(c));
   StageScope t(c, GS3D_STAGE_IDENTIFY);
+  CK(cudaMemsetAsync(c->tile_offsets.p, 0, ((size_t)c->total_tiles + 1) * sizeof(uint32_t),
+                     c->stream),
+     "clear tile offsets");
   CK(launch_identify(static_cast<uint2*>(c->keys_a.p), u32(c->ref_counter), c->capacity,
                      c->total_tiles, u32(c->tile_offsets), &ctrl_of(c)->error, c->sm_count,
                      c->stream),
@@ -1276,7 +1287,7 @@ int gs3d_rasterize_tiles(gs3d_ctx* c) {
   if (!c) return GS3D_ERR_INVALID_ARG;
   TRY(require_frame(c, "rasterize_tiles"));
   TRY(set_device(c));
-  return raster_stage(c);
+  return raster_stage(c, false);
 }
 
 int gs3d_rebin(gs3d_ctx* c, const gs3d_camera* cam, uint32_t width, uint32_t height) {

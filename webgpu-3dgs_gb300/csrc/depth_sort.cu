@@ -77,12 +77,14 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t x, uint32_t* s_wsum
 }
 
 // Histograms of every digit place, and the clear of the passes' look-back
-// status.  Sixteen keys a thread a round, loaded before the first add.
+// status and of what later kernels of the frame want zeroed (a memset costs a
+// launch: the six of a frame were 12 us of a 20k-splat frame's 160).  Sixteen keys a thread a round, loaded before the first add.
 constexpr int kHistThreads = 256, kHistItems = 16;
 __global__ void __launch_bounds__(kHistThreads)
     depth_histogram_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ count,
                            const DepthRange* __restrict__ range, uint32_t* __restrict__ g_hist,
-                           uint32_t* __restrict__ status, size_t status_stride) {
+                           uint32_t* __restrict__ status, size_t status_stride,
+                           ClearList clear) {
   __shared__ uint32_t s_hist[kDepthPasses][kBins];
   for (int k = threadIdx.x; k < kDepthPasses * (int)kBins; k += kHistThreads)
     (&s_hist[0][0])[k] = 0u;
@@ -93,6 +95,9 @@ __global__ void __launch_bounds__(kHistThreads)
   const size_t words = (size_t)((n + kPart - 1) / kPart) * kBins;
   for (int p = 0; p < kDepthPasses; ++p)
     for (size_t k = gtid; k < words; k += gstride) status[p * status_stride + k] = 0u;
+#pragma unroll
+  for (int c = 0; c < ClearList::kMax; ++c)
+    for (size_t k = gtid; k < clear.words[c]; k += gstride) clear.p[c][k] = 0u;
   Digits d[kDepthPasses];
 #pragma unroll
   for (int p = 0; p < kDepthPasses; ++p) d[p] = digits_of(range, p);
@@ -338,8 +343,8 @@ size_t depth_sort_status_words(uint32_t n) { return status_stride(n) * kDepthPas
 cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const DepthRange* range,
                               uint32_t* keys_a, uint32_t* ids_a, uint32_t* keys_b,
                               uint32_t* ids_b, uint32_t* status, uint32_t* g_hist,
-                              uint32_t* part_counters, uint32_t* err, int sm_count,
-                              cudaStream_t s) {
+                              uint32_t* part_counters, uint32_t* err, const ClearList& clear,
+                              int sm_count, cudaStream_t s) {
   int per_sm = 0;
   cudaError_t e = pass_setup(&per_sm);
   if (e != cudaSuccess) return e;
@@ -347,7 +352,7 @@ cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const De
   const size_t parts = ((size_t)capacity + kPart - 1) / kPart;
   const size_t rounds = ((size_t)capacity + kHistThreads * kHistItems - 1) / (kHistThreads * kHistItems);
   depth_histogram_kernel<<<(unsigned)std::min<size_t>((size_t)sm_count * 8, std::max<size_t>(rounds, 1)),
-                           kHistThreads, 0, s>>>(keys_a, count, range, g_hist, status, stride);
+                           kHistThreads, 0, s>>>(keys_a, count, range, g_hist, status, stride, clear);
   const unsigned grid =
       (unsigned)std::min<size_t>((size_t)sm_count * per_sm, std::max<size_t>(parts, 1));
   for (int p = 0; p < kDepthPasses; ++p) {

@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(kThreads)
 struct CellArgs {
   const unsigned long long* ref_total;
   uint32_t* ref_counter;  // written: min(*ref_total, 2^32 - 1)
+  uint32_t* entry_total;  // zeroed where nothing is emitted
 };
 template <int TP, int BINS, bool CELLS>
 __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
                        const uint32_t* __restrict__ ref_counter, CellArgs cells,
                        uint32_t capacity, uint2* __restrict__ keys,
                        uint32_t* __restrict__ values, int4 shifts,
-                       uint4 masks, uint32_t* __restrict__ g_hist,
+                       uint4 masks, StatusClear sort_status, uint32_t* __restrict__ g_hist,
                        uint32_t* __restrict__ chunk_ticket, uint32_t* __restrict__ err) {
   __shared__ uint32_t s_off[kThreads + 1];
   // per splat, read as two 16-byte words by every ref it owns:
@@ -131,8 +132,22 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
   if (CELLS && blockIdx.x == 0 && threadIdx.x == 0)
     *cells.ref_counter = frame_refs > 0xffffffffull ? 0xffffffffu : (uint32_t)frame_refs;
   if (frame_refs > capacity) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) latch_error(err, DEVERR_CAPACITY);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      latch_error(err, DEVERR_CAPACITY);
+      if (CELLS) *cells.entry_total = 0u;
+    }
     return;
+  }
+  {  // look-back status of the digit passes over what is emitted here
+    const size_t parts = (total + sort_status.part - 1) / sort_status.part;
+    const size_t stride = (size_t)gridDim.x * kThreads;
+#pragma unroll
+    for (int p = 0; p < TP; ++p) {
+      uint32_t* st = sort_status.status + sort_status.stride[p];
+      const size_t words = parts * sort_status.bins[p];
+      for (size_t k = (size_t)blockIdx.x * kThreads + threadIdx.x; k < words; k += stride)
+        st[k] = 0u;
+    }
   }
   const uint32_t* __restrict__ sorted_keys = sorted.keys();
   const uint32_t* __restrict__ sorted_ids = sorted.ids();
@@ -329,7 +344,7 @@ cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
                          const DepthSorted& sorted, const uint32_t* sorted_offsets,
                          const uint32_t* counter, CellArgs cells,
                          uint32_t capacity, uint2* keys, uint32_t* values, const SortPlan& plan,
-                         uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
+                         const StatusClear& sort_status, uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                          cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const uint32_t chunks = (n + kThreads - 1) / kThreads;
@@ -349,7 +364,7 @@ cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
     emit_sorted_kernel<TP, BINS, CELLS>                                                       \
         <<<std::min(chunks, sms * emit_blocks_per_sm<TP, BINS, CELLS>()), kThreads, 0, s>>>(  \
             views, n_views, n, proj, rect8, sorted, sorted_offsets, counter, cells,           \
-            capacity, keys, values, sh, mk, g_hist, chunk_ticket, err);                \
+            capacity, keys, values, sh, mk, sort_status, g_hist, chunk_ticket, err);   \
     break;
   if (wide) {
     switch (plan.passes) {
@@ -381,26 +396,25 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
                                const DepthSorted& sorted,
                                const uint32_t* sorted_offsets, const uint32_t* ref_counter,
                                uint32_t capacity, uint2* keys, uint32_t* values,
-                               const SortPlan& tile_plan, uint32_t* g_hist,
-                               uint32_t* chunk_ticket, uint32_t* err, int sm_count,
+                               const SortPlan& tile_plan, const StatusClear& sort_status,
+                               uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                                cudaStream_t s) {
   return emit_ordered<false>(views, n_views, n, proj, rect8, sorted, sorted_offsets,
                              ref_counter, CellArgs{}, capacity, keys, values,
-                             tile_plan, g_hist, chunk_ticket, err, sm_count, s);
+                             tile_plan, sort_status, g_hist, chunk_ticket, err, sm_count, s);
 }
 
 cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t n,
                               const gs3d_projected_splat* proj, const uint32_t* rect8,
                               const DepthSorted& sorted, const uint32_t* sorted_offsets,
-                              const uint32_t* entry_total,
-                              const unsigned long long* ref_total, uint32_t* ref_counter,
+                              uint32_t* entry_total, const unsigned long long* ref_total, uint32_t* ref_counter,
                               uint32_t capacity, uint2* keys, uint32_t* values,
-                              const SortPlan& cell_plan, uint32_t* g_hist, uint32_t* chunk_ticket,
-                              uint32_t* err, int sm_count, cudaStream_t s) {
+                              const SortPlan& cell_plan, const StatusClear& sort_status,
+                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count, cudaStream_t s) {
   return emit_ordered<true>(views, n_views, n, proj, rect8, sorted, sorted_offsets, entry_total,
-                            CellArgs{ref_total, ref_counter},
-                            capacity, keys, values, cell_plan, g_hist, chunk_ticket, err,
-                            sm_count, s);
+                            CellArgs{ref_total, ref_counter, entry_total},
+                            capacity, keys, values, cell_plan, sort_status, g_hist, chunk_ticket,
+                            err, sm_count, s);
 }
 
 cudaError_t launch_emit(const FrameUniforms* d_frame, uint32_t n,

@@ -377,7 +377,15 @@ size_t sort_status_words_max(uint32_t capacity);
 // (entries past the live count are read and ignored).
 uint32_t sort_capacity_round(uint32_t capacity);
 // Tile-id passes of the fused rebin: histograms already in
-// g_hist[p * kTileHistStride + digit].
+// g_hist[p * kTileHistStride + digit], the status words that the passes of a
+// count use (tile_sort_status) cleared.
+struct StatusClear {
+  uint32_t* status;
+  size_t stride[kMaxTilePasses];  // first word of each pass
+  uint32_t bins[kMaxTilePasses];  // words per partition of `part` keys
+  uint32_t passes, part;
+};
+StatusClear tile_sort_status(const SortPlan& plan, uint32_t capacity, uint32_t* status);
 cudaError_t launch_sort_tile_passes(const SortPlan& plan, const uint32_t* ref_counter,
                                     uint32_t capacity, uint2* keys_a, uint32_t* vals_a,
                                     uint2* keys_b, uint32_t* vals_b, uint32_t* status,
@@ -394,11 +402,17 @@ cudaError_t launch_sort_u32(const SortPlan& plan, const uint32_t* count, uint32_
 // depth_sort_capacity(capacity) entries; g_hist[4][512] zeroed.
 size_t depth_sort_capacity(uint32_t n);
 size_t depth_sort_status_words(uint32_t n);
+// clear: arrays of words that are zeroed on the way.
+struct ClearList {
+  static constexpr int kMax = 4;
+  uint32_t* p[kMax];
+  size_t words[kMax];
+};
 cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const DepthRange* range,
                               uint32_t* keys_a, uint32_t* ids_a, uint32_t* keys_b,
                               uint32_t* ids_b, uint32_t* status, uint32_t* g_hist,
-                              uint32_t* part_counters, uint32_t* err, int sm_count,
-                              cudaStream_t s);
+                              uint32_t* part_counters, uint32_t* err, const ClearList& clear,
+                              int sm_count, cudaStream_t s);
 // Raster work order: tile indices sorted by decreasing expected cost
 // (schedule = GS3D_SCHEDULE_KEY_COUNT: the tile's key count), so the
 // persistent raster CTAs start the longest tiles first.
@@ -455,7 +469,8 @@ cudaError_t launch_gate_update(const float* pred, const uint32_t* costs, uint32_
 cudaError_t launch_log_costs(const uint32_t* costs, uint32_t n, float* out, cudaStream_t s);
 
 // Emit in depth-sorted order over all splat-views of a batch (global tile
-// ids, global splat-view values) + histograms of the tile-id digit places.
+// ids, global splat-view values) + histograms of the tile-id digit places, and
+// the clear of the status words their passes will use.
 // rect8: the preprocess's one-word tile rectangles (null: read the
 // rectangles from the projected records).
 cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t total,
@@ -463,19 +478,19 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
                                const DepthSorted& sorted,
                                const uint32_t* sorted_offsets, const uint32_t* ref_counter,
                                uint32_t capacity, uint2* keys, uint32_t* values,
-                               const SortPlan& tile_plan, uint32_t* g_hist,
-                               uint32_t* chunk_ticket, uint32_t* err, int sm_count,
+                               const SortPlan& tile_plan, const StatusClear& sort_status,
+                               uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                                cudaStream_t s);
 // The same for cell entries: one per (splat-view, cell), keys [cell and
 // rectangle inside it | depth], and *ref_counter = the frame's refs.
 cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t total,
                               const gs3d_projected_splat* proj, const uint32_t* rect8,
                               const DepthSorted& sorted, const uint32_t* sorted_offsets,
-                              const uint32_t* entry_total,
-                              const unsigned long long* ref_total, uint32_t* ref_counter,
+                              uint32_t* entry_total, const unsigned long long* ref_total, uint32_t* ref_counter,
                               uint32_t capacity, uint2* keys, uint32_t* values,
-                              const SortPlan& cell_plan, uint32_t* g_hist, uint32_t* chunk_ticket,
-                              uint32_t* err, int sm_count, cudaStream_t s);
+                              const SortPlan& cell_plan, const StatusClear& sort_status,
+                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count, cudaStream_t s);
+// tile_offsets zeroed by the caller.
 cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint32_t capacity,
                             uint32_t num_tiles, uint32_t* tile_offsets, uint32_t* err,
                             int sm_count, cudaStream_t s);
@@ -492,7 +507,7 @@ struct RasterArgs {
   const uint32_t* tile_offsets;
   const uint32_t* values;
   uint2* image;
-  uint32_t* tile_costs;   // may be null
+  uint32_t* tile_costs;   // zeroed; may be null
   const uint32_t* order;  // may be null
   unsigned long long* queue_counter;
   void* pool;             // raster_pool_bytes(), zeroed once: blocks handed on between warps

@@ -74,9 +74,6 @@ __global__ void __launch_bounds__(kThreads)
 cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint32_t capacity,
                             uint32_t num_tiles, uint32_t* tile_offsets, uint32_t* err,
                             int sm_count, cudaStream_t s) {
-  cudaError_t e =
-      cudaMemsetAsync(tile_offsets, 0, ((size_t)num_tiles + 1) * sizeof(uint32_t), s);
-  if (e != cudaSuccess) return e;
   identify_kernel<<<sm_count * 8, kThreads, 0, s>>>(keys, ref_counter, capacity, num_tiles,
                                                     tile_offsets, err);
   return cudaGetLastError();

@@ -1260,11 +1260,6 @@ cudaError_t launch_raster(const RasterArgs& args, int sm_count, cudaStream_t s) 
   RasterConfig cfg;
   cudaError_t e = raster_config(a, &cfg);
   if (e != cudaSuccess) return e;
-  // every work item folds its cost into its tile's by maximum
-  if (a.tile_costs != nullptr) {
-    e = cudaMemsetAsync(a.tile_costs, 0, (size_t)a.num_tiles * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-  }
   const uint32_t ctas = (uint32_t)sm_count * (uint32_t)cfg.per_sm;
   uint64_t max_ctas = a.num_tiles;
   if (cfg.mode == 2) {

@@ -856,11 +856,9 @@ cudaError_t run_passes(const SortPlan& plan, const uint32_t* ref_counter, uint32
     pd.shift[p] = plan.shift[p];
     pd.mask[p] = digit_mask(plan.nbits[p]);
   }
-  if (!hist_ready) {
+  if (!hist_ready) {  // else the caller has cleared the status too
     e = launch_histogram<K>(plan.passes, pd, keys_a, ref_counter, capacity, g_hist, status,
                             stride, sm_count * 4, s);
-  } else {
-    e = cudaMemsetAsync(status, 0, status_off[plan.passes] * sizeof(uint32_t), s);
   }
   if (e != cudaSuccess) return e;
   for (int p = 0; p < plan.passes; ++p) {
@@ -917,6 +915,22 @@ size_t sort_status_words_max(uint32_t capacity) {
   // the larger of 8 passes of 256 bins and 4 tile passes, 3 of them 2048-bin
   const size_t parts = ((size_t)capacity + kPart - 1) / kPart + 1;
   return parts * std::max<size_t>(kMaxSortPasses * kRadixBins, 3 * kWideBins + kRadixBins);
+}
+
+StatusClear tile_sort_status(const SortPlan& plan, uint32_t capacity, uint32_t* status) {
+  // as run_passes lays them out
+  const size_t parts_cap = ((size_t)capacity + kPart - 1) / kPart + 1;
+  StatusClear c{};
+  c.status = status;
+  c.passes = (uint32_t)plan.passes;
+  c.part = kPart;
+  size_t off = 0;
+  for (int p = 0; p < plan.passes && p < kMaxTilePasses; ++p) {
+    c.bins[p] = plan.nbits[p] == kWideBits ? kWideBins : (uint32_t)kRadixBins;
+    c.stride[p] = off;
+    off += parts_cap * c.bins[p];
+  }
+  return c;
 }
 
 cudaError_t launch_sort(const SortPlan& plan, const uint32_t* ref_counter, uint32_t capacity,
