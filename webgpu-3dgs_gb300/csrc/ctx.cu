@@ -576,18 +576,26 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
                           static_cast<float*>(c->tile_feats.p), c->total_tiles,
                           static_cast<float*>(c->tile_preds.p), c->stream),
          "cost MLP inference");
-      CK(launch_learned_keys(static_cast<float*>(c->tile_preds.p), c->total_tiles,
-                             static_cast<SchedGate*>(c->gate.p), u32(c->tile_offsets),
-                             u32(c->sched_keys_a), u32(c->sched_order_a),
-                             static_cast<float*>(c->tile_est.p), c->stream),
-         "learned schedule keys");
     }
-    CK(launch_schedule(c->schedule, u32(c->tile_offsets), c->total_tiles,
-                       &dviews(c)->batch_tiles, u32(c->sched_keys_a), u32(c->sched_order_a),
-                       u32(c->sched_keys_b), u32(c->sched_order_b),
-                       static_cast<float*>(c->tile_est.p), u32(c->sched_status), ctrl_of(c),
-                       raster_ctas, strips, split_all, c->sm_count, c->stream),
-       "raster schedule");
+    if (c->total_tiles <= kOrderTiles) {
+      CK(launch_order(c->schedule, u32(c->tile_offsets), static_cast<float*>(c->tile_preds.p),
+                      static_cast<SchedGate*>(c->gate.p), c->total_tiles, raster_ctas, strips,
+                      split_all, u32(c->sched_order_a), &ctrl_of(c)->raster_heavy, c->stream),
+         "raster schedule");
+    } else {
+      if (learned)
+        CK(launch_learned_keys(static_cast<float*>(c->tile_preds.p), c->total_tiles,
+                               static_cast<SchedGate*>(c->gate.p), u32(c->tile_offsets),
+                               u32(c->sched_keys_a), u32(c->sched_order_a),
+                               static_cast<float*>(c->tile_est.p), c->stream),
+           "learned schedule keys");
+      CK(launch_schedule(c->schedule, u32(c->tile_offsets), c->total_tiles,
+                         &dviews(c)->batch_tiles, u32(c->sched_keys_a), u32(c->sched_order_a),
+                         u32(c->sched_keys_b), u32(c->sched_order_b),
+                         static_cast<float*>(c->tile_est.p), u32(c->sched_status), ctrl_of(c),
+                         raster_ctas, strips, split_all, c->sm_count, c->stream),
+         "raster schedule");
+    }
     order = u32(c->sched_order_a);
     heavy = &ctrl_of(c)->raster_heavy;
   } else if (split_all) {  // row-major order, every tile split

@@ -440,6 +440,15 @@ cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t raster_cta
                                uint32_t strips, float floor, bool all, uint32_t* heavy,
                                cudaStream_t s);
 
+// The same order (by buckets of 1/32 octave) and split in one block, for at most
+// kOrderTiles tiles: 8,160 tiles 50 -> 9 us, launches included; its time grows
+// with the tiles, the radix sort's hardly.
+constexpr uint32_t kOrderTiles = 65536;
+cudaError_t launch_order(uint32_t schedule, const uint32_t* tile_offsets, const float* pred,
+                         const SchedGate* gate, uint32_t num_tiles, uint32_t workers,
+                         uint32_t items_per_tile, bool split_all, uint32_t* order,
+                         uint32_t* heavy, cudaStream_t s);
+
 // ---- learned schedule (learned.cu) ----
 constexpr int kFeatures = 16;
 constexpr int kHidden = 64;

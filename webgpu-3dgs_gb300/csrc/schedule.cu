@@ -9,7 +9,8 @@
 //
 // Key-count schedule: expected cost = the tile's key count (the plain
 // schedule the learned one falls back to).  Learned schedule: expected cost
-// = the cost MLP's prediction (learned.cu); both sort 16-bit keys.
+// = the cost MLP's prediction (learned.cu).  Up to kOrderTiles tiles are
+// ordered by one block (order_kernel), more by a radix sort of 16-bit keys.
 //
 // Both also split: the tiles whose expected cost per work item exceeds half of
 // a raster worker's fair share of the frame (the head of the order) are shaded
@@ -76,7 +77,101 @@ __global__ void __launch_bounds__(kHeavyThreads)
   }
 }
 
+// The whole order in one block, for up to kOrderTiles tiles: buckets of 1/32
+// octave of the expected cost, largest first (any order inside a bucket: the
+// queue needs long tiles early, not an exact sort), and the tiles to split.
+// Costs are walked three times (sum; bucket and heavy counts; placement)
+// instead of six launches for keys, heavy count, histogram and two digit
+// passes.
+constexpr int kOrderThreads = 1024;
+constexpr uint32_t kBuckets = 1024;  // 32 octaves
+__device__ __forceinline__ uint32_t cost_bucket(float est) {
+  // bits of 1 + est in [1, 2^32]: exponent and five bits of mantissa
+  const uint32_t b = (__float_as_uint(fminf(fmaxf(est, 0.0f), 4.29e9f) + 1.0f) >> 18) - (127u << 5);
+  return kBuckets - 1u - min(b, kBuckets - 1u);
+}
+template <bool LEARNED>
+__global__ void __launch_bounds__(kOrderThreads)
+    order_kernel(const uint32_t* __restrict__ tile_offsets, const float* __restrict__ pred,
+                 const SchedGate* __restrict__ gate, uint32_t n, uint32_t workers,
+                 uint32_t items_per_tile, float floor_keys, float floor_cost, uint32_t split_all,
+                 uint32_t* __restrict__ order, uint32_t* __restrict__ heavy) {
+  __shared__ uint32_t s_bucket[kBuckets];
+  __shared__ float s_sum[kOrderThreads / 32];
+  __shared__ uint32_t s_warp[kOrderThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool learned = LEARNED && gate->use_learned != 0u;
+  auto cost = [&](uint32_t t) -> float {
+    if (learned) return expm1f(fminf(fmaxf(__ldg(pred + t), 0.0f), 15.99f));
+    const uint32_t lo = __ldg(tile_offsets + t), hi = __ldg(tile_offsets + t + 1);
+    return hi > lo ? (float)(hi - lo) : 0.0f;
+  };
+  s_bucket[tid] = 0u;
+  __syncthreads();
+  float sum = 0.0f;
+  for (uint32_t t = tid; t < n; t += kOrderThreads) {
+    const float c = cost(t);
+    sum += c;
+    atomicAdd(&s_bucket[cost_bucket(c)], 1u);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (lane == 0) s_sum[warp] = sum;
+  __syncthreads();
+  float total = 0.0f;
+  for (int w = 0; w < kOrderThreads / 32; ++w) total += s_sum[w];
+  // a work item costs about the tile's cost; the frame about total * items
+  const float thr = fmaxf(0.5f * total * (float)items_per_tile / (float)max(workers, 1u),
+                          learned ? floor_cost : floor_keys);
+  // bucket starts (a bucket a thread)
+  {
+    const uint32_t c = s_bucket[tid];
+    uint32_t inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    s_bucket[tid] = before + inc - c;
+  }
+  __syncthreads();
+  uint32_t over = 0;
+  for (uint32_t t = tid; t < n; t += kOrderThreads) {
+    const float c = cost(t);
+    order[atomicAdd(&s_bucket[cost_bucket(c)], 1u)] = t;
+    over += c > thr ? 1u : 0u;
+  }
+  over = __reduce_add_sync(0xffffffffu, over);
+  __syncthreads();  // s_warp is rewritten
+  if (lane == 0) s_warp[warp] = over;
+  __syncthreads();
+  if (tid == 0) {
+    uint32_t c = 0;
+    for (int w = 0; w < kOrderThreads / 32; ++w) c += s_warp[w];
+    *heavy = split_all ? n : c;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_order(uint32_t schedule, const uint32_t* tile_offsets, const float* pred,
+                         const SchedGate* gate, uint32_t num_tiles, uint32_t workers,
+                         uint32_t items_per_tile, bool split_all, uint32_t* order,
+                         uint32_t* heavy, cudaStream_t s) {
+  if (schedule == GS3D_SCHEDULE_LEARNED)
+    order_kernel<true><<<1, kOrderThreads, 0, s>>>(
+        tile_offsets, pred, gate, num_tiles, workers, items_per_tile, (float)kHeavyKeys,
+        (float)kHeavyCost, split_all ? 1u : 0u, order, heavy);
+  else
+    order_kernel<false><<<1, kOrderThreads, 0, s>>>(
+        tile_offsets, nullptr, nullptr, num_tiles, workers, items_per_tile, (float)kHeavyKeys,
+        (float)kHeavyCost, split_all ? 1u : 0u, order, heavy);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t raster_ctas,
                                uint32_t strips, float floor, bool all, uint32_t* heavy,
