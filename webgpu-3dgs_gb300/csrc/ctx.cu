@@ -65,6 +65,7 @@ struct gs3d_ctx {
   // writer of the target) waits for the last one (copy_done)
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t frame_done = nullptr, copy_done = nullptr;
+  bool copies_pending = false;  // copy_stream has work that no wait has covered
   int sm_count = 0;
   std::string err = "no error";
 
@@ -248,10 +249,19 @@ int set_device(gs3d_ctx* c) {
   return GS3D_OK;
 }
 
-// Reads the latched device error word (stream must be idle) and clears it.
-int check_device_errors(gs3d_ctx* c) {
-  CK(cudaMemcpy(c->h_word, &ctrl_of(c)->error, sizeof(uint32_t), cudaMemcpyDeviceToHost),
+// Waits for the stream and the copy-outs under way, then reports and clears the
+// latched device errors.  The error word comes back in stream order, so a frame
+// is waited for once (a blocking read after the wait cost another round trip,
+// 9 us).
+int sync_and_check(gs3d_ctx* c) {
+  CK(cudaMemcpyAsync(c->h_word, &ctrl_of(c)->error, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                     c->stream),
      "read error word");
+  CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+  if (c->copies_pending) {
+    CK(cudaStreamSynchronize(c->copy_stream), "copy-out stream");
+    c->copies_pending = false;
+  }
   const uint32_t e = c->h_word[0];
   if (e == 0) return GS3D_OK;
   CK(cudaMemset(&ctrl_of(c)->error, 0, sizeof(uint32_t)), "clear error word");
@@ -314,12 +324,6 @@ struct StageScope {
     c->pending.push_back({stage, a, b});
   }
 };
-
-int sync_and_check(gs3d_ctx* c) {
-  CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-  if (c->copy_stream) CK(cudaStreamSynchronize(c->copy_stream), "copy-out stream");
-  return check_device_errors(c);
-}
 
 int upload_scene(gs3d_ctx* c, SceneBufs& sc, uint32_t n, const float* positions,
                  const float* scales, const float* rotations, const float* colors,
@@ -1717,6 +1721,7 @@ int gs3d_copy_buffer_async(gs3d_ctx* c, gs3d_buffer which, void* dst, size_t byt
     // off the rebin stream: the next rebin runs while this frame copies out
     CK(cudaEventRecord(c->frame_done, c->stream), "frame event");
     CK(cudaStreamWaitEvent(c->copy_stream, c->frame_done, 0), "copy waits for the frame");
+    c->copies_pending = true;
     CK(cudaMemcpyAsync(dst, b->p, bytes, cudaMemcpyDeviceToHost, c->copy_stream),
        "async copy-out");
     CK(cudaEventRecord(c->copy_done, c->copy_stream), "copy event");
