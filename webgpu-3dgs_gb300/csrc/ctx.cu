@@ -110,7 +110,8 @@ struct gs3d_ctx {
   cudaEvent_t upload_ev[kUploadSlots] = {};
   int upload_slot = 0;
 
-  DevBuf ctrl;
+  DevBuf ctrl, ply_words;
+  bool reads_host = false;     // kernels may read pageable host memory (host page tables)
   uint32_t* h_word = nullptr;  // pinned scratch for small reads
   uint64_t alloc_gen = 0;      // bumped by every device (re)allocation
 
@@ -934,6 +935,7 @@ int gs3d_create(gs3d_ctx** out, const gs3d_config* cfg) {
     return bail(GS3D_ERR_NO_DEVICE);
   }
   c->sm_count = prop.multiProcessorCount;
+  c->reads_host = prop.pageableMemoryAccess && prop.pageableMemoryAccessUsesHostPageTables;
   if (cfg->stream) {
     c->stream = static_cast<cudaStream_t>(cfg->stream);
   } else {
@@ -984,7 +986,7 @@ int gs3d_destroy(gs3d_ctx* c) {
                     &c->sched_keys_b,  &c->sched_order_a, &c->sched_order_b, &c->sched_status,
                     &c->d_views,       &c->ctrl,          &c->model_params,  &c->model_mean,
                     &c->model_inv_std, &c->tile_feats,    &c->tile_preds,    &c->composite_out,
-                    &c->tile_est,      &c->gate,          &c->raster_pool};
+                    &c->tile_est,      &c->gate,          &c->raster_pool,   &c->ply_words};
   for (DevBuf* b : bufs) release(*b);
   for (int i = 0; i < kUploadSlots; ++i)
     if (c->upload_ev[i]) cudaEventDestroy(c->upload_ev[i]);
@@ -1101,10 +1103,9 @@ int gs3d_load_ply(gs3d_ctx* c, const void* data, size_t size, uint32_t target,
   SceneBufs fresh;
   SceneBufs& sc = target == 0 ? c->scenes[0] : fresh;
   const size_t v4 = (size_t)n * 16;
-  DevBuf d_rows, d_words;
+  DevBuf d_rows;
   auto cleanup = [&](int rc) {
     release(d_rows);
-    release(d_words);
     if (&sc == &fresh) {
       release(fresh.pos);
       release(fresh.scale);
@@ -1118,29 +1119,32 @@ int gs3d_load_ply(gs3d_ctx* c, const void* data, size_t size, uint32_t target,
   if ((rc = ensure(c, sc.pos, v4, "splat_positions")) || (rc = ensure(c, sc.scale, v4, "splat_scales")) ||
       (rc = ensure(c, sc.rot, v4, "splat_rotations")) || (rc = ensure(c, sc.color, v4, "splat_colors")) ||
       (lay.sh_k && (rc = ensure(c, sc.sh, (size_t)n * 3 * lay.sh_k * sizeof(float), "splat_sh_rest"))) ||
-      (rc = ensure(c, d_rows, std::max<size_t>((size_t)n * lay.stride, 16), "ply rows")) ||
-      (rc = ensure(c, d_words, 64, "ply status")))
+      // where the device walks the host's page tables the decode reads the rows
+      // in place: 300k rows of 248 bytes 826 -> 483 us (a buffer for them 155 us
+      // to allocate and free, its copy 430, the decode after it 150; the link
+      // alone is 377)
+      (!c->reads_host && (rc = ensure(c, d_rows, std::max<size_t>((size_t)n * lay.stride, 16), "ply rows"))) ||
+      (rc = ensure(c, c->ply_words, 64, "ply status")))
     return cleanup(rc);
   uint32_t words[7] = {0u, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-  cudaError_t e = cudaMemcpyAsync(d_words.p, words, sizeof(words), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess && n)
+  cudaError_t e = cudaMemcpyAsync(c->ply_words.p, words, sizeof(words), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess && n && !c->reads_host)
     e = cudaMemcpyAsync(d_rows.p, rows, (size_t)n * lay.stride, cudaMemcpyHostToDevice, c->stream);
-  uint32_t* dw = static_cast<uint32_t*>(d_words.p);
+  uint32_t* dw = u32(c->ply_words);
   if (e == cudaSuccess)
-    e = launch_ply_decode(static_cast<const uint8_t*>(d_rows.p), n, lay,
+    e = launch_ply_decode(c->reads_host ? rows : static_cast<const uint8_t*>(d_rows.p), n, lay,
                           lay.format == GS3D_PLY_BINARY_BE, static_cast<float4*>(sc.pos.p),
                           static_cast<float4*>(sc.scale.p), static_cast<float4*>(sc.rot.p),
                           static_cast<float4*>(sc.color.p), static_cast<float*>(sc.sh.p), dw,
                           dw + 1, c->stream);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(words, d_words.p, sizeof(words), cudaMemcpyDeviceToHost, c->stream);
+    e = cudaMemcpyAsync(words, c->ply_words.p, sizeof(words), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cleanup(cuda_fail(c, e, "ply decode"));
   if (words[0] != 0)
     return cleanup(fail(c, GS3D_ERR_INVALID_ARG, "Invalid Gaussian Splat PLY row: missing '%s'",
                         ply_required_name((int)words[0] - 1)));
   release(d_rows);
-  release(d_words);
   sc.n = n;
   sc.sh_degree = deg;
   if (&sc == &fresh) {

@@ -386,6 +386,7 @@ struct DecodeArgs {
   const uint8_t* rows;
   uint64_t n;
   uint32_t stride, big, sh_k;  // sh_k: coefficients per channel
+  uint32_t tile_rows;          // rows staged at a time, 0: too wide to stage
   PlyField req[kPlyRequired];
   PlyField rest[kPlyMaxRest];
   float4 *pos, *scale, *rot, *color;
@@ -394,12 +395,40 @@ struct DecodeArgs {
   uint32_t* bounds;
 };
 
-__global__ void __launch_bounds__(256) ply_decode_kernel(DecodeArgs a) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = i < a.n;
+// A block takes kDecodeThreads rows at most, a thread a row.  The rows' bytes
+// are staged in shared memory by 16-byte copies first (they may lie in host
+// memory, behind the link: 300k rows of 248 bytes are read in 0.38 ms there,
+// and several blocks per SM keep it busy while others are at the f64
+// activations), and the SH block is written with unit stride.
+constexpr int kDecodeThreads = 128;
+constexpr uint32_t kDecodeBytes = 40 * 1024;  // staged rows, with their ragged ends
+__global__ void __launch_bounds__(kDecodeThreads) ply_decode_kernel(DecodeArgs a) {
+  extern __shared__ __align__(16) uint8_t s_rows[];
+  __shared__ PlyField s_rest[kPlyMaxRest];
+  const uint32_t tile = a.tile_rows ? a.tile_rows : kDecodeThreads;
+  const uint64_t first = (uint64_t)blockIdx.x * tile;
+  const uint32_t count = (uint32_t)(a.n - first < tile ? a.n - first : tile);
+  const uint8_t* base = a.rows + first * a.stride;
+  if (a.tile_rows) {
+    // whole 16-byte words: the first and the last also hold bytes beside the
+    // rows, of the same page
+    const uint32_t lead = (uint32_t)((uintptr_t)base & 15u);
+    const uint32_t words = (lead + count * a.stride + 15u) / 16u;
+    const uint4* src = reinterpret_cast<const uint4*>(base - lead);
+    for (uint32_t k = threadIdx.x; k < words; k += kDecodeThreads)
+      cp_async16(s_rows + 16 * k, src + k);
+    cp_async_commit();
+    base = s_rows + lead;
+  }
+  const uint32_t kc = 3 * a.sh_k;
+  if (threadIdx.x < kc) s_rest[threadIdx.x] = a.rest[threadIdx.x];
+  cp_async_wait<0>();
+  __syncthreads();
+  const bool live = threadIdx.x < count;
+  const uint64_t i = first + threadIdx.x;
   float px = 0.f, py = 0.f, pz = 0.f;
   if (live) {
-    const uint8_t* row = a.rows + i * a.stride;
+    const uint8_t* row = base + (size_t)threadIdx.x * a.stride;
     double v[kPlyRequired];
 #pragma unroll
     for (int k = 0; k < kPlyRequired; ++k) {
@@ -420,13 +449,13 @@ __global__ void __launch_bounds__(256) ply_decode_kernel(DecodeArgs a) {
     const double inv = len > 0.0 ? 1.0 / len : 1.0;
     a.rot[i] = make_float4((float)(v[7] * inv), (float)(v[8] * inv), (float)(v[9] * inv),
                            (float)(v[10] * inv));
-    if (a.sh_k) {
-      float* dst = a.sh + i * 3 * a.sh_k;
-      for (uint32_t c = 0; c < 3; ++c)
-        for (uint32_t k = 0; k < a.sh_k; ++k) {
-          const PlyField f = a.rest[c * a.sh_k + k];
-          dst[c * a.sh_k + k] = (float)read_scalar(row + f.offset, f.type, a.big);
-        }
+  }
+  if (kc) {
+    float* dst = a.sh + first * kc;
+    for (uint32_t e = threadIdx.x; e < count * kc; e += kDecodeThreads) {
+      const uint32_t r = e / kc;
+      const PlyField f = s_rest[e - r * kc];
+      dst[e] = (float)read_scalar(base + (size_t)r * a.stride + f.offset, f.type, a.big);
     }
   }
   // position bounds: warp reduction, one atomic per warp and word
@@ -434,12 +463,10 @@ __global__ void __launch_bounds__(256) ply_decode_kernel(DecodeArgs a) {
                     live ? f2ord(pz) : 0xffffffffu};
   uint32_t hi[3] = {live ? f2ord(px) : 0u, live ? f2ord(py) : 0u, live ? f2ord(pz) : 0u};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      lo[c] = min(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-      hi[c] = max(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
-    }
+  for (int c = 0; c < 3; ++c) {
+    lo[c] = __reduce_min_sync(0xffffffffu, lo[c]);
+    hi[c] = __reduce_max_sync(0xffffffffu, hi[c]);
+  }
   if ((threadIdx.x & 31) == 0)
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -470,8 +497,13 @@ cudaError_t launch_ply_decode(const uint8_t* rows, uint64_t n, const PlyLayout& 
   a.sh = sh;
   a.bad = bad;
   a.bounds = bounds;
-  const uint64_t blocks = (n + 255) / 256;
-  ply_decode_kernel<<<(unsigned)blocks, 256, 0, s>>>(a);
+  // two ragged ends of at most 15 bytes
+  a.tile_rows = lay.stride ? std::min<uint32_t>((kDecodeBytes - 32u) / lay.stride, kDecodeThreads)
+                           : kDecodeThreads;
+  const uint32_t tile = a.tile_rows ? a.tile_rows : kDecodeThreads;
+  const size_t smem = a.tile_rows ? ((size_t)tile * lay.stride + 32 + 15) / 16 * 16 : 0;
+  const uint64_t blocks = (n + tile - 1) / tile;
+  ply_decode_kernel<<<(unsigned)blocks, kDecodeThreads, smem, s>>>(a);
   return cudaGetLastError();
 }
 
