@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(kThreads)
                       const unsigned long long* __restrict__ ref_total, uint32_t capacity,
                       uint32_t num_cells, uint32_t* __restrict__ cell_start,
                       uint32_t* __restrict__ chunk_cell) {
+  after_predecessor(entries, entry_total, ref_total);
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t m = (blockIdx.x * kThreads + threadIdx.x) >> 5;
   if (m >= num_cells) return;
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kThreads)
                        const uint32_t* __restrict__ chunk_cell, uint32_t num_cells,
                        uint32_t* __restrict__ counts) {
   __shared__ uint32_t s_cnt[2][kCellTiles];
+  after_predecessor(entries, cell_start, chunk_cell);
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t slots = chunk_slot(__ldg(cell_start + num_cells), num_cells);
   if (threadIdx.x < 2 * kCellTiles) (&s_cnt[0][0])[threadIdx.x] = 0u;
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(kScanThreads)
                       const uint32_t* __restrict__ cell_start, uint32_t* __restrict__ counts,
                       uint32_t* __restrict__ tile_counts) {
   __shared__ uint32_t s_sum[kSegments][kCellTiles];
+  after_predecessor(views, cell_start);
   const uint32_t m = blockIdx.x, t = threadIdx.x % kCellTiles, seg = threadIdx.x / kCellTiles;
   const uint32_t a = __ldg(cell_start + m), b = __ldg(cell_start + m + 1);
   const uint32_t chunks = (b - a + kChunkEntries - 1) / kChunkEntries;
@@ -212,6 +215,7 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ uint32_t s_cnt[kWarps][kCellTiles];  // counts, then exclusive positions
   __shared__ uint2 s_tile[kCellTiles];  // destination - position in the chunk, global tile
   __shared__ uint32_t s_half, s_total, s_next;
+  after_predecessor(cell_start, ref_total);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t slots = chunk_slot(__ldg(cell_start + num_cells), num_cells);
   const unsigned long long total = *ref_total;
@@ -319,13 +323,13 @@ cudaError_t launch_bin_count(const ViewDesc* views, uint32_t n_views, uint32_t n
                              const uint2* entries, const uint32_t* entry_total,
                              const unsigned long long* ref_total, uint32_t capacity,
                              uint32_t* cell_start, uint32_t* chunk_cell, uint32_t* chunk_counts,
-                             uint32_t* tile_counts, int sm_count, cudaStream_t s) {
-  cell_table_kernel<<<(num_cells + kWarps - 1) / kWarps, kThreads, 0, s>>>(
-      entries, entry_total, ref_total, capacity, num_cells, cell_start, chunk_cell);
-  chunk_count_kernel<<<sm_count * 8, kThreads, 0, s>>>(entries, cell_start, chunk_cell, num_cells,
-                                                       chunk_counts);
-  chunk_scan_kernel<<<num_cells, kScanThreads, 0, s>>>(views, n_views, cell_start, chunk_counts,
-                                                       tile_counts);
+                             uint32_t* tile_counts, int sm_count, LaunchStream s) {
+  launch_after(cell_table_kernel, (num_cells + kWarps - 1) / kWarps, kThreads, 0, s, entries,
+               entry_total, ref_total, capacity, num_cells, cell_start, chunk_cell);
+  launch_after(chunk_count_kernel, sm_count * 8, kThreads, 0, s, entries, cell_start, chunk_cell,
+               num_cells, chunk_counts);
+  launch_after(chunk_scan_kernel, num_cells, kScanThreads, 0, s, views, n_views, cell_start,
+               chunk_counts, tile_counts);
   return cudaGetLastError();
 }
 
@@ -334,10 +338,10 @@ cudaError_t launch_bin_place(const ViewDesc* views, uint32_t n_views, uint32_t n
                              const uint32_t* chunk_cell, const uint32_t* chunk_counts,
                              const uint32_t* tile_offsets, const unsigned long long* ref_total,
                              uint32_t capacity, uint2* keys, uint32_t* values, uint32_t* ticket,
-                             uint32_t* err, int sm_count, cudaStream_t s) {
-  chunk_place_kernel<<<sm_count * 8, kThreads, 0, s>>>(
-      views, n_views, entries, ids, cell_start, chunk_cell, num_cells, chunk_counts, tile_offsets,
-      ref_total, capacity, keys, values, ticket, err);
+                             uint32_t* err, int sm_count, LaunchStream s) {
+  launch_after(chunk_place_kernel, sm_count * 8, kThreads, 0, s, views, n_views, entries, ids,
+               cell_start, chunk_cell, num_cells, chunk_counts, tile_offsets, ref_total, capacity,
+               keys, values, ticket, err);
   return cudaGetLastError();
 }
 

@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(kHistThreads)
                            uint32_t* __restrict__ status, size_t status_stride,
                            ClearList clear) {
   __shared__ uint32_t s_hist[kDepthPasses][kBins];
+  after_predecessor(keys, count, range);
   for (int k = threadIdx.x; k < kDepthPasses * (int)kBins; k += kHistThreads)
     (&s_hist[0][0])[k] = 0u;
   __syncthreads();
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   __shared__ uint32_t s_wsum[kWarps];
   __shared__ uint32_t s_part[2];
   __shared__ uint64_t s_bar[2];
+  after_predecessor(count_in, range, hist);
   const Digits digit = digits_of(range, pass);
   if (pass == 3 && digit.mask != 255u) return;  // three passes did
   if (blockDim.x != kThreads) {  // the indexing below is written for this block size
@@ -344,23 +346,23 @@ cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const De
                               uint32_t* keys_a, uint32_t* ids_a, uint32_t* keys_b,
                               uint32_t* ids_b, uint32_t* status, uint32_t* g_hist,
                               uint32_t* part_counters, uint32_t* err, const ClearList& clear,
-                              int sm_count, cudaStream_t s) {
+                              int sm_count, LaunchStream s) {
   int per_sm = 0;
   cudaError_t e = pass_setup(&per_sm);
   if (e != cudaSuccess) return e;
   const size_t stride = status_stride(capacity);
   const size_t parts = ((size_t)capacity + kPart - 1) / kPart;
   const size_t rounds = ((size_t)capacity + kHistThreads * kHistItems - 1) / (kHistThreads * kHistItems);
-  depth_histogram_kernel<<<(unsigned)std::min<size_t>((size_t)sm_count * 8, std::max<size_t>(rounds, 1)),
-                           kHistThreads, 0, s>>>(keys_a, count, range, g_hist, status, stride, clear);
+  launch_after(depth_histogram_kernel,
+               (unsigned)std::min<size_t>((size_t)sm_count * 8, std::max<size_t>(rounds, 1)),
+               kHistThreads, 0, s, keys_a, count, range, g_hist, status, stride, clear);
   const unsigned grid =
       (unsigned)std::min<size_t>((size_t)sm_count * per_sm, std::max<size_t>(parts, 1));
   for (int p = 0; p < kDepthPasses; ++p) {
     const bool even = p % 2 == 0;
-    depth_pass_kernel<<<grid, kThreads, kSmem, s>>>(
-        even ? keys_a : keys_b, even ? ids_a : ids_b, even ? keys_b : keys_a,
-        even ? ids_b : ids_a, count, range, p, g_hist + (size_t)p * kBins, status + p * stride,
-        part_counters + p, err);
+    launch_after(depth_pass_kernel, grid, kThreads, kSmem, s, even ? keys_a : keys_b,
+                 even ? ids_a : ids_b, even ? keys_b : keys_a, even ? ids_b : ids_a, count, range,
+                 p, g_hist + (size_t)p * kBins, status + p * stride, part_counters + p, err);
   }
   return cudaGetLastError();
 }

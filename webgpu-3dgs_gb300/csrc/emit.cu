@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
   __shared__ uint32_t s_hist[TP > 0 ? TP : 1][BINS];
   __shared__ uint32_t s_first, s_next;  // tickets: the block's first chunk, its next one
 
+  after_predecessor(ref_counter, cells.ref_total, sorted.range);
   const uint32_t total = *ref_counter;
   const unsigned long long frame_refs = CELLS ? *cells.ref_total : total;
   if (CELLS && blockIdx.x == 0 && threadIdx.x == 0)
@@ -345,7 +346,7 @@ cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
                          const uint32_t* counter, CellArgs cells,
                          uint32_t capacity, uint2* keys, uint32_t* values, const SortPlan& plan,
                          const StatusClear& sort_status, uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
-                         cudaStream_t s) {
+                         LaunchStream s) {
   if (n == 0) return cudaSuccess;
   const uint32_t chunks = (n + kThreads - 1) / kThreads;
   const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 1u;
@@ -361,10 +362,10 @@ cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
   for (int p = 0; p < plan.passes; ++p) wide = wide || plan.nbits[p] > 8;
 #define GS3D_EMIT_CASE(TP, BINS)                                                              \
   case TP:                                                                                    \
-    emit_sorted_kernel<TP, BINS, CELLS>                                                       \
-        <<<std::min(chunks, sms * emit_blocks_per_sm<TP, BINS, CELLS>()), kThreads, 0, s>>>(  \
-            views, n_views, n, proj, rect8, sorted, sorted_offsets, counter, cells,           \
-            capacity, keys, values, sh, mk, sort_status, g_hist, chunk_ticket, err);   \
+    launch_after(emit_sorted_kernel<TP, BINS, CELLS>,                                         \
+                 std::min(chunks, sms * emit_blocks_per_sm<TP, BINS, CELLS>()), kThreads, 0,  \
+                 s, views, n_views, n, proj, rect8, sorted, sorted_offsets, counter, cells,   \
+                 capacity, keys, values, sh, mk, sort_status, g_hist, chunk_ticket, err);     \
     break;
   if (wide) {
     switch (plan.passes) {
@@ -398,7 +399,7 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
                                uint32_t capacity, uint2* keys, uint32_t* values,
                                const SortPlan& tile_plan, const StatusClear& sort_status,
                                uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
-                               cudaStream_t s) {
+                               LaunchStream s) {
   return emit_ordered<false>(views, n_views, n, proj, rect8, sorted, sorted_offsets,
                              ref_counter, CellArgs{}, capacity, keys, values,
                              tile_plan, sort_status, g_hist, chunk_ticket, err, sm_count, s);
@@ -410,7 +411,7 @@ cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t 
                               uint32_t* entry_total, const unsigned long long* ref_total, uint32_t* ref_counter,
                               uint32_t capacity, uint2* keys, uint32_t* values,
                               const SortPlan& cell_plan, const StatusClear& sort_status,
-                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count, cudaStream_t s) {
+                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count, LaunchStream s) {
   return emit_ordered<true>(views, n_views, n, proj, rect8, sorted, sorted_offsets, entry_total,
                             CellArgs{ref_total, ref_counter, entry_total},
                             capacity, keys, values, cell_plan, sort_status, g_hist, chunk_ticket,

@@ -211,6 +211,21 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// A kernel that launch_after starts as a programmatic dependent begins with
+// this: it returns when the predecessor on the stream has completed with its
+// writes visible (the predecessor waited for its own, so all of the stream's
+// earlier work has).  The pointers passed are the ones read first: they leave
+// as unknown values, so that no read-only load through them can be scheduled
+// before the wait.  No kernel of this library triggers its dependents early:
+// blocks that are resident and wait keep other streams' kernels off the chip
+// (with a trigger at the kernels' start a frame of 500k splats, three contexts
+// at a time, went from 512 to 560 us; with none to 487 us).
+template <typename... P>
+__device__ __forceinline__ void after_predecessor(P&... read_first) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (..., ([&] { asm volatile("" : "+l"(read_first)::"memory"); }()));
+}
+
 // mbarrier + bulk (TMA, non-tensor) copy helpers.
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
@@ -270,6 +285,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 
 __device__ __forceinline__ void latch_error(uint32_t* err, uint32_t bit) { atomicOr(err, bit); }
 
+// The stream that a launcher enqueues on, and whether its kernels are
+// programmatic dependents of their predecessors: launched while those drain,
+// not after.
+struct LaunchStream {
+  cudaStream_t s;
+  bool dependent;
+  LaunchStream(cudaStream_t stream, bool dep = false) : s(stream), dependent(dep) {}
+  operator cudaStream_t() const { return s; }
+};
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                         LaunchStream on, A&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = on.s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = on.dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Per-device launch set-up (shared-memory attributes, occupancy) is cached
 // in arrays of this many devices.
 constexpr int kMaxDevices = 64;
@@ -327,7 +367,7 @@ cudaError_t launch_preprocess(const ViewDesc* views, uint32_t n_views, uint32_t 
 // Exclusive scan of counts in the order of gather (as they are when it is null).
 cudaError_t launch_scan(const uint32_t* counts, const DepthSorted* gather, uint32_t* offsets,
                         uint32_t n, unsigned long long* status, uint32_t* tile_counter,
-                        uint32_t epoch, uint32_t* total_out, uint32_t* err, cudaStream_t s);
+                        uint32_t epoch, uint32_t* total_out, uint32_t* err, LaunchStream s);
 size_t scan_status_words(uint32_t n);
 // Exclusive scan, in the order of `gather`, of the cells that every splat-view
 // covers: its rectangle in rect8 (all ones: culled), or where rect8 is null in
@@ -336,13 +376,13 @@ cudaError_t launch_scan_cells(const uint32_t* counts, const uint32_t* rect8,
                               const gs3d_projected_splat* proj, const DepthSorted& gather,
                               uint32_t* offsets, uint32_t n, unsigned long long* status,
                               uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
-                              unsigned long long* ref_total, uint32_t* err, cudaStream_t s);
+                              unsigned long long* ref_total, uint32_t* err, LaunchStream s);
 // tile_offsets[n + 1] of n tile counts, in identify_tile_ranges.wgsl's
 // convention (tiles after the last populated one keep 0).
 cudaError_t launch_scan_tiles(const uint32_t* tile_counts, uint32_t* tile_offsets, uint32_t n,
                               const unsigned long long* ref_total, unsigned long long* status,
                               uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
-                              uint32_t* err, cudaStream_t s);
+                              uint32_t* err, LaunchStream s);
 // Binned rebin (binning.cu), over the entries sorted by cell: chunk counts and
 // tile totals; then, once the tile offsets are known, the refs.
 size_t chunk_slots_max(uint32_t capacity, uint32_t num_cells);
@@ -350,13 +390,13 @@ cudaError_t launch_bin_count(const ViewDesc* views, uint32_t n_views, uint32_t n
                              const uint2* entries, const uint32_t* entry_total,
                              const unsigned long long* ref_total, uint32_t capacity,
                              uint32_t* cell_start, uint32_t* chunk_cell, uint32_t* chunk_counts,
-                             uint32_t* tile_counts, int sm_count, cudaStream_t s);
+                             uint32_t* tile_counts, int sm_count, LaunchStream s);
 cudaError_t launch_bin_place(const ViewDesc* views, uint32_t n_views, uint32_t num_cells,
                              const uint2* entries, const uint32_t* ids, const uint32_t* cell_start,
                              const uint32_t* chunk_cell, const uint32_t* chunk_counts,
                              const uint32_t* tile_offsets, const unsigned long long* ref_total,
                              uint32_t capacity, uint2* keys, uint32_t* values, uint32_t* ticket,
-                             uint32_t* err, int sm_count, cudaStream_t s);
+                             uint32_t* err, int sm_count, LaunchStream s);
 // Message of the calling thread's last failing context-free call.
 const char* noalloc_last_error();
 // Sets the message gs3d_last_error(NULL) returns on the calling thread.
@@ -390,7 +430,7 @@ cudaError_t launch_sort_tile_passes(const SortPlan& plan, const uint32_t* ref_co
                                     uint32_t capacity, uint2* keys_a, uint32_t* vals_a,
                                     uint2* keys_b, uint32_t* vals_b, uint32_t* status,
                                     uint32_t* g_hist, uint32_t* part_counters, uint32_t* err,
-                                    int sm_count, cudaStream_t s);
+                                    int sm_count, LaunchStream s);
 // Stable LSD passes of `plan` (word ignored) over 32-bit keys; the histograms
 // are computed here.  count is read on the device.
 cudaError_t launch_sort_u32(const SortPlan& plan, const uint32_t* count, uint32_t capacity,
@@ -412,7 +452,7 @@ cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const De
                               uint32_t* keys_a, uint32_t* ids_a, uint32_t* keys_b,
                               uint32_t* ids_b, uint32_t* status, uint32_t* g_hist,
                               uint32_t* part_counters, uint32_t* err, const ClearList& clear,
-                              int sm_count, cudaStream_t s);
+                              int sm_count, LaunchStream s);
 // Raster work order: tile indices sorted by decreasing expected cost
 // (schedule = GS3D_SCHEDULE_KEY_COUNT: the tile's key count), so the
 // persistent raster CTAs start the longest tiles first.
@@ -447,7 +487,7 @@ constexpr uint32_t kOrderTiles = 65536;
 cudaError_t launch_order(uint32_t schedule, const uint32_t* tile_offsets, const float* pred,
                          const SchedGate* gate, uint32_t num_tiles, uint32_t workers,
                          uint32_t items_per_tile, bool split_all, uint32_t* order,
-                         uint32_t* heavy, cudaStream_t s);
+                         uint32_t* heavy, LaunchStream s);
 
 // ---- learned schedule (learned.cu) ----
 constexpr int kFeatures = 16;
@@ -489,7 +529,7 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
                                uint32_t capacity, uint2* keys, uint32_t* values,
                                const SortPlan& tile_plan, const StatusClear& sort_status,
                                uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
-                               cudaStream_t s);
+                               LaunchStream s);
 // The same for cell entries: one per (splat-view, cell), keys [cell and
 // rectangle inside it | depth], and *ref_counter = the frame's refs.
 cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t total,
@@ -498,11 +538,12 @@ cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t 
                               uint32_t* entry_total, const unsigned long long* ref_total, uint32_t* ref_counter,
                               uint32_t capacity, uint2* keys, uint32_t* values,
                               const SortPlan& cell_plan, const StatusClear& sort_status,
-                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count, cudaStream_t s);
+                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err,
+                              int sm_count, LaunchStream s);
 // tile_offsets zeroed by the caller.
 cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint32_t capacity,
                             uint32_t num_tiles, uint32_t* tile_offsets, uint32_t* err,
-                            int sm_count, cudaStream_t s);
+                            int sm_count, LaunchStream s);
 // Rasterizes every tile of the batch.  Persistent CTAs pull tile indices
 // from a device work queue (order[k] = k-th tile to render, identity when
 // order is null) through *queue_counter, which must be zero at launch, as must
@@ -529,7 +570,7 @@ struct RasterArgs {
   bool fine;              // single blocks instead of regions, set by launch_raster
 };
 size_t raster_pool_bytes();
-cudaError_t launch_raster(const RasterArgs& a, int sm_count, cudaStream_t s);
+cudaError_t launch_raster(const RasterArgs& a, int sm_count, LaunchStream s);
 // Work items per tile and resident workers (warps; CTAs where a CTA shades a
 // tile) of the raster launch for these args.
 cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* items_per_tile,

@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(kThreads)
     identify_kernel(const uint2* __restrict__ keys, const uint32_t* __restrict__ ref_counter,
                     uint32_t capacity, uint32_t num_tiles, uint32_t* __restrict__ tile_offsets,
                     uint32_t* __restrict__ err) {
+  after_predecessor(keys, ref_counter);
   const uint32_t n = live_refs(ref_counter, capacity);
   const uint32_t pairs = (n + 1) / 2;
   const uint32_t lane = threadIdx.x & 31;
@@ -73,9 +74,9 @@ __global__ void __launch_bounds__(kThreads)
 
 cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint32_t capacity,
                             uint32_t num_tiles, uint32_t* tile_offsets, uint32_t* err,
-                            int sm_count, cudaStream_t s) {
-  identify_kernel<<<sm_count * 8, kThreads, 0, s>>>(keys, ref_counter, capacity, num_tiles,
-                                                    tile_offsets, err);
+                            int sm_count, LaunchStream s) {
+  launch_after(identify_kernel, sm_count * 8, kThreads, 0, s, keys, ref_counter, capacity,
+               num_tiles, tile_offsets, err);
   return cudaGetLastError();
 }
 

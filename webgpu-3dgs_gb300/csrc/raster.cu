@@ -1038,6 +1038,7 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
   extern __shared__ __align__(16) unsigned char smem[];
   WarpSmem& w = reinterpret_cast<WarpSmem*>(smem)[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
+  after_predecessor(a.heavy);
   if (lane == 0) {
     w.kept[kKept].a = make_float4(0.f, 0.f, -1.f, 0.f);
     w.kept[kKept].b = make_float4(0.f, 0.f, 0.f, -1.f);
@@ -1254,7 +1255,7 @@ cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* items_per_
 
 size_t raster_pool_bytes() { return kPoolSlots * sizeof(PoolSlot); }
 
-cudaError_t launch_raster(const RasterArgs& args, int sm_count, cudaStream_t s) {
+cudaError_t launch_raster(const RasterArgs& args, int sm_count, LaunchStream s) {
   if (args.num_tiles == 0) return cudaSuccess;
   RasterArgs a = args;
   RasterConfig cfg;
@@ -1270,7 +1271,9 @@ cudaError_t launch_raster(const RasterArgs& args, int sm_count, cudaStream_t s) 
   } else {
     a.heavy = nullptr;  // split items exist in the warp variant only
   }
-  cfg.kern<<<(uint32_t)std::min<uint64_t>(max_ctas, ctas), cfg.threads, cfg.smem, s>>>(a);
+  const uint32_t grid = (uint32_t)std::min<uint64_t>(max_ctas, ctas);
+  if (cfg.mode == 2) return launch_after(cfg.kern, grid, cfg.threads, cfg.smem, s, a);
+  cfg.kern<<<grid, cfg.threads, cfg.smem, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ unsigned long long s_refs[kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
+  after_predecessor(in, order.range, ex.rect8, ex.proj);
   const uint32_t* gather = order.range != nullptr ? order.ids() : nullptr;
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
   __syncthreads();
@@ -232,14 +233,15 @@ size_t scan_status_words(uint32_t n) { return (n + kTile - 1) / kTile + 1; }
 
 cudaError_t launch_scan(const uint32_t* counts, const DepthSorted* gather, uint32_t* offsets,
                         uint32_t n, unsigned long long* status, uint32_t* tile_counter,
-                        uint32_t epoch, uint32_t* total_out, uint32_t* err, cudaStream_t s) {
+                        uint32_t epoch, uint32_t* total_out, uint32_t* err, LaunchStream s) {
   if (n == 0) {
     scan_empty_kernel<<<1, 1, 0, s>>>(offsets, total_out);
     return cudaGetLastError();
   }
   const uint32_t tiles = (n + kTile - 1) / kTile;
-  scan_kernel<Scan::counts><<<tiles, kThreads, 0, s>>>(counts, gather ? *gather : DepthSorted{}, ScanExtra{}, offsets, n,
-                                                       status, tile_counter, epoch, total_out, err);
+  launch_after(scan_kernel<Scan::counts>, tiles, kThreads, 0, s, counts,
+               gather ? *gather : DepthSorted{}, ScanExtra{}, offsets, n, status, tile_counter,
+               epoch, total_out, err);
   return cudaGetLastError();
 }
 
@@ -247,7 +249,7 @@ cudaError_t launch_scan_cells(const uint32_t* counts, const uint32_t* rect8,
                               const gs3d_projected_splat* proj, const DepthSorted& gather,
                               uint32_t* offsets, uint32_t n, unsigned long long* status,
                               uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
-                              unsigned long long* ref_total, uint32_t* err, cudaStream_t s) {
+                              unsigned long long* ref_total, uint32_t* err, LaunchStream s) {
   if (n == 0) {
     scan_empty_kernel<<<1, 1, 0, s>>>(offsets, total_out);
     return cudaGetLastError();
@@ -255,22 +257,22 @@ cudaError_t launch_scan_cells(const uint32_t* counts, const uint32_t* rect8,
   const uint32_t tiles = (n + kTile - 1) / kTile;
   const ScanExtra ex{rect8, proj, ref_total};
   if (rect8 != nullptr)
-    scan_kernel<Scan::cells8><<<tiles, kThreads, 0, s>>>(counts, gather, ex, offsets, n, status,
-                                                         tile_counter, epoch, total_out, err);
+    launch_after(scan_kernel<Scan::cells8>, tiles, kThreads, 0, s, counts, gather, ex, offsets, n,
+                 status, tile_counter, epoch, total_out, err);
   else
-    scan_kernel<Scan::cells16><<<tiles, kThreads, 0, s>>>(counts, gather, ex, offsets, n, status,
-                                                          tile_counter, epoch, total_out, err);
+    launch_after(scan_kernel<Scan::cells16>, tiles, kThreads, 0, s, counts, gather, ex, offsets, n,
+                 status, tile_counter, epoch, total_out, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_scan_tiles(const uint32_t* tile_counts, uint32_t* tile_offsets, uint32_t n,
                               const unsigned long long* ref_total, unsigned long long* status,
                               uint32_t* tile_counter, uint32_t epoch, uint32_t* total_out,
-                              uint32_t* err, cudaStream_t s) {
+                              uint32_t* err, LaunchStream s) {
   const uint32_t tiles = (n + kTile - 1) / kTile;
   const ScanExtra ex{nullptr, nullptr, const_cast<unsigned long long*>(ref_total)};
-  scan_kernel<Scan::tiles><<<tiles, kThreads, 0, s>>>(tile_counts, DepthSorted{}, ex, tile_offsets, n,
-                                                      status, tile_counter, epoch, total_out, err);
+  launch_after(scan_kernel<Scan::tiles>, tiles, kThreads, 0, s, tile_counts, DepthSorted{}, ex,
+               tile_offsets, n, status, tile_counter, epoch, total_out, err);
   return cudaGetLastError();
 }
 

@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(kOrderThreads)
   __shared__ float s_sum[kOrderThreads / 32];
   __shared__ uint32_t s_warp[kOrderThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  after_predecessor(tile_offsets, pred, gate);
   const bool learned = LEARNED && gate->use_learned != 0u;
   auto cost = [&](uint32_t t) -> float {
     if (learned) return expm1f(fminf(fmaxf(__ldg(pred + t), 0.0f), 15.99f));
@@ -161,15 +162,15 @@ __global__ void __launch_bounds__(kOrderThreads)
 cudaError_t launch_order(uint32_t schedule, const uint32_t* tile_offsets, const float* pred,
                          const SchedGate* gate, uint32_t num_tiles, uint32_t workers,
                          uint32_t items_per_tile, bool split_all, uint32_t* order,
-                         uint32_t* heavy, cudaStream_t s) {
+                         uint32_t* heavy, LaunchStream s) {
   if (schedule == GS3D_SCHEDULE_LEARNED)
-    order_kernel<true><<<1, kOrderThreads, 0, s>>>(
-        tile_offsets, pred, gate, num_tiles, workers, items_per_tile, (float)kHeavyKeys,
-        (float)kHeavyCost, split_all ? 1u : 0u, order, heavy);
+    launch_after(order_kernel<true>, 1, kOrderThreads, 0, s, tile_offsets, pred, gate, num_tiles,
+                 workers, items_per_tile, (float)kHeavyKeys, (float)kHeavyCost,
+                 split_all ? 1u : 0u, order, heavy);
   else
-    order_kernel<false><<<1, kOrderThreads, 0, s>>>(
-        tile_offsets, nullptr, nullptr, num_tiles, workers, items_per_tile, (float)kHeavyKeys,
-        (float)kHeavyCost, split_all ? 1u : 0u, order, heavy);
+    launch_after(order_kernel<false>, 1, kOrderThreads, 0, s, tile_offsets, nullptr, nullptr,
+                 num_tiles, workers, items_per_tile, (float)kHeavyKeys, (float)kHeavyCost,
+                 split_all ? 1u : 0u, order, heavy);
   return cudaGetLastError();
 }
 

@@ -263,6 +263,7 @@ __global__ void __launch_bounds__(kPassThreads, 1024 / kPassThreads)
   __shared__ uint32_t s_part[2];  // partition id of each buffer
   __shared__ uint64_t s_bar[2];
 
+  after_predecessor(ref_counter, hist);
   if (blockDim.x != kPassThreads) {  // the indexing below is written for this block size
     if (threadIdx.x == 0) latch_error(err, DEVERR_RANGE);
     return;
@@ -510,6 +511,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   __shared__ uint32_t s_part[2];
   __shared__ uint64_t s_bar[2];
 
+  after_predecessor(ref_counter, hist);
   if (blockDim.x != kWideThreads) {  // the indexing below is written for this block size
     if (threadIdx.x == 0) latch_error(err, DEVERR_RANGE);
     return;
@@ -770,26 +772,24 @@ template <typename K>
 cudaError_t launch_pass(int nbits, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout,
                         const uint32_t* ref_counter, uint32_t capacity, int word, int shift,
                         const uint32_t* hist, uint32_t* status, uint32_t* part_counter,
-                        uint32_t* err, int sm_count, size_t parts_cap, cudaStream_t s) {
+                        uint32_t* err, int sm_count, size_t parts_cap, LaunchStream s) {
   int per_sm = 0;
   cudaError_t e;
 #define GS3D_PASS(NB)                                                                        \
   e = onesweep_setup<K, NB>(&per_sm);                                                       \
   if (e != cudaSuccess) return e;                                                           \
-  onesweep_kernel<K, NB><<<(int)std::min<size_t>((size_t)sm_count * per_sm, parts_cap),      \
-                           kPassThreads, pass_smem<K>(), s>>>(kin, vin, kout, vout,          \
-                                                              ref_counter, capacity, word,   \
-                                                              shift, hist, status,           \
-                                                              part_counter, err);            \
+  launch_after(onesweep_kernel<K, NB>,                                                      \
+               (unsigned)std::min<size_t>((size_t)sm_count * per_sm, parts_cap),            \
+               kPassThreads, pass_smem<K>(), s, kin, vin, kout, vout, ref_counter, capacity, \
+               word, shift, hist, status, part_counter, err);                                \
   break;
   if (nbits == kWideBits) {  // 2048-bin digits: (tile | depth) keys only
     if constexpr (std::is_same<K, uint2>::value) {
       e = onesweep_wide_setup();
       if (e != cudaSuccess) return e;
-      onesweep_wide_kernel<<<(int)std::min<size_t>((size_t)sm_count, parts_cap), kWideThreads,
-                             wide_pass_smem<uint2>(), s>>>(kin, vin, kout, vout, ref_counter,
-                                                           capacity, word, shift, hist, status,
-                                                           part_counter, err);
+      launch_after(onesweep_wide_kernel, (unsigned)std::min<size_t>((size_t)sm_count, parts_cap),
+                   kWideThreads, wide_pass_smem<uint2>(), s, kin, vin, kout, vout, ref_counter,
+                   capacity, word, shift, hist, status, part_counter, err);
       return cudaGetLastError();
     } else {
       return cudaErrorInvalidValue;
@@ -838,7 +838,7 @@ cudaError_t run_passes(const SortPlan& plan, const uint32_t* ref_counter, uint32
                        K* keys_a, uint32_t* vals_a, K* keys_b, uint32_t* vals_b,
                        uint32_t* status, uint32_t* g_hist, size_t hist_stride,
                        uint32_t* part_counters, uint32_t* err, bool hist_ready, int sm_count,
-                       cudaStream_t s) {
+                       LaunchStream s) {
   cudaError_t e = cudaSuccess;
   const size_t parts_cap = ((size_t)capacity + kPart - 1) / kPart + 1;
   const size_t stride = parts_cap * kRadixBins;
@@ -949,7 +949,7 @@ cudaError_t launch_sort_tile_passes(const SortPlan& plan, const uint32_t* ref_co
                                     uint32_t capacity, uint2* keys_a, uint32_t* vals_a,
                                     uint2* keys_b, uint32_t* vals_b, uint32_t* status,
                                     uint32_t* g_hist, uint32_t* part_counters, uint32_t* err,
-                                    int sm_count, cudaStream_t s) {
+                                    int sm_count, LaunchStream s) {
   return run_passes<uint2>(plan, ref_counter, capacity, keys_a, vals_a, keys_b, vals_b, status,
                            g_hist, kTileHistStride, part_counters, err, true, sm_count, s);
 }
