@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
   }
   const uint32_t* __restrict__ sorted_keys = sorted.keys();
   const uint32_t* __restrict__ sorted_ids = sorted.ids();
+  const uint32_t* __restrict__ sorted_rects = sorted.rects();
   for (int k = threadIdx.x; k < TP * BINS; k += kThreads) (&s_hist[0][0])[k] = 0u;
   const int sh[4] = {shifts.x, shifts.y, shifts.z, shifts.w};
   const uint32_t mk[4] = {masks.x, masks.y, masks.z, masks.w};
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
   // fetched while the current chunk expands, and its rectangles gathered
   // before the barrier that ends the chunk (while the warps that finished
   // wait there), so a chunk starts with its fields in registers.
-  uint32_t p_id = 0, p_key = 0, p_off = 0, p_end = 0;
+  uint32_t p_id = 0, p_key = 0, p_off = 0, p_end = 0, p_word = 0;
   uint4 p_rect = make_uint4(0u, 0u, 0u, 0u);  // [x0, y0, x1, y1]
   auto fetch = [&](uint32_t c) {
     const uint32_t i = c * kThreads + threadIdx.x;
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
       p_id = __ldg(sorted_ids + i);
       p_key = __ldg(sorted_keys + i);
       p_off = __ldg(sorted_offsets + i);
+      if (CELLS && rect8 != nullptr) p_word = __ldg(sorted_rects + i);
     }
     if (threadIdx.x == 0 && c < chunks) p_end = __ldg(sorted_offsets + min(n, (c + 1) * kThreads));
   };
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
   auto gather = [&](uint32_t c) {
     if (c >= chunks || c * kThreads + threadIdx.x >= n) return;
     if (rect8 != nullptr) {
-      uint32_t rr = __ldg(rect8 + p_id);
+      uint32_t rr = CELLS ? p_word : __ldg(rect8 + p_id);
       if (rr == kCulledRect) rr = 0u;
       const uint32_t x0 = rr & 0xffu, y0 = (rr >> 8) & 0xffu;
       p_rect = make_uint4(x0, y0, x0 + ((rr >> 16) & 0xffu), y0 + (rr >> 24));
@@ -224,10 +226,11 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
     if (threadIdx.x == 0) s_off[last - first] = p_end;
     __syncthreads();  // the chunk's fields and the next ticket are in shared memory
     const uint32_t next = s_next;
-    fetch(next);
-
     const uint32_t nloc = last - first;
     const uint32_t begin = s_off[0], end = s_off[nloc];
+    if (begin == total) break;  // nothing here or in any later chunk: culled splats sort last
+    fetch(next);
+
     // block-uniform (shared values): an inconsistent chunk is skipped
     if (end < begin || end > total) {
       if (threadIdx.x == 0) latch_error(err, DEVERR_RANGE);

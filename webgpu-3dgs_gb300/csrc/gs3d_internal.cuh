@@ -116,12 +116,18 @@ __host__ __device__ inline bool depth_three_passes(uint32_t lo, uint32_t hi) {
 // Where the depth sort leaves its result: the B arrays after three passes.
 struct DepthSorted {
   const DepthRange* range;
-  const uint32_t *keys_a, *ids_a, *keys_b, *ids_b;
+  const uint32_t* keys_a;
+  uint32_t* ids_a;
+  const uint32_t* keys_b;
+  uint32_t* ids_b;
   __device__ __forceinline__ bool in_b() const {
     return depth_three_passes(~__ldg(&range->max_not), __ldg(&range->max));
   }
   __device__ __forceinline__ const uint32_t* keys() const { return in_b() ? keys_b : keys_a; }
   __device__ __forceinline__ const uint32_t* ids() const { return in_b() ? ids_b : ids_a; }
+  // the other id array, free after the sort: the scan leaves the one-word
+  // rectangles there in depth order
+  __device__ __forceinline__ uint32_t* rects() const { return in_b() ? ids_a : ids_b; }
 };
 
 constexpr int kMaxSortPasses = 8;

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kThreads)
   uint32_t v[kItems];
   if (KIND == Scan::cells8 || KIND == Scan::cells16) {
     unsigned long long refs = 0;
-    uint32_t id[kItems];
+    uint32_t id[kItems], rect[kItems] = {};
 #pragma unroll
     for (int k = 0; k < kItems; ++k) id[k] = (base + k < n) ? __ldg(gather + base + k) : 0u;
 #pragma unroll
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kThreads)
       v[k] = 0u;
       if (base + k >= n) continue;
       if (KIND == Scan::cells8) {
-        const uint32_t r = __ldg(ex.rect8 + id[k]);
+        const uint32_t r = rect[k] = __ldg(ex.rect8 + id[k]);
         const uint32_t x0 = r & 0xffu, y0 = (r >> 8) & 0xffu;
         if (r != kCulledRect)
           v[k] = rect_cells(x0, y0, x0 + ((r >> 16) & 0xffu), y0 + (r >> 24), refs);
@@ -99,6 +99,11 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) refs += __shfl_xor_sync(0xffffffffu, refs, o);
     if (lane == 0) s_refs[warp] = refs;
+    if (KIND == Scan::cells8 && base < n) {  // whole groups of 8 fit the array
+      uint4* r4 = reinterpret_cast<uint4*>(order.rects() + base);
+      r4[0] = make_uint4(rect[0], rect[1], rect[2], rect[3]);
+      r4[1] = make_uint4(rect[4], rect[5], rect[6], rect[7]);
+    }
   } else if (gather != nullptr) {  // counts read through a permutation (fused rebin)
 #pragma unroll
     for (int k = 0; k < kItems; ++k) v[k] = (base + k < n) ? __ldg(in + __ldg(gather + base + k)) : 0u;
