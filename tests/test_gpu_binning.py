@@ -2,7 +2,7 @@
 cell), sorted by cell, expanded in place) against the six reference stages:
 keys, values and tile ranges bit for bit, at the edges of its tiling - grids a
 tile over or under whole cells, cells of no entry, of one, of several chunks of
-1024, chunks of more refs than one window of 4096 holds, splats over the whole
+1024, chunks of more refs than one window of 10,240 holds, splats over the whole
 grid, grids of more than 256 tiles per axis, cell counts around a digit.  The
 cells serve scenes of 300,000 splats or more, so each scene is filled up to that
 with splats behind the camera."""
@@ -65,6 +65,22 @@ def test_refs_equal_the_reference_stages(renderer, n, spread, scale, tile, w, h)
     want = refs(r, data, tile, w, h, True)
     got = refs(r, data, tile, w, h, False)
     assert want[0] > 0 and want[3].size > 257
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+    r.setTileSize(16, 16)
+
+
+@pytest.mark.parametrize("scale", [0.1, 0.2, 0.3, 0.45, 0.7])
+def test_chunks_around_one_window(renderer, scale):
+    """Chunks of 4 to 40 refs an entry: placed a tile a lane up to one window
+    of refs, an entry a lane beyond it."""
+    r = renderer
+    data = cloud(6000, 77, 1.0, scale)
+    r.setSplatData(data)
+    r.setTileSize(8, 8)
+    want = refs(r, data, (8, 8), 400, 300, True)
+    got = refs(r, data, (8, 8), 400, 300, False)
+    assert want[0] > 0
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
     r.setTileSize(16, 16)

@@ -35,7 +35,14 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kGroups = kChunkEntries / kThreads;  // groups of 32 entries per warp
 static_assert(kGroups * kThreads == kChunkEntries, "whole groups");
-constexpr uint32_t kWindow = 4096;  // refs placed through shared memory at a time
+// Refs placed through shared memory at a time.  A chunk of no more is put in
+// tile order by a tile a lane; in a chunk of more, whose windows hold the refs
+// of a few tiles each, a tile a lane left most lanes idle (143 instructions per
+// 32 refs), so there a warp places a tile's refs together, an entry a lane.
+// refs + ranges of 3M heavy-tailed splats at 4K (40M refs) 666 -> 394 us, a 3M
+// frame 152 -> 141, 8 views of 3M 519 -> 503; windows of 4096 and of 16384
+// were slower (12 views: 428 and 443 us, 416 with this one).
+constexpr uint32_t kWindow = 10240;
 
 // A warp's transpose of a 32x32 bit matrix: lane i holds row i and gets column i.
 __device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
@@ -199,7 +206,9 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // Places the refs of every chunk.  A window of them at a time is put in tile
 // order in shared memory (2 bytes a ref: tile of the cell and entry of the
-// chunk), then written out with unit stride, each tile's run contiguous.
+// chunk), then written out with unit stride, each tile's run contiguous (with
+// the runs of 32 entries written straight to memory, 3M heavy-tailed splats at
+// 4K took 1210 us).
 __global__ void __launch_bounds__(kThreads)
     chunk_place_kernel(const ViewDesc* __restrict__ views, uint32_t n_views,
                        const uint2* __restrict__ entries, const uint32_t* __restrict__ ids,
@@ -218,8 +227,8 @@ __global__ void __launch_bounds__(kThreads)
   after_predecessor(cell_start, ref_total);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t slots = chunk_slot(__ldg(cell_start + num_cells), num_cells);
-  const unsigned long long total = *ref_total;
-  if (total > capacity) return;  // latched by the emit
+  if (*ref_total > capacity) return;  // latched by the emit
+  const uint32_t total = (uint32_t)*ref_total;
   for (;;) {
     if (threadIdx.x == 0) s_next = atomicAdd(ticket, 1u);
     __syncthreads();  // also: the previous chunk's readers are done
@@ -277,23 +286,36 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();
     const uint32_t refs = s_total;
+    const bool dense = refs > kWindow;
     uint32_t pos0 = s_cnt[warp][lane], pos1 = s_cnt[warp][lane + 32];
     for (uint32_t wb = 0; wb < refs; wb += kWindow) {
       const uint32_t we = min(refs, wb + kWindow);
+      if (dense) {  // a tile of the window at a time, an entry a lane
 #pragma unroll
-      for (int g = 0; g < kGroups; ++g) {
-        const uint32_t e0 = (warp * kGroups + g) * 32;
-        while (c.w[g][0] && pos0 < we) {
-          const uint32_t bit = __ffs(c.w[g][0]) - 1;
-          c.w[g][0] &= c.w[g][0] - 1;
-          s_slot[pos0 - wb] = (uint16_t)((lane << 10) | (e0 + bit));
-          ++pos0;
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t pos = h ? pos1 : pos0, cnt = h ? n1 : n0;
+          for (uint32_t tiles = __ballot_sync(0xffffffffu, cnt && pos < we && pos + cnt > wb);
+               tiles != 0u; tiles &= tiles - 1u) {
+            const int tl = __ffs(tiles) - 1;
+            uint32_t at = __shfl_sync(0xffffffffu, pos, tl) - wb;  // may start before the window
+            const uint32_t code = ((h * 32 + tl) << 10) | (warp * kGroups * 32 + lane);
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g) {
+              const uint32_t who = __shfl_sync(0xffffffffu, c.w[g][h], tl);
+              const uint32_t to = at + __popc(who & lanemask_lt());
+              if (((who >> lane) & 1u) && to < we - wb) s_slot[to] = (uint16_t)(code + g * 32);
+              at += __popc(who);
+            }
+          }
         }
-        while (c.w[g][1] && pos1 < we) {
-          const uint32_t bit = __ffs(c.w[g][1]) - 1;
-          c.w[g][1] &= c.w[g][1] - 1;
-          s_slot[pos1 - wb] = (uint16_t)(((lane + 32) << 10) | (e0 + bit));
-          ++pos1;
+      } else {  // the window is the whole chunk: a tile a lane
+        uint16_t *p0 = s_slot + pos0, *p1 = s_slot + pos1;
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) {
+          const uint32_t code = (lane << 10) | ((warp * kGroups + g) * 32);
+          for (uint32_t w = c.w[g][0]; w; w &= w - 1) *p0++ = (uint16_t)(code + __ffs(w) - 1);
+          for (uint32_t w = c.w[g][1]; w; w &= w - 1)
+            *p1++ = (uint16_t)(code + (32u << 10) + __ffs(w) - 1);
         }
       }
       __syncthreads();
