@@ -205,21 +205,24 @@ __global__ void __launch_bounds__(kThreads, 2)
       // past the end: the last digit, after every item of it
       dr[i] = in ? digit(key[i]) : digit.mask;
     }
+    // (the last fetch of a block finds no partition left)
+    if (__any_sync(0xffffffffu, part < num_parts)) {
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-      const uint32_t d = dr[i];
-      uint32_t peers = 0xffffffffu;
+      for (int i = 0; i < kItems; ++i) {
+        const uint32_t d = dr[i];
+        uint32_t peers = 0xffffffffu;
 #pragma unroll
-      for (int k = 0; k < kBits; ++k) {
-        const uint32_t bit = (d >> k) & 1u;
-        const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-        peers &= bit ? bal : ~bal;
+        for (int k = 0; k < kBits; ++k) {
+          const uint32_t bit = (d >> k) & 1u;
+          const uint32_t bal = __ballot_sync(0xffffffffu, bit);
+          peers &= bit ? bal : ~bal;
+        }
+        const uint32_t prior = wh[d];
+        __syncwarp();
+        if ((__ffs(peers) - 1) == lane) wh[d] = (uint16_t)(prior + __popc(peers));
+        __syncwarp();
+        dr[i] = d | ((prior + __popc(peers & lanemask_lt())) << kBits);
       }
-      const uint32_t prior = wh[d];
-      __syncwarp();
-      if ((__ffs(peers) - 1) == lane) wh[d] = (uint16_t)(prior + __popc(peers));
-      __syncwarp();
-      dr[i] = d | ((prior + __popc(peers & lanemask_lt())) << kBits);
     }
     // A: counts complete, input buffer read, the fetch had landed for everyone
     if (!__syncthreads_and(landed)) {  // bounded wait gave up: stop this block
