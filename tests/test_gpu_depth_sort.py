@@ -56,6 +56,21 @@ def test_order_equals_the_reference_stages(renderer, n, near, far):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 130_000, 311_296, 311_297])
+def test_order_at_the_partition_sizes(renderer, n):
+    """Partitions of 2048 keys up to 311,296 splats, then of 5120."""
+    r = renderer
+    w, h = 640, 480
+    data = along_the_view(n, 2.0, 60.0, n)
+    u = scenes.camera_at((0.0, 0.0, 0.0), w, h, target=(0.0, 0.0, -1.0)).getUniformData(w, h)
+    r.setSplatData(data)
+    want = frame(r, data, u, w, h, True)
+    got = frame(r, data, u, w, h, False)
+    assert want[0] > 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+
+
 def test_one_splat_among_culled_ones(renderer):
     r = renderer
     w, h = 400, 300

@@ -12,16 +12,16 @@
 // sorted arrays are then the B buffers (DepthSorted).
 //
 // With 512 bins every one of a block's 512 threads owns a digit in the offset
-// and look-back phases (of 256 bins, half of them idled there).  A partition
-// takes 10 keys a thread: 12, as 8-bit passes take, would leave one block per SM
-// beside the 16 KB of per-warp counts.
+// and look-back phases (of 256 bins, half of them idled there).
 //
 // Culled splats carry key 2^32 - 1 and are capped to the last key of the span:
 // they sort last, and where they tie with a splat at its very end they have no
 // refs to put in front of it.
 //
-// Measured (GB300), 4 x 8-bit passes -> 3 x 9-bit, histogram included: see
-// launch_sort_depth.
+// Measured (GB300), 4 x 8-bit passes -> 3 x 9-bit, histogram included: 24M
+// splat-views 795 -> 676 us, 3M 177 -> 144, 20k 69 -> 55.  A pass moves 16 bytes
+// a key; what bounds it is the ranking (issue slots 53% busy) and, below 1M
+// keys, the chain of one partition.
 #include <algorithm>
 #include <mutex>
 
@@ -32,15 +32,31 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kItems = 10;
-constexpr uint32_t kPart = kThreads * kItems;  // 5120 keys per partition
+// Keys a thread ranks: 10 (12, as 8-bit passes take, would leave one block per
+// SM beside the 16 KB of per-warp counts).  While partitions of 4 keys a thread
+// number at most one per SM, a pass is bound by one partition's chain, of which
+// ranking is 0.3 us a key: sort of 20k splats 37 -> 29 us, 100k 41 -> 34 (400k
+// with 4 keys 46 -> 47; 6 keys up to two partitions per SM: 43, but a 500k frame
+// with others beside it 464 -> 468).
+constexpr int kItems = 10, kItemsSmall = 4;
+template <int ITEMS>
+constexpr uint32_t part_of() {
+  return (uint32_t)(kThreads * ITEMS);
+}
+constexpr uint32_t kSmallSplats = 152 * part_of<kItemsSmall>();
 constexpr uint32_t kBins = 512;                // one per thread
 constexpr int kBits = 9;
 constexpr uint32_t kFlagAgg = 1u, kFlagInc = 2u;
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
 constexpr int kLookback = 16;
-constexpr size_t kBuf = (size_t)kPart * 2 * sizeof(uint32_t);
-constexpr size_t kSmem = 2 * kBuf + (size_t)kWarps * kBins * sizeof(uint16_t);
+template <int ITEMS>
+constexpr size_t buf_of() {
+  return (size_t)part_of<ITEMS>() * 2 * sizeof(uint32_t);
+}
+template <int ITEMS>
+constexpr size_t smem_of() {
+  return 2 * buf_of<ITEMS>() + (size_t)kWarps * kBins * sizeof(uint16_t);
+}
 
 // Digit p of a key under the frame's mapping.
 struct Digits {
@@ -84,7 +100,7 @@ __global__ void __launch_bounds__(kHistThreads)
     depth_histogram_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ count,
                            const DepthRange* __restrict__ range, uint32_t* __restrict__ g_hist,
                            uint32_t* __restrict__ status, size_t status_stride,
-                           ClearList clear) {
+                           uint32_t part, ClearList clear) {
   __shared__ uint32_t s_hist[kDepthPasses][kBins];
   after_predecessor(keys, count, range);
   for (int k = threadIdx.x; k < kDepthPasses * (int)kBins; k += kHistThreads)
@@ -93,7 +109,7 @@ __global__ void __launch_bounds__(kHistThreads)
   const uint32_t n = *count;
   const size_t gtid = (size_t)blockIdx.x * kHistThreads + threadIdx.x;
   const size_t gstride = (size_t)gridDim.x * kHistThreads;
-  const size_t words = (size_t)((n + kPart - 1) / kPart) * kBins;
+  const size_t words = (size_t)((n + part - 1) / part) * kBins;
   for (int p = 0; p < kDepthPasses; ++p)
     for (size_t k = gtid; k < words; k += gstride) status[p * status_stride + k] = 0u;
 #pragma unroll
@@ -136,6 +152,7 @@ __global__ void __launch_bounds__(kHistThreads)
 // One pass.  Partitions are claimed in order, late (after the look-back of the
 // current one), and fetched into the other buffer while the current one is
 // written out; barriers and waits as in sort.cu's onesweep_kernel.
+template <int ITEMS>
 __global__ void __launch_bounds__(kThreads, 2)
     depth_pass_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ ids_in,
                       uint32_t* __restrict__ keys_out, uint32_t* __restrict__ ids_out,
@@ -143,6 +160,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                       int pass, const uint32_t* __restrict__ hist, uint32_t* __restrict__ status,
                       uint32_t* __restrict__ part_counter, uint32_t* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char smem[];
+  constexpr size_t kBuf = buf_of<ITEMS>();
+  constexpr uint32_t kPart = part_of<ITEMS>();
   // [kWarps][512] per-warp digit counts, then positions of the warps' items
   uint16_t* s_whist = reinterpret_cast<uint16_t*>(smem + 2 * kBuf);
   __shared__ uint32_t s_dest[kBins];
@@ -194,10 +213,10 @@ __global__ void __launch_bounds__(kThreads, 2)
     const uint32_t part = landed ? s_part[b] : num_parts;
     const uint32_t count = part < num_parts ? min(kPart, n - part * kPart) : 0u;
 
-    uint32_t key[kItems], id[kItems], dr[kItems];  // dr: digit | rank in warp << 9
-    const uint32_t wloc = warp * (32u * kItems) + lane;
+    uint32_t key[ITEMS], id[ITEMS], dr[ITEMS];  // dr: digit | rank in warp << 9
+    const uint32_t wloc = warp * (32u * ITEMS) + lane;
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
       const uint32_t loc = wloc + i * 32u;
       const bool in = loc < count;
       key[i] = in ? s_keys[loc] : 0u;
@@ -208,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     // (the last fetch of a block finds no partition left)
     if (__any_sync(0xffffffffu, part < num_parts)) {
 #pragma unroll
-      for (int i = 0; i < kItems; ++i) {
+      for (int i = 0; i < ITEMS; ++i) {
         const uint32_t d = dr[i];
         uint32_t peers = 0xffffffffu;
 #pragma unroll
@@ -255,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
     // ---- reorder the partition in place ----
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
       const uint32_t pos = wh[dr[i] & (kBins - 1u)] + (dr[i] >> kBits);
       s_keys[pos] = key[i];
       s_ids[pos] = id[i];
@@ -315,8 +334,10 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
 }
 
+template <int ITEMS>
 cudaError_t pass_setup(int* per_sm) {
-  // once per device; contexts on other host threads may launch concurrently
+  // once per device and instance; contexts on other host threads may launch
+  // concurrently
   static std::mutex mu;
   static int v[kMaxDevices] = {};
   int dev = 0;
@@ -324,11 +345,12 @@ cudaError_t pass_setup(int* per_sm) {
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mu);
   if (v[dev] == 0) {
-    e = cudaFuncSetAttribute(depth_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kSmem);
+    e = cudaFuncSetAttribute(depth_pass_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem_of<ITEMS>());
     if (e != cudaSuccess) return e;
     int n = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, depth_pass_kernel, kThreads, kSmem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, depth_pass_kernel<ITEMS>, kThreads,
+                                                      smem_of<ITEMS>());
     if (e != cudaSuccess) return e;
     v[dev] = n > 0 ? n : 1;
   }
@@ -336,38 +358,51 @@ cudaError_t pass_setup(int* per_sm) {
   return cudaSuccess;
 }
 
-size_t status_stride(uint32_t capacity) {
-  return (((size_t)capacity + kPart - 1) / kPart + 1) * kBins;
+size_t parts_of(uint32_t n, uint32_t part) { return ((size_t)n + part - 1) / part; }
+
+template <int ITEMS>
+cudaError_t run_sort(const uint32_t* count, uint32_t n, const DepthRange* range, uint32_t* keys_a,
+                     uint32_t* ids_a, uint32_t* keys_b, uint32_t* ids_b, uint32_t* status,
+                     uint32_t* g_hist, uint32_t* part_counters, uint32_t* err,
+                     const ClearList& clear, int sm_count, LaunchStream s) {
+  int per_sm = 0;
+  cudaError_t e = pass_setup<ITEMS>(&per_sm);
+  if (e != cudaSuccess) return e;
+  constexpr uint32_t part = part_of<ITEMS>();
+  const size_t parts = std::max<size_t>(parts_of(n, part), 1);
+  const size_t stride = parts * kBins;
+  const size_t rounds = std::max<size_t>(parts_of(n, kHistThreads * kHistItems), 1);
+  launch_after(depth_histogram_kernel, (unsigned)std::min<size_t>((size_t)sm_count * 8, rounds),
+               kHistThreads, 0, s, keys_a, count, range, g_hist, status, stride, part, clear);
+  const unsigned grid = (unsigned)std::min<size_t>((size_t)sm_count * per_sm, parts);
+  for (int p = 0; p < kDepthPasses; ++p) {
+    const bool even = p % 2 == 0;
+    launch_after(depth_pass_kernel<ITEMS>, grid, kThreads, smem_of<ITEMS>(), s,
+                 even ? keys_a : keys_b, even ? ids_a : ids_b, even ? keys_b : keys_a,
+                 even ? ids_b : ids_a, count, range, p, g_hist + (size_t)p * kBins,
+                 status + p * stride, part_counters + p, err);
+  }
+  return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t depth_sort_capacity(uint32_t n) { return (size_t)n + kPart; }
-size_t depth_sort_status_words(uint32_t n) { return status_stride(n) * kDepthPasses; }
+size_t depth_sort_capacity(uint32_t n) { return (size_t)n + part_of<kItems>(); }
+// enough for every smaller count too
+size_t depth_sort_status_words(uint32_t n) {
+  const size_t parts = std::max(parts_of(std::min(n, kSmallSplats), part_of<kItemsSmall>()),
+                                parts_of(n, part_of<kItems>()));
+  return (parts + 1) * kBins * kDepthPasses;
+}
 
 cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const DepthRange* range,
                               uint32_t* keys_a, uint32_t* ids_a, uint32_t* keys_b,
                               uint32_t* ids_b, uint32_t* status, uint32_t* g_hist,
                               uint32_t* part_counters, uint32_t* err, const ClearList& clear,
                               int sm_count, LaunchStream s) {
-  int per_sm = 0;
-  cudaError_t e = pass_setup(&per_sm);
-  if (e != cudaSuccess) return e;
-  const size_t stride = status_stride(capacity);
-  const size_t parts = ((size_t)capacity + kPart - 1) / kPart;
-  const size_t rounds = ((size_t)capacity + kHistThreads * kHistItems - 1) / (kHistThreads * kHistItems);
-  launch_after(depth_histogram_kernel,
-               (unsigned)std::min<size_t>((size_t)sm_count * 8, std::max<size_t>(rounds, 1)),
-               kHistThreads, 0, s, keys_a, count, range, g_hist, status, stride, clear);
-  const unsigned grid =
-      (unsigned)std::min<size_t>((size_t)sm_count * per_sm, std::max<size_t>(parts, 1));
-  for (int p = 0; p < kDepthPasses; ++p) {
-    const bool even = p % 2 == 0;
-    launch_after(depth_pass_kernel, grid, kThreads, kSmem, s, even ? keys_a : keys_b,
-                 even ? ids_a : ids_b, even ? keys_b : keys_a, even ? ids_b : ids_a, count, range,
-                 p, g_hist + (size_t)p * kBins, status + p * stride, part_counters + p, err);
-  }
-  return cudaGetLastError();
+  const auto run = capacity <= kSmallSplats ? run_sort<kItemsSmall> : run_sort<kItems>;
+  return run(count, capacity, range, keys_a, ids_a, keys_b, ids_b, status, g_hist, part_counters,
+             err, clear, sm_count, s);
 }
 
 }  // namespace gs3d
