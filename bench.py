@@ -180,53 +180,50 @@ def algorithmic_bytes(n, R, tiles, tile_passes, sh_floats, fused, views_per_scen
     """Minimum bytes each stage must move for one view (inputs read once,
     outputs written once), the numerator of the per-stage roofline.  The
     batched preprocess reads a scene's splats once per launch for all
-    `views_per_scene` views of it, so a view is charged that share of the read."""
+    `views_per_scene` views of it, so a view is charged that share of the read.
+    The fused path sorts one entry per (splat, cell of 8x8 tiles) by cell and
+    then writes every ref once, with the tile ranges; a splat with refs is
+    charged one entry, the usual case and the least."""
     full_passes = 4 + tile_passes
+    entries = min(n, R)
     return {
         # splat SoA (64 B) + SH rest read once per scene and launch; per
         # splat-view the record and count, fused: + depth key, depth id and
         # the one-word tile rectangle
         "preprocess-splats": n * (64 + 4 * sh_floats) / views_per_scene
                              + n * (64 + 4 + (12 if fused else 0)),
-        "depth-sort": 4 * n + 4 * 16 * n,
-        "prefix-scan": 12 * n if fused else 8 * n,
+        "depth-sort": 4 * n + 3 * 16 * n,
+        # fused: depth id and one-word rectangle read, the latter and the offset written
+        "prefix-scan": 16 * n if fused else 8 * n,
         # fused: depth id, depth key, offset and one-word rectangle per splat-view
-        "emit-tile-refs": n * (4 + 4 + 4 + 4) + 12 * R if fused else n * (24 + 4) + 12 * R,
-        "radix-sort": tile_passes * 24 * R if fused else 8 * R + full_passes * 24 * R,
-        "identify-tile-ranges": 4 * R + 4 * (tiles + 1),
+        "emit-tile-refs": n * (4 + 4 + 4 + 4) + 12 * entries if fused
+                          else n * (24 + 4) + 12 * R,
+        "radix-sort": 24 * entries if fused else 8 * R + full_passes * 24 * R,
+        # fused: the entries counted (8 B), then placed (12 B) as refs (12 B)
+        "identify-tile-ranges": 20 * entries + 12 * R + 4 * (tiles + 1) if fused
+                                else 4 * R + 4 * (tiles + 1),
         "rasterize-tiles": 44 * R + 8 * WIDTH * HEIGHT,
     }
 
 
-# DRAM bytes per unit of the HBM-bound kernels, from ncu captures of a
-# 2-view batch of the same workload (profiles/), scaled to a launch by the
-# units it processes: tile-digit pass per ref (by tile size); preprocess per
-# scene splat read + per splat-view written; emit per (splat-view, ref) with
-# one-word rectangles.
-DRAM_PER_REF_PASS = {(32, 32): 22.4, (16, 16): 25.1, (64, 32): 21.2}
+# DRAM bytes of the preprocess, from an ncu capture of a 2-view batch of the same
+# workload (profiles/): per scene splat read, per splat-view written.
 DRAM_PREPROCESS = (732.1e6 / 3e6, 434.7e6 / 6e6)
-DRAM_EMIT = {(32, 32): (365.2e6, 6e6, 23.7e6), (64, 32): (273.4e6, 6e6, 16.99e6)}
 
 
-def dominant_traffic(stage, tile, refs_per_launch, splats_per_launch, scene_splats):
+def dominant_traffic(stage, splats_per_launch, scene_splats):
     """Measured DRAM bytes of one launch of the dominant HBM-bound kernel, or
     None where no capture covers it."""
-    if stage == "radix-sort" and tile in DRAM_PER_REF_PASS:
-        return int(DRAM_PER_REF_PASS[tile] * refs_per_launch)
     if stage == "preprocess-splats":
         return int(DRAM_PREPROCESS[0] * scene_splats + DRAM_PREPROCESS[1] * splats_per_launch)
-    if stage == "emit-tile-refs" and tile in DRAM_EMIT:
-        b, n, r = DRAM_EMIT[tile]
-        return int(b * (0.5 * splats_per_launch / n + 0.5 * refs_per_launch / r))
     return None
 
 
-# Pipe use of the raster kernel (ncu --set full, one launch of the headline
-# path's raster at 32x32 tiles, 2-view batch;
-# profiles/raster_culled2_t32_2views_3M_sh3_1080p.md).
-RASTER_NCU = {"kernel": "raster_kernel_culled2", "issue_active": 0.732, "pipe_fma": 0.442,
-              "pipe_alu": 0.589, "pipe_xu": 0.173, "warps_active": 0.497,
-              "source": "profiles/raster_culled2_t32_2views_3M_sh3_1080p.md (raster_t32c)"}
+# Pipe use of the raster kernel (ncu, one launch of the headline path's raster at
+# 64x32 tiles, 2-view batch; profiles/raster_warps_2views_3M_sh3_1080p.md).
+RASTER_NCU = {"kernel": "raster_kernel_warps", "issue_active": 0.606, "pipe_fma": 0.247,
+              "pipe_alu": 0.435, "pipe_xu": 0.095, "warps_active": 0.308,
+              "source": "profiles/raster_warps_2views_3M_sh3_1080p.md"}
 
 
 def raster_work(view=0, tile=TILE):
@@ -526,12 +523,14 @@ def run_ours(args, rank, world):
     dom = max(hbm, key=lambda s: batched_roof[s]["ms"])
     learned_on = batched_schedule == _lib.SCHEDULE_LEARNED
     # kernels of one batched rebin: preprocess, depth sort (histogram + 4 passes), scan, emit,
-    # tile-digit passes, identify, schedule (features + MLP + keys + split count + histogram
-    # + 2 passes + gate for the learned order; keys + split count + histogram + 2 passes for
-    # key counts; none for row-major), raster
-    sched_kernels = {_lib.SCHEDULE_ROW_MAJOR: 0, _lib.SCHEDULE_KEY_COUNT: 5,
-                     _lib.SCHEDULE_LEARNED: 8}[best_sched]
-    launches_per_batch = 1 + 5 + 1 + 1 + tuned_passes + 1 + sched_kernels + 1
+    # cell-digit passes, cell table, chunk counts, their scan, tile scan and placement, the
+    # schedule (order; features + MLP + order + gate for the learned order; none for
+    # row-major), raster
+    sched_kernels = {_lib.SCHEDULE_ROW_MAJOR: 0, _lib.SCHEDULE_KEY_COUNT: 1,
+                     _lib.SCHEDULE_LEARNED: 4}[best_sched]
+    cells = B * -(-WIDTH // (8 * tuned.tile_w)) * -(-HEIGHT // (8 * tuned.tile_h))
+    cell_passes = -(-(cells - 1).bit_length() // tuned.digit_bits)
+    launches_per_batch = 1 + 5 + 1 + 1 + cell_passes + 5 + sched_kernels + 1
     return {
         "value": views * world / (batched_ms * 1e-3), "ms_per_step": batched_ms / args.steps,
         "views": views, "per_stage": batched_roof, "dominant": dom, "peak": peak,
@@ -553,16 +552,17 @@ def run_ours(args, rank, world):
         "tuning": {"tile": [tuned.tile_w, tuned.tile_h], "digit_bits": tuned.digit_bits,
                    "raster_batch": tuned.raster_batch, "candidates": tune_table},
         "tile_passes_batched": tuned_passes,
-        "traffic": dominant_traffic(dom, (tuned.tile_w, tuned.tile_h), tuned_R * B, N_SPLATS * B,
-                                    N_SPLATS),
+        "traffic": dominant_traffic(dom, N_SPLATS * B, N_SPLATS),
         "launch_units": {"refs": int(tuned_R * B), "splat_views": N_SPLATS * B},
         "batch_median": batch_median, "c0_gpu_views_per_s": c0_gpu,
         # bytes the sort moves per view: the reference's eight 8-bit passes over
         # 12-byte refs at its 16x16 tiles (one histogram read + 8 scatters)
-        # against this path's 4 depth passes over splats + its tile-digit passes
+        # against this path's 3 depth passes over splats, its cell-digit pass over one
+        # entry per splat with refs (the least) and the refs written once
         "sort_bytes_per_view": {
             "reference_8_pass_16x16": int(8 * mean_R + 8 * 24 * mean_R),
-            "this_path": int(4 * N_SPLATS + 4 * 16 * N_SPLATS + tuned_passes * 24 * tuned_R)},
+            "this_path": int(4 * N_SPLATS + 3 * 16 * N_SPLATS
+                             + 24 * min(N_SPLATS, tuned_R) + 12 * tuned_R)},
     }
 
 

@@ -97,7 +97,7 @@ typedef struct gs3d_config {
  * same layout only rewrite the view table and replay the graph.  Stage
  * timing events are not recorded in graph mode. */
 #define GS3D_FLAG_CUDA_GRAPH      4u
-/* Shades every tile of the two-pixel raster as half-strip work items (the
+/* Shades every tile whose sides divide by 8 as half-block work items (the
  * split the key-count and learned schedules give their heaviest tiles), for
  * tests and measurements.  The image is unchanged. */
 #define GS3D_FLAG_SPLIT_ALL_TILES 8u
@@ -136,10 +136,11 @@ typedef struct gs3d_view_info {
     uint32_t scene;
 } gs3d_view_info;
 
-/* Raster work order (the persistent raster CTAs pull tiles from a queue).
- * The key-count and learned orders also split: tiles whose expected cost
- * per strip exceeds half of one raster CTA's fair share of the frame (the
- * head of the order) are shaded as two half-strip work items per strip.
+/* Raster work order (the persistent raster warps pull regions of 16x16 pixels
+ * from a queue).  The key-count and learned orders also split: tiles whose
+ * expected cost exceeds half of one raster warp's fair share of the frame and
+ * a floor (16,384 keys, a predicted 1024 splats) head the order and are shaded
+ * as two work items per 8x8 block.
  * The learned order falls back to the key count on its own while the
  * measured prediction error exceeds its bound (gs3d_set_schedule_gate). */
 #define GS3D_SCHEDULE_ROW_MAJOR 0u  /* the reference's dispatch order          */
@@ -158,7 +159,7 @@ typedef struct gs3d_schedule_status {
     float bound;           /* the gate's bound on mae_log                           */
     uint32_t frames;       /* learned frames measured since gs3d_set_cost_model     */
     uint32_t fallbacks;    /* of those, frames rendered in key-count order          */
-    uint32_t split_tiles;  /* tiles of the last raster shaded as half strips        */
+    uint32_t split_tiles;  /* tiles of the last raster shaded as half blocks        */
 } gs3d_schedule_status;
 
 /* Cost MLP (extension): 16 tile features -> 64 -> 64 -> 1, ReLU, predicting
@@ -276,14 +277,15 @@ int gs3d_set_schedule(struct gs3d_ctx* ctx, uint32_t schedule);
  * tile_w x tile_h. */
 typedef struct gs3d_tuning {
     uint32_t tile_w, tile_h;  /* tile pixel size: up to 1024 pixels, or up to 2048
-                                 with tile_w a multiple of 8 and tile_h of 16 (such
-                                 tiles are shaded by the culled two-pixel raster
-                                 only: the stage-wise rebin rejects them)             */
+                                 with tile_w a multiple of 8 and tile_h of 16 (the
+                                 stage-wise rebin rejects tiles above 1024 pixels)    */
     uint32_t digit_bits;      /* widest radix digit of the tile-id passes: 4, 6, 8 or
                                  11 (fused rebin; the stage-wise sort uses at most 8);
                                  8 when narrower digits would need over 4 passes     */
-    uint32_t raster_batch;    /* splats staged per raster batch: a multiple of 32 in
-                                 [32, 1024]; 0 = one per tile pixel (at most 1024)    */
+    uint32_t raster_batch;    /* splats staged per raster batch where a tile is shaded
+                                 by one CTA (sides that do not divide by 8): a multiple
+                                 of 32 in [32, 1024]; 0 = one per tile pixel (at most
+                                 1024)                                                */
 } gs3d_tuning;
 
 typedef struct gs3d_tune_result {

@@ -651,9 +651,10 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
 // Do the refs go through cells (binning.cu) or through the digit passes over
 // the refs themselves?  Cells take three launches more, so they pay where the
 // refs outweigh a launch: sum of the stages from scan to tile ranges, passes ->
-// cells, 20k splats 51 -> 69 us, 100k 79 -> 87 us, 400k 110 -> 109 us, 3M (16x16
-// tiles) 623 -> 294 us, 8 views of 3M (64x32) 1743 -> 1306 us, 3M heavy-tailed
-// splats at 4K (32x32) 3317 -> 815 us.
+// cells when they were first compared, 20k splats 51 -> 69 us, 100k 79 -> 87,
+// 400k 110 -> 109, 3M (16x16 tiles) 623 -> 294, 8 views of 3M (64x32) 1743 ->
+// 1306, 3M heavy-tailed splats at 4K (32x32) 3317 -> 815 (now 39 us by passes at
+// 20k, and by cells 84 at 400k, 265, 1250 and 505).
 constexpr uint32_t kCellsMinSplats = 300000;
 bool use_cells(const gs3d_ctx* c) {
   bool fits = c->total_cells <= kMaxCells && c->total_splats >= kCellsMinSplats;

@@ -178,7 +178,8 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
   // the depth bits come in order from the depth sort, the ref count from the
   // scan's offsets (0 for culled splats, whose rectangle is zeroed) (or,
   // where every view's tile grid fits 8 bits, the 4-byte word of the
-  // preprocess's compact rectangle array, which stays in L2)
+  // preprocess's compact rectangle array; for cells the scan has put those words
+  // in depth order)
   auto gather = [&](uint32_t c) {
     if (c >= chunks || c * kThreads + threadIdx.x >= n) return;
     if (rect8 != nullptr) {
@@ -215,11 +216,11 @@ __global__ void __launch_bounds__(kThreads, BINS <= 256 ? 8 : 1)
         s_rb[threadIdx.x] = make_uint4(__ldg(&views[v].cell_base) + cy0 * cx + cx0, p_key, id,
                                        p_rect.z | (p_rect.w << 16));
       } else {
-      const uint32_t tx = __ldg(&views[v].f.tile_count[0]);
-      // ref k of the splat: row = k / w, tile = first + row * tx + (k - row * w)
-      //                                      = first + row * (tx - w) + k
-      s_ra[threadIdx.x] = make_uint4(w * h, w, __float_as_uint(1.0f / (float)w), tx - w);
-      s_rb[threadIdx.x] = make_uint4(__ldg(&views[v].f.tile_base) + y0 * tx + x0, p_key, id, 0u);
+        const uint32_t tx = __ldg(&views[v].f.tile_count[0]);
+        // ref k of the splat: row = k / w, tile = first + row * tx + (k - row * w)
+        //                                      = first + row * (tx - w) + k
+        s_ra[threadIdx.x] = make_uint4(w * h, w, __float_as_uint(1.0f / (float)w), tx - w);
+        s_rb[threadIdx.x] = make_uint4(__ldg(&views[v].f.tile_base) + y0 * tx + x0, p_key, id, 0u);
       }
     }
     const uint32_t last = min(n, first + kThreads);
@@ -348,7 +349,8 @@ cudaError_t emit_ordered(const ViewDesc* views, uint32_t n_views, uint32_t n,
                          const DepthSorted& sorted, const uint32_t* sorted_offsets,
                          const uint32_t* counter, CellArgs cells,
                          uint32_t capacity, uint2* keys, uint32_t* values, const SortPlan& plan,
-                         const StatusClear& sort_status, uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
+                         const StatusClear& sort_status, uint32_t* g_hist,
+                         uint32_t* chunk_ticket, uint32_t* err, int sm_count,
                          LaunchStream s) {
   if (n == 0) return cudaSuccess;
   const uint32_t chunks = (n + kThreads - 1) / kThreads;
@@ -401,8 +403,8 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
                                const uint32_t* sorted_offsets, const uint32_t* ref_counter,
                                uint32_t capacity, uint2* keys, uint32_t* values,
                                const SortPlan& tile_plan, const StatusClear& sort_status,
-                               uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count,
-                               LaunchStream s) {
+                               uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err,
+                               int sm_count, LaunchStream s) {
   return emit_ordered<false>(views, n_views, n, proj, rect8, sorted, sorted_offsets,
                              ref_counter, CellArgs{}, capacity, keys, values,
                              tile_plan, sort_status, g_hist, chunk_ticket, err, sm_count, s);
@@ -411,10 +413,12 @@ cudaError_t launch_emit_sorted(const ViewDesc* views, uint32_t n_views, uint32_t
 cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t n,
                               const gs3d_projected_splat* proj, const uint32_t* rect8,
                               const DepthSorted& sorted, const uint32_t* sorted_offsets,
-                              uint32_t* entry_total, const unsigned long long* ref_total, uint32_t* ref_counter,
+                              uint32_t* entry_total, const unsigned long long* ref_total,
+                              uint32_t* ref_counter,
                               uint32_t capacity, uint2* keys, uint32_t* values,
                               const SortPlan& cell_plan, const StatusClear& sort_status,
-                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err, int sm_count, LaunchStream s) {
+                              uint32_t* g_hist, uint32_t* chunk_ticket, uint32_t* err,
+                              int sm_count, LaunchStream s) {
   return emit_ordered<true>(views, n_views, n, proj, rect8, sorted, sorted_offsets, entry_total,
                             CellArgs{ref_total, ref_counter, entry_total},
                             capacity, keys, values, cell_plan, sort_status, g_hist, chunk_ticket,

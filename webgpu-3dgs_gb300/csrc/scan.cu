@@ -9,8 +9,9 @@
 // offsets[n] = ref_counter[0] = total.
 //
 // Status words are 64-bit: [63:34] launch epoch, [33:32] flag, [31:0] value.
-// The epoch changes every launch, so the status array never needs clearing;
-// entries carrying another epoch read as "not ready".  Prefixes are summed in
+// Entries carrying another epoch than the launch's read as "not ready"; the
+// depth sort's first kernel also zeroes the words, since a replayed graph repeats
+// its epoch.  Prefixes are summed in
 // 64 bits; a total that does not fit 32 bits saturates at 0xffffffff and
 // latches DEVERR_CAPACITY (no rebin can hold that many refs).
 #include "gs3d_internal.cuh"
@@ -56,9 +57,10 @@ __device__ __forceinline__ uint32_t rect_cells(uint32_t x0, uint32_t y0, uint32_
 
 template <Scan KIND>
 __global__ void __launch_bounds__(kThreads)
-    scan_kernel(const uint32_t* __restrict__ in, DepthSorted order, ScanExtra ex, uint32_t* __restrict__ out, uint32_t n,
-                unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket,
-                uint32_t epoch, uint32_t* __restrict__ total_out, uint32_t* __restrict__ err) {
+    scan_kernel(const uint32_t* __restrict__ in, DepthSorted order, ScanExtra ex,
+                uint32_t* __restrict__ out, uint32_t n, unsigned long long* __restrict__ status,
+                uint32_t* __restrict__ ticket, uint32_t epoch, uint32_t* __restrict__ total_out,
+                uint32_t* __restrict__ err) {
   __shared__ uint32_t s_tile, s_prefix;
   __shared__ uint32_t s_warp[kThreads / 32];
   __shared__ unsigned long long s_refs[kThreads / 32];
@@ -99,7 +101,11 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) refs += __shfl_xor_sync(0xffffffffu, refs, o);
     if (lane == 0) s_refs[warp] = refs;
-    if (KIND == Scan::cells8 && base < n) {  // whole groups of 8 fit the array
+    // Rectangles in depth order for the emit (whole groups of 8 fit the array).
+    // The gather is what bounds this kernel: one L2 request a splat-view, 100 G
+    // a second (24M splat-views 264 us; wider look-back windows and tiles of
+    // 1024 to 8192 made no difference).
+    if (KIND == Scan::cells8 && base < n) {
       uint4* r4 = reinterpret_cast<uint4*>(order.rects() + base);
       r4[0] = make_uint4(rect[0], rect[1], rect[2], rect[3]);
       r4[1] = make_uint4(rect[4], rect[5], rect[6], rect[7]);

@@ -187,7 +187,7 @@ class GaussianSplatRenderer:
         return {f: getattr(st, f) for f, _ in st._fields_}
 
     def setSplitAllTiles(self, on: bool) -> None:
-        """Shades every tile as half-strip work items (testing the split; the
+        """Shades every tile as half-block work items (testing the split; the
         image is unchanged)."""
         self._flags = (getattr(self, "_flags", 0) & ~_lib.FLAG_SPLIT_ALL_TILES) | \
             (_lib.FLAG_SPLIT_ALL_TILES if on else 0)
