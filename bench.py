@@ -176,16 +176,16 @@ def cpu_c0_stages(threads):
             "stage_ms": {k: round(v * 1e3, 2) for k, v in t.items()}}
 
 
-def algorithmic_bytes(n, R, tiles, tile_passes, sh_floats, fused, views_per_scene=1):
+def algorithmic_bytes(n, R, tiles, tile_passes, sh_floats, fused, views_per_scene=1,
+                      entries=0):
     """Minimum bytes each stage must move for one view (inputs read once,
     outputs written once), the numerator of the per-stage roofline.  The
     batched preprocess reads a scene's splats once per launch for all
     `views_per_scene` views of it, so a view is charged that share of the read.
     The fused path sorts one entry per (splat, cell of 8x8 tiles) by cell and
-    then writes every ref once, with the tile ranges; a splat with refs is
-    charged one entry, the usual case and the least."""
+    then writes every ref once, with the tile ranges; `entries` is the splats
+    with refs, which have one each at least."""
     full_passes = 4 + tile_passes
-    entries = min(n, R)
     return {
         # splat SoA (64 B) + SH rest read once per scene and launch; per
         # splat-view the record and count, fused: + depth key, depth id and
@@ -417,6 +417,9 @@ def run_ours(args, rank, world):
                     "samples": len(per_view_ms)}
     check(lib.gs3d_set_flags(ctx, 0))
     eager_ms, batched_stages, _ = timed("batched", best_sched)  # per-stage events
+    counts = np.empty(N_SPLATS * len(batches[-1]), np.uint32)  # refs of the last batch's splats
+    check(lib.gs3d_read_buffer(ctx, 6, counts.ctypes.data_as(C.c_void_p), counts.nbytes))
+    visible = float(np.count_nonzero(counts)) / len(batches[-1])
     # each work order on the tuned batched path (same image): graph-replay
     # views/s and the raster's eager per-stage time
     sched_batched = {}
@@ -510,7 +513,8 @@ def run_ours(args, rank, world):
     peak, peak_kind = peaks()
 
     def roof(stages, fused, R, tiles, passes, tile_px, views_per_scene=1):
-        algo = algorithmic_bytes(N_SPLATS, R, tiles, passes, 45, fused, views_per_scene)
+        algo = algorithmic_bytes(N_SPLATS, R, tiles, passes, 45, fused, views_per_scene,
+                                 visible)
         out = {}
         for name, (ms, n) in stages.items():
             gbs = algo[name] / (ms * 1e-3) / 1e9
@@ -562,7 +566,7 @@ def run_ours(args, rank, world):
         "sort_bytes_per_view": {
             "reference_8_pass_16x16": int(8 * mean_R + 8 * 24 * mean_R),
             "this_path": int(4 * N_SPLATS + 3 * 16 * N_SPLATS
-                             + 24 * min(N_SPLATS, tuned_R) + 12 * tuned_R)},
+                             + 24 * visible + 12 * tuned_R)},
     }
 
 

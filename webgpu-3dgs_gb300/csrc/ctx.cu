@@ -653,7 +653,7 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
 // refs outweigh a launch: sum of the stages from scan to tile ranges, passes ->
 // cells when they were first compared, 20k splats 51 -> 69 us, 100k 79 -> 87,
 // 400k 110 -> 109, 3M (16x16 tiles) 623 -> 294, 8 views of 3M (64x32) 1743 ->
-// 1306, 3M heavy-tailed splats at 4K (32x32) 3317 -> 815 (now 39 us by passes at
+// 1306, 3M heavy-tailed splats at 4K (32x32) 3317 -> 815 (now 41 us by passes at
 // 20k, and by cells 84 at 400k, 265, 1250 and 505).
 constexpr uint32_t kCellsMinSplats = 300000;
 bool use_cells(const gs3d_ctx* c) {

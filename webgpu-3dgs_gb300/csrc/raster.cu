@@ -37,8 +37,8 @@
 //
 // Bound: instruction issue (61% busy, ALU 43%, 20 warps an SM; DRAM under 10%).
 // One strip of a tile per CTA -> independent warps over regions, cull per
-// region, blocks handed on: 8 views of 3M splats 3540 -> 2530 us, 12 mixed views
-// 4420 -> 3800, one 3M frame 500 -> 350, 100k 124 -> 60.
+// region, blocks handed on: 8 views of 3M splats 3935 -> 2530 us, 12 mixed views
+// 5580 -> 3800, one 3M frame 425 -> 350, 100k 74 -> 60.
 #include <algorithm>
 #include <map>
 #include <mutex>
