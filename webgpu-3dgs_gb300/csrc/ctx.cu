@@ -533,8 +533,9 @@ SortPlan tile_digit_plan(uint32_t num_tiles, uint32_t digit_bits) {
   return tp;
 }
 
-// A fused rebin's kernels are launched while their predecessors drain up to
-// this many splat-views (frame of 20k splats 171 -> 142 us, 100k 229 -> 209,
+// A fused rebin's kernels, and the passes of the stage-wise sort, are launched
+// while their predecessors drain up to this many splat-views (six stages of 150k
+// splats 136 -> 132 us; frame of 20k splats 171 -> 142 us, 100k 229 -> 209,
 // 400k 376 -> 344, 3M 983 -> 956; eight views of 3M, whose kernels run for
 // 200 us and more, 5664 -> 5708).
 constexpr uint32_t kDependentSplats = 1u << 23;
@@ -1292,7 +1293,7 @@ int gs3d_radix_sort(gs3d_ctx* c) {
     StageScope t(c, GS3D_STAGE_SORT);
     CK(launch_sort(plan, u32(c->ref_counter), c->capacity, static_cast<uint2*>(c->keys_a.p),
                    u32(c->vals_a), static_cast<uint2*>(c->keys_b.p), u32(c->vals_b),
-                   u32(c->sort_status), ctrl_of(c), c->sm_count, c->stream),
+                   u32(c->sort_status), ctrl_of(c), c->sm_count, chain_stream(c)),
        "radix sort");
   }
   if (plan.passes % 2) {  // sorted data ended in the B buffers: rename

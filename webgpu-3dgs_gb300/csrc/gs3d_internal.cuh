@@ -414,7 +414,7 @@ cudaError_t launch_emit(const FrameUniforms* d_frame, uint32_t n,
                         uint32_t* values, uint32_t* err, cudaStream_t s);
 cudaError_t launch_sort(const SortPlan& plan, const uint32_t* ref_counter, uint32_t capacity,
                         uint2* keys_a, uint32_t* vals_a, uint2* keys_b, uint32_t* vals_b,
-                        uint32_t* status, Ctrl* ctrl, int sm_count, cudaStream_t s);
+                        uint32_t* status, Ctrl* ctrl, int sm_count, LaunchStream s);
 size_t sort_status_words(uint32_t capacity, int passes);
 // Status words any sort plan of a capacity needs (11-bit tile passes included).
 size_t sort_status_words_max(uint32_t capacity);

@@ -941,7 +941,7 @@ StatusClear tile_sort_status(const SortPlan& plan, uint32_t capacity, uint32_t* 
 
 cudaError_t launch_sort(const SortPlan& plan, const uint32_t* ref_counter, uint32_t capacity,
                         uint2* keys_a, uint32_t* vals_a, uint2* keys_b, uint32_t* vals_b,
-                        uint32_t* status, Ctrl* ctrl, int sm_count, cudaStream_t s) {
+                        uint32_t* status, Ctrl* ctrl, int sm_count, LaunchStream s) {
   // the sort may run more than once per frame: its tickets and histograms
   cudaError_t e = cudaMemsetAsync(ctrl->sort_part_counter, 0, sizeof(ctrl->sort_part_counter), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(ctrl->sort_hist, 0, sizeof(ctrl->sort_hist), s);
