@@ -381,7 +381,7 @@ struct BackwardSmem {
   float w2[kHidden][kPitch];  // [unit of layer 2][unit of layer 1]
   float x[kTile * kPitchX];
   float h1[kTile * kPitch], d2[kTile * kPitch], d1[kTile * kPitch];
-  float b1[kHidden];
+  float b1[kHidden], b2[kHidden], w3[kHidden], b3;  // the block's sums
 };
 // Gradient of the mean squared error (y - target)^2 over n samples, added
 // into grads (same layout as params; must be zeroed by the caller).  The weight
@@ -403,7 +403,8 @@ __global__ void __launch_bounds__(kTrainThreads, 2)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int k = tid; k < kHidden * kHidden; k += kTrainThreads)
     sm.w2[k / kHidden][k % kHidden] = __ldg(W2 + k);
-  if (tid < kHidden) sm.b1[tid] = 0.f;
+  if (tid < kHidden) sm.b1[tid] = sm.b2[tid] = sm.w3[tid] = 0.f;
+  if (tid == 0) sm.b3 = 0.f;
   const float w3[2] = {__ldg(W3 + lane), __ldg(W3 + 32 + lane)};
   const int s0 = tid / 16 * 4, u0 = tid % 16 * 4;
   float g2[4][4] = {};     // d W2[s0 + i][u0 + u] (rows: units of layer 2)
@@ -485,12 +486,19 @@ __global__ void __launch_bounds__(kTrainThreads, 2)
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    atomicAdd(gB2 + h * 32 + lane, gb2[h]);
-    atomicAdd(gW3 + h * 32 + lane, gw3[h]);
+    atomicAdd(&sm.b2[h * 32 + lane], gb2[h]);
+    atomicAdd(&sm.w3[h * 32 + lane], gw3[h]);
   }
-  if (lane == 0) atomicAdd(gB3, gb3);
+  if (lane == 0) atomicAdd(&sm.b3, gb3);
   __syncthreads();
-  if (tid < kHidden) atomicAdd(gB1 + tid, sm.b1[tid]);
+  // one add per block into each gradient: the fewer, the smaller the rounding of
+  // their sum
+  if (tid < kHidden) {
+    atomicAdd(gB1 + tid, sm.b1[tid]);
+    atomicAdd(gB2 + tid, sm.b2[tid]);
+    atomicAdd(gW3 + tid, sm.w3[tid]);
+  }
+  if (tid == 0) atomicAdd(gB3, sm.b3);
 }
 
 // Blocks of a training launch: the resident ones, at most one per tile.
