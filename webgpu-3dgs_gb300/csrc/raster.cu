@@ -72,10 +72,13 @@ struct SplatStage {  // first 48 bytes of a ProjectedSplat, prepared in place (p
 
 constexpr float kHalfLog2e = 0.72134752044448170f;
 constexpr float kExactFormBound = 4096.0f;
-constexpr float kCircleOnly = 3.0e38f;  // vis of splats culled by their circle alone
 // How a splat's alpha is evaluated: fast form whose op exp(power) stays below
 // the 0.99 clamp; fast form with the clamp; exact form (which clamps).
 constexpr uint32_t kSimple = 0u, kClamped = 1u, kExact = 2u;
+// vis of splats culled by their circle alone, 3.0e38.  Its two low bits are clear:
+// prepare leaves the kind there, and every kind has to stay at or above it.
+constexpr float kCircleOnly = 0x1.c363c8p+127f;
+static_assert((__builtin_bit_cast(uint32_t, kCircleOnly) & 3u) == 0u, "room for the kind");
 
 struct Pixel {
   float cr, cg, cb, T;
