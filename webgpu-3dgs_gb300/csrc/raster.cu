@@ -95,7 +95,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // opacity | color, valid) into the raster form.  vis = the largest Q at which
 // alpha can still reach 1/255, with a 1% margin, in the units of the splat's
 // form (-1: never visible; kCircleOnly or more: use the circle only: a conic
-// with a non-positive diagonal, or a non-finite opacity or conic).
+// with a non-positive diagonal, or anything not finite, whose NaN alphas pass as
+// 0.99 whatever the opacity).
 //
 // vis also carries the rounding of the quadratic form, so that the cull stays
 // conservative for any conic, needles included (condition numbers of 10^3
@@ -115,13 +116,15 @@ __device__ __forceinline__ void prepare(SplatStage& s, float ext) {
   const float4 a = s.a, b = s.b;
   const float A = b.x, B = b.y, C = b.z, op = b.w;
   const float sum = fabsf(A) + 2.0f * fabsf(B) + fabsf(C);
+  // the form's terms anywhere near the circle, NaN or infinite where the mean, the
+  // radius or the conic is; lim is NaN there
+  const float reach = a.w + ext, near = fmaf(0.0f, a.x + a.y, sum * reach * reach);
+  const float lim = fmaf(0.0f, near, op * 255.0f);
   float vis;
-  const float lim = op * 255.0f;
   if (lim < 0.999f) {
     vis = -1.0f;  // alpha = opacity * exp(power) <= opacity < 1/255 everywhere
   } else {
-    const float reach = a.w + ext;
-    vis = __log2f(lim) * 1.01f + 1e-3f + (kHalfLog2e * 9.5367431640625e-07f) * sum * reach * reach;
+    vis = __log2f(lim) * 1.01f + 1e-3f + (kHalfLog2e * 9.5367431640625e-07f) * near;
     // false for NaNs too
     if (!(lim > 1.0f && A > 0.0f && C > 0.0f && vis < 1.0e38f)) vis = kCircleOnly;
   }
@@ -386,6 +389,12 @@ __device__ __forceinline__ void stage_batch(const gs3d_projected_splat* __restri
   cp_async_commit();
 }
 
+// x clamped to [lo, hi]; NaN where a bound is (fminf and fmaxf drop it).
+__device__ __forceinline__ float clamp_nan(float x, float lo, float hi) {
+  asm("max.NaN.f32 %0, %0, %1;\n min.NaN.f32 %0, %0, %2;" : "+f"(x) : "f"(lo), "f"(hi));
+  return x;
+}
+
 // Can the splat reach alpha >= 1/255 inside the rectangle of pixel centres
 // [x0,x1] x [y0,y1]?  Minimum of the splat's q over the rectangle
 // (scale-invariant, so either form works), compared with vis; plus the radius
@@ -395,14 +404,14 @@ __device__ __forceinline__ void stage_batch(const gs3d_projected_splat* __restri
 // made indefinite.  Along an edge q is convex (the conic's diagonal is
 // positive), so its minimum there is at the clamped stationary point.
 // Conservative by the margins folded into vis (prepare) and the circle.  NaN
-// means, radii, conics or opacities are never culled (the per-pixel tests
-// decide, as in the reference).
+// means (one coordinate or both), radii, conics or opacities are never culled (the
+// per-pixel tests decide, as in the reference): no comparison with a NaN culls.
 __device__ __forceinline__ bool rect_may_hit(const float4 a, const float4 b, float2 xr,
                                              float2 yr) {
   // the box corners relative to the mean (x - m computed as x + (-m))
   const float2 xd = __fadd2_rn(xr, bcast(-a.x)), yd = __fadd2_rn(yr, bcast(-a.y));
   const float x0 = xd.x, x1 = xd.y, y0 = yd.x, y1 = yd.y;
-  const float ex = fminf(fmaxf(0.0f, x0), x1), ey = fminf(fmaxf(0.0f, y0), y1);
+  const float ex = clamp_nan(0.0f, x0, x1), ey = clamp_nan(0.0f, y0, y1);
   const float vis = b.w;
   if (ex * ex + ey * ey > a.z * 1.0001f + 1e-3f || vis < 0.0f) return false;
   const float qa = b.x, qb = b.y, qc = b.z;
