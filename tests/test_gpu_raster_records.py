@@ -1,5 +1,6 @@
-"""The raster on projected records written as they are: conics, means and radii
-that are not finite, opacities around every bound.  A splat may be skipped for a block of pixels only where no
+"""The raster on projected records written as they are: conics that are not
+positive definite or not finite, means and radii that are not finite, opacities
+around every bound.  A splat may be skipped for a block of pixels only where no
 pixel of it passes the per-pixel tests, which a NaN alpha does (as 0.99).  Tiles
 of 15x15 pixels are shaded pixel by pixel, without a cull, and an image does not
 depend on the tile grid: every other shape has to give that image bit for bit."""
@@ -83,6 +84,10 @@ CASES = {
     "nan conic": (holed(np.nan), FAINT + STRONG, RADII, None),
     "infinite conic": (holed(np.inf), FAINT + STRONG, RADII, None),
     "huge conic": (holed(3e38), FAINT + STRONG, RADII, None),
+    "zero conic": (holed(0.0), FAINT + STRONG, RADII, None),
+    "negative definite": (around(-1, -1, 0.2), FAINT + STRONG, RADII, None),
+    "one diagonal negative": (around(-1, 1, 0.2), FAINT + STRONG, RADII, None),
+    "indefinite": (around(1, 1, 6.0), FAINT + STRONG, RADII, None),
     "odd opacities": (around(1, 1, 0.15), ODD, RADII, None),
     "nan mean": (around(1, 1, 0.15), FAINT + STRONG, RADII, np.nan),
     "infinite mean": (around(1, 1, 0.15), FAINT + STRONG, RADII, np.inf),

@@ -72,6 +72,7 @@ struct SplatStage {  // first 48 bytes of a ProjectedSplat, prepared in place (p
 
 constexpr float kHalfLog2e = 0.72134752044448170f;
 constexpr float kExactFormBound = 4096.0f;
+constexpr float kInf = __builtin_huge_valf();
 // How a splat's alpha is evaluated: fast form whose op exp(power) stays below
 // the 0.99 clamp; fast form with the clamp; exact form (which clamps).
 constexpr uint32_t kSimple = 0u, kClamped = 1u, kExact = 2u;
@@ -120,20 +121,24 @@ __device__ __forceinline__ void prepare(SplatStage& s, float ext) {
   // radius or the conic is; lim is NaN there
   const float reach = a.w + ext, near = fmaf(0.0f, a.x + a.y, sum * reach * reach);
   const float lim = fmaf(0.0f, near, op * 255.0f);
+  const float r2 = a.w * a.w;
+  const float terms = sum * r2;
+  const bool fast = terms <= kExactFormBound;
+  // q >= t / 800 then, far above its rounding; a projected splat's fast form has
+  // B^2 < 0.992 A C (its condition number is below 455)
+  const bool positive = A > 0.0f && B * B <= 0.995f * A * C;
   float vis;
-  if (lim < 0.999f) {
+  if (lim < 0.999f && (positive || !fast)) {
     vis = -1.0f;  // alpha = opacity * exp(power) <= opacity < 1/255 everywhere
   } else {
     vis = __log2f(lim) * 1.01f + 1e-3f + (kHalfLog2e * 9.5367431640625e-07f) * near;
     // false for NaNs too
     if (!(lim > 1.0f && A > 0.0f && C > 0.0f && vis < 1.0e38f)) vis = kCircleOnly;
   }
-  const float r2 = a.w * a.w;
-  const float terms = sum * r2;
   s.a = make_float4(a.x, a.y, r2, op);
-  if (terms <= kExactFormBound) {
+  if (fast) {
     // no clamp where ex2 of a value <= 0 (to 2 ulp) times op stays below it
-    const bool simple = op <= 0.9899f && fabsf(a.x) + fabsf(a.y) < 3.0e38f;
+    const bool simple = lim <= 0.9899f * 255.0f && positive;
     vis = __uint_as_float((__float_as_uint(vis) & ~3u) | (simple ? kSimple : kClamped));
     s.b = make_float4(kHalfLog2e * A, 2.0f * kHalfLog2e * B, kHalfLog2e * C, vis);
     s.c.w = 0.0f;
@@ -287,8 +292,7 @@ __device__ __forceinline__ float2 exact_alpha(float pfx, float2 pfy, const Splat
 }
 // The same for a splat of either form: both are evaluated and one is taken, so
 // that four of a step overlap (a branch per splat costs more than the few
-// operations that the forms do not share).  The q < 0 and clamp tests cannot
-// act on a fast-form splat that has none.
+// operations that the forms do not share).  The fast form has no q < 0 test.
 __device__ __forceinline__ float any_alpha(float pfx, float pfy, const SplatStage& s, bool exact) {
   const float4 a = s.a, b = s.b;
   const float dx = pfx - a.x;
@@ -299,9 +303,9 @@ __device__ __forceinline__ float any_alpha(float pfx, float pfy, const SplatStag
   const float qe = __fadd_rn(__fadd_rn(__fmul_rn(u, dx), __fmul_rn(v, dy)), w);
   const float qf = fmaf(u, dx, fmaf(v, dy, w));
   const float d2 = exact ? __fadd_rn(__fmul_rn(dx, dx), dyy) : fmaf(dx, dx, dyy);
-  const float q = exact ? qe : qf;
+  const float q = exact ? qe : qf, least = exact ? 0.0f : -kInf;
   const float alpha = fminf(0.99f, a.w * ex2_approx(__fmul_rn(q, exact ? -kHalfLog2e : -1.0f)));
-  return !(d2 > a.z) && !(q < 0.0f) && !(alpha < 1.0f / 255.0f) ? alpha : 0.0f;
+  return !(d2 > a.z) && !(q < least) && !(alpha < 1.0f / 255.0f) ? alpha : 0.0f;
 }
 __device__ __forceinline__ float2 any_alpha(float pfx, float2 pfy, const SplatStage& s,
                                             bool exact) {
@@ -321,12 +325,13 @@ __device__ __forceinline__ float2 any_alpha(float pfx, float2 pfy, const SplatSt
                                exact ? __fadd_rn(__fadd_rn(t1, t2.y), w.y) : qf.y);
   const float2 d2 =
       make_float2(exact ? __fadd_rn(dxx, dyy.x) : df.x, exact ? __fadd_rn(dxx, dyy.y) : df.y);
+  const float least = exact ? 0.0f : -kInf;
   const float2 ev = __fmul2_rn(q, bcast(exact ? -kHalfLog2e : -1.0f));
   const float2 am = __fmul2_rn(bcast(a.w), make_float2(ex2_approx(ev.x), ex2_approx(ev.y)));
   const float2 alpha = make_float2(fminf(0.99f, am.x), fminf(0.99f, am.y));
   return make_float2(
-      !(d2.x > a.z) && !(q.x < 0.0f) && !(alpha.x < 1.0f / 255.0f) ? alpha.x : 0.0f,
-      !(d2.y > a.z) && !(q.y < 0.0f) && !(alpha.y < 1.0f / 255.0f) ? alpha.y : 0.0f);
+      !(d2.x > a.z) && !(q.x < least) && !(alpha.x < 1.0f / 255.0f) ? alpha.x : 0.0f,
+      !(d2.y > a.z) && !(q.y < least) && !(alpha.y < 1.0f / 255.0f) ? alpha.y : 0.0f);
 }
 
 // The blend state of a lane's pixels: one (Px1) or two of a column (Px2).
