@@ -65,6 +65,11 @@ def around(sign_a, sign_c, mix):
     return f
 
 
+def steep(rng, r):
+    """Terms of some hundreds at the edge: exp underflows inside the circle."""
+    return 80 * around(1, 1, 0.15)(rng, r)
+
+
 def holed(value):
     """Positive definite ones, one entry of every other splat replaced."""
     def f(rng, r):
@@ -89,6 +94,7 @@ CASES = {
     "one diagonal negative": (around(-1, 1, 0.2), FAINT + STRONG, RADII, None),
     "indefinite": (around(1, 1, 6.0), FAINT + STRONG, RADII, None),
     "odd opacities": (around(1, 1, 0.15), ODD, RADII, None),
+    "odd opacities, steep": (steep, ODD, RADII, None),
     "nan mean": (around(1, 1, 0.15), FAINT + STRONG, RADII, np.nan),
     "infinite mean": (around(1, 1, 0.15), FAINT + STRONG, RADII, np.inf),
     "odd radii": (around(1, 1, 0.15), FAINT + STRONG, [2, 60, np.nan, np.inf, 1e20, 0.0], None),

@@ -118,8 +118,9 @@ __device__ __forceinline__ void prepare(SplatStage& s, float ext) {
   const float A = b.x, B = b.y, C = b.z, op = b.w;
   const float sum = fabsf(A) + 2.0f * fabsf(B) + fabsf(C);
   // the form's terms anywhere near the circle, NaN or infinite where the mean, the
-  // radius or the conic is; lim is NaN there
-  const float reach = a.w + ext, near = fmaf(0.0f, a.x + a.y, sum * reach * reach);
+  // radius, the conic or the opacity is (an infinite one gives NaN where exp
+  // underflows); lim is NaN there
+  const float reach = a.w + ext, near = fmaf(0.0f, a.x + a.y + op, sum * reach * reach);
   const float lim = fmaf(0.0f, near, op * 255.0f);
   const float r2 = a.w * a.w;
   const float terms = sum * r2;
