@@ -101,6 +101,9 @@ typedef struct gs3d_config {
  * split the key-count and learned schedules give their heaviest tiles), for
  * tests and measurements.  The image is unchanged. */
 #define GS3D_FLAG_SPLIT_ALL_TILES 8u
+/* Raster warps without work give up waiting for some after a few polls instead
+ * of about a second, for tests.  The image is unchanged. */
+#define GS3D_FLAG_BRIEF_WAITS     16u
 
 /* Stage indices of gs3d_read_stage_times (the reference's profiler labels,
  * GaussianSplatRenderer.ts:1144-1260, plus the fused path's depth sort). */
@@ -190,7 +193,11 @@ typedef enum gs3d_buffer {
     GS3D_BUF_SPLAT_TARGET      = 14, /* rgba16float x W x H (premultiplied)        */
     GS3D_BUF_TILE_COSTS        = 15, /* u32 x T: splats iterated before the tile's
                                         last pixel terminated (extension)          */
-    GS3D_BUF_COUNT_            = 16
+    GS3D_BUF_RASTER_POOL       = 16, /* u32 x 8, of the last raster: blocks sent to
+                                        waiting warps, places taken by those, warps
+                                        waiting, warps present, waits that ran out,
+                                        blocks taken back; 0, 0 (extension)         */
+    GS3D_BUF_COUNT_            = 17
 } gs3d_buffer;
 
 /* ---- lifetime ----------------------------------------------------------- */

@@ -95,6 +95,7 @@ struct gs3d_ctx {
   DevBuf model_params, model_mean, model_inv_std, tile_feats, tile_preds;
   DevBuf tile_est;    // expected cost per tile of the last ordered raster
   DevBuf raster_pool; // blocks handed on between raster warps
+  DevBuf pool_words;  // their counters (in the control block, not owned)
   DevBuf gate;        // SchedGate: the learned schedule's fallback gate
   float gate_bound = 0.5f;
 
@@ -454,10 +455,7 @@ int set_views(gs3d_ctx* c, const gs3d_view* views, uint32_t n_views, bool upload
   TRY(ensure(c, c->tile_feats, std::max<uint64_t>(tiles, 1) * kFeatures * 4, "tile features"));
   TRY(ensure(c, c->tile_preds, std::max<uint64_t>(tiles, 1) * 4, "tile cost predictions"));
   TRY(ensure(c, c->tile_est, std::max<uint64_t>(tiles, 1) * 4, "tile expected costs"));
-  if (!c->raster_pool.p) {
-    TRY(ensure(c, c->raster_pool, raster_pool_bytes(), "raster pool"));
-    CK(cudaMemsetAsync(c->raster_pool.p, 0, raster_pool_bytes(), c->stream), "raster pool");
-  }
+  TRY(ensure(c, c->raster_pool, raster_pool_bytes(), "raster pool"));
   TRY(ensure(c, c->d_views, (size_t)n_views * sizeof(ViewDesc), "view table"));
   if (c->capacity < 1) TRY(ensure_key_capacity(c, 1));
   TRY(ensure(c, c->tile_counts, std::max<uint64_t>(tiles, 1) * 4, "tile counts"));
@@ -569,7 +567,7 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
   const bool learned = c->schedule == GS3D_SCHEDULE_LEARNED && c->total_tiles > 1;
   if (!cleared) {
     CK(cudaMemsetAsync(&ctrl_of(c)->raster_queue, 0,
-                       offsetof(Ctrl, raster_pool) + sizeof(Ctrl::raster_pool) -
+                       offsetof(Ctrl, raster_places) + sizeof(Ctrl::raster_places) -
                            offsetof(Ctrl, raster_queue),
                        c->stream),
        "reset raster queue");
@@ -630,8 +628,9 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
   a.order = order;
   a.queue_counter = &ctrl_of(c)->raster_queue;
   a.pool = c->raster_pool.p;
-  a.pool_ctrl = &ctrl_of(c)->raster_pool;
-  a.err = &ctrl_of(c)->error;
+  a.pool_ctrl = ctrl_of(c)->raster_pool;
+  a.pool_places = ctrl_of(c)->raster_places;
+  a.wait_polls = (c->flags & GS3D_FLAG_BRIEF_WAITS) ? 2u : kSpinLimit;
   // the previous frame's splat target may still be copying out (captured as
   // an external event wait in graph mode; a never-recorded event is no wait;
   // an eager frame with no copy out puts nothing between its kernels)
@@ -972,6 +971,8 @@ int gs3d_create(gs3d_ctx** out, const gs3d_config* cfg) {
   if (ensure(c, c->ctrl, sizeof(Ctrl), "control block") != GS3D_OK ||
       ensure(c, c->ref_counter, 16, "ref_counter") != GS3D_OK)
     return bail(GS3D_ERR_OOM);
+  c->pool_words.p = ctrl_of(c)->raster_pool;
+  c->pool_words.bytes = sizeof(Ctrl::raster_pool);
   if (cudaMallocHost(&c->h_word, 64) != cudaSuccess) return bail(GS3D_ERR_OOM);
   for (int i = 0; i < kUploadSlots; ++i)
     if (cudaEventCreateWithFlags(&c->upload_ev[i], cudaEventDisableTiming) != cudaSuccess)
@@ -1242,8 +1243,9 @@ int gs3d_preprocess(gs3d_ctx* c) {
   if (!c) return GS3D_ERR_INVALID_ARG;
   TRY(require_single(c, "preprocess"));
   TRY(set_device(c));
-  // start of a frame: counters, histograms and the error latch
-  CK(cudaMemsetAsync(c->ctrl.p, 0, sizeof(Ctrl), c->stream), "reset control block");
+  // start of a frame: counters, histograms and the error latch (the raster clears its own)
+  CK(cudaMemsetAsync(c->ctrl.p, 0, offsetof(Ctrl, raster_places), c->stream),
+     "reset control block");
   StageScope t(c, GS3D_STAGE_PREPROCESS);
   CK(launch_preprocess(dviews(c), 1, c->total_blocks, c->max_sh,
                        static_cast<gs3d_projected_splat*>(c->proj.p), u32(c->counts), nullptr,
@@ -1640,7 +1642,7 @@ int gs3d_read_stage_times(gs3d_ctx* c, double* ms, uint32_t* n) {
 int gs3d_set_flags(gs3d_ctx* c, uint32_t flags) {
   if (!c) return GS3D_ERR_INVALID_ARG;
   if (flags & ~(GS3D_FLAG_STAGEWISE_REBIN | GS3D_FLAG_STAGE_TIMING | GS3D_FLAG_CUDA_GRAPH |
-                GS3D_FLAG_SPLIT_ALL_TILES))
+                GS3D_FLAG_SPLIT_ALL_TILES | GS3D_FLAG_BRIEF_WAITS))
     return fail(c, GS3D_ERR_INVALID_ARG, "unknown flag bits 0x%x", flags);
   c->flags = flags;
   return GS3D_OK;
@@ -1671,6 +1673,7 @@ static DevBuf* named(gs3d_ctx* c, gs3d_buffer which) {
     case GS3D_BUF_TILE_OFFSETS: return &c->tile_offsets;
     case GS3D_BUF_SPLAT_TARGET: return &c->image;
     case GS3D_BUF_TILE_COSTS: return &c->tile_costs;
+    case GS3D_BUF_RASTER_POOL: return &c->pool_words;
     default: return nullptr;
   }
 }

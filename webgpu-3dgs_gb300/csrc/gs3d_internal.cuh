@@ -137,6 +137,8 @@ constexpr int kRadixBins = 256;
 constexpr int kTileHistStride = 2048;
 constexpr int kMaxTilePasses = kMaxSortPasses - 4;
 
+constexpr uint32_t kRasterPlaces = 4096;  // blocks handed on in a raster launch
+
 // Per-frame control block, zeroed at the start of every rebin.
 struct Ctrl {
   uint32_t error;
@@ -158,7 +160,8 @@ struct Ctrl {
   // their own (both are polled), cleared together
   alignas(128) unsigned long long raster_queue;  // next work item
   uint32_t raster_heavy;  // tiles whose work is split (the head of an order by cost)
-  alignas(128) uint32_t raster_pool[4];          // blocks handed on between warps
+  alignas(128) uint32_t raster_pool[8];          // blocks handed on between warps
+  alignas(128) uint32_t raster_places[kRasterPlaces];
 };
 
 // Fallback gate of the learned raster schedule, kept on the device across
@@ -176,7 +179,8 @@ struct SchedGate {
 
 // Bounded spins: a device wait gives up after this many polls (with
 // __nanosleep back-off this is on the order of a second), latches
-// DEVERR_TIMEOUT and returns instead of hanging the GPU.
+// DEVERR_TIMEOUT and returns instead of hanging the GPU.  (Not an error: a raster
+// warp that stops waiting for work, which its owner then does itself.)
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 // ---------------------------------------------------------------------------
@@ -553,7 +557,7 @@ cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint
 // Rasterizes every tile of the batch.  Persistent CTAs pull tile indices
 // from a device work queue (order[k] = k-th tile to render, identity when
 // order is null) through *queue_counter, which must be zero at launch, as must
-// the four words of pool_ctrl.
+// the words of pool_ctrl and pool_places.
 struct RasterArgs {
   const ViewDesc* views;
   uint32_t n_views;
@@ -566,9 +570,10 @@ struct RasterArgs {
   uint32_t* tile_costs;   // zeroed; may be null
   const uint32_t* order;  // may be null
   unsigned long long* queue_counter;
-  void* pool;             // raster_pool_bytes(), zeroed once: blocks handed on between warps
-  void* pool_ctrl;
-  uint32_t* err;
+  void* pool;             // raster_pool_bytes(): blocks handed on between warps
+  uint32_t* pool_ctrl;    // Ctrl::raster_pool
+  uint32_t* pool_places;  // Ctrl::raster_places
+  uint32_t wait_polls;    // polls after which a warp without work stops waiting for some
   uint32_t batch;         // splats staged per batch (0 = tile_w * tile_h)
   // tiles at the head of the order whose blocks are shaded as two half-block
   // items (device count, warp variant only; may be null: none)

@@ -764,6 +764,7 @@ struct WarpSmem {
   SplatStage kept[kKept + 1];  // c.w = position in the tile's list; [kKept] hits nothing
   float4 state[kRegionBlocks][2][32];  // a block's pixels, per lane
   uint16_t list[kKept + 16];
+  uint32_t n_sent, sent[kRegionBlocks - 1];  // places of blocks to come back for (lane 0)
 };
 
 __device__ __forceinline__ void load_px(const float4 (&st)[2][32], uint32_t lane, Px2& p) {
@@ -803,20 +804,30 @@ __device__ __forceinline__ void store_px(float4 (&st)[2][32], uint32_t lane, con
 // warp keeps its CTA's shared memory from kernels of other streams (3 eager
 // 1005x672 views at a time: 442 us alone and 199 us with three contexts in
 // turn; with every warp waiting 442 and 299, with none 672 and 248).
-constexpr uint32_t kPoolSlots = 4096;    // blocks handed on in a launch
+//
+// A block sent to a place stays its sender's until somebody takes it (compare and
+// swap): the warp that waits there, or the sender, which comes back for what it
+// has sent when it is done with the rest of its region.  So no block depends on
+// anybody's waiting: a place may be sent to before it is taken, a warp that has
+// waited wait_polls polls (a second and more) just leaves, and a place that it left
+// behind keeps nothing.  (Blocks sent to places already taken only: 16 views of
+// 640x360 1089 -> 1147 us.)
 constexpr uint32_t kHelperCtas = 64;     // the others leave when the queue is empty
 constexpr uint32_t kHandOnLeft = 512;    // list entries left below which nothing is handed on
 struct PoolSlot {
   float4 state[2][32];
   uint32_t tile, view_x, view_y, k;
-  uint32_t ready;  // 1 from when it is written until it is read (0 between launches)
-  uint32_t pad[3];
 };
-// The counters of RasterArgs::pool_ctrl, all zero at launch: blocks handed on,
-// places taken, warps waiting, warps started and not yet gone.
+enum : uint32_t { PLACE_EMPTY = 0u, PLACE_BLOCK = 1u, PLACE_TAKEN = 2u };
+// RasterArgs::pool_ctrl, all zero at launch: blocks sent, places taken, warps
+// waiting, warps started and not yet gone, waits that ran out, blocks that their
+// senders took back.
 struct PoolCtrl {
-  uint32_t handed, places, waiting, present;
+  uint32_t sent, places, waiting, present, expired, taken_back;
 };
+__device__ __forceinline__ PoolCtrl* pool_ctrl(const RasterArgs& a) {
+  return reinterpret_cast<PoolCtrl*>(a.pool_ctrl);
+}
 __device__ __forceinline__ uint4 pool_look(const RasterArgs& a) {
   uint4 v;
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -825,43 +836,45 @@ __device__ __forceinline__ uint4 pool_look(const RasterArgs& a) {
                : "memory");
   return v;
 }
-__device__ __forceinline__ void hand_on(const RasterArgs& a, const float4 (&st)[2][32],
-                                        uint32_t slot, uint32_t tile, uint32_t x, uint32_t y,
-                                        uint32_t k) {
+__device__ __forceinline__ void send_block(const RasterArgs& a, const float4 (&st)[2][32],
+                                           uint32_t place, uint32_t tile, uint32_t x, uint32_t y,
+                                           uint32_t k) {
   const uint32_t lane = threadIdx.x & 31;
-  PoolSlot& s = static_cast<PoolSlot*>(a.pool)[slot];
+  PoolSlot& s = static_cast<PoolSlot*>(a.pool)[place];
   __stcg(&s.state[0][lane], st[0][lane]);
   __stcg(&s.state[1][lane], st[1][lane]);
   if (lane == 0) __stcg(reinterpret_cast<uint4*>(&s.tile), make_uint4(tile, x, y, k));
   __threadfence();
   __syncwarp();
-  if (lane == 0) st_relaxed_u32(&s.ready, 1u);
+  if (lane == 0) st_relaxed_u32(a.pool_places + place, PLACE_BLOCK);
 }
-// Lane 0 of a warp without work: waits for a block and returns its slot, or ~0u
-// once nobody is left who could hand one on.  Blocks go to places in order, a
-// warp that got one comes back for the next place, and none leaves while a
-// block is on its way to its place or another warp still works.
+// Lane 0: takes the block at a place that has been sent one; false if somebody has.
+__device__ __forceinline__ bool take_block(const RasterArgs& a, uint32_t place) {
+  const bool mine = atomicCAS(a.pool_places + place, PLACE_BLOCK, PLACE_TAKEN) == PLACE_BLOCK;
+  __threadfence();
+  return mine;
+}
+// Lane 0 of a warp without work: takes a place and waits for a block; its place, or
+// ~0u once every warp waits (nobody has a block to send) or the polls run out.
 __device__ __forceinline__ uint32_t wait_for_block(const RasterArgs& a) {
-  PoolCtrl* c = static_cast<PoolCtrl*>(a.pool_ctrl);
+  PoolCtrl* c = pool_ctrl(a);
   atomicAdd(&c->waiting, 1u);
-  const uint32_t place = atomicAdd(&c->places, 1u);
-  if (place < kPoolSlots) {
-    uint32_t* ready = &static_cast<PoolSlot*>(a.pool)[place].ready;
-    for (uint32_t polls = 0; polls < (1u << 22); ++polls) {  // a second and more
-      if (ld_relaxed_u32(ready) != 0u) {
-        atomicSub(&c->waiting, 1u);
-        __threadfence();
-        st_relaxed_u32(ready, 0u);
-        return place;
-      }
-      if ((polls & 3u) == 3u) {
-        const uint4 v = pool_look(a);
-        // everyone waits: nobody hands on any more
-        if (v.z >= v.w && place >= ld_relaxed_u32(&c->handed)) break;
-      }
-      __nanosleep(300);
+  uint32_t place = atomicAdd(&c->places, 1u), polls = 0;
+  for (; place < kRasterPlaces && polls < a.wait_polls; ++polls) {
+    if (ld_relaxed_u32(a.pool_places + place) != PLACE_EMPTY) {
+      atomicSub(&c->waiting, 1u);
+      if (take_block(a, place)) return place;
+      atomicAdd(&c->waiting, 1u);  // its sender has
+      place = atomicAdd(&c->places, 1u);
+      continue;
     }
+    if ((polls & 3u) == 3u) {
+      const uint4 v = pool_look(a);
+      if (v.z >= v.w) break;
+    }
+    __nanosleep(300);
   }
+  if (polls == a.wait_polls) atomicAdd(&c->expired, 1u);
   atomicSub(&c->waiting, 1u);
   atomicSub(&c->present, 1u);
   return ~0u;
@@ -1002,14 +1015,17 @@ __device__ uint32_t shade_region(const RasterArgs& a, const TileGeom& g, uint32_
         if (look && lane == 0) pool = pool_look(a);
         flush();
         if (look && (alive & (alive - 1u)) != 0u) {
-          const int places = __shfl_sync(0xffffffffu, (int)min(pool.y, kPoolSlots) - (int)pool.x, 0);
+          const int places =
+              __shfl_sync(0xffffffffu, (int)min(pool.y, kRasterPlaces) - (int)pool.x, 0);
           for (int i = 0; i < places && (alive & (alive - 1u)) != 0u; ++i) {
-            uint32_t slot = 0;
-            if (lane == 0) slot = atomicAdd(&static_cast<PoolCtrl*>(a.pool_ctrl)->handed, 1u);
-            slot = __shfl_sync(0xffffffffu, slot, 0);
-            if (slot >= kPoolSlots) break;
+            uint32_t place = 0;
+            if (lane == 0) place = atomicAdd(&pool_ctrl(a)->sent, 1u);
+            place = __shfl_sync(0xffffffffu, place, 0);
+            if (place >= kRasterPlaces) break;
             const uint32_t b = 31 - __clz(alive);
-            hand_on(a, w.state[b], slot, g.tile, x0 + (b % nbx) * 8, y0 + (b / nbx) * kRows, at);
+            send_block(a, w.state[b], place, g.tile, x0 + (b % nbx) * 8, y0 + (b / nbx) * kRows,
+                       at);
+            if (lane == 0) w.sent[w.n_sent++] = place;
             alive &= ~(1u << b);
             owned &= ~(1u << b);
           }
@@ -1055,7 +1071,8 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
     w.kept[kKept].a = make_float4(0.f, 0.f, -1.f, 0.f);
     w.kept[kKept].b = make_float4(0.f, 0.f, 0.f, -1.f);
     w.kept[kKept].c = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (HAND_ON) atomicAdd(&static_cast<PoolCtrl*>(a.pool_ctrl)->present, 1u);
+    w.n_sent = 0;
+    if (HAND_ON) atomicAdd(&pool_ctrl(a)->present, 1u);
   }
   __syncwarp();
   const uint32_t bw = a.tile_w / 8, blocks = bw * (a.tile_h / 8);
@@ -1067,16 +1084,28 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
   bool queued = true;  // the queue may still hold items
   for (;;) {
     unsigned long long item = items;
-    if (queued) {
+    uint32_t t, x, y, nbx = 1, nby = 1, slot = ~0u;
+    if (HAND_ON) {  // a block of the region just shaded that nobody has taken
+      if (lane == 0) {
+        while (w.n_sent && slot == ~0u) {
+          const uint32_t place = w.sent[--w.n_sent];
+          if (take_block(a, place)) {
+            atomicAdd(&pool_ctrl(a)->taken_back, 1u);
+            slot = place;
+          }
+        }
+      }
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+    }
+    if (slot == ~0u && queued) {
       if (lane == 0) item = atomicAdd(a.queue_counter, 1ull);
       item = __shfl_sync(0xffffffffu, item, 0);
       queued = item < items;
     }
-    uint32_t t, x, y, nbx = 1, nby = 1, slot = ~0u;
     const bool in_heavy = item < heavy_items;
     bool fine = a.fine;
     TileGeom g;
-    if (queued) {
+    if (item < items) {
       uint32_t sub;
       if (in_heavy) {
         t = (uint32_t)(item / (2 * blocks));
@@ -1105,13 +1134,15 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
       }
     } else {
       if (!HAND_ON) break;
-      if (blockIdx.x >= kHelperCtas) {
-        if (lane == 0) atomicSub(&static_cast<PoolCtrl*>(a.pool_ctrl)->present, 1u);
-        break;
+      if (slot == ~0u) {
+        if (blockIdx.x >= kHelperCtas) {
+          if (lane == 0) atomicSub(&pool_ctrl(a)->present, 1u);
+          break;
+        }
+        if (lane == 0) slot = wait_for_block(a);
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        if (slot == ~0u) break;
       }
-      if (lane == 0) slot = wait_for_block(a);
-      slot = __shfl_sync(0xffffffffu, slot, 0);
-      if (slot == ~0u) break;
       const uint4 info =
           __ldcg(reinterpret_cast<const uint4*>(&static_cast<PoolSlot*>(a.pool)[slot].tile));
       t = info.x;
@@ -1265,7 +1296,7 @@ cudaError_t raster_shape(const RasterArgs& a, int sm_count, uint32_t* items_per_
   return cudaSuccess;
 }
 
-size_t raster_pool_bytes() { return kPoolSlots * sizeof(PoolSlot); }
+size_t raster_pool_bytes() { return kRasterPlaces * sizeof(PoolSlot); }
 
 cudaError_t launch_raster(const RasterArgs& args, int sm_count, LaunchStream s) {
   if (args.num_tiles == 0) return cudaSuccess;

@@ -30,6 +30,7 @@ FLAG_STAGEWISE_REBIN = 1
 FLAG_STAGE_TIMING = 2
 FLAG_CUDA_GRAPH = 4
 FLAG_SPLIT_ALL_TILES = 8
+FLAG_BRIEF_WAITS = 16
 STAGE_NAMES = ["preprocess-splats", "depth-sort", "prefix-scan", "emit-tile-refs", "radix-sort",
                "identify-tile-ranges", "rasterize-tiles"]
 
@@ -39,7 +40,7 @@ BUFFERS = {
     "splat_sh_rest": 4, "projected_splats": 5, "splat_ref_counts": 6,
     "splat_ref_offsets": 7, "ref_counter": 8, "sort_keys_a": 9, "sort_values_a": 10,
     "sort_keys_b": 11, "sort_values_b": 12, "tile_offsets": 13, "splat_target": 14,
-    "tile_costs": 15,
+    "tile_costs": 15, "raster_pool": 16,
 }
 
 

@@ -193,6 +193,13 @@ class GaussianSplatRenderer:
             (_lib.FLAG_SPLIT_ALL_TILES if on else 0)
         self._call("gs3d_set_flags", self._flags)
 
+    def setBriefWaits(self, on: bool) -> None:
+        """Raster warps give up waiting for blocks at once (testing what becomes
+        of the blocks; the image is unchanged)."""
+        self._flags = (getattr(self, "_flags", 0) & ~_lib.FLAG_BRIEF_WAITS) | \
+            (_lib.FLAG_BRIEF_WAITS if on else 0)
+        self._call("gs3d_set_flags", self._flags)
+
     def setTuning(self, tile: int | tuple[int, int] = 16, digit_bits: int = 8,
                   raster_batch: int = 0) -> None:
         """Speed knobs that leave every image bit-identical: square (or
@@ -454,6 +461,7 @@ class GaussianSplatRenderer:
             "tile_offsets": (np.uint32, (tiles + 1,)),
             "splat_target": (np.float16, (h, w, 4)),
             "tile_costs": (np.uint32, (tiles,)),
+            "raster_pool": (np.uint32, (8,)),
         }
         dtype, shape = shapes[name]
         out = np.zeros(shape, dtype)
