@@ -544,9 +544,9 @@ LaunchStream chain_stream(const gs3d_ctx* c) {
 
 // cleared: the fused rebin has zeroed the work queue and the tile costs.
 int raster_stage(gs3d_ctx* c, bool cleared) {
-  if ((uint64_t)c->tile_w * c->tile_h > 1024 && (c->flags & GS3D_FLAG_STAGEWISE_REBIN))
+  if ((uint64_t)c->tile_w * c->tile_h > 1024 && !cleared)
     return fail(c, GS3D_ERR_INVALID_ARG,
-                "tiles of %ux%u pixels are for the fused rebin; the stage-wise rebin takes tiles "
+                "tiles of %ux%u pixels are for the fused rebin; the stage entry points take tiles "
                 "of at most 1024 pixels",
                 c->tile_w, c->tile_h);
   StageScope t(c, GS3D_STAGE_RASTER);
