@@ -110,8 +110,22 @@ def test_every_tile_shape_gives_the_unculled_image(renderer, case, w, h):
     with np.errstate(all="ignore"):
         p = records(rng, w, h, conic, opacity, radius, mean)
     want = image(renderer, (15, 15), w, h, p)
-    assert want.any()
+    assert want.any() or case == "negative definite"  # its powers are all positive
     for tile in [(16, 16), (32, 32), (12, 8)]:
         for split in (False, True):
             got = image(renderer, tile, w, h, p, split)
             assert np.array_equal(got, want), (tile, split, int((got != want).any(-1).sum()))
+
+
+@pytest.mark.parametrize("case", ["negative definite", "one diagonal negative", "indefinite"])
+def test_forms_that_are_not_positive_match_the_oracle(renderer, oracle, case):
+    """A positive power skips the splat there, as in the reference."""
+    w, h, tile = 323, 197, (16, 16)
+    conic, opacity, radius, _ = CASES[case]
+    p = records(np.random.default_rng(50), w, h, conic, opacity, radius, None)
+    got = image(renderer, tile, w, h, p).view(np.float16).astype(np.float32)
+    tiles = (-(-w // tile[0])) * (-(-h // tile[1]))
+    want = oracle.rasterize(w, h, *tile, p, np.arange(tiles + 1, dtype=np.uint32) * LISTED,
+                            np.tile(np.arange(LISTED, dtype=np.uint32), tiles))
+    want = want[0] if isinstance(want, tuple) else want
+    assert np.abs(got - want).max() <= 2.0 / 255.0

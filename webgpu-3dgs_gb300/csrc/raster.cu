@@ -59,7 +59,8 @@ namespace {
 // Splats take the exact form when the terms of q can reach 2^12 inside the
 // radius, (|conic.x| + 2 |conic.y| + |conic.z|) r^2 > 2^12: there the terms
 // cancel (elongated splats seen far from their mean), and the rounding order
-// decides the result.  Below that bound the fast form's q differs from the
+// decides the result.  So do conics that are not positive definite (by rounding of
+// a huge covariance): theirs is the q < 0 test.  Below that bound the fast form's q differs from the
 // reference's by about 2^-11 at most, so each alpha differs by a relative
 // 1e-3 and a pixel, whose blend weights alpha_i T_i sum to at most 1, by
 // about that much.  b.w = vis, in q's units; its two lowest bits hold the
@@ -72,7 +73,6 @@ struct SplatStage {  // first 48 bytes of a ProjectedSplat, prepared in place (p
 
 constexpr float kHalfLog2e = 0.72134752044448170f;
 constexpr float kExactFormBound = 4096.0f;
-constexpr float kInf = __builtin_huge_valf();
 // How a splat's alpha is evaluated: fast form whose op exp(power) stays below
 // the 0.99 clamp; fast form with the clamp; exact form (which clamps).
 constexpr uint32_t kSimple = 0u, kClamped = 1u, kExact = 2u;
@@ -124,12 +124,12 @@ __device__ __forceinline__ void prepare(SplatStage& s, float ext) {
   const float lim = fmaf(0.0f, near, op * 255.0f);
   const float r2 = a.w * a.w;
   const float terms = sum * r2;
-  const bool fast = terms <= kExactFormBound;
-  // q >= t / 800 then, far above its rounding; a projected splat's fast form has
-  // B^2 < 0.992 A C (its condition number is below 455)
-  const bool positive = A > 0.0f && B * B <= 0.995f * A * C;
+  // the second bound gives q >= t / 800, far above its rounding; a splat whose
+  // covariance did not lose it to rounding has B^2 < 0.992 A C where the first holds
+  // (a condition number below 455)
+  const bool fast = terms <= kExactFormBound && A > 0.0f && B * B <= 0.995f * A * C;
   float vis;
-  if (lim < 0.999f && (positive || !fast)) {
+  if (lim < 0.999f) {
     vis = -1.0f;  // alpha = opacity * exp(power) <= opacity < 1/255 everywhere
   } else {
     vis = __log2f(lim) * 1.01f + 1e-3f + (kHalfLog2e * 9.5367431640625e-07f) * near;
@@ -139,7 +139,7 @@ __device__ __forceinline__ void prepare(SplatStage& s, float ext) {
   s.a = make_float4(a.x, a.y, r2, op);
   if (fast) {
     // no clamp where ex2 of a value <= 0 (to 2 ulp) times op stays below it
-    const bool simple = lim <= 0.9899f * 255.0f && positive;
+    const bool simple = lim <= 0.9899f * 255.0f;
     vis = __uint_as_float((__float_as_uint(vis) & ~3u) | (simple ? kSimple : kClamped));
     s.b = make_float4(kHalfLog2e * A, 2.0f * kHalfLog2e * B, kHalfLog2e * C, vis);
     s.c.w = 0.0f;
@@ -168,11 +168,10 @@ __device__ __forceinline__ float splat_alpha(float pfx, float pfy, const SplatSt
   const float dy = pfy - a.y;
   if (!exact) {
     // fast form: q < 0 cannot occur (no power > 0 test needed): these splats'
-    // conics have condition numbers below 455 (their terms, at least 9 times
-    // the condition number, stay within kExactFormBound), so q, computed to
-    // a relative 1e-3, and the reference's s keep the sign of the positive
-    // definite form at every pixel centre, which lies 6e-8 pixels or more
-    // from the mean unless exactly on it
+    // conics are positive definite by a margin (prepare), so q, computed to
+    // a relative 1e-3, and the reference's s keep the sign of the form at every
+    // pixel centre, which lies 6e-8 pixels or more from the mean unless exactly
+    // on it
     const float d2 = fmaf(dx, dx, dy * dy);
     const float q = fmaf(b.x * dx, dx, fmaf(b.y * dx, dy, b.z * dy * dy));  // -power log2(e)
     const float alpha = fminf(0.99f, a.w * ex2_approx(-q));
@@ -293,7 +292,8 @@ __device__ __forceinline__ float2 exact_alpha(float pfx, float2 pfy, const Splat
 }
 // The same for a splat of either form: both are evaluated and one is taken, so
 // that four of a step overlap (a branch per splat costs more than the few
-// operations that the forms do not share).  The fast form has no q < 0 test.
+// operations that the forms do not share).  The q < 0 and clamp tests cannot
+// act on a fast-form splat that has none.
 __device__ __forceinline__ float any_alpha(float pfx, float pfy, const SplatStage& s, bool exact) {
   const float4 a = s.a, b = s.b;
   const float dx = pfx - a.x;
@@ -304,9 +304,9 @@ __device__ __forceinline__ float any_alpha(float pfx, float pfy, const SplatStag
   const float qe = __fadd_rn(__fadd_rn(__fmul_rn(u, dx), __fmul_rn(v, dy)), w);
   const float qf = fmaf(u, dx, fmaf(v, dy, w));
   const float d2 = exact ? __fadd_rn(__fmul_rn(dx, dx), dyy) : fmaf(dx, dx, dyy);
-  const float q = exact ? qe : qf, least = exact ? 0.0f : -kInf;
+  const float q = exact ? qe : qf;
   const float alpha = fminf(0.99f, a.w * ex2_approx(__fmul_rn(q, exact ? -kHalfLog2e : -1.0f)));
-  return !(d2 > a.z) && !(q < least) && !(alpha < 1.0f / 255.0f) ? alpha : 0.0f;
+  return !(d2 > a.z) && !(q < 0.0f) && !(alpha < 1.0f / 255.0f) ? alpha : 0.0f;
 }
 __device__ __forceinline__ float2 any_alpha(float pfx, float2 pfy, const SplatStage& s,
                                             bool exact) {
@@ -326,13 +326,12 @@ __device__ __forceinline__ float2 any_alpha(float pfx, float2 pfy, const SplatSt
                                exact ? __fadd_rn(__fadd_rn(t1, t2.y), w.y) : qf.y);
   const float2 d2 =
       make_float2(exact ? __fadd_rn(dxx, dyy.x) : df.x, exact ? __fadd_rn(dxx, dyy.y) : df.y);
-  const float least = exact ? 0.0f : -kInf;
   const float2 ev = __fmul2_rn(q, bcast(exact ? -kHalfLog2e : -1.0f));
   const float2 am = __fmul2_rn(bcast(a.w), make_float2(ex2_approx(ev.x), ex2_approx(ev.y)));
   const float2 alpha = make_float2(fminf(0.99f, am.x), fminf(0.99f, am.y));
   return make_float2(
-      !(d2.x > a.z) && !(q.x < least) && !(alpha.x < 1.0f / 255.0f) ? alpha.x : 0.0f,
-      !(d2.y > a.z) && !(q.y < least) && !(alpha.y < 1.0f / 255.0f) ? alpha.y : 0.0f);
+      !(d2.x > a.z) && !(q.x < 0.0f) && !(alpha.x < 1.0f / 255.0f) ? alpha.x : 0.0f,
+      !(d2.y > a.z) && !(q.y < 0.0f) && !(alpha.y < 1.0f / 255.0f) ? alpha.y : 0.0f);
 }
 
 // The blend state of a lane's pixels: one (Px1) or two of a column (Px2).
@@ -1084,7 +1083,7 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
   bool queued = true;  // the queue may still hold items
   for (;;) {
     unsigned long long item = items;
-    uint32_t t, x, y, nbx = 1, nby = 1, slot = ~0u;
+    uint32_t slot = ~0u;
     if (HAND_ON) {  // a block of the region just shaded that nobody has taken
       if (lane == 0) {
         while (w.n_sent && slot == ~0u) {
@@ -1097,15 +1096,16 @@ __global__ void __launch_bounds__(kItemWarps * 32, 5) raster_kernel_warps(Raster
       }
       slot = __shfl_sync(0xffffffffu, slot, 0);
     }
-    if (slot == ~0u && queued) {
+    if (queued && (!HAND_ON || slot == ~0u)) {
       if (lane == 0) item = atomicAdd(a.queue_counter, 1ull);
       item = __shfl_sync(0xffffffffu, item, 0);
       queued = item < items;
     }
+    uint32_t t, x, y, nbx = 1, nby = 1;
     const bool in_heavy = item < heavy_items;
     bool fine = a.fine;
     TileGeom g;
-    if (item < items) {
+    if (HAND_ON ? item < items : queued) {
       uint32_t sub;
       if (in_heavy) {
         t = (uint32_t)(item / (2 * blocks));
