@@ -3,10 +3,12 @@ order have lists of thousands of splats, so their warps still work when the queu
 has run empty, and warps that wait take over blocks of theirs.  The image and the
 costs are those of half-block items, which are never handed on - also where the
 waiting warps leave before a block comes, which its sender then takes back."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from gs3d import GaussianSplatRenderer, Scene, scenes
+from gs3d import GaussianSplatRenderer, Scene, _lib, learned, scenes
 from gs3d.renderer import PROJ_DTYPE
 
 pytestmark = pytest.mark.gpu
@@ -84,3 +86,39 @@ def test_blocks_that_nobody_waits_for_are_taken_back(frame):
         got, gotc, pool = frame()  # nothing is left behind for the next launch
         assert pool[0] > pool[5] and pool[4] == 0
         assert np.array_equal(got, image) and np.array_equal(gotc, costs)
+
+
+def test_an_order_by_predictions_hands_on_too(built_lib):
+    """A prediction may rank a long list last: batches of any size in learned order
+    hand blocks on (here an untrained model's order, 11 regions a warp), and give
+    the row-major order's images."""
+    w, h = 1920, 1080
+    data = scenes.scene_opacity_mix(300_000, 100_000, seed=3)
+    eyes = scenes.random_eyes(4, 9.0, 16.0, seed=9)
+    views = [(0, scenes.camera_at(e, w, h).getUniformData(w, h), w, h) for e in eyes]
+    r = GaussianSplatRenderer(Scene())
+    r.init()
+    try:
+        r.setSplatData(data)
+        r.setTuning(16, 8, 0)
+
+        def batch():
+            r.rebinBatch(views)
+            return ([r.readViewImage(v).view(np.uint16).copy() for v in range(4)],
+                    r.readBuffer("raster_pool"))
+        want, _ = batch()
+        f32 = lambda *a: np.ascontiguousarray(*a, np.float32)  # noqa: E731
+        p, mean, std = f32(learned.init_params(1)), f32(np.zeros(16)), f32(np.ones(16))
+        r.setScheduleGate(1e9)  # the model is not trained
+        r._call("gs3d_set_cost_model", *(a.ctypes.data_as(C.c_void_p) for a in (p, mean, std)))
+        r.setSchedule(_lib.SCHEDULE_LEARNED)
+        taken = 0
+        for _ in range(3):
+            got, pool = batch()
+            assert r.getScheduleStatus()["active"] == _lib.SCHEDULE_LEARNED
+            taken += int(pool[0]) - int(pool[5])
+            for a, b in zip(got, want):
+                assert np.array_equal(a, b)
+        assert taken > 0
+    finally:
+        r.destroy()

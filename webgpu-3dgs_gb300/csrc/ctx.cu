@@ -626,6 +626,7 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
   a.image = static_cast<uint2*>(c->image.p);
   a.tile_costs = u32(c->tile_costs);
   a.order = order;
+  a.predicted = learned;
   a.queue_counter = &ctrl_of(c)->raster_queue;
   a.pool = c->raster_pool.p;
   a.pool_ctrl = ctrl_of(c)->raster_pool;

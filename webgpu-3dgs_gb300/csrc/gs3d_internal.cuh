@@ -569,6 +569,7 @@ struct RasterArgs {
   uint2* image;
   uint32_t* tile_costs;   // zeroed; may be null
   const uint32_t* order;  // may be null
+  bool predicted;         // the order is by predicted costs
   unsigned long long* queue_counter;
   void* pool;             // raster_pool_bytes(): blocks handed on between warps
   uint32_t* pool_ctrl;    // Ctrl::raster_pool

@@ -1279,9 +1279,12 @@ cudaError_t raster_config(const RasterArgs& a, RasterConfig* cfg) {
 // blocks).
 constexpr float kFineWaves = 1.75f;
 // Blocks are handed on in the row-major order, which cannot know the long lists
-// beforehand, and in orders by cost up to this many regions a warp (16 views of
-// 640x360 with 5 regions a warp: raster 975 -> 871 us; with 20 and more the
-// tail is short and the check costs 2%).
+// beforehand; in an order by predicted costs, which may be wrong about one (eight
+// views of opaque and translucent clusters at 1080p in learned order, raster at
+// 16x16 tiles 7199 -> 3559 us, 32x32 5023 -> 3656, 64x32 5373 -> 3644; of evenly
+// spread ones 2432 -> 2442); and in the order by key counts up to this many regions
+// a warp (16 views of 640x360 with 5 regions a warp: raster 975 -> 871 us; with 20
+// and more the tail is short and the check costs 2%).
 constexpr float kHandOnWaves = 8.0f;
 
 }  // namespace
@@ -1309,7 +1312,8 @@ cudaError_t launch_raster(const RasterArgs& args, int sm_count, LaunchStream s) 
   if (cfg.mode == 2) {
     const float waves = (float)a.num_tiles * (float)cfg.regions / (float)(ctas * kItemWarps);
     a.fine = waves <= kFineWaves;
-    if (!a.fine && (a.order == nullptr || waves < kHandOnWaves)) cfg.kern = raster_kernel_warps<true>;
+    if (!a.fine && (a.order == nullptr || a.predicted || waves < kHandOnWaves))
+      cfg.kern = raster_kernel_warps<true>;
     max_ctas = ((uint64_t)a.num_tiles * cfg.blocks * 2 + kItemWarps - 1) / kItemWarps;
   } else {
     a.heavy = nullptr;  // split items exist in the warp variant only
