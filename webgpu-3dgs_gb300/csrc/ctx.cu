@@ -1162,6 +1162,8 @@ int gs3d_load_ply(gs3d_ctx* c, const void* data, size_t size, uint32_t target,
     e = cudaMemcpyAsync(words, c->ply_words.p, sizeof(words), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cleanup(cuda_fail(c, e, "ply decode"));
+  if (words[0] == kPlyTimeout)
+    return cleanup(fail(c, GS3D_ERR_TIMEOUT, "ply decode: rows did not arrive in time"));
   if (words[0] != 0)
     return cleanup(fail(c, GS3D_ERR_INVALID_ARG, "Invalid Gaussian Splat PLY row: missing '%s'",
                         ply_required_name((int)words[0] - 1)));

@@ -629,7 +629,8 @@ bool ply_ascii_rows(const uint8_t* data, size_t size, const PlyLayout& lay,
 // Decodes n vertex rows on the device into the four vec4 SoA arrays and the
 // SH block (lay.sh_k coefficients per channel, channel-major), activating as
 // the reference's loader does; the first non-finite required value latches
-// 1 + its field index in *bad; bounds = 6 ordered-u32 words (min xyz, max xyz).
+// 1 + its field index in *bad (kPlyTimeout: rows that did not arrive); bounds = 6 ordered-u32 words (min xyz, max xyz).
+constexpr uint32_t kPlyTimeout = 0xffffffffu;
 cudaError_t launch_ply_decode(const uint8_t* rows, uint64_t n, const PlyLayout& lay,
                               bool big_endian, float4* pos, float4* scale,
                               float4* rot, float4* color, float* sh, uint32_t* bad,

@@ -396,15 +396,18 @@ struct DecodeArgs {
 };
 
 // A block takes kDecodeThreads rows at most, a thread a row.  The rows' bytes
-// are staged in shared memory by 16-byte copies first (they may lie in host
+// are staged in shared memory by one bulk copy first (they may lie in host
 // memory, behind the link: 300k rows of 248 bytes are read in 0.38 ms there,
 // and several blocks per SM keep it busy while others are at the f64
-// activations), and the SH block is written with unit stride.
+// activations), and the SH block is written with unit stride.  Copies of 16 bytes
+// a thread depended on where the rows begin: 300k rows of 236 bytes 485 to 905 us
+// over the offsets from a 128-byte line, 422 to 438 by the bulk copy.
 constexpr int kDecodeThreads = 128;
 constexpr uint32_t kDecodeBytes = 40 * 1024;  // staged rows, with their ragged ends
 __global__ void __launch_bounds__(kDecodeThreads) ply_decode_kernel(DecodeArgs a) {
   extern __shared__ __align__(16) uint8_t s_rows[];
   __shared__ PlyField s_rest[kPlyMaxRest];
+  __shared__ uint64_t s_bar;
   const uint32_t tile = a.tile_rows ? a.tile_rows : kDecodeThreads;
   const uint64_t first = (uint64_t)blockIdx.x * tile;
   const uint32_t count = (uint32_t)(a.n - first < tile ? a.n - first : tile);
@@ -415,15 +418,24 @@ __global__ void __launch_bounds__(kDecodeThreads) ply_decode_kernel(DecodeArgs a
     const uint32_t lead = (uint32_t)((uintptr_t)base & 15u);
     const uint32_t words = (lead + count * a.stride + 15u) / 16u;
     const uint4* src = reinterpret_cast<const uint4*>(base - lead);
-    for (uint32_t k = threadIdx.x; k < words; k += kDecodeThreads)
-      cp_async16(s_rows + 16 * k, src + k);
-    cp_async_commit();
+    if (threadIdx.x == 0) {
+      mbar_init(&s_bar, 1);
+      fence_mbar_init();
+      mbar_expect_tx(&s_bar, words * 16u);
+      bulk_g2s(s_rows, src, words * 16u, &s_bar);
+    }
     base = s_rows + lead;
   }
   const uint32_t kc = 3 * a.sh_k;
   if (threadIdx.x < kc) s_rest[threadIdx.x] = a.rest[threadIdx.x];
-  cp_async_wait<0>();
   __syncthreads();
+  if (a.tile_rows && !__syncthreads_and(mbar_wait(&s_bar, 0))) {
+    if (threadIdx.x == 0) {
+      atomicCAS(a.bad, 0u, kPlyTimeout);
+      mbar_wait(&s_bar, 0);  // one more bounded wait
+    }
+    return;
+  }
   const bool live = threadIdx.x < count;
   const uint64_t i = first + threadIdx.x;
   float px = 0.f, py = 0.f, pz = 0.f;
