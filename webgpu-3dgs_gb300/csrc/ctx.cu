@@ -20,6 +20,8 @@
 // Every rebin runs over a device-side view table (ViewDesc); a single-view
 // rebin is a batch of one, gs3d_rebin_batch renders many views, of several
 // scenes and uneven sizes, in one launch sequence.
+#include <unistd.h>
+
 #include <algorithm>
 #include <cstdarg>
 #include <cstddef>
@@ -1101,6 +1103,21 @@ int gs3d_composite(gs3d_ctx* c, uint32_t view, uint32_t mode, uint32_t debug_ref
   return GS3D_OK;
 }
 
+namespace {
+// Reads a byte of every page: pages of a memory-mapped file that no one has read
+// are brought in by the host here, not one device fault after the other, and what
+// the host cannot read never reaches the device.  7 to 13 us of 430 where 74 MB are
+// present in pages of 64 KB; a mapped file's first load 496 us (2751 when the rows
+// were copied first).
+void touch_pages(const uint8_t* p, size_t bytes) {
+  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  uint8_t seen = 0;
+  for (size_t i = 0; i < bytes; i += page) seen |= p[i];
+  if (bytes) seen |= p[bytes - 1];
+  asm volatile("" ::"r"(seen));
+}
+}  // namespace
+
 int gs3d_load_ply(gs3d_ctx* c, const void* data, size_t size, uint32_t target,
                   uint32_t* out_scene, gs3d_ply_info* info) {
   if (!c || !data) return fail(c, GS3D_ERR_INVALID_ARG, "null argument");
@@ -1141,9 +1158,9 @@ int gs3d_load_ply(gs3d_ctx* c, const void* data, size_t size, uint32_t target,
       (rc = ensure(c, sc.rot, v4, "splat_rotations")) || (rc = ensure(c, sc.color, v4, "splat_colors")) ||
       (lay.sh_k && (rc = ensure(c, sc.sh, (size_t)n * 3 * lay.sh_k * sizeof(float), "splat_sh_rest"))) ||
       // where the device walks the host's page tables the decode reads the rows
-      // in place: 300k rows of 248 bytes 826 -> 483 us (a buffer for them 155 us
-      // to allocate and free, its copy 430, the decode after it 150; the link
-      // alone is 377)
+      // in place: 300k rows of 236 bytes from a buffer loaded before 852 -> 436 us
+      // (a buffer for them 155 us to allocate and free, its copy 430, the decode
+      // after it 150; the link alone is 377), from a new one 1089 -> 600
       (!c->reads_host && (rc = ensure(c, d_rows, std::max<size_t>((size_t)n * lay.stride, 16), "ply rows"))) ||
       (rc = ensure(c, c->ply_words, 64, "ply status")))
     return cleanup(rc);
@@ -1152,6 +1169,7 @@ int gs3d_load_ply(gs3d_ctx* c, const void* data, size_t size, uint32_t target,
   if (e == cudaSuccess && n && !c->reads_host)
     e = cudaMemcpyAsync(d_rows.p, rows, (size_t)n * lay.stride, cudaMemcpyHostToDevice, c->stream);
   uint32_t* dw = u32(c->ply_words);
+  if (c->reads_host) touch_pages(rows, (size_t)n * lay.stride);
   if (e == cudaSuccess)
     e = launch_ply_decode(c->reads_host ? rows : static_cast<const uint8_t*>(d_rows.p), n, lay,
                           lay.format == GS3D_PLY_BINARY_BE, static_cast<float4*>(sc.pos.p),
