@@ -1179,7 +1179,11 @@ int gs3d_load_ply(gs3d_ctx* c, const void* data, size_t size, uint32_t target,
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(words, c->ply_words.p, sizeof(words), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return cleanup(cuda_fail(c, e, "ply decode"));
+  if (e != cudaSuccess) {
+    // a decode under way still reads the caller's rows and writes the new scene
+    cudaStreamSynchronize(c->stream);
+    return cleanup(cuda_fail(c, e, "ply decode"));
+  }
   if (words[0] == kPlyTimeout)
     return cleanup(fail(c, GS3D_ERR_TIMEOUT, "ply decode: rows did not arrive in time"));
   if (words[0] != 0)
