@@ -310,7 +310,7 @@ int gs3d_get_tuning(struct gs3d_ctx* ctx, gs3d_tuning* out);
  * of tile size {8x8, 16x16, 32x32, 32x64, 64x32} x digit width {4, 8, 11} x
  * raster batch {128, 256, 512}, applies the fastest and writes up to max_results
  * measurements (n_results = candidates measured; candidates whose refs
- * exceed the 2^30 limit of one rebin are skipped).  Blocking. */
+ * exceed one rebin's limit are skipped).  Blocking. */
 int gs3d_autotune(struct gs3d_ctx* ctx, const gs3d_view* views, uint32_t n_views,
                   uint32_t reps, gs3d_tune_result* results, uint32_t max_results,
                   uint32_t* n_results);

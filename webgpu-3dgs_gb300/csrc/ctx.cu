@@ -559,12 +559,9 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
   a.num_tiles = c->total_tiles;
   a.tile_w = c->tile_w;
   a.tile_h = c->tile_h;
-  // raster_batch 0 stages one splat per tile pixel, at most 1024 (the staged
-  // batches of a 2048-pixel tile would not fit shared memory)
-  a.batch = c->raster_batch ? c->raster_batch
-                            : ((uint64_t)c->tile_w * c->tile_h > 1024 ? 1024u : 0u);
-  uint32_t strips = 1, raster_ctas = 1;
-  CK(raster_shape(a, c->sm_count, &strips, &raster_ctas), "raster shape");
+  a.batch = c->raster_batch;
+  uint32_t items_per_tile = 1, workers = 1;
+  CK(raster_shape(a, c->sm_count, &items_per_tile, &workers), "raster shape");
   const bool split_all = (c->flags & GS3D_FLAG_SPLIT_ALL_TILES) != 0;
   const bool learned = c->schedule == GS3D_SCHEDULE_LEARNED && c->total_tiles > 1;
   if (!cleared) {
@@ -596,8 +593,8 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
     }
     if (c->total_tiles <= kOrderTiles) {
       CK(launch_order(c->schedule, u32(c->tile_offsets), static_cast<float*>(c->tile_preds.p),
-                      static_cast<SchedGate*>(c->gate.p), c->total_tiles, raster_ctas, strips,
-                      split_all, u32(c->sched_order_a), &ctrl_of(c)->raster_heavy, stream),
+                      static_cast<SchedGate*>(c->gate.p), c->total_tiles, workers,
+                      items_per_tile, split_all, u32(c->sched_order_a), &ctrl_of(c)->raster_heavy, stream),
          "raster schedule");
     } else {
       if (learned)
@@ -610,13 +607,13 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
                          &dviews(c)->batch_tiles, u32(c->sched_keys_a), u32(c->sched_order_a),
                          u32(c->sched_keys_b), u32(c->sched_order_b),
                          static_cast<float*>(c->tile_est.p), u32(c->sched_status), ctrl_of(c),
-                         raster_ctas, strips, split_all, c->sm_count, c->stream),
+                         workers, items_per_tile, split_all, c->sm_count, c->stream),
          "raster schedule");
     }
     order = u32(c->sched_order_a);
     heavy = &ctrl_of(c)->raster_heavy;
   } else if (split_all) {  // row-major order, every tile split
-    CK(launch_heavy_count(nullptr, c->total_tiles, raster_ctas, strips, 0.0f, true,
+    CK(launch_heavy_count(nullptr, c->total_tiles, workers, items_per_tile, 0.0f, true,
                           &ctrl_of(c)->raster_heavy, c->stream),
        "split all tiles");
     heavy = &ctrl_of(c)->raster_heavy;
@@ -1406,8 +1403,8 @@ int gs3d_set_tuning(gs3d_ctx* c, const gs3d_tuning* t) {
     return fail(c, GS3D_ERR_INVALID_ARG,
                 "raster_batch must be 0 or a multiple of 32 up to 1024 (got %u)",
                 t->raster_batch);
-  // up to 1024 pixels; up to 2048 where the two-pixel raster shades the tile
-  // as row strips of at most 512 threads (sides multiples of 8 and 16)
+  // up to 1024 pixels (a thread a pixel); up to 2048 with sides that divide by 8
+  // and 16, whose regions the raster's warps shade one by one
   const uint64_t area = (uint64_t)t->tile_w * t->tile_h;
   const bool wide = area > 1024 && area <= 2048 && t->tile_w % 8 == 0 && t->tile_h % 16 == 0;
   if (t->tile_w == 0 || t->tile_h == 0 || (area > 1024 && !wide))

@@ -465,7 +465,7 @@ cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const De
                               int sm_count, LaunchStream s);
 // Raster work order: tile indices sorted by decreasing expected cost
 // (schedule = GS3D_SCHEDULE_KEY_COUNT: the tile's key count), so the
-// persistent raster CTAs start the longest tiles first.
+// raster starts the longest tiles first.
 // keys_a/order_a and est (the expected cost of every tile) must already be
 // written for GS3D_SCHEDULE_LEARNED (launch_learned_keys); for the key-count
 // schedule they are computed here.  Also sets ctrl->raster_heavy
@@ -473,7 +473,7 @@ cudaError_t launch_sort_depth(const uint32_t* count, uint32_t capacity, const De
 cudaError_t launch_schedule(uint32_t schedule, const uint32_t* tile_offsets, uint32_t num_tiles,
                             const uint32_t* num_tiles_dev, uint32_t* keys_a, uint32_t* order_a,
                             uint32_t* keys_b, uint32_t* order_b, float* est, uint32_t* status,
-                            Ctrl* ctrl, uint32_t raster_ctas, uint32_t strips, bool split_all,
+                            Ctrl* ctrl, uint32_t workers, uint32_t items_per_tile, bool split_all,
                             int sm_count, cudaStream_t s);
 // Tiles of fewer keys, or of a smaller predicted cost, are never split.  Most
 // long lists are opaque and end after a few thousand splats, so the bound on
@@ -483,11 +483,11 @@ cudaError_t launch_schedule(uint32_t schedule, const uint32_t* tile_offsets, uin
 constexpr uint32_t kHeavyKeys = 16384, kHeavyCost = 1024;
 // The per-tile split: *heavy = the number of tiles (the head of an order by
 // decreasing est) whose expected cost per work item exceeds half of one raster
-// worker's fair share of the frame, sum(est) * strips / raster_ctas, and floor;
+// worker's fair share of the frame, sum(est) * items_per_tile / workers, and floor;
 // those tiles are shaded as half-block work items.  all: every tile (est may be
 // null).
-cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t raster_ctas,
-                               uint32_t strips, float floor, bool all, uint32_t* heavy,
+cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t workers,
+                               uint32_t items_per_tile, float floor, bool all, uint32_t* heavy,
                                cudaStream_t s);
 
 // The same order (by buckets of 1/32 octave) and split in one block, for at most
@@ -554,7 +554,7 @@ cudaError_t launch_emit_cells(const ViewDesc* views, uint32_t n_views, uint32_t 
 cudaError_t launch_identify(const uint2* keys, const uint32_t* ref_counter, uint32_t capacity,
                             uint32_t num_tiles, uint32_t* tile_offsets, uint32_t* err,
                             int sm_count, LaunchStream s);
-// Rasterizes every tile of the batch.  Persistent CTAs pull tile indices
+// Rasterizes every tile of the batch.  Resident workers pull work items
 // from a device work queue (order[k] = k-th tile to render, identity when
 // order is null) through *queue_counter, which must be zero at launch, as must
 // the words of pool_ctrl and pool_places.

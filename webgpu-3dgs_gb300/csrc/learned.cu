@@ -2,12 +2,12 @@
 // MLP (warp-level bf16 mma inference, fp32 training kernels) and the work
 // order it produces.
 //
-// The raster's cost per tile is the number of splats its CTA iterates before
-// the tile's last pixel terminates (recorded in tile_costs).  The key count
+// The raster's cost per tile is the number of splats iterated before the tile's
+// last pixel terminates (recorded in tile_costs).  The key count
 // is a poor proxy for it in dense, opaque regions where pixels terminate
-// early.  The MLP predicts log(1 + cost) from 16 features; the persistent
-// raster CTAs then take tiles in decreasing predicted cost.  The schedule
-// only changes which CTA renders a tile and when, never a pixel's arithmetic.
+// early.  The MLP predicts log(1 + cost) from 16 features; the raster's warps
+// then take the tiles' regions in decreasing predicted cost.  The schedule only
+// changes which warp renders a region and when, never a pixel's arithmetic.
 //
 // Parameter vector (f32, kMlpParams entries):
 //   W1[64][16] | b1[64] | W2[64][64] | b2[64] | w3[64] | b3

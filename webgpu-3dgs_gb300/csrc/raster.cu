@@ -13,8 +13,9 @@
 //  * plain (any tile): one CTA per tile, one thread per pixel, the sorted
 //    splats staged in batches of RasterArgs::batch by double-buffered cp.async,
 //    left as soon as every pixel has terminated (the reference keeps looping);
-//  * culled (sides that divide by 8 and 4): the same, and each warp owns an 8x4
-//    block and tests every staged splat once against it;
+//  * culled (an area that divides by 32): the same, and each warp owns a block of
+//    8x4 pixels, or where the sides do not divide so 32 pixels in row order, and
+//    tests every staged splat once against its pixels' box;
 //  * warps (sides that divide by 8, all usual tiles): independent warps over
 //    regions of 2x2 blocks of 8x8 pixels, two pixels a lane (see there).
 // A splat is converted once per CTA or warp into its raster form (r^2, the
@@ -200,64 +201,26 @@ __device__ __forceinline__ bool blend_alpha(Pixel& p, const float4 c, float alph
   return ok && p.T < 1.0e-4f;
 }
 
-template <bool EARLY_OUT>
-__device__ __forceinline__ bool blend_one(float pfx, float pfy, const SplatStage& s, Pixel& p,
-                                          bool live) {
-  if (EARLY_OUT) {  // outside the radius (d^2 as splat_alpha forms it): alpha would be 0
-    const float dx = pfx - s.a.x, dy = pfy - s.a.y;
-    const float d2 = s.c.w == 0.0f ? fmaf(dx, dx, dy * dy)
-                                   : __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-    if (d2 > s.a.z) return false;
-  }
+// The plain variant's splat; true when the pixel terminates.
+__device__ __forceinline__ bool blend_one(float pfx, float pfy, const SplatStage& s, Pixel& p) {
+  // outside the radius (d^2 as splat_alpha forms it): alpha would be 0
+  const float dx = pfx - s.a.x, dy = pfy - s.a.y;
+  const float d2 = s.c.w == 0.0f ? fmaf(dx, dx, dy * dy)
+                                 : __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+  if (d2 > s.a.z) return false;
   bool ok;
   const float alpha = splat_alpha(pfx, pfy, s, s.c.w != 0.0f, ok);
-  return blend_alpha(p, s.c, alpha, ok && live);
+  return blend_alpha(p, s.c, alpha, ok);
 }
 
-// Two pixels of one column in the halves of a float2 (the two-pixel
-// variant).  Every component is computed by the scalar operation of
-// splat_alpha / blend_alpha, in the same order and rounding (the paired
-// FP32 instructions of sm_100 round each half like their scalar forms), so
-// each pixel is bit-identical to the one-pixel variants.
+// Two pixels of one column in the halves of a float2.  Every component is computed
+// by the scalar operation of splat_alpha / blend_alpha, in the same order and
+// rounding (the paired FP32 instructions of sm_100 round each half like their
+// scalar forms), so each pixel is bit-identical to the one-pixel forms.
 __device__ __forceinline__ float2 bcast(float x) { return make_float2(x, x); }
 
-__device__ __forceinline__ float2 splat_alpha2(float pfx, float2 pfy, const SplatStage& s,
-                                               bool exact, bool& ok0, bool& ok1) {
-  const float4 a = s.a, b = s.b;
-  const float dx = pfx - a.x;
-  const float2 dy = __fadd2_rn(pfy, bcast(-a.y));
-  float2 d2, q, ev;
-  if (!exact) {  // fast form (splat-uniform branch; no q < 0 test, see splat_alpha)
-    d2 = __ffma2_rn(bcast(dx), bcast(dx), __fmul2_rn(dy, dy));
-    q = __ffma2_rn(bcast(b.x * dx), bcast(dx),
-                   __ffma2_rn(bcast(b.y * dx), dy, __fmul2_rn(__fmul2_rn(bcast(b.z), dy), dy)));
-    const float2 e = make_float2(ex2_approx(-q.x), ex2_approx(-q.y));
-    const float2 am = __fmul2_rn(bcast(a.w), e);
-    const float2 alpha = make_float2(fminf(0.99f, am.x), fminf(0.99f, am.y));
-    ok0 = !(d2.x > a.z) && !(alpha.x < 1.0f / 255.0f);
-    ok1 = !(d2.y > a.z) && !(alpha.y < 1.0f / 255.0f);
-    return alpha;
-  } else {  // exact form in the reference's order, the column's dx terms shared; the
-            // products are paired, every sum a scalar __fadd_rn (never merged into an FMA)
-    const float dxx = __fmul_rn(dx, dx);
-    const float t1 = __fmul_rn(__fmul_rn(b.x, dx), dx);
-    const float2 dyy = __fmul2_rn(dy, dy);
-    const float2 t2 = __fmul2_rn(bcast(__fmul_rn(b.y, dx)), dy);
-    const float2 t3 = __fmul2_rn(__fmul2_rn(bcast(b.z), dy), dy);
-    d2 = make_float2(__fadd_rn(dxx, dyy.x), __fadd_rn(dxx, dyy.y));
-    q = make_float2(__fadd_rn(__fadd_rn(t1, t2.x), t3.x), __fadd_rn(__fadd_rn(t1, t2.y), t3.y));
-    ev = __fmul2_rn(q, bcast(-kHalfLog2e));
-  }
-  const float2 e = make_float2(ex2_approx(ev.x), ex2_approx(ev.y));
-  const float2 am = __fmul2_rn(bcast(a.w), e);
-  const float2 alpha = make_float2(fminf(0.99f, am.x), fminf(0.99f, am.y));
-  ok0 = !(d2.x > a.z) && !(q.x < 0.0f) && !(alpha.x < 1.0f / 255.0f);
-  ok1 = !(d2.y > a.z) && !(q.y < 0.0f) && !(alpha.y < 1.0f / 255.0f);
-  return alpha;
-}
-
-// splat_alpha and splat_alpha2 of a simple splat, 0 where it is skipped: the
-// same operations without the clamp, which cannot act.
+// splat_alpha of a simple splat, 0 where it is skipped: the same operations without
+// the clamp, which cannot act.
 __device__ __forceinline__ float simple_alpha(float pfx, float pfy, const SplatStage& s) {
   const float4 a = s.a, b = s.b;
   const float dx = pfx - a.x;
@@ -285,10 +248,25 @@ __device__ __forceinline__ float exact_alpha(float pfx, float pfy, const SplatSt
   const float alpha = splat_alpha(pfx, pfy, s, true, ok);
   return ok ? alpha : 0.0f;
 }
+// (the products are paired, every sum a scalar __fadd_rn, never merged into an FMA)
 __device__ __forceinline__ float2 exact_alpha(float pfx, float2 pfy, const SplatStage& s) {
-  bool ok0, ok1;
-  const float2 alpha = splat_alpha2(pfx, pfy, s, true, ok0, ok1);
-  return make_float2(ok0 ? alpha.x : 0.0f, ok1 ? alpha.y : 0.0f);
+  const float4 a = s.a, b = s.b;
+  const float dx = pfx - a.x;
+  const float2 dy = __fadd2_rn(pfy, bcast(-a.y));
+  const float dxx = __fmul_rn(dx, dx);
+  const float t1 = __fmul_rn(__fmul_rn(b.x, dx), dx);
+  const float2 dyy = __fmul2_rn(dy, dy);
+  const float2 t2 = __fmul2_rn(bcast(__fmul_rn(b.y, dx)), dy);
+  const float2 t3 = __fmul2_rn(__fmul2_rn(bcast(b.z), dy), dy);
+  const float2 d2 = make_float2(__fadd_rn(dxx, dyy.x), __fadd_rn(dxx, dyy.y));
+  const float2 q =
+      make_float2(__fadd_rn(__fadd_rn(t1, t2.x), t3.x), __fadd_rn(__fadd_rn(t1, t2.y), t3.y));
+  const float2 ev = __fmul2_rn(q, bcast(-kHalfLog2e));
+  const float2 am = __fmul2_rn(bcast(a.w), make_float2(ex2_approx(ev.x), ex2_approx(ev.y)));
+  const float2 alpha = make_float2(fminf(0.99f, am.x), fminf(0.99f, am.y));
+  return make_float2(
+      !(d2.x > a.z) && !(q.x < 0.0f) && !(alpha.x < 1.0f / 255.0f) ? alpha.x : 0.0f,
+      !(d2.y > a.z) && !(q.y < 0.0f) && !(alpha.y < 1.0f / 255.0f) ? alpha.y : 0.0f);
 }
 // The same for a splat of either form: both are evaluated and one is taken, so
 // that four of a step overlap (a branch per splat costs more than the few
@@ -640,7 +618,7 @@ __device__ void raster_tile_plain(const RasterArgs& a, const TileGeom& g, SplatS
     __syncthreads();
     if (!done) {
       for (uint32_t j = 0; j < cnt; ++j) {
-        if (blend_one<true>(pfx, pfy, cur[j], p, true)) {
+        if (blend_one(pfx, pfy, cur[j], p)) {
           done = true;
           used = bi * D + j + 1;
           break;

@@ -1,11 +1,11 @@
-// schedule.cu - work order of the persistent raster CTAs.
+// schedule.cu - work order of the raster.
 //
 // The reference dispatches one workgroup per tile in row-major order
 // (GaussianSplatRenderer.ts:1259-1265).  Per-tile raster cost spans orders of
 // magnitude, and a long tile that starts late stretches the whole pass, so
-// the persistent raster pulls tiles from a queue ordered by decreasing
+// the raster's workers pull tiles from a queue ordered by decreasing
 // expected cost (longest-processing-time first).  The order only changes
-// which CTA renders a tile and when; every pixel's arithmetic is unchanged.
+// which worker renders a tile and when; every pixel's arithmetic is unchanged.
 //
 // Key-count schedule: expected cost = the tile's key count (the plain
 // schedule the learned one falls back to).  Learned schedule: expected cost
@@ -39,12 +39,12 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // One block: the sum of the expected costs, then the count of tiles above
-// half of a raster CTA's fair share (deterministic: fixed per-thread order,
+// half of a raster worker's fair share (deterministic: fixed per-thread order,
 // fixed tree reduction).
 constexpr int kHeavyThreads = 1024;
 __global__ void __launch_bounds__(kHeavyThreads)
-    heavy_count_kernel(const float* __restrict__ est, uint32_t n, uint32_t raster_ctas,
-                       uint32_t strips, float floor, uint32_t all,
+    heavy_count_kernel(const float* __restrict__ est, uint32_t n, uint32_t workers,
+                       uint32_t items_per_tile, float floor, uint32_t all,
                        uint32_t* __restrict__ heavy) {
   __shared__ float s_sum[kHeavyThreads / 32];
   __shared__ uint32_t s_cnt[kHeavyThreads / 32];
@@ -61,9 +61,9 @@ __global__ void __launch_bounds__(kHeavyThreads)
   __syncthreads();
   float total = 0.0f;
   for (int w = 0; w < kHeavyThreads / 32; ++w) total += s_sum[w];
-  // a work item costs about est; the frame about sum(est) * strips
+  // a work item costs about est; the frame about sum(est) * items_per_tile
   const float thr =
-      fmaxf(0.5f * total * (float)strips / (float)max(raster_ctas, 1u), floor);
+      fmaxf(0.5f * total * (float)items_per_tile / (float)max(workers, 1u), floor);
   uint32_t cnt = 0;
   for (uint32_t t = threadIdx.x; t < n; t += kHeavyThreads) cnt += __ldg(est + t) > thr ? 1u : 0u;
 #pragma unroll
@@ -174,10 +174,10 @@ cudaError_t launch_order(uint32_t schedule, const uint32_t* tile_offsets, const 
   return cudaGetLastError();
 }
 
-cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t raster_ctas,
-                               uint32_t strips, float floor, bool all, uint32_t* heavy,
+cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t workers,
+                               uint32_t items_per_tile, float floor, bool all, uint32_t* heavy,
                                cudaStream_t s) {
-  heavy_count_kernel<<<1, kHeavyThreads, 0, s>>>(est, n, raster_ctas, strips, floor,
+  heavy_count_kernel<<<1, kHeavyThreads, 0, s>>>(est, n, workers, items_per_tile, floor,
                                                  all ? 1u : 0u, heavy);
   return cudaGetLastError();
 }
@@ -185,7 +185,7 @@ cudaError_t launch_heavy_count(const float* est, uint32_t n, uint32_t raster_cta
 cudaError_t launch_schedule(uint32_t schedule, const uint32_t* tile_offsets, uint32_t num_tiles,
                             const uint32_t* num_tiles_dev, uint32_t* keys_a, uint32_t* order_a,
                             uint32_t* keys_b, uint32_t* order_b, float* est, uint32_t* status,
-                            Ctrl* ctrl, uint32_t raster_ctas, uint32_t strips, bool split_all,
+                            Ctrl* ctrl, uint32_t workers, uint32_t items_per_tile, bool split_all,
                             int sm_count, cudaStream_t s) {
   if (num_tiles == 0) return cudaSuccess;
   cudaError_t e = cudaSuccess;
@@ -195,7 +195,7 @@ cudaError_t launch_schedule(uint32_t schedule, const uint32_t* tile_offsets, uin
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  e = launch_heavy_count(est, num_tiles, raster_ctas, strips,
+  e = launch_heavy_count(est, num_tiles, workers, items_per_tile,
                          schedule == GS3D_SCHEDULE_LEARNED ? (float)kHeavyCost : (float)kHeavyKeys,
                          split_all, &ctrl->raster_heavy, s);
   if (e != cudaSuccess) return e;
