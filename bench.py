@@ -206,9 +206,11 @@ def algorithmic_bytes(n, R, tiles, tile_passes, sh_floats, fused, views_per_scen
     }
 
 
-# DRAM bytes of the preprocess, from an ncu capture of a 2-view batch of the same
-# workload (profiles/): per scene splat read, per splat-view written.
+# DRAM bytes from ncu captures of batches of the same workload (profiles/): the
+# preprocess of 2 views, per scene splat read and per splat-view written; the depth
+# sort's histogram and three passes of 8 views, per splat-view.
 DRAM_PREPROCESS = (732.1e6 / 3e6, 434.7e6 / 6e6)
+DRAM_DEPTH_SORT = 1152.2e6 / 24e6
 
 
 def dominant_traffic(stage, splats_per_launch, scene_splats):
@@ -216,13 +218,15 @@ def dominant_traffic(stage, splats_per_launch, scene_splats):
     None where no capture covers it."""
     if stage == "preprocess-splats":
         return int(DRAM_PREPROCESS[0] * scene_splats + DRAM_PREPROCESS[1] * splats_per_launch)
+    if stage == "depth-sort":
+        return int(DRAM_DEPTH_SORT * splats_per_launch)
     return None
 
 
 # Pipe use of the raster kernel (ncu, one launch of the headline path's raster at
 # 64x32 tiles, 2-view batch; profiles/raster_warps_2views_3M_sh3_1080p.md).
-RASTER_NCU = {"kernel": "raster_kernel_warps", "issue_active": 0.606, "pipe_fma": 0.247,
-              "pipe_alu": 0.435, "pipe_xu": 0.095, "warps_active": 0.308,
+RASTER_NCU = {"kernel": "raster_kernel_warps", "issue_active": 0.669, "pipe_fma": 0.290,
+              "pipe_alu": 0.464, "pipe_xu": 0.101, "warps_active": 0.305,
               "source": "profiles/raster_warps_2views_3M_sh3_1080p.md"}
 
 
@@ -952,7 +956,7 @@ def main():
                          "peak": res["peak"], "unit": "GB/s", "frac": dom["frac_hbm"],
                          "peak_kind": res["peak_kind"], "traffic": res["traffic"],
                          "traffic_per": "launch (one pass over one batch), ncu DRAM "
-                                        "bytes of a 2-view capture scaled by units",
+                                        "bytes of a capture scaled by units",
                          "launch_units": res["launch_units"]},
             "roofline_raster": raster_roof,
             "stages": res["per_stage"],

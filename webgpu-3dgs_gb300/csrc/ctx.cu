@@ -650,11 +650,14 @@ int raster_stage(gs3d_ctx* c, bool cleared) {
 
 // Do the refs go through cells (binning.cu) or through the digit passes over
 // the refs themselves?  Cells take three launches more, so they pay where the
-// refs outweigh a launch: sum of the stages from scan to tile ranges, passes ->
-// cells when they were first compared, 20k splats 51 -> 69 us, 100k 79 -> 87,
-// 400k 110 -> 109, 3M (16x16 tiles) 623 -> 294, 8 views of 3M (64x32) 1743 ->
-// 1306, 3M heavy-tailed splats at 4K (32x32) 3317 -> 815 (now 41 us by passes at
-// 20k, and by cells 84 at 400k, 265, 1250 and 505).
+// refs outweigh a launch.  The line lies where scenes of few refs a splat cross it;
+// the more refs a splat has, the further below it cells would be faster already.
+// Sum of the stages from scan to tile ranges, passes / cells, us:
+//   refs a splat      50k         100k         300k          800k splats
+//   2.6 (640x360)     50 / 57      56 / 62      74 / 73      108 / 92
+//   9 (1080p)         74 / 63      85 / 79     124 / 97      218 / 123
+//   28 (8x8 tiles)   150 / 90     189 / 104    290 / 143     580 / 214
+//   240 (4K)        1131 / 149   1461 / 184   2567 / 318    5123 / 627
 constexpr uint32_t kCellsMinSplats = 300000;
 bool use_cells(const gs3d_ctx* c) {
   bool fits = c->total_cells <= kMaxCells && c->total_splats >= kCellsMinSplats;

@@ -18,8 +18,8 @@
 // they sort last, and where they tie with a splat at its very end they have no
 // refs to put in front of it.
 //
-// Measured (GB300), 4 x 8-bit passes -> 3 x 9-bit, histogram included: 24M
-// splat-views 795 -> 676 us, 3M 177 -> 144, 20k 69 -> 55.  A pass moves 16 bytes
+// Measured (GB300), 4 x 8-bit passes -> these, histogram included: 24M splat-views
+// 795 -> 653 us, 3M 177 -> 120, 400k 79 -> 47, 20k 69 -> 29.  A pass moves 16 bytes
 // a key; what bounds it is the ranking (issue slots 53% busy) and, below 1M
 // keys, the chain of one partition.
 #include <algorithm>

@@ -36,10 +36,10 @@
 // the log2 domain) and the blend (fused multiply-adds) differ from the reference
 // only in rounding, which the 2/255 image tolerance covers.
 //
-// Bound: instruction issue (61% busy, ALU 43%, 20 warps an SM; DRAM under 10%).
-// One strip of a tile per CTA -> independent warps over regions, cull per
-// region, blocks handed on: 8 views of 3M splats 3935 -> 2530 us, 12 mixed views
-// 5580 -> 3800, one 3M frame 425 -> 350, 100k 74 -> 60.
+// Bound: instruction issue (67 to 74% busy, ALU 46 to 53%, 20 warps an SM; DRAM
+// under 10%).  One strip of a tile per CTA -> independent warps over regions, cull
+// per region, blocks handed on: 8 views of 3M splats 3935 -> 2518 us, 12 mixed
+// views 5580 -> 3784, one 3M frame 425 -> 344, 100k 74 -> 61.
 #include <algorithm>
 #include <map>
 #include <mutex>
